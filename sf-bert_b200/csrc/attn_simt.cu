@@ -5,7 +5,7 @@
 // Thread layout shared by all matmul kernels: 256 threads as a 16x16 grid; thread (ty,tx) owns
 // rows ty+16m and columns tx+16n of a tile, so the 16 lanes of a half-warp own one set of rows
 // and row reductions are four shuffles.
-#include "attn.cuh"
+#include "simt_tile.cuh"
 #include <float.h>
 #include <math.h>
 
@@ -34,50 +34,100 @@ __device__ __forceinline__ void load_tile_kmajor(float (*dst)[BS + 1], const voi
 }
 
 // ------------------------------------------------------------------------------------------------
-// SDDMM: one CTA per non-zero block
+// SDDMM.  A CTA (four warps) makes one 64x64 block, a 32x32 quarter per warp, or four consecutive 32x32 blocks of the LUT,
+// one per warp.  Consecutive blocks mostly share their block-row (the LUT is in row-major scan order): its query rows
+// are then staged once for the four.  Both operands come chunk by chunk (32 of d) through two buffers; the scores leave
+// through shared memory, eight per lane, so that a row is written in whole pieces of 16 or 32 bytes.
 template <int BS, int AB_DT, int C_DT>
-__global__ void __launch_bounds__(256) sddmm_nt_kernel(const uint2 *__restrict__ lut, const void *__restrict__ A,
-                                                      const void *__restrict__ Bm, void *__restrict__ C, AttnDims p)
+__global__ void __launch_bounds__(tile::kThreads, 3) sddmm_nt_kernel(const uint2 *__restrict__ lut, const void *__restrict__ A,
+                                                                   const void *__restrict__ Bm, void *__restrict__ C, AttnDims p, bool vec)
 {
-    constexpr int KC = 32, T = BS / 16;
-    __shared__ float As[KC][BS + 1];
-    __shared__ float Bs[KC][BS + 1];
-    const uint32_t bid = blockIdx.x, b = blockIdx.y, h = blockIdx.z;
-    const uint2 e = lut[(size_t)h * p.lut_stride + bid];
+    using namespace tile;
+    constexpr uint32_t PER = BS == 32 ? 4 : 1;               // blocks per CTA
+    constexpr uint32_t ROWS = PER * BS;                      // staged rows of each operand: 128 or 64
+    constexpr uint32_t BUF = 2 * ROWS * kStride;
+    extern __shared__ __align__(16) float sm[];              // [2][A rows | B rows]
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane_row(lane), lc = lane_quad(lane);
+    const uint32_t bid0 = blockIdx.x * PER, b = blockIdx.y, h = blockIdx.z;
+    const uint32_t nblk = min(PER, p.blocks - bid0);
     const size_t HD = (size_t)p.H * p.d;
-    const size_t baseA = ((size_t)b * p.nb_a * BS + (size_t)e.x * BS) * HD + (size_t)h * p.d;
-    const size_t baseB = ((size_t)b * p.nb_b * BS + (size_t)e.y * BS) * HD + (size_t)h * p.d;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-
-    float acc[T][T];
+    const size_t head = (size_t)h * p.d;
+    size_t offA[PER], offB[PER];
+    bool shared_rows = true;
+    {
+        const uint2 *e = lut + (size_t)h * p.lut_stride + bid0;
+        const uint32_t x0 = e[0].x;
 #pragma unroll
-    for (int m = 0; m < T; m++)
-#pragma unroll
-        for (int n = 0; n < T; n++) acc[m][n] = 0.f;
-
-    for (uint32_t k0 = 0; k0 < p.d; k0 += KC) {
-        load_tile_kmajor<AB_DT, BS, KC>(As, A, baseA, HD, k0, p.d);
-        load_tile_kmajor<AB_DT, BS, KC>(Bs, Bm, baseB, HD, k0, p.d);
-        __syncthreads();
-#pragma unroll 8
-        for (int k = 0; k < KC; k++) {
-            float a[T], bb[T];
-#pragma unroll
-            for (int m = 0; m < T; m++) a[m] = As[k][ty + 16 * m];
-#pragma unroll
-            for (int n = 0; n < T; n++) bb[n] = Bs[k][tx + 16 * n];
-#pragma unroll
-            for (int m = 0; m < T; m++)
-#pragma unroll
-                for (int n = 0; n < T; n++) acc[m][n] = fmaf(a[m], bb[n], acc[m][n]);
+        for (uint32_t k = 0; k < PER; k++) {
+            const uint2 en = k < nblk ? e[k] : e[0];
+            offA[k] = ((size_t)b * p.nb_a + en.x) * BS * HD + head;
+            offB[k] = ((size_t)b * p.nb_b + en.y) * BS * HD + head;
+            shared_rows = shared_rows && en.x == x0;
         }
-        __syncthreads();
     }
-    const size_t baseC = (((size_t)b * p.H + h) * p.blocks + bid) * BS * BS;
+    auto issue = [&](uint32_t c) {
+        float *buf = sm + (c & 1) * BUF;
+        const uint32_t k0 = c * kChunk, left = p.d - k0;
 #pragma unroll
-    for (int m = 0; m < T; m++)
+        for (uint32_t g = 0; g < PER; g++)
+            if (g < nblk) {
+                if (g == 0 || !shared_rows) stage<AB_DT, BS, (int)kChunk>(buf + g * BS * kStride, kStride, A, offA[g] + k0, HD, left, vec);
+                stage<AB_DT, BS, (int)kChunk>(buf + (ROWS + g * BS) * kStride, kStride, Bm, offB[g] + k0, HD, left, vec);
+            }
+        cp_commit();
+    };
+    const bool live = BS == 64 || warp < nblk;
+    const uint32_t r0 = BS == 64 ? 32 * (warp >> 1) : (shared_rows ? 0 : 32 * warp), c0 = BS == 64 ? 32 * (warp & 1) : 32 * warp;
+    uint64_t acc[4][8];
 #pragma unroll
-        for (int n = 0; n < T; n++) Elem<C_DT>::store(C, baseC + (size_t)(ty + 16 * m) * BS + tx + 16 * n, acc[m][n]);
+    for (int m = 0; m < 4; m++)
+#pragma unroll
+        for (int n = 0; n < 8; n++) acc[m][n] = 0;
+    const uint32_t chunks = (p.d + kChunk - 1) / kChunk;
+    issue(0);
+    for (uint32_t c = 0; c < chunks; c++) {
+        cp_wait_all();
+        __syncthreads();
+        if (c + 1 < chunks) issue(c + 1);
+        const float *buf = sm + (c & 1) * BUF;
+        if (live) mma_nt(acc, buf + (r0 + lr) * kStride, kStride, buf + (ROWS + c0 + lc) * kStride, kStride);
+    }
+    __syncthreads();
+    if (!live) return;
+    float *t = sm + warp * 32 * kStride;
+#pragma unroll
+    for (int m = 0; m < 4; m++)
+#pragma unroll
+        for (int n = 0; n < 8; n++) t[(lr + 8 * m) * kStride + lc + 4 * n] = half_sum(acc[m][n]);
+    __syncwarp();
+    const size_t baseC = (((size_t)b * p.H + h) * p.blocks + bid0 + (BS == 64 ? 0 : warp)) * BS * BS + (BS == 64 ? (size_t)r0 * BS + c0 : 0);
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+        const float *row = t + (lr + 8 * m) * kStride + lc * 8;
+        const float4 u = *(const float4 *)row, w = *(const float4 *)(row + 4);
+        const float v[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
+        const size_t at = baseC + (size_t)(lr + 8 * m) * BS + lc * 8;
+        if (vec) {
+            if (C_DT == SFB_F32) {
+                *(float4 *)((float *)C + at) = u;
+                *(float4 *)((float *)C + at + 4) = w;
+            } else {
+                uint32_t q[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    if (C_DT == SFB_BF16) q[k] = to_bhalf_bits(v[2 * k]) | ((uint32_t)to_bhalf_bits(v[2 * k + 1]) << 16);
+                    else {
+                        __half2 hh = __floats2half2_rn(v[2 * k], v[2 * k + 1]);
+                        q[k] = *reinterpret_cast<uint32_t *>(&hh);
+                    }
+                }
+                *(uint4 *)((uint16_t *)C + at) = make_uint4(q[0], q[1], q[2], q[3]);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; k++) Elem<C_DT>::store(C, at + k, v[k]);
+        }
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -438,62 +488,72 @@ __global__ void __launch_bounds__(BS * BS / 8 / SPLIT) softmax_grad_kernel(const
 }
 
 // ------------------------------------------------------------------------------------------------
-// SpMM: one CTA per (block-row, 64-wide slice of d).  TRANS = false: O = sum over the row's blocks of P . V (NN, the
+// SpMM: one CTA per (block-row, slice of up to 128 of d).  TRANS = false: O = sum over the row's blocks of P . V (NN, the
 // lut is the nn_lut).  TRANS = true: the backward products dV = P^T dO and dK = dS^T Q -- the lut is the tn_lut,
 // "row" i is a block COLUMN, an entry names a block of that column and the block-row its B rows come from, and
-// the block is used transposed.
-template <int BS, int A_DT, int BC_DT, bool TRANS>
-__global__ void __launch_bounds__(256) spmm_nn_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Pm,
-                                                     const void *__restrict__ V, void *__restrict__ O, AttnDims p)
+// the block is used transposed (read as it lies, four neighbouring rows of P^T per 16-byte load).
+// A chunk is 32 elements of the contraction: one 32x32 block, or half of a 64x64 one, with its 32 rows of V.
+template <int BS, int DS> struct SpmmCfg {
+    static constexpr int WC = BS == 32 ? 4 : 2;                          // warps side by side along d
+    static constexpr int TN = DS / WC / 4;                               // columns per thread
+    static constexpr uint32_t a_floats = BS == 32 ? 32 * tile::kStride : 64 * tile::kStride > 32 * (64 + 4) ? 64 * tile::kStride : 32 * (64 + 4);
+    static constexpr uint32_t buf = a_floats + 32 * (DS + 4);
+};
+template <int BS, int DS, int A_DT, int BC_DT, bool TRANS>
+__global__ void __launch_bounds__(tile::kThreads, 4) spmm_nn_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Pm,
+                                                                  const void *__restrict__ V, void *__restrict__ O, AttnDims p, bool avec,
+                                                                  bool vec)
 {
-    constexpr int TM = BS / 16, TN = 4;
-    __shared__ float Ps[BS][BS + 16];
-    __shared__ float Vs[BS][64];
-    const uint32_t nslice = (p.d + 63) / 64;
-    const uint32_t i = blockIdx.x / nslice, n0 = (blockIdx.x % nslice) * 64;
+    using namespace tile;
+    typedef SpmmCfg<BS, DS> Cfg;
+    constexpr int TN = Cfg::TN;
+    constexpr uint32_t PARTS = BS / 32;                                  // chunks per block
+    constexpr uint32_t a_stride = TRANS ? BS + 4 : kStride;
+    extern __shared__ __align__(16) float sm[];                          // [2][P chunk | V chunk]
+    const uint32_t nslice = (p.d + DS - 1) / DS;
+    const uint32_t i = blockIdx.x / nslice, d0 = (blockIdx.x % nslice) * DS;
     const uint32_t b = blockIdx.y, h = blockIdx.z;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane_row(lane), lc = lane_quad(lane);
     const uint2 *nn = lut + (size_t)h * p.lut_stride;
     const uint2 head = nn[i];
     const size_t HD = (size_t)p.H * p.d;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const size_t bh = (size_t)b * p.H + h;
+    const uint32_t r0 = BS == 64 ? 32 * (warp >> 1) : 0, n0 = (BS == 64 ? warp & 1 : warp) * (DS / Cfg::WC);
+    const uint32_t chunks = head.y * PARTS;
 
-    float acc[TM][TN];
+    auto issue = [&](uint32_t c) {
+        const uint2 ent = nn[head.x + c / PARTS];
+        const uint32_t part = c % PARTS;
+        float *buf = sm + (c & 1) * Cfg::buf;
+        const size_t baseP = (bh * p.blocks + ent.x) * BS * BS, baseV = ((size_t)b * p.nb_b + ent.y) * BS * HD + (size_t)h * p.d + d0;
+        if (TRANS) stage<A_DT, 32, BS>(buf, a_stride, Pm, baseP + part * 32 * BS, BS, BS, avec);
+        else stage<A_DT, BS, 32>(buf, a_stride, Pm, baseP + part * 32, BS, 32, avec);
+        stage<BC_DT, 32, DS>(buf + Cfg::a_floats, DS + 4, V, baseV + (size_t)part * 32 * HD, HD, p.d - d0, vec);
+        cp_commit();
+    };
+    uint64_t acc[4][TN / 2];
 #pragma unroll
-    for (int m = 0; m < TM; m++)
+    for (int m = 0; m < 4; m++)
 #pragma unroll
-        for (int n = 0; n < TN; n++) acc[m][n] = 0.f;
-
-    for (uint32_t e = 0; e < head.y; e++) {
-        const uint2 ent = nn[head.x + e];
-        const size_t baseP = (((size_t)b * p.H + h) * p.blocks + ent.x) * BS * BS;
-        const size_t baseV = ((size_t)b * p.nb_b * BS + (size_t)ent.y * BS) * HD + (size_t)h * p.d + n0;
-        for (uint32_t t = threadIdx.x; t < BS * BS; t += 256) Ps[t / BS][t % BS] = Elem<A_DT>::load(Pm, baseP + t);
-        for (uint32_t t = threadIdx.x; t < BS * 64; t += 256) {
-            uint32_t c = t / 64, n = t % 64;
-            Vs[c][n] = (n0 + n < p.d) ? Elem<BC_DT>::load(V, baseV + (size_t)c * HD + n) : 0.f;
-        }
+        for (int n = 0; n < TN / 2; n++) acc[m][n] = 0;
+    if (chunks) issue(0);
+    for (uint32_t c = 0; c < chunks; c++) {
+        cp_wait_all();
         __syncthreads();
-#pragma unroll 8
-        for (int c = 0; c < BS; c++) {
-            float a[TM], bb[TN];
-#pragma unroll
-            for (int m = 0; m < TM; m++) a[m] = TRANS ? Ps[c][ty + 16 * m] : Ps[ty + 16 * m][c];
-#pragma unroll
-            for (int n = 0; n < TN; n++) bb[n] = Vs[c][tx + 16 * n];
-#pragma unroll
-            for (int m = 0; m < TM; m++)
-#pragma unroll
-                for (int n = 0; n < TN; n++) acc[m][n] = fmaf(a[m], bb[n], acc[m][n]);
-        }
-        __syncthreads();
+        if (c + 1 < chunks) issue(c + 1);
+        const float *buf = sm + (c & 1) * Cfg::buf;
+        const float *v = buf + Cfg::a_floats + n0 + lane_col<TN>(lc);
+        if (TRANS) mma_tn<TN>(acc, buf + r0 + 4 * lr, a_stride, v, DS + 4);
+        else mma_nn<TN>(acc, buf + (r0 + lr) * a_stride, a_stride, v, DS + 4);
     }
     // rows without blocks are written as zeros (blocksparse.h:949-962)
-    const size_t baseO = ((size_t)b * p.nb_a * BS + (size_t)i * BS) * HD + (size_t)h * p.d + n0;
+    const size_t baseO = ((size_t)b * p.nb_a + i) * BS * HD + (size_t)h * p.d + d0 + n0;
+    const uint32_t left = p.d > d0 + n0 ? p.d - d0 - n0 : 0;
 #pragma unroll
-    for (int m = 0; m < TM; m++)
-#pragma unroll
-        for (int n = 0; n < TN; n++)
-            if (n0 + tx + 16 * n < p.d) Elem<BC_DT>::store(O, baseO + (size_t)(ty + 16 * m) * HD + tx + 16 * n, acc[m][n]);
+    for (int m = 0; m < 4; m++) {
+        const uint32_t r = r0 + (TRANS ? 4 * lr + m : lr + 8 * m);
+        store_cols<BC_DT, TN>(O, baseO + (size_t)r * HD, lc, acc[m], 1.f, left, vec);
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -619,104 +679,167 @@ __global__ void __launch_bounds__(256) fused_sddmm_softmax_kernel(const uint2 *_
     }
 }
 
-// SDDMM + softmax + SpMM with an online softmax; S and P never leave the SM.
-template <int BS, int DMAX, int DT>
-__global__ void __launch_bounds__(256) fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q,
-                                                             const void *__restrict__ K, const void *__restrict__ V,
-                                                             void *__restrict__ O,
-                                                             const typename MaskWord<BS>::type *__restrict__ mask,
-                                                             AttnDims p, float scale_log2e)
+// SDDMM + softmax + SpMM with an online softmax; S and P never leave the SM.  One CTA (four warps) per block-row.
+// A step takes four 32x32 key blocks (a 32x32 score tile per warp) or one 64x64 block (a quarter per warp): Q . K^T over
+// chunks of 32 of d, the softmax in registers (row maxima meet in shared memory), P to shared memory, then O += P . V in
+// chunks of 32 keys, each warp on its share of O's columns (and, for 64 rows, of its rows).  Keys and values flow through
+// the same two buffers as one sequence of chunks.  Score and O rows of a thread are the same, so O is rescaled in place.
+template <int BS, int D> struct FaCfg {
+    static constexpr uint32_t G = BS == 32 ? 4 : 1;                      // key blocks per step
+    static constexpr uint32_t NK = G * BS;                               // keys per step
+    static constexpr uint32_t WC = BS == 32 ? 4 : 2;                     // warps side by side (score columns, O columns)
+    static constexpr int TN = D / (int)WC / 4;
+    static constexpr uint32_t kbuf = NK * tile::kStride, vbuf = 32 * (D + 4), buf = kbuf > vbuf ? kbuf : vbuf;
+    static constexpr uint32_t p_stride = NK + 4, q_stride = D + 4;
+    static constexpr uint32_t floats = BS * q_stride + 2 * buf + BS * p_stride + WC * BS;
+    static constexpr int ctas = BS == 64 && D == 128 ? 2 : 3;            // what registers and shared memory allow per SM
+};
+template <int BS, int D, int DT>
+__global__ void __launch_bounds__(tile::kThreads, (FaCfg<BS, D>::ctas))
+fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q, const void *__restrict__ K, const void *__restrict__ V,
+                       void *__restrict__ O, const typename MaskWord<BS>::type *__restrict__ mask, AttnDims p, float scale_log2e, bool vec)
 {
+    using namespace tile;
     typedef typename MaskWord<BS>::type W;
-    constexpr int T = BS / 16, TD = DMAX / 16;
-    extern __shared__ float smem[];
-    float (*Qs)[BS + 1] = (float (*)[BS + 1])smem;
-    float (*Ks)[BS + 1] = (float (*)[BS + 1])(smem + DMAX * (BS + 1));
-    float (*Vs)[DMAX] = (float (*)[DMAX])(smem + 2 * DMAX * (BS + 1));
-    float (*Ps)[BS + 16] = (float (*)[BS + 16])(smem + 2 * DMAX * (BS + 1) + BS * DMAX);
-    const uint32_t i = blockIdx.x, b = blockIdx.y, h = blockIdx.z;
+    typedef FaCfg<BS, D> Cfg;
+    constexpr int TN = Cfg::TN;
+    constexpr uint32_t G = Cfg::G, NK = Cfg::NK, WC = Cfg::WC, QS = Cfg::q_stride, PS = Cfg::p_stride;
+    extern __shared__ __align__(16) float sm[];
+    float *Qs = sm, *bufs = Qs + BS * QS, *Ps = bufs + 2 * Cfg::buf, *red = Ps + BS * PS;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane_row(lane), lc = lane_quad(lane);
+    // rows are dealt from both ends: the long rows of the layouts at hand sit there and start first
+    const uint32_t i = (blockIdx.x & 1u) ? p.nb_a - 1u - (blockIdx.x >> 1) : blockIdx.x >> 1, b = blockIdx.y, h = blockIdx.z;
     const uint2 *nn = lut + (size_t)h * p.lut_stride;
     const uint2 head = nn[i];
     const size_t HD = p.in_pitch ? (size_t)p.in_pitch : (size_t)p.H * p.d;      // row pitch of q, k, v
     const size_t HDo = p.out_pitch ? (size_t)p.out_pitch : (size_t)p.H * p.d;   // row pitch of o
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     const W *mh = mask ? mask + (size_t)h * p.mask_stride : nullptr;
+    const uint32_t r0 = BS == 64 ? 32 * (warp >> 1) : 0, wc = BS == 64 ? warp & 1 : warp;   // this warp's rows and column share
+    const uint32_t n0 = wc * (D / WC);
+    const uint32_t kchunks = (p.d + kChunk - 1) / kChunk;
+    const uint32_t cnt = head.y;
 
-    if (head.y)
-        for (uint32_t k0 = 0; k0 < p.d; k0 += 32)
-            load_tile_kmajor<DT, BS, 32>(Qs + k0, Q, ((size_t)b * p.nb_a * BS + (size_t)i * BS) * HD + (size_t)h * p.d, HD, k0, p.d);
-
-    float mx[T], sum[T], acc[T][TD];
+    // the sequence of chunks: per step the key chunks, then the value chunks
+    uint32_t is_e = 0, is_k = 0, is_n = 0;                               // next chunk to issue: step's first entry, index in the step, overall
+    size_t koff[G];
+    auto issue = [&]() {
+        const uint32_t nblk = min(G, cnt - is_e);
+        if (is_k == 0) {
 #pragma unroll
-    for (int m = 0; m < T; m++) {
+            for (uint32_t g = 0; g < G; g++)
+                koff[g] = ((size_t)b * p.nb_b + nn[head.x + is_e + (g < nblk ? g : 0)].y) * BS * HD + (size_t)h * p.d;
+        }
+        float *buf = bufs + (is_n & 1) * Cfg::buf;
+        if (is_k < kchunks) {
+            const uint32_t k0 = is_k * kChunk;
+#pragma unroll
+            for (uint32_t g = 0; g < G; g++)
+                if (g < nblk) stage<DT, BS, (int)kChunk>(buf + g * BS * kStride, kStride, K, koff[g] + k0, HD, p.d - k0, vec);
+        } else {
+            const uint32_t vc = is_k - kchunks;
+            const size_t base = G > 1 ? (vc == 0 ? koff[0] : vc == 1 ? koff[1 % G] : vc == 2 ? koff[2 % G] : koff[3 % G]) : koff[0] + (size_t)vc * 32 * HD;
+            stage<DT, 32, D>(buf, D + 4, V, base, HD, p.d, vec);
+        }
+        cp_commit();
+        is_n++;
+        if (++is_k == kchunks + nblk * (BS / 32)) {
+            is_k = 0;
+            is_e += G;
+        }
+    };
+
+    if (cnt) {
+        stage<DT, BS, D>(Qs, QS, Q, ((size_t)b * p.nb_a + i) * BS * HD + (size_t)h * p.d, HD, p.d, vec);
+        issue();
+    }
+    float mx[4], sum[4];
+    uint64_t acc[4][TN / 2];
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
         mx[m] = -INFINITY;
         sum[m] = 0.f;
 #pragma unroll
-        for (int n = 0; n < TD; n++) acc[m][n] = 0.f;
+        for (int n = 0; n < TN / 2; n++) acc[m][n] = 0;
     }
-
-    for (uint32_t e = 0; e < head.y; e++) {
-        const uint2 ent = nn[head.x + e];
-        const size_t baseKV = ((size_t)b * p.nb_b * BS + (size_t)ent.y * BS) * HD + (size_t)h * p.d;
-        __syncthreads();
-        for (uint32_t k0 = 0; k0 < p.d; k0 += 32) load_tile_kmajor<DT, BS, 32>(Ks + k0, K, baseKV, HD, k0, p.d);
-        for (uint32_t t = threadIdx.x; t < BS * DMAX; t += 256) {
-            uint32_t c = t / DMAX, n = t % DMAX;
-            Vs[c][n] = n < p.d ? Elem<DT>::load(V, baseKV + (size_t)c * HD + n) : 0.f;
+    uint32_t c = 0;
+    for (uint32_t e = 0; e < cnt; e += G) {
+        const uint32_t nblk = min(G, cnt - e);
+        const bool live = G == 1 || warp < nblk;
+        uint64_t s2[4][8];
+#pragma unroll
+        for (int m = 0; m < 4; m++)
+#pragma unroll
+            for (int n = 0; n < 8; n++) s2[m][n] = 0;
+        for (uint32_t kc = 0; kc < kchunks; kc++, c++) {
+            cp_wait_all();
+            __syncthreads();
+            issue();                                                     // a value chunk follows every key chunk of a step
+            const float *buf = bufs + (c & 1) * Cfg::buf;
+            if (live) mma_nt(s2, Qs + (r0 + lr) * QS + kc * kChunk, QS, buf + (32 * wc + lc) * kStride, kStride);
+        }
+        const uint32_t blk = nn[head.x + e + (G > 1 && live ? warp : 0)].x;
+        float s[4][8], bm[4];
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            const W w = live ? (mh ? __ldg(mh + (size_t)blk * BS + r0 + lr + 8 * m) : ~(W)0) : (W)0;
+            bm[m] = -INFINITY;
+#pragma unroll
+            for (int n = 0; n < 8; n++) {
+                const uint32_t col = (BS == 64 ? 32 * wc : 0) + lc + 4 * n;
+                s[m][n] = ((w >> col) & 1) ? half_sum(s2[m][n]) * scale_log2e : -INFINITY;
+                bm[m] = fmaxf(bm[m], s[m][n]);
+            }
+            bm[m] = fmaxf(bm[m], __shfl_xor_sync(0xffffffffu, bm[m], 1));
+            bm[m] = fmaxf(bm[m], __shfl_xor_sync(0xffffffffu, bm[m], 4));
+            if (lc == 0) red[wc * BS + r0 + lr + 8 * m] = bm[m];
         }
         __syncthreads();
-        float s[T][T];
-        score_tile<BS>(s, Qs, Ks, p.d, tx, ty);
 #pragma unroll
-        for (int m = 0; m < T; m++) {
-            const uint32_t r = ty + 16 * m;
-            const W w = mh ? __ldg(mh + (size_t)ent.x * BS + r) : ~(W)0;
-            float bm = -INFINITY;
+        for (int m = 0; m < 4; m++) {
+            const uint32_t r = r0 + lr + 8 * m;
+            float mn = mx[m];
 #pragma unroll
-            for (int n = 0; n < T; n++) {
-                const uint32_t c = tx + 16 * n;
-                s[m][n] = ((w >> c) & 1) ? s[m][n] * scale_log2e : -INFINITY;
-                bm = fmaxf(bm, s[m][n]);
-            }
-            bm = half_warp_max(bm);
-            float alpha = 1.f;
-            if (bm > mx[m]) {
-                alpha = exp2f(mx[m] - bm);
-                mx[m] = bm;
-            }
+            for (uint32_t k = 0; k < WC; k++) mn = fmaxf(mn, red[k * BS + r]);
+            const float alpha = mn > mx[m] ? exp2f(mx[m] - mn) : 1.f;
+            mx[m] = mn;
             float ps = 0.f;
 #pragma unroll
-            for (int n = 0; n < T; n++) {
-                float pv = mx[m] > -INFINITY ? exp2f(s[m][n] - mx[m]) : 0.f;
-                Ps[r][tx + 16 * n] = pv;
+            for (int n = 0; n < 8; n++) {
+                const float pv = mn > -INFINITY ? exp2f(s[m][n] - mn) : 0.f;
+                Ps[r * PS + 32 * wc + lc + 4 * n] = pv;
                 ps += pv;
             }
-            sum[m] = sum[m] * alpha + half_warp_sum(ps);
+            sum[m] = fmaf(sum[m], alpha, ps);                            // this thread's columns only; the shares meet at the end
+            const uint64_t a2 = pair(alpha, alpha);
 #pragma unroll
-            for (int n = 0; n < TD; n++) acc[m][n] *= alpha;
+            for (int n = 0; n < TN / 2; n++) acc[m][n] = fma2(acc[m][n], a2, 0ull);
         }
-        __syncthreads();
-#pragma unroll 4
-        for (int c = 0; c < BS; c++) {
-            float a[T], bb[TD];
-#pragma unroll
-            for (int m = 0; m < T; m++) a[m] = Ps[ty + 16 * m][c];
-#pragma unroll
-            for (int n = 0; n < TD; n++) bb[n] = Vs[c][tx + 16 * n];
-#pragma unroll
-            for (int m = 0; m < T; m++)
-#pragma unroll
-                for (int n = 0; n < TD; n++) acc[m][n] = fmaf(a[m], bb[n], acc[m][n]);
+        const uint32_t vchunks = nblk * (BS / 32);
+        for (uint32_t vc = 0; vc < vchunks; vc++, c++) {
+            cp_wait_all();
+            __syncthreads();
+            if (vc + 1 < vchunks || e + G < cnt) issue();
+            const float *buf = bufs + (c & 1) * Cfg::buf;
+            mma_nn<TN>(acc, Ps + (r0 + lr) * PS + vc * 32, PS, buf + n0 + lane_col<TN>(lc), D + 4);
         }
     }
-    const size_t baseO = ((size_t)b * p.nb_a * BS + (size_t)i * BS) * HDo + (size_t)h * p.d;
+    __syncthreads();
 #pragma unroll
-    for (int m = 0; m < T; m++) {
-        const float inv = sum[m] > 0.f ? 1.f / sum[m] : 0.f;
+    for (int m = 0; m < 4; m++) {
+        sum[m] += __shfl_xor_sync(0xffffffffu, sum[m], 1);
+        sum[m] += __shfl_xor_sync(0xffffffffu, sum[m], 4);
+        if (lc == 0) red[wc * BS + r0 + lr + 8 * m] = sum[m];
+    }
+    __syncthreads();
+    const size_t baseO = (((size_t)b * p.nb_a + i) * BS) * HDo + (size_t)h * p.d + n0;
+    const uint32_t left = p.d > n0 ? p.d - n0 : 0;
 #pragma unroll
-        for (int n = 0; n < TD; n++)
-            if ((uint32_t)(tx + 16 * n) < p.d)
-                Elem<DT>::store(O, baseO + (size_t)(ty + 16 * m) * HDo + tx + 16 * n, acc[m][n] * inv);
+    for (int m = 0; m < 4; m++) {
+        const uint32_t r = r0 + lr + 8 * m;
+        float l = 0.f;
+#pragma unroll
+        for (uint32_t k = 0; k < WC; k++) l += red[k * BS + r];
+        store_cols<DT, TN>(O, baseO + (size_t)r * HDo, lc, acc[m], l > 0.f ? 1.f / l : 0.f, left, vec);
     }
 }
 
@@ -729,15 +852,40 @@ __global__ void __launch_bounds__(256) fused_attention_kernel(const uint2 *__res
     else if (dt == SFB_BF16) { constexpr int NAME = SFB_BF16; __VA_ARGS__ } \
     else { constexpr int NAME = SFB_F16; __VA_ARGS__ }
 
+template <typename K>
+static int set_smem(K kernel, size_t bytes)
+{
+    if (bytes > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e != cudaSuccess) return fail("cudaFuncSetAttribute(%zu bytes): %s", bytes, cudaGetErrorString(e));
+    }
+    return 0;
+}
+
+// 16-byte accesses to rows of a [.., pitch] tensor whose heads are d wide
+static bool rows_vec(const void *ptr, int dtype, uint64_t pitch, uint32_t d)
+{
+    const uint32_t per = dtype == SFB_F32 ? 4 : 8;
+    return ((uintptr_t)ptr & 15) == 0 && pitch % per == 0 && d % per == 0;
+}
+
 int simt_sddmm_nt(cudaStream_t s, const void *lut, const void *a, const void *b, void *c, int ab_dtype, int c_dtype,
                   uint32_t bs, const AttnDims &p)
 {
-    dim3 grid(p.blocks, p.B, p.H);
+    const uint64_t HD = (uint64_t)p.H * p.d;
+    const bool vec = rows_vec(a, ab_dtype, HD, p.d) && rows_vec(b, ab_dtype, HD, p.d) && ((uintptr_t)c & 15) == 0;
+#define SD_LAUNCH(CD)                                                                                             \
+    {                                                                                                             \
+        constexpr uint32_t per = BS == 32 ? 4 : 1;                                                                \
+        const size_t bytes = sizeof(float) * 4 * per * BS * tile::kStride;                                        \
+        auto kern = sddmm_nt_kernel<BS, AB, CD>;                                                                  \
+        if (set_smem(kern, bytes)) return 1;                                                                      \
+        kern<<<dim3((p.blocks + per - 1) / per, p.B, p.H), tile::kThreads, bytes, s>>>((const uint2 *)lut, a, b, c, p, vec); \
+    }
     DISPATCH_BS(bs, DISPATCH_DT(ab_dtype, AB, {
-        if (c_dtype == SFB_F32) sddmm_nt_kernel<BS, AB, SFB_F32><<<grid, 256, 0, s>>>((const uint2 *)lut, a, b, c, p);
-        else if (c_dtype == SFB_BF16) sddmm_nt_kernel<BS, AB, SFB_BF16><<<grid, 256, 0, s>>>((const uint2 *)lut, a, b, c, p);
-        else sddmm_nt_kernel<BS, AB, SFB_F16><<<grid, 256, 0, s>>>((const uint2 *)lut, a, b, c, p);
+        if (c_dtype == SFB_F32) SD_LAUNCH(SFB_F32) else if (c_dtype == SFB_BF16) SD_LAUNCH(SFB_BF16) else SD_LAUNCH(SFB_F16)
     }))
+#undef SD_LAUNCH
     return check_launch("sfb_bst_sgemm_nt");
 }
 
@@ -785,11 +933,26 @@ int simt_softmax(cudaStream_t s, const void *lut, const void *mask, const void *
 int simt_spmm_nn(cudaStream_t s, const void *lut, const void *a, const void *b, void *c, int a_dtype, int bc_dtype,
                  uint32_t bs, const AttnDims &p, bool trans)
 {
-    dim3 grid(p.nb_a * ((p.d + 63) / 64), p.B, p.H);
+    const uint64_t HD = (uint64_t)p.H * p.d;
+    const bool avec = ((uintptr_t)a & 15) == 0, vec = rows_vec(b, bc_dtype, HD, p.d) && rows_vec(c, bc_dtype, HD, p.d);
+#define SP_LAUNCH(DSV)                                                                                            \
+    {                                                                                                             \
+        const size_t bytes = sizeof(float) * 2 * SpmmCfg<BS, DSV>::buf;                                           \
+        const dim3 grid(p.nb_a * ((p.d + DSV - 1) / DSV), p.B, p.H);                                              \
+        if (trans) {                                                                                              \
+            auto kern = spmm_nn_kernel<BS, DSV, AD, BD, true>;                                                    \
+            if (set_smem(kern, bytes)) return 1;                                                                  \
+            kern<<<grid, tile::kThreads, bytes, s>>>((const uint2 *)lut, a, b, c, p, avec, vec);                  \
+        } else {                                                                                                  \
+            auto kern = spmm_nn_kernel<BS, DSV, AD, BD, false>;                                                   \
+            if (set_smem(kern, bytes)) return 1;                                                                  \
+            kern<<<grid, tile::kThreads, bytes, s>>>((const uint2 *)lut, a, b, c, p, avec, vec);                  \
+        }                                                                                                         \
+    }
     DISPATCH_BS(bs, DISPATCH_DT(a_dtype, AD, DISPATCH_DT(bc_dtype, BD, {
-        if (trans) spmm_nn_kernel<BS, AD, BD, true><<<grid, 256, 0, s>>>((const uint2 *)lut, a, b, c, p);
-        else spmm_nn_kernel<BS, AD, BD, false><<<grid, 256, 0, s>>>((const uint2 *)lut, a, b, c, p);
+        if (p.d <= 32) SP_LAUNCH(32) else if (p.d <= 64) SP_LAUNCH(64) else SP_LAUNCH(128)
     })))
+#undef SP_LAUNCH
     return check_launch("sfb_bst_sgemm_xn");
 }
 
@@ -812,16 +975,6 @@ int simt_softmax_grad(cudaStream_t s, const void *lut, const void *dy, const voi
     })
 #undef SG_LAUNCH
     return check_launch("sfb_masked_softmax_grad");
-}
-
-template <typename K>
-static int set_smem(K kernel, size_t bytes)
-{
-    if (bytes > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess) return fail("cudaFuncSetAttribute(%zu bytes): %s", bytes, cudaGetErrorString(e));
-    }
-    return 0;
 }
 
 int simt_fused_sddmm_softmax(cudaStream_t s, const void *nn_lut, const void *a, const void *b, const void *mask, void *y,
@@ -851,16 +1004,18 @@ int simt_fused_attention(cudaStream_t s, const void *nn_lut, const void *q, cons
     SFB_REQUIRE(p.d <= 128, "sfb_fused_attention: state_dim %u > 128 not supported", p.d);
     dim3 grid(p.nb_a, p.B, p.H);
     const float sl = scale * LOG2E_F;
-#define LAUNCH_FA(DMAX)                                                                                          \
+    const uint64_t HD = (uint64_t)p.H * p.d, in = p.in_pitch ? p.in_pitch : HD, on = p.out_pitch ? p.out_pitch : HD;
+    const bool vec = rows_vec(q, dtype, in, p.d) && rows_vec(k, dtype, in, p.d) && rows_vec(v, dtype, in, p.d) && rows_vec(o, dtype, on, p.d);
+#define LAUNCH_FA(DV)                                                                                            \
     {                                                                                                            \
         typedef typename MaskWord<BS>::type W;                                                                   \
-        size_t bytes = sizeof(float) * (2 * DMAX * (BS + 1) + BS * DMAX + BS * (BS + 16));                       \
-        auto kern = fused_attention_kernel<BS, DMAX, DT>;                                                        \
+        const size_t bytes = sizeof(float) * FaCfg<BS, DV>::floats;                                              \
+        auto kern = fused_attention_kernel<BS, DV, DT>;                                                          \
         if (set_smem(kern, bytes)) return 1;                                                                     \
-        kern<<<grid, 256, bytes, s>>>((const uint2 *)nn_lut, q, k, v, o, (const W *)mask, p, sl);                \
+        kern<<<grid, tile::kThreads, bytes, s>>>((const uint2 *)nn_lut, q, k, v, o, (const W *)mask, p, sl, vec); \
     }
     DISPATCH_BS(bs, DISPATCH_DT(dtype, DT, {
-        if (p.d <= 64) LAUNCH_FA(64) else LAUNCH_FA(128)
+        if (p.d <= 32) LAUNCH_FA(32) else if (p.d <= 64) LAUNCH_FA(64) else LAUNCH_FA(128)
     }))
 #undef LAUNCH_FA
     return check_launch("sfb_fused_attention");
