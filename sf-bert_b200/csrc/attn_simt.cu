@@ -852,12 +852,15 @@ fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q
     else if (dt == SFB_BF16) { constexpr int NAME = SFB_BF16; __VA_ARGS__ } \
     else { constexpr int NAME = SFB_F16; __VA_ARGS__ }
 
+// the kernel's dynamic shared memory, asked for once per device and kernel
 template <typename K>
-static int set_smem(K kernel, size_t bytes)
+static int set_smem(DeviceOnce &once, K kernel, size_t bytes)
 {
-    if (bytes > 48 * 1024) {
+    const int dev = current_device();
+    if (bytes > 48 * 1024 && !once.done(dev)) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         if (e != cudaSuccess) return fail("cudaFuncSetAttribute(%zu bytes): %s", bytes, cudaGetErrorString(e));
+        once.mark(dev);
     }
     return 0;
 }
@@ -879,7 +882,7 @@ int simt_sddmm_nt(cudaStream_t s, const void *lut, const void *a, const void *b,
         constexpr uint32_t per = BS == 32 ? 4 : 1;                                                                \
         const size_t bytes = sizeof(float) * 4 * per * BS * tile::kStride;                                        \
         auto kern = sddmm_nt_kernel<BS, AB, CD>;                                                                  \
-        if (set_smem(kern, bytes)) return 1;                                                                      \
+        static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                                                      \
         kern<<<dim3((p.blocks + per - 1) / per, p.B, p.H), tile::kThreads, bytes, s>>>((const uint2 *)lut, a, b, c, p, vec); \
     }
     DISPATCH_BS(bs, DISPATCH_DT(ab_dtype, AB, {
@@ -941,11 +944,11 @@ int simt_spmm_nn(cudaStream_t s, const void *lut, const void *a, const void *b, 
         const dim3 grid(p.nb_a * ((p.d + DSV - 1) / DSV), p.B, p.H);                                              \
         if (trans) {                                                                                              \
             auto kern = spmm_nn_kernel<BS, DSV, AD, BD, true>;                                                    \
-            if (set_smem(kern, bytes)) return 1;                                                                  \
+            static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                                                  \
             kern<<<grid, tile::kThreads, bytes, s>>>((const uint2 *)lut, a, b, c, p, avec, vec);                  \
         } else {                                                                                                  \
             auto kern = spmm_nn_kernel<BS, DSV, AD, BD, false>;                                                   \
-            if (set_smem(kern, bytes)) return 1;                                                                  \
+            static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                                                  \
             kern<<<grid, tile::kThreads, bytes, s>>>((const uint2 *)lut, a, b, c, p, avec, vec);                  \
         }                                                                                                         \
     }
@@ -988,7 +991,7 @@ int simt_fused_sddmm_softmax(cudaStream_t s, const void *nn_lut, const void *a, 
         typedef typename MaskWord<BS>::type W;                                                                   \
         size_t bytes = sizeof(float) * 2 * DMAX * (BS + 1);                                                      \
         auto kern = fused_sddmm_softmax_kernel<BS, DMAX, AB, YD>;                                                \
-        if (set_smem(kern, bytes)) return 1;                                                                     \
+        static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                                                     \
         kern<<<grid, 256, bytes, s>>>((const uint2 *)nn_lut, a, b, (const W *)mask, y, p, sl);                   \
     }
     DISPATCH_BS(bs, DISPATCH_DT(ab_dtype, AB, DISPATCH_DT(y_dtype, YD, {
@@ -1011,7 +1014,7 @@ int simt_fused_attention(cudaStream_t s, const void *nn_lut, const void *q, cons
         typedef typename MaskWord<BS>::type W;                                                                   \
         const size_t bytes = sizeof(float) * FaCfg<BS, DV>::floats;                                              \
         auto kern = fused_attention_kernel<BS, DV, DT>;                                                          \
-        if (set_smem(kern, bytes)) return 1;                                                                     \
+        static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                                                     \
         kern<<<grid, tile::kThreads, bytes, s>>>((const uint2 *)nn_lut, q, k, v, o, (const W *)mask, p, sl, vec); \
     }
     DISPATCH_BS(bs, DISPATCH_DT(dtype, DT, {

@@ -340,7 +340,7 @@ static int launch_ln(cudaStream_t s, void *out, void *sum_out, float *mean, floa
     // are still striding: measured 0.62 against 0.66 of copy bandwidth); the warps loop over the remaining rows
     const uint32_t want = (m + rows_per_cta - 1) / rows_per_cta;
     const size_t smem = 3 * (size_t)hidden * sizeof(float);
-    const int sms = device_sm_count(current_device());
+    const int dev = current_device(), sms = device_sm_count(dev);
     SFB_REQUIRE(sms > 0, "sfb_bias_residual_layernorm: cannot query the device");
 #ifndef SFB_LN_PREFETCH
 #define SFB_LN_PREFETCH true
@@ -348,9 +348,14 @@ static int launch_ln(cudaStream_t s, void *out, void *sum_out, float *mean, floa
 #define LN_LAUNCH(C, R)                                                                                                        \
     do {                                                                                                                       \
         auto kern = bias_residual_layernorm_kernel<DT, C, R, SFB_LN_PREFETCH>;                                                 \
-        int per_sm = 0;                                                                                                        \
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * rows_per_cta, smem) != cudaSuccess || per_sm < 1) \
-            per_sm = 1;                                                                                                        \
+        static std::atomic<uint64_t> known[64];                        /* per device: (shared memory, CTAs per SM) last asked for */ \
+        const uint64_t seen = known[dev & 63].load(std::memory_order_relaxed);                                                 \
+        int per_sm = (int)(uint32_t)seen;                                                                                      \
+        if (per_sm < 1 || (seen >> 32) != smem) {                                                                              \
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * rows_per_cta, smem) != cudaSuccess || per_sm < 1) \
+                per_sm = 1;                                                                                                    \
+            known[dev & 63].store(((uint64_t)smem << 32) | (uint32_t)per_sm, std::memory_order_relaxed);                       \
+        }                                                                                                                      \
         const uint32_t resident = (uint32_t)per_sm * (uint32_t)sms;                                                            \
         launch_overlapped(kern, dim3(want < resident ? want : resident), dim3(32 * rows_per_cta), smem, s, out, sum_out, mean, rstd, x, \
                           bias, resid, gain, beta, m, hidden);                                                                 \

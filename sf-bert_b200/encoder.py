@@ -43,7 +43,9 @@ def encoder_layer(sfb, x, w, lay, heads, ln_order="post", projections="library")
     x2d = x.reshape(m, hidden)
     scale = 1.0 / math.sqrt(d)
     if projections == "tensor":
-        return _encoder_layer_tensor(sfb, x2d, w, lay, heads, ln_order, scale).view(B, L, hidden)
+        # 1 + 1 + 2 projections with the biases and the GELU in their epilogues (Q, K and V as one product, read in place by
+        # the attention as column slices), the attention and two LayerNorm launches, issued from C++
+        return sfb.encoder_layer_tensor(x2d, w, lay, heads, ln_order, scale).view(B, L, hidden)
 
     def attn(h2d):
         q = torch.addmm(w.bq.to(h2d.dtype), h2d, w.wq).view(B, L, heads, d)
@@ -64,34 +66,4 @@ def encoder_layer(sfb, x, w, lay, heads, ln_order="post", projections="library")
     y = torch.mm(f, w.w2)
     out, _, _, _ = sfb.bias_residual_layernorm(y, w.b2, x1, w.g2, w.be2)
     return out.view(B, L, hidden)
-
-
-def _encoder_layer_tensor(sfb, x2d, w, lay, heads, ln_order, scale):
-    """The same layer with every projection on sfb.linear: biases and the GELU ride in the GEMM epilogues, so the
-    layer is 1 + 1 + 2 projections, the attention and two LayerNorm launches."""
-    m, hidden = x2d.shape
-    d = hidden // heads
-    L = lay.nb * lay.block_size
-    B = m // L
-
-    def attn(h2d):
-        # one product for the three projections (the activations are read once, and three times the column tiles fill
-        # the last wave of the GEMM's grid better); the attention reads Q, K and V in place as column slices of the
-        # [m, 3 * hidden] result, rows 3 * hidden elements apart
-        wqkv, bqkv = w.fused_qkv()
-        qkv = sfb.linear(h2d, wqkv, bqkv).view(B, L, 3, heads, d)
-        return sfb.fused_attention_slice(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], lay, scale).view(m, hidden)
-
-    if ln_order == "pre":
-        h, _, _, _ = sfb.bias_residual_layernorm(x2d, None, None, w.g1, w.be1)
-        a = sfb.linear(attn(h), w.wo)
-        h2, x1, _, _ = sfb.bias_residual_layernorm(a, w.bo, x2d, w.g2, w.be2, want_sum=True)
-        f = sfb.linear(h2, w.w1, w.b1, sfb.ACT_GELU)
-        return x1 + sfb.linear(f, w.w2, w.b2)
-    a = sfb.linear(attn(x2d), w.wo)
-    x1, _, _, _ = sfb.bias_residual_layernorm(a, w.bo, x2d, w.g1, w.be1)
-    f = sfb.linear(x1, w.w1, w.b1, sfb.ACT_GELU)
-    y = sfb.linear(f, w.w2)
-    out, _, _, _ = sfb.bias_residual_layernorm(y, w.b2, x1, w.g2, w.be2)
-    return out
 
