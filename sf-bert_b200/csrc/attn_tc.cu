@@ -338,13 +338,17 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
     SharedState *sh = (SharedState *)(smem + kOffState);
     UEntry *lists = (UEntry *)(smem + kOffList);
 
-    const uint32_t hw_warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t hw_warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t warp = hw_warp;
     const uint32_t L = p.nb * 64;
     volatile uint32_t *abort_flag = &sh->abort_flag;
     const uint32_t fmt = BF16 ? 1u : 0u;
 
     if (threadIdx.x == 0) {
+        prefetch_map(qmap);
+        prefetch_map(kmap);
+        prefetch_map(vmap);
+        prefetch_map(omap);
         for (int s = 0; s < kStreams; s++) {
             StreamState *st = &sh->st[s];
             mbar_init(&st->q_full, 1);
@@ -415,7 +419,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
         } else {
         // ===== MMA issuer of stream s:  S(0) | S(1) O(0) | S(2) O(1) | ...  =====
         const uint32_t s = warp - 12;
-        if (lane == 0) {
+        if (elect_one()) {
             StreamState *st = &sh->st[s];
             const uint32_t tbase = tmem + s * kStreamCols;
             const uint32_t t_o = tbase + 96;     // S(even) = tbase, S(odd) = tbase + 32, P(even) = tbase, P(odd) = tbase + 64

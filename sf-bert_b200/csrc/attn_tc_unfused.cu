@@ -92,7 +92,7 @@ sddmm_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant_
     uint8_t *stage_out = tiles + kSdStages * kStage;         // two 8 KB tiles of 16-bit scores on their way out
     SdShared *st = (SdShared *)(stage_out + 2 * kTileBytes);
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t b = blockIdx.y, h = blockIdx.z;
     const uint32_t k0 = blockIdx.x * kChunk;
     const uint32_t T = min(kChunk, p.blocks - k0);
@@ -102,6 +102,10 @@ sddmm_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant_
     const uint32_t fmt = p.is_bf16 ? 1u : 0u;
 
     if (threadIdx.x == 0) {
+        prefetch_map(qmap);
+        prefetch_map(kmap);
+        prefetch_map(omap);
+        prefetch_map(pmap);
         // GRAD: a stage is free when the MMA has read Q and K AND the 128 drain threads have read P
         for (uint32_t s = 0; s < kSdStages; s++) { mbar_init(&st->in_full[s], 1); mbar_init(&st->in_empty[s], GRAD ? 129 : 1); }
         for (int s = 0; s < 2; s++) { mbar_init(&st->s_full[s], 1); mbar_init(&st->s_empty[s], 128); }
@@ -123,7 +127,7 @@ sddmm_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant_
     const int32_t xq = (int32_t)(h * 64);
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t n_q = 0;                                  // query tiles requested so far
             for (uint32_t t = 0; t < T; t++) {
                 const uint32_t s = t % kSdStages;
@@ -150,7 +154,7 @@ sddmm_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = instr_desc(fmt, fmt, 128, 64, 0);
             uint32_t n_q = 0, qi = 0;
             for (uint32_t t = 0; t < T; t++) {
@@ -293,7 +297,7 @@ spmm_tc_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
     constexpr uint32_t kStageBytes = kQBytes + kTileBytes;
     UShared *st = (UShared *)(tiles + kUStages * kStageBytes);
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t pair = blockIdx.x, b = blockIdx.y, h = blockIdx.z;
     const bool has_row1 = pair * 2 + 1 < p.nb;
     const uint32_t L = p.nb * 64;
@@ -302,6 +306,8 @@ spmm_tc_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
     const uint32_t fmt = p.is_bf16 ? 1u : 0u;
 
     if (threadIdx.x == 0) {
+        prefetch_map(pmap);
+        prefetch_map(vmap);
         for (int s = 0; s < kUStages; s++) { mbar_init(&st->in_full[s], 1); mbar_init(&st->in_empty[s], 1); }
         mbar_init(&st->o_final, 1);
         mbar_init(&st->drained, 1);
@@ -322,7 +328,7 @@ spmm_tc_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
     const uint32_t tmem = st->tmem_base;
 
     if (warp == 0) {
-        if (lane == 0 && T > 0) {
+        if (T > 0 && elect_one()) {
             const uint32_t bh_rows = ((b * p.H + h) * p.blocks) * 64;    // first row of this (b,h) in the 2-D view of P
             for (uint32_t t = 0; t < T; t++) {
                 const uint32_t s = t % kUStages;
@@ -338,7 +344,7 @@ spmm_tc_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && T > 0) {
+        if (T > 0 && elect_one()) {
             const uint32_t idesc = instr_desc(fmt, fmt, 128, 64, 1) | (p.trans ? 1u << 15 : 0u);   // bit 15: A is MN-major
             const uint32_t a_step = p.trans ? 128u : 2u;   // descriptor units of 16 bytes per 16 of K
             for (uint32_t t = 0; t < T; t++) {
@@ -433,7 +439,7 @@ fused_p_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constan
     UShared *st = (UShared *)(k_tiles + kUStages * kTileBytes);
     float2 *comb = (float2 *)(st + 1);         // [column half][row]: (max, sum) after sweep 1
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t pair = blockIdx.x, b = blockIdx.y, h = blockIdx.z;
     const uint32_t L = p.nb * 64;
     const uint2 *nn = p.nn_lut + (size_t)h * p.lut_stride;
@@ -441,6 +447,8 @@ fused_p_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constan
     const uint32_t fmt = p.is_bf16 ? 1u : 0u;
 
     if (threadIdx.x == 0) {
+        prefetch_map(qmap);
+        prefetch_map(kmap);
         mbar_init(&st->q_full, 1);
         for (int s = 0; s < kUStages; s++) { mbar_init(&st->in_full[s], 1); mbar_init(&st->in_empty[s], 1); }
         for (int s = 0; s < 2; s++) { mbar_init(&st->s_full[s], 1); mbar_init(&st->s_empty[s], 256); }
@@ -465,7 +473,7 @@ fused_p_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constan
     const int32_t xq = (int32_t)(h * 64);
 
     if (warp == 0) {
-        if (lane == 0 && T > 0) {
+        if (T > 0 && elect_one()) {
             mbar_expect_tx(&st->q_full, kQBytes);
             tma_load_2d(smem_u32(q_tile), &qmap, &st->q_full, xq, (int32_t)(b * L + pair * 128));
             for (uint32_t t = 0; t < T2; t++) {
@@ -477,7 +485,7 @@ fused_p_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constan
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && T > 0) {
+        if (T > 0 && elect_one()) {
             const uint32_t idesc = instr_desc(fmt, fmt, 128, 64, 0);
             const uint64_t q_desc = smem_desc_sw128(smem_u32(q_tile));
             bool alive = mbar_wait(&st->q_full, 0, abort_flag, 42);

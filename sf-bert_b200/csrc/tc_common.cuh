@@ -29,6 +29,17 @@ static __device__ uint32_t g_status = 0;
 // ---- PTX wrappers -------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// one lane of a converged warp; the compiler keeps the branch's addresses and descriptors in uniform registers, which the
+// TMA and tcgen05 instructions take their operands from
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// this thread's warp, as a value the compiler knows to be the same in all lanes
+__device__ __forceinline__ uint32_t uniform_warp() { return __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); }
+
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
@@ -107,6 +118,12 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
         ::"r"(dst), "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y)
         : "memory");
+}
+
+// brings a tensor map into the descriptor cache ahead of the first copy that uses it
+__device__ __forceinline__ void prefetch_map(const CUtensorMap &map)
+{
+    asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&map) : "memory");
 }
 
 __device__ __forceinline__ void tcgen05_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
