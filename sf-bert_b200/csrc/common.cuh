@@ -46,26 +46,39 @@ __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepco
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename... KArgs, typename... Args>
-static inline cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args)
+static inline cudaError_t launch_overlapped_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                                    unsigned cluster, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (cluster > 1) {                 // `cluster` neighbouring CTAs form a cluster (0 or 1: as the kernel declares)
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        n++;
+    }
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = n + 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
     if (e != cudaSuccess) {
-        // a driver or a capture mode that refuses the attribute: the same launch, fully serialised
+        // a driver or a capture mode that refuses the overlap: the same launch, fully serialised
         (void)cudaGetLastError();
-        cfg.numAttrs = 0;
+        cfg.numAttrs = n;
         e = cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
     }
     return e;
+}
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args)
+{
+    return launch_overlapped_cluster(kernel, grid, block, smem, s, 0u, args...);
 }
 
 // ---- device: element conversion -------------------------------------------------------------

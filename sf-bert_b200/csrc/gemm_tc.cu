@@ -12,7 +12,6 @@
 // Every wait on an mbarrier is bounded; on a timeout the CTA records a status word and leaves through the
 // common teardown.
 #include "tc_common.cuh"
-#include <cstdlib>
 
 namespace sfb {
 namespace tc {
@@ -20,19 +19,13 @@ namespace tc {
 constexpr uint32_t kGBM = 128, kGBN = 256, kGBK = 64;
 constexpr uint32_t kGABytes = kGBM * kGBK * 2;           // 16 KB per 128 rows
 constexpr uint32_t kGBBytes = kGBK * kGBN * 2;           // 32 KB: four 64 x 64 boxes
-// MT = row sub-tiles of 128 per CTA tile.  MT = 1: 128 x 256 tiles, two accumulators, the epilogue of a tile runs
-// under the MMAs of the next.  MT = 2: 256 x 256 tiles -- both sub-tiles multiply the same w boxes, so a third less
-// travels from L2 per flop, which is what long-k products are bound by -- at the price of a single accumulator set.
-template <int MT> struct GCfg {
-    static constexpr int stages = MT == 1 ? 4 : 3;
-    static constexpr int acc_bufs = MT == 1 ? 2 : 1;
-    static constexpr uint32_t stage_bytes = MT * kGABytes + kGBBytes;
-    static constexpr size_t smem = 1024 + stages * stage_bytes + 256;
-};
-constexpr int kGMaxStages = 4;
+constexpr uint32_t kBiasBytes = 2 * 2 * 128 * 4;          // the epilogue's bias: [accumulator][column half][128]
+constexpr int kGStages = 4, kGBufs = 2;
+constexpr uint32_t kGStageBytes = kGABytes + kGBBytes;
+constexpr size_t kGSmem = 1024 + kGStages * kGStageBytes + kBiasBytes + 256;
 
 struct GShared {
-    uint64_t full[kGMaxStages], empty[kGMaxStages], acc_full[2], acc_empty[2], drained;
+    uint64_t full[kGStages], empty[kGStages], acc_full[2], acc_empty[2], drained;
     uint32_t tmem_base, abort_flag;
 };
 static_assert(sizeof(GShared) <= 256, "GShared outgrew its slot");
@@ -59,6 +52,15 @@ __device__ __forceinline__ void tile_coords(const GParams &p, uint32_t t, uint32
     tn = b * p.band + (rem - tm * width);
 }
 
+// Four of the bias values of the 128 columns from n0 on, for this lane.  The epilogue reads them from shared memory: from
+// global memory they cost it a trip to the cache per 16 columns, one after another.  Each epilogue warp keeps the values
+// of its tile (fetched a tile ahead) in the slot of its column half and the tile's accumulator; the four warps that
+// share a slot write the same values, and none is more than one tile ahead of another, so two slots are enough.
+__device__ __forceinline__ float4 fetch_bias(const GParams &p, uint32_t n0, uint32_t lane)
+{
+    return p.bias && n0 + lane * 4 < p.N ? __ldg((const float4 *)(p.bias + n0 + lane * 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
 __device__ __forceinline__ float gelu_ref(float t)
 {
     // x * sigmoid(1.702 x), the reference's GELU (gelu_gpu_v2, cuda_kernels.h:561-581), as
@@ -72,7 +74,7 @@ __device__ __forceinline__ float gelu_ref(float t)
 
 // One thread's share of a 128-row accumulator: row `row` of the output, 128 columns from n0 on, read from TMEM at
 // tcol 32 columns at a time (the next 32 travel while these are written), bias and activation applied, 32-byte stores.
-__device__ __forceinline__ void drain_rows(const GParams &p, uint32_t tcol, uint32_t row, uint32_t n0)
+__device__ __forceinline__ void drain_rows(const GParams &p, uint32_t tcol, const float *bias, uint32_t row, uint32_t n0)
 {
     const bool row_ok = row < p.M;
     const size_t off = (size_t)row * p.N + n0;
@@ -94,7 +96,7 @@ __device__ __forceinline__ void drain_rows(const GParams &p, uint32_t tcol, uint
                 if (p.bias) {
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
-                        const float4 bb = __ldg((const float4 *)(p.bias + col) + j);   // the same address in every lane: one broadcast
+                        const float4 bb = *(const float4 *)(bias + c0 + q * 16 + 4 * j);   // the same address in every lane: one broadcast
                         x[4 * j] += bb.x; x[4 * j + 1] += bb.y; x[4 * j + 2] += bb.z; x[4 * j + 3] += bb.w;
                     }
                 }
@@ -118,8 +120,8 @@ __device__ __forceinline__ void drain_rows(const GParams &p, uint32_t tcol, uint
 // the tile to the TMA, twice per 128 columns.  The writes reach memory as whole 128-byte rows instead of 32 bytes per
 // thread and instruction, and the storing threads are free as soon as the tile is in shared memory.
 // row0 = first of the warp's 32 rows, n0 = first of its 128 columns.
-__device__ __forceinline__ void drain_rows_staged(const GParams &p, const CUtensorMap *omap, uint32_t tcol, uint8_t *stage, uint32_t row0,
-                                                  uint32_t n0, uint32_t lane)
+__device__ __forceinline__ void drain_rows_staged(const GParams &p, const CUtensorMap *omap, uint32_t tcol, uint8_t *stage, const float *bias,
+                                                  uint32_t row0, uint32_t n0, uint32_t lane)
 {
     uint8_t *srow = stage + lane * 128;
     uint32_t v[2][32];
@@ -136,14 +138,13 @@ __device__ __forceinline__ void drain_rows_staged(const GParams &p, const CUtens
         uint32_t(&cur)[32] = v[c & 1];
 #pragma unroll
         for (uint32_t q = 0; q < 2; q++) {
-            const uint32_t col = n0 + c0 + q * 16;
             float x[16];
 #pragma unroll
             for (int j = 0; j < 16; j++) x[j] = __uint_as_float(cur[q * 16 + j]);
-            if (p.bias && col < p.N) {      // N is a multiple of 16: a group of 16 is inside or outside as a whole
+            if (p.bias) {
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
-                    const float4 bb = __ldg((const float4 *)(p.bias + col) + j);
+                    const float4 bb = *(const float4 *)(bias + c0 + q * 16 + 4 * j);
                     x[4 * j] += bb.x; x[4 * j + 1] += bb.y; x[4 * j + 2] += bb.z; x[4 * j + 3] += bb.w;
                 }
             }
@@ -171,24 +172,24 @@ __device__ __forceinline__ void drain_rows_staged(const GParams &p, const CUtens
     }
 }
 
-template <int MT>
 __global__ void __launch_bounds__(320, 1)
 linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap, const GParams p)
 {
-    constexpr int kGStages = GCfg<MT>::stages, kBufs = GCfg<MT>::acc_bufs;
-    constexpr uint32_t kGStageBytes = GCfg<MT>::stage_bytes, kBBase = MT * kGABytes;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *tiles = smem;                                   // stage s: A (16 KB) then B (32 KB)
-    GShared *st = (GShared *)(tiles + kGStages * kGStageBytes);
+    float *bias_s = (float *)(tiles + kGStages * kGStageBytes);
+    GShared *st = (GShared *)((uint8_t *)bias_s + kBiasBytes);
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = uniform_warp(), lane = threadIdx.x & 31;
     volatile uint32_t *abort_flag = &st->abort_flag;
     const uint32_t fmt = p.is_bf16 ? 1u : 0u;
     const uint32_t n_tiles = p.tiles_m * p.tiles_n;
     const uint32_t kblocks = (p.K + kGBK - 1) / kGBK;
 
     if (threadIdx.x == 0) {
+        prefetch_map(amap);
+        prefetch_map(bmap);
         for (int s = 0; s < kGStages; s++) { mbar_init(&st->full[s], 1); mbar_init(&st->empty[s], 1); }
         for (int s = 0; s < 2; s++) { mbar_init(&st->acc_full[s], 1); mbar_init(&st->acc_empty[s], 256); }
         mbar_init(&st->drained, 1);
@@ -209,26 +210,24 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
 
     if (warp == 0) {
         // ===== TMA producer =====
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t g = 0;   // k-blocks loaded so far (ring position)
             for (uint32_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-                const int32_t m0 = (int32_t)((t % p.tiles_m) * (MT * kGBM)), n0 = (int32_t)((t / p.tiles_m) * kGBN);
+                const int32_t m0 = (int32_t)((t % p.tiles_m) * kGBM), n0 = (int32_t)((t / p.tiles_m) * kGBN);
                 bool alive = true;
                 for (uint32_t kb = 0; kb < kblocks; kb++, g++) {
                     const uint32_t s = g % kGStages;
                     if (g >= kGStages && !mbar_wait(&st->empty[s], ((g / kGStages) - 1) & 1, abort_flag, 41)) { alive = false; break; }
                     const uint32_t base = smem_u32(tiles + s * kGStageBytes);
                     mbar_expect_tx(&st->full[s], kGStageBytes);   // boxes beyond the tensor arrive as zeros and still count
-#pragma unroll
-                    for (uint32_t mt = 0; mt < MT; mt++)
-                        tma_load_2d(base + mt * kGABytes, &amap, &st->full[s], (int32_t)(kb * kGBK), m0 + (int32_t)(mt * kGBM));
+                    tma_load_2d(base, &amap, &st->full[s], (int32_t)(kb * kGBK), m0);
                     if (p.w_transposed) {
                         // 256 rows of w, 64 of k: one box
-                        tma_load_2d(base + kBBase, &bmap, &st->full[s], (int32_t)(kb * kGBK), n0);
+                        tma_load_2d(base + kGABytes, &bmap, &st->full[s], (int32_t)(kb * kGBK), n0);
                     } else {
 #pragma unroll
                         for (uint32_t j = 0; j < 4; j++)
-                            tma_load_2d(base + kBBase + j * kTileBytes, &bmap, &st->full[s], n0 + (int32_t)(j * 64), (int32_t)(kb * kGBK));
+                            tma_load_2d(base + kGABytes + j * kTileBytes, &bmap, &st->full[s], n0 + (int32_t)(j * 64), (int32_t)(kb * kGBK));
                     }
                 }
                 if (!alive) break;
@@ -236,14 +235,14 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
         }
     } else if (warp == 1) {
         // ===== MMA issuer =====
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = instr_desc(fmt, fmt, kGBM, kGBN, p.w_transposed ? 0 : 1);
             const uint32_t b_step = p.w_transposed ? 2u : 128u;   // descriptor units of 16 bytes per 16 of K
             uint32_t g = 0, i = 0;
             for (uint32_t t = blockIdx.x; t < n_tiles; t += gridDim.x, i++) {
-                const uint32_t buf = i % kBufs;
+                const uint32_t buf = i % kGBufs;
                 bool alive = true;
-                if (i >= (uint32_t)kBufs && !mbar_wait(&st->acc_empty[buf], ((i / kBufs) - 1) & 1, abort_flag, 42)) break;
+                if (i >= (uint32_t)kGBufs && !mbar_wait(&st->acc_empty[buf], ((i / kGBufs) - 1) & 1, abort_flag, 42)) break;
                 tcgen05_fence_after();
                 for (uint32_t kb = 0; kb < kblocks; kb++, g++) {
                     const uint32_t s = g % kGStages;
@@ -251,14 +250,11 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
                     tcgen05_fence_after();
                     const uint32_t base = smem_u32(tiles + s * kGStageBytes);
                     // MN-major: the next 64 columns are one box further on; K-major: 256 rows of 128 bytes
-                    const uint64_t b_desc = p.w_transposed ? smem_desc_sw128(base + kBBase) : smem_desc_sw128(base + kBBase, kTileBytes);
+                    const uint64_t b_desc = p.w_transposed ? smem_desc_sw128(base + kGABytes) : smem_desc_sw128(base + kGABytes, kTileBytes);
+                    const uint64_t a_desc = smem_desc_sw128(base);
 #pragma unroll
-                    for (uint32_t mt = 0; mt < MT; mt++) {
-                        const uint64_t a_desc = smem_desc_sw128(base + mt * kGABytes);
-#pragma unroll
-                        for (uint32_t kk = 0; kk < 4; kk++)   // 16 of K per MMA: +32 bytes in A's swizzled rows, +16 rows (2048 bytes) in B
-                            umma_f16(tmem + (buf * MT + mt) * kGBN, a_desc + 2 * kk, b_desc + b_step * kk, idesc, (kb | kk) ? 1u : 0u);
-                    }
+                    for (uint32_t kk = 0; kk < 4; kk++)   // 16 of K per MMA: +32 bytes in A's swizzled rows, +16 rows (2048 bytes) in B
+                        umma_f16(tmem + buf * kGBN, a_desc + 2 * kk, b_desc + b_step * kk, idesc, (kb | kk) ? 1u : 0u);
                     umma_commit(&st->empty[s]);
                 }
                 if (!alive) break;
@@ -272,16 +268,17 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
         const uint32_t r = quarter * 32 + lane;
         const uint32_t lane_field = (quarter * 32) << 16;
         uint32_t i = 0;
+        float4 next = fetch_bias(p, (blockIdx.x / p.tiles_m) * kGBN + chalf * 128, lane);
         for (uint32_t t = blockIdx.x; t < n_tiles; t += gridDim.x, i++) {
-            const uint32_t buf = i % kBufs;
+            const uint32_t buf = i % kGBufs;
             const uint32_t n0 = (t / p.tiles_m) * kGBN + chalf * 128;
-            if (!mbar_wait_warp(&st->acc_full[buf], (i / kBufs) & 1, abort_flag, 44)) break;
+            float *bias = bias_s + ((i & 1) * 2 + chalf) * 128;
+            *(float4 *)(bias + lane * 4) = next;
+            __syncwarp();
+            if (t + gridDim.x < n_tiles) next = fetch_bias(p, ((t + gridDim.x) / p.tiles_m) * kGBN + chalf * 128, lane);
+            if (!mbar_wait_warp(&st->acc_full[buf], (i / kGBufs) & 1, abort_flag, 44)) break;
             tcgen05_fence_after();
-#pragma unroll 1
-            for (uint32_t mt = 0; mt < MT; mt++) {
-            const uint32_t m0 = (t % p.tiles_m) * (MT * kGBM) + mt * kGBM;
-            drain_rows(p, tmem + (buf * MT + mt) * kGBN + chalf * 128 + lane_field, m0 + r, n0);
-            }
+            drain_rows(p, tmem + buf * kGBN + chalf * 128 + lane_field, bias, (t % p.tiles_m) * kGBM + r, n0);
             tcgen05_fence_before();
             mbar_arrive(&st->acc_empty[buf]);
         }
@@ -334,7 +331,9 @@ constexpr uint32_t kPStagingBytes = 8 * 32 * 128;     // one 32-row x 64-column 
 constexpr uint32_t kPABytes = kGBM * kGBK * 2;            // 16 KB: this CTA's 128 rows of x
 constexpr uint32_t kPBBytes = kGBK * (kGBN / 2) * 2;      // 16 KB: this CTA's 128 columns of w
 constexpr uint32_t kPStageBytes = kPABytes + kPBBytes;
-constexpr size_t kPSmem = 1024 + kPStages * kPStageBytes + kPStagingBytes + 256;
+// the shared window starts on a multiple of 1024 (aligned below): there is no room left for slack
+constexpr size_t kPSmem = kPStages * kPStageBytes + kPStagingBytes + kBiasBytes + 256;
+static_assert(kPSmem <= 227 * 1024, "shared memory budget");
 
 struct PShared {
     uint64_t full[kPStages], empty[kPStages], acc_full[2], acc_empty[2], drained;
@@ -393,13 +392,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1)
 linear_tc_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap,
                       const __grid_constant__ CUtensorMap omap, const GParams p)
 {
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t *tiles = smem;                                   // stage s: A (16 KB) then this CTA's half of B (16 KB)
+    extern __shared__ __align__(1024) uint8_t smem_aligned[];
+    uint8_t *tiles = smem_aligned;                                   // stage s: A (16 KB) then this CTA's half of B (16 KB)
     uint8_t *staging = tiles + kPStages * kPStageBytes;      // the epilogue warps' output tiles (4 KB each)
-    PShared *st = (PShared *)(staging + kPStagingBytes);
+    float *bias_s = (float *)(staging + kPStagingBytes);
+    PShared *st = (PShared *)((uint8_t *)bias_s + kBiasBytes);
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();                 // 0: issues the MMAs of the pair
     const uint32_t pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     volatile uint32_t *abort_flag = &st->abort_flag;
@@ -408,6 +407,9 @@ linear_tc_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_con
     const uint32_t kblocks = (p.K + kGBK - 1) / kGBK;
 
     if (threadIdx.x == 0) {
+        prefetch_map(amap);
+        prefetch_map(bmap);
+        prefetch_map(omap);
         for (uint32_t s = 0; s < kPStages; s++) { mbar_init(&st->full[s], 1); mbar_init(&st->empty[s], 1); }
         for (int s = 0; s < 2; s++) { mbar_init(&st->acc_full[s], 1); mbar_init(&st->acc_empty[s], 16); }   // 8 epilogue warps of each CTA
         mbar_init(&st->drained, 1);
@@ -429,7 +431,7 @@ linear_tc_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_con
 
     if (warp == 0) {
         // ===== TMA producer (both CTAs): own rows of x, own half of the w tile; bytes counted on the even CTA's barrier =====
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t g = 0;
             for (uint32_t t = pair; t < n_tiles; t += pairs) {
                 uint32_t tm, tn;
@@ -457,7 +459,7 @@ linear_tc_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_con
         }
     } else if (warp == 1) {
         // ===== MMA issuer: one thread of the even CTA for the pair =====
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             const uint32_t idesc = instr_desc(fmt, fmt, 256, kGBN, p.w_transposed ? 0 : 1);
             const uint32_t b_step = p.w_transposed ? 2u : 128u;
             uint32_t g = 0, i = 0;
@@ -489,16 +491,23 @@ linear_tc_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_con
         const uint32_t chalf = (warp - 2) >> 2;
         const uint32_t lane_field = (quarter * 32) << 16;
         const uint32_t acc_empty0[2] = {mapa_rank(smem_u32(&st->acc_empty[0]), 0), mapa_rank(smem_u32(&st->acc_empty[1]), 0)};
-        uint32_t i = 0;
+        uint32_t i = 0, tm, tn;
+        tile_coords(p, pair, tm, tn);
+        float4 next = fetch_bias(p, tn * kGBN + chalf * 128, lane);
         for (uint32_t t = pair; t < n_tiles; t += pairs, i++) {
             const uint32_t buf = i & 1;
-            uint32_t tm, tn;
-            tile_coords(p, t, tm, tn);
             const uint32_t n0 = tn * kGBN + chalf * 128;
             const uint32_t m0 = tm * 256 + rank * kGBM;
+            float *bias = bias_s + (buf * 2 + chalf) * 128;
+            *(float4 *)(bias + lane * 4) = next;
+            __syncwarp();
+            if (t + pairs < n_tiles) {
+                tile_coords(p, t + pairs, tm, tn);
+                next = fetch_bias(p, tn * kGBN + chalf * 128, lane);
+            }
             if (!mbar_wait_warp(&st->acc_full[buf], (i >> 1) & 1, abort_flag, 54)) break;
             tcgen05_fence_after();
-            drain_rows_staged(p, &omap, tmem + buf * kGBN + chalf * 128 + lane_field, staging + (warp - 2) * 4096, m0 + quarter * 32, n0, lane);
+            drain_rows_staged(p, &omap, tmem + buf * kGBN + chalf * 128 + lane_field, staging + (warp - 2) * 4096, bias, m0 + quarter * 32, n0, lane);
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(buf ? acc_empty0[1] : acc_empty0[0]);
@@ -528,6 +537,212 @@ linear_tc_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_con
     }
 }
 
+// ---- few tiles: the contraction split over a cluster -------------------------------------------------------------
+// With fewer 128 x 256 tiles than SMs the kernels above leave most of the chip idle, and the tiles that do run walk the
+// whole of k one after another (m = 320, n = 768, k = 3072: 9 CTAs, 20 us).  Here a tile is 128 x BN and a cluster of
+// `split` CTAs shares it, each multiplying its share of the k-blocks; the fp32 accumulators meet in distributed shared
+// memory: every CTA leaves its own in shared memory, and after the cluster's barrier each adds up its share of the
+// rows from all of them, rank 0 first (the sum does not depend on timing), applies bias and activation and stores.
+// One tile per CTA and deep stages: with few CTAs pulling through L2 the distance to it is what a k-block waits for.
+// Measured, launches in sequence: m 320, n 768, k 3072 17.7 -> 8.6 us (two CTAs per 128 x 64 tile), m 320, n 768, k 768
+// 8.4 -> 4.9 us (128 x 64), m 2048, n 768, k 3072 20.6 -> 14.0 us (128 x 128).
+template <int BN, int ST> struct SCfg {
+    static constexpr uint32_t stages = ST;
+    static constexpr uint32_t stage_bytes = kGABytes + kGBK * BN * 2;
+    static constexpr uint32_t acc_stride = BN + 4;                                  // floats
+    static constexpr uint32_t acc_bytes = kGBM * acc_stride * 4;
+    static constexpr uint32_t body = stages * stage_bytes > acc_bytes ? stages * stage_bytes : acc_bytes;
+    static constexpr size_t smem = 1024 + body + BN * 4 + 256;
+};
+struct SShared {
+    uint64_t full[8], empty[8], acc_full, drained;
+    uint32_t tmem_base, abort_flag;
+};
+static_assert(sizeof(SShared) <= 256, "SShared outgrew its slot");
+
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr)
+{
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
+    return v;
+}
+
+// eight neighbouring outputs of one row: bias, activation, one 16-byte store
+__device__ __forceinline__ void finish8(const GParams &p, float (&x)[8], const float *bias, uint32_t row, uint32_t col)
+{
+    if (p.bias) {
+        const float4 b0 = *(const float4 *)bias, b1 = *(const float4 *)(bias + 4);
+        x[0] += b0.x; x[1] += b0.y; x[2] += b0.z; x[3] += b0.w;
+        x[4] += b1.x; x[5] += b1.y; x[6] += b1.z; x[7] += b1.w;
+    }
+    if (p.act == 1) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) x[j] = gelu_ref(x[j]);
+    }
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) w[j] = pack2(x[2 * j], x[2 * j + 1], p.is_bf16);
+    *(uint4 *)((uint16_t *)p.out + (size_t)row * p.N + col) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+template <int BN, int ST>
+__global__ void __launch_bounds__(256, 1)
+linear_tc_split_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap, const GParams p, const uint32_t split)
+{
+    typedef SCfg<BN, ST> Cfg;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    float *bias_s = (float *)(smem + Cfg::body);           // the tile's bias: a read from L2 per column group would be on the critical path
+    SShared *st = (SShared *)(smem + Cfg::body + BN * 4);
+    float *acc_s = (float *)smem;                          // the accumulator's place once the stages are spent
+
+    const uint32_t warp = uniform_warp(), lane = threadIdx.x & 31;
+    volatile uint32_t *abort_flag = &st->abort_flag;
+    const uint32_t fmt = p.is_bf16 ? 1u : 0u;
+    const uint32_t tile = blockIdx.x / split, rank = blockIdx.x - tile * split;    // the cluster is `split` neighbouring CTAs
+    const uint32_t tm = tile % p.tiles_m, tn = tile / p.tiles_m;
+    const uint32_t kblocks = (p.K + kGBK - 1) / kGBK;
+    const uint32_t kb0 = kblocks * rank / split, kb1 = kblocks * (rank + 1) / split;   // split <= kblocks: never empty
+
+    if (threadIdx.x == 0) {
+        prefetch_map(amap);
+        prefetch_map(bmap);
+        for (uint32_t s = 0; s < ST; s++) { mbar_init(&st->full[s], 1); mbar_init(&st->empty[s], 1); }
+        mbar_init(&st->acc_full, 1);
+        mbar_init(&st->drained, 1);
+        st->abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        __syncwarp();
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&st->tmem_base)), "r"((uint32_t)BN) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    const uint32_t tmem = st->tmem_base;
+    grid_dependency_wait();
+    grid_launch_dependents();
+
+    if (warp == 0) {
+        if (elect_one()) {
+            for (uint32_t kb = kb0; kb < kb1; kb++) {
+                const uint32_t g = kb - kb0, s = g % ST;
+                if (g >= ST && !mbar_wait(&st->empty[s], ((g / ST) - 1) & 1, abort_flag, 61)) break;
+                const uint32_t base = smem_u32(smem + s * Cfg::stage_bytes);
+                mbar_expect_tx(&st->full[s], Cfg::stage_bytes);       // boxes beyond the tensor arrive as zeros and still count
+                tma_load_2d(base, &amap, &st->full[s], (int32_t)(kb * kGBK), (int32_t)(tm * kGBM));
+                if (p.w_transposed) {
+                    tma_load_2d(base + kGABytes, &bmap, &st->full[s], (int32_t)(kb * kGBK), (int32_t)(tn * BN));
+                } else {
+#pragma unroll
+                    for (uint32_t j = 0; j < BN / 64; j++)
+                        tma_load_2d(base + kGABytes + j * kTileBytes, &bmap, &st->full[s], (int32_t)(tn * BN + j * 64), (int32_t)(kb * kGBK));
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (elect_one()) {
+            const uint32_t idesc = instr_desc(fmt, fmt, kGBM, BN, p.w_transposed ? 0 : 1);
+            const uint32_t b_step = p.w_transposed ? 2u : 128u;
+            bool alive = true;
+            for (uint32_t kb = kb0; kb < kb1; kb++) {
+                const uint32_t g = kb - kb0, s = g % ST;
+                if (!mbar_wait(&st->full[s], (g / ST) & 1, abort_flag, 62)) { alive = false; break; }
+                tcgen05_fence_after();
+                const uint32_t base = smem_u32(smem + s * Cfg::stage_bytes);
+                const uint64_t a_desc = smem_desc_sw128(base);
+                const uint64_t b_desc = p.w_transposed ? smem_desc_sw128(base + kGABytes) : smem_desc_sw128(base + kGABytes, kTileBytes);
+#pragma unroll
+                for (uint32_t kk = 0; kk < 4; kk++) umma_f16(tmem, a_desc + 2 * kk, b_desc + b_step * kk, idesc, (g | kk) ? 1u : 0u);
+                umma_commit(&st->empty[s]);
+            }
+            if (alive) umma_commit(&st->acc_full);
+        }
+    }
+    else if (warp == 2 && p.bias) {
+        for (uint32_t c = lane; c < BN; c += 32) bias_s[c] = tn * BN + c < p.N ? __ldg(p.bias + tn * BN + c) : 0.f;
+    }
+    __syncwarp();
+    // ===== all eight warps drain the accumulator: 32 rows and half of the columns each =====
+    const bool ok = mbar_wait_warp(&st->acc_full, 0, abort_flag, 63);
+    __syncthreads();                                       // the bias is in place
+    const uint32_t quarter = warp & 3, ch = warp >> 2, r = quarter * 32 + lane, lane_field = (quarter * 32) << 16;
+    if (ok) {
+        tcgen05_fence_after();
+#pragma unroll
+        for (uint32_t c0 = 0; c0 < BN / 2; c0 += 32) {
+            const uint32_t c = ch * (BN / 2) + c0;
+            uint32_t v[32];
+            TMEM_LD_32((v), tmem + c + lane_field);
+            tmem_wait_ld();
+            if (split == 1) {
+                const uint32_t row = tm * kGBM + r;
+#pragma unroll
+                for (uint32_t q = 0; q < 4; q++) {
+                    const uint32_t col = tn * BN + c + q * 8;
+                    if (row < p.M && col < p.N) {
+                        float x[8];
+#pragma unroll
+                        for (int j = 0; j < 8; j++) x[j] = __uint_as_float(v[q * 8 + j]);
+                        finish8(p, x, bias_s + c + q * 8, row, col);
+                    }
+                }
+            } else {
+                float4 *d = (float4 *)(acc_s + r * Cfg::acc_stride + c);
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    d[j] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+            }
+        }
+        tcgen05_fence_before();
+    }
+    if (split > 1) {
+        // every CTA of the cluster reaches both barriers, also after a timeout (the status word then says that the sums are not to be used)
+        cluster_sync_all();
+        const uint32_t rows = kGBM / split, first = rank * rows;      // split is 2, 4 or 8
+        const uint32_t mine = smem_u32(acc_s);
+        constexpr uint32_t PIECES = BN / 8;
+        for (uint32_t t = threadIdx.x; t < rows * PIECES; t += 256) {
+            const uint32_t rr = first + t / PIECES, c = (t % PIECES) * 8;
+            const uint32_t row = tm * kGBM + rr, col = tn * BN + c;
+            if (row >= p.M || col >= p.N) continue;
+            const uint32_t at = mine + (rr * Cfg::acc_stride + c) * 4;
+            float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+            for (uint32_t k = 0; k < split; k++) {
+                const uint32_t a = mapa_rank(at, k);
+                const float4 u = ld_cluster_f4(a), w = ld_cluster_f4(a + 16);
+                x[0] += u.x; x[1] += u.y; x[2] += u.z; x[3] += u.w;
+                x[4] += w.x; x[5] += w.y; x[6] += w.z; x[7] += w.w;
+            }
+            finish8(p, x, bias_s + c, row, col);
+        }
+        __syncwarp();
+        cluster_sync_all();                                           // the others have read this CTA's accumulator
+    }
+
+    // ---- teardown (also the way out after a timeout) ----
+    __syncthreads();
+    if (st->abort_flag) {
+        if (warp == 1 && lane == 0) {
+            umma_commit(&st->drained);
+            for (uint32_t k = 0; k < kWaitLimit && !mbar_try_wait(&st->drained, 0); k++) {}
+        }
+        if (warp == 0 && lane == 0) {
+            const uint64_t t0 = clock64();
+            while (clock64() - t0 < 2000000ull) {}
+        }
+        __syncthreads();
+    }
+    if (warp == 0) {
+        __syncwarp();
+        tcgen05_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)BN) : "memory");
+    }
+}
+
 // [rows, cols] 16-bit row-major tensor, boxes of box_rows x 64 elements, 128-byte swizzle
 static int make_map_2d(CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols, int is_bf16, uint32_t box_rows)
 {
@@ -546,6 +761,67 @@ static int make_map_2d(CUtensorMap *map, const void *base, uint64_t rows, uint64
 
 }  // namespace tc
 
+template <int BN, int ST>
+static int launch_split(cudaStream_t s, const CUtensorMap &am, const void *w, const tc::GParams &g, uint32_t split, int dev)
+{
+    using namespace tc;
+    static DeviceOnce once;
+    if (!once.done(dev)) {
+        if (cudaFuncSetAttribute(linear_tc_split_kernel<BN, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCfg<BN, ST>::smem) != cudaSuccess)
+            return fail("sfb_linear: cannot reserve %zu bytes of shared memory", SCfg<BN, ST>::smem);
+        once.mark(dev);
+    }
+    CUtensorMap bm;
+    if (g.w_transposed ? make_map_2d(&bm, w, g.N, g.K, g.is_bf16, BN) : make_map_2d(&bm, w, g.K, g.N, g.is_bf16, kGBK)) return 1;
+    GParams prm = g;
+    prm.tiles_m = (g.M + kGBM - 1) / kGBM;
+    prm.tiles_n = (g.N + BN - 1) / BN;
+    launch_overlapped_cluster(linear_tc_split_kernel<BN, ST>, dim3(prm.tiles_m * prm.tiles_n * split), dim3(256), SCfg<BN, ST>::smem, s, split, am, bm,
+                              prm, split);
+    return check_launch("sfb_linear");
+}
+
+// Which kernel and which tile: the one with the least estimated time, in microseconds.  Each estimate is a fixed part (the
+// hand-over from the kernel before, the first load, the last tile's epilogue) plus the k-blocks of 64 that a CTA walks
+// one after another, times what one costs -- which grows with the share of the SMs that pull operands through L2.
+// Fitted to 36 shapes (m 64-32768, n 256-4096, k 256-4096, bf16, launches in sequence); within 8 % of all of them, and
+// the shape's fastest variant or one within 4 % of it is the one taken:
+//   128 x 64 and 128 x 128 tiles, one per CTA, only while all of them run at once: 2.7 + 0.165 and 3.7 + 0.175 per
+//     k-block; sharing a tile between 2 (4) CTAs costs 1.9 (2.2) more, and clusters of four are only placed at once in a
+//     third of the SMs (with twice as many CTAs they took two rounds);
+//   128 x 256 tiles, persistent: 5.0 + 0.25 per k-block and round;  256 x 256 tiles on CTA pairs: 5.4 + 0.27.
+struct LinearPlan {
+    int kind;                  // 0: 128 x 256, 1: CTA pairs, 2: one tile per cluster
+    uint32_t bn, split;
+};
+static LinearPlan plan_linear(uint32_t m, uint32_t n, uint32_t k, uint32_t sms)
+{
+    using namespace tc;
+    const uint32_t kb = (k + kGBK - 1) / kGBK, tiles_m = (m + kGBM - 1) / kGBM, tiles_n = (n + kGBN - 1) / kGBN;
+    auto waves = [&](uint64_t tiles, uint32_t slots, double fixed, double per, double load) {
+        const uint64_t rounds = (tiles + slots - 1) / slots;
+        const double share = tiles < slots ? (double)tiles / slots : 1.0;
+        return fixed + (double)kb * (double)rounds * (per + load * share);
+    };
+    LinearPlan best = {0, kGBN, 1};
+    double t_best = waves((uint64_t)tiles_m * tiles_n, sms, 5.0, 0.25, 0.13);
+    if (kUsePairs && sms >= 2) {
+        const double t = waves((uint64_t)((m + 255) / 256) * tiles_n, sms / 2, 5.4, 0.27, 0.09);
+        if (t < t_best) { t_best = t; best = {1, kGBN, 1}; }
+    }
+    for (uint32_t bn = 64; bn <= 128; bn += 64) {
+        const uint64_t tiles = (uint64_t)tiles_m * ((n + bn - 1) / bn);
+        for (uint32_t split = 1; split <= 4 && split <= kb; split *= 2) {
+            const uint64_t ctas = tiles * split;
+            if (ctas > (split == 4 ? sms / 3 : sms)) break;
+            const double t = (bn == 64 ? 2.7 : 3.7) + (split == 1 ? 0.0 : split == 2 ? 1.9 : 2.2) +
+                             (double)((kb + split - 1) / split) * ((bn == 64 ? 0.165 : 0.175) + 0.04 * (double)ctas / sms);
+            if (t < t_best) { t_best = t; best = {2, bn, split}; }
+        }
+    }
+    return best;
+}
+
 int tc_linear(cudaStream_t s, void *out, const void *x, const void *w, const float *bias, uint32_t m, uint32_t n, uint32_t k,
               int dtype, int act, bool w_transposed)
 {
@@ -553,21 +829,15 @@ int tc_linear(cudaStream_t s, void *out, const void *x, const void *w, const flo
     const int is_bf16 = dtype == SFB_BF16;
     CUtensorMap am, bm;
     if (make_map_2d(&am, x, m, k, is_bf16, kGBM)) return 1;
-    if (w_transposed ? make_map_2d(&bm, w, n, k, is_bf16, kGBN) : make_map_2d(&bm, w, k, n, is_bf16, kGBK)) return 1;
-    static DeviceOnce once;
     const int dev = current_device();
     const int sms = device_sm_count(dev);
     if (sms <= 0) return fail("sfb_linear: cannot read the SM count");
-    if (!once.done(dev)) {
-        if (cudaFuncSetAttribute(linear_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GCfg<1>::smem) != cudaSuccess ||
-            cudaFuncSetAttribute(linear_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GCfg<2>::smem) != cudaSuccess)
-            return fail("sfb_linear: cannot reserve %zu bytes of shared memory", GCfg<1>::smem);
-        once.mark(dev);
-    }
+    const LinearPlan plan = plan_linear(m, n, k, (uint32_t)sms);
     const uint32_t tiles_n = (n + kGBN - 1) / kGBN;
-    // CTA pairs on 256 x 256 tiles whenever there is at least one tile per pair of SMs
-    const uint32_t pair_tiles = ((m + 255) / 256) * tiles_n;
-    if (kUsePairs && sms >= 2 && pair_tiles >= (uint32_t)(sms / 2)) {
+    GParams prm = {out, bias, m, n, k, 0, tiles_n, is_bf16, act, w_transposed ? 1 : 0, 1};
+    if (plan.kind == 2)
+        return plan.bn == 64 ? launch_split<64, 8>(s, am, w, prm, plan.split, dev) : launch_split<128, 6>(s, am, w, prm, plan.split, dev);
+    if (plan.kind == 1) {
         CUtensorMap bp;
         if (w_transposed ? make_map_2d(&bp, w, n, k, is_bf16, kGBN / 2) : make_map_2d(&bp, w, k, n, is_bf16, kGBK)) return 1;
         static DeviceOnce once_pair;
@@ -578,19 +848,26 @@ int tc_linear(cudaStream_t s, void *out, const void *x, const void *w, const flo
         }
         CUtensorMap om;      // out as [m, n], boxes of 32 rows x 64 columns for the epilogue's stores
         if (make_map_2d(&om, out, m, n, is_bf16, 32)) return 1;
-        GParams prm = {out, bias, m, n, k, (m + 255) / 256, tiles_n, is_bf16, act, w_transposed ? 1 : 0, tiles_n < kPBand ? tiles_n : kPBand};
-        const uint32_t pairs = pair_tiles < (uint32_t)(sms / 2) ? pair_tiles : (uint32_t)(sms / 2);
+        prm.tiles_m = (m + 255) / 256;
+        prm.band = tiles_n < kPBand ? tiles_n : kPBand;
+        const uint64_t pair_tiles = (uint64_t)prm.tiles_m * tiles_n;
+        const uint32_t pairs = pair_tiles < (uint64_t)(sms / 2) ? (uint32_t)pair_tiles : (uint32_t)(sms / 2);
         launch_overlapped(linear_tc_pair_kernel, dim3(2 * pairs), dim3(320), kPSmem, s, am, bp, om, prm);
         // a device or a partition that cannot place the clusters refuses the launch: the single-CTA kernel takes over
         if (cudaGetLastError() == cudaSuccess) { clear_error(); return 0; }
     }
-    // long-k products are bound by what travels from L2: 256-row tiles, as long as they still fill the SMs twice over
-    const int mt = (k >= 2048 && (uint64_t)((m + 255) / 256) * tiles_n >= 2ull * sms) ? 2 : 1;
-    GParams prm = {out, bias, m, n, k, (m + mt * kGBM - 1) / (mt * kGBM), tiles_n, is_bf16, act, w_transposed ? 1 : 0, 1};
-    const uint32_t tiles = prm.tiles_m * prm.tiles_n;
-    const uint32_t grid = tiles < (uint32_t)sms ? tiles : (uint32_t)sms;
-    if (mt == 2) launch_overlapped(linear_tc_kernel<2>, dim3(grid), dim3(320), GCfg<2>::smem, s, am, bm, prm);
-    else launch_overlapped(linear_tc_kernel<1>, dim3(grid), dim3(320), GCfg<1>::smem, s, am, bm, prm);
+    if (w_transposed ? make_map_2d(&bm, w, n, k, is_bf16, kGBN) : make_map_2d(&bm, w, k, n, is_bf16, kGBK)) return 1;
+    static DeviceOnce once;
+    if (!once.done(dev)) {
+        if (cudaFuncSetAttribute(linear_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGSmem) != cudaSuccess)
+            return fail("sfb_linear: cannot reserve %zu bytes of shared memory", kGSmem);
+        once.mark(dev);
+    }
+    prm.tiles_m = (m + kGBM - 1) / kGBM;
+    prm.band = 1;
+    const uint64_t tiles = (uint64_t)prm.tiles_m * prm.tiles_n;
+    const uint32_t grid = tiles < (uint64_t)sms ? (uint32_t)tiles : (uint32_t)sms;
+    launch_overlapped(linear_tc_kernel, dim3(grid), dim3(320), kGSmem, s, am, bm, prm);
     return check_launch("sfb_linear");
 }
 

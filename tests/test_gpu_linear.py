@@ -35,6 +35,27 @@ def test_linear_against_oracle(sfb, oracle, dtype, m, n, k, act, with_bias):
     assert np.abs(got.float().cpu().numpy() - want).max() <= 2e-2 * np.abs(want).max()
 
 
+@pytest.mark.parametrize("transposed", [False, True])
+@pytest.mark.parametrize("m,n,k,act", [
+    (1, 16, 8, 0),                   # the smallest: one row, one column group, an eighth of a k-block
+    (129, 80, 72, 1),                # one row and 16 columns into the second tiles
+    (64, 192, 520, 1),               # nine k-blocks over four CTAs per tile
+    (320, 768, 3072, 0),             # two CTAs per 128 x 64 tile
+    (640, 1040, 4096, 1),            # two CTAs per 128 x 128 tile, the last one 16 columns wide
+    (2048, 1024, 1032, 0),           # 128 x 128 tiles, eight elements into the last k-block
+])
+def test_linear_few_tiles(sfb, oracle, m, n, k, act, transposed):
+    x, xn = _mk(oracle, (m, k), 420, "bf16")
+    w, wn = _mk(oracle, (n, k) if transposed else (k, n), 421, "bf16", 0.05)
+    b = torch.from_numpy(oracle.fill_normal((n,), 422, 0.5)).cuda()
+    got = (sfb.linear_nt if transposed else sfb.linear)(x, w, b, act)
+    again = (sfb.linear_nt if transposed else sfb.linear)(x, w, b, act)
+    assert sfb.device_status() == 0 and torch.equal(got, again)      # the shares of a tile are added in a fixed order
+    rows = np.unique(np.r_[np.arange(0, m, 37), m - 1])
+    want = oracle.linear(xn[rows], np.ascontiguousarray(wn.T) if transposed else wn, b.cpu().numpy(), act)
+    assert np.abs(got[rows].float().cpu().numpy() - want).max() <= 2e-2 * np.abs(want).max()
+
+
 def test_linear_more_tiles_than_sms_and_batched_input(sfb, oracle):
     """A [B, L, hidden] activation (leading dimensions flattened) with enough tiles that every CTA loops."""
     B, L, hidden, n = 2, 4096, 768, 2304
