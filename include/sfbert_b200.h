@@ -248,6 +248,12 @@ int sfb_linear(sfb_stream_t stream, void *out, const void *x, const void *w, con
 int sfb_linear_nt(sfb_stream_t stream, void *out, const void *x, const void *wt, const float *bias, uint32_t m,
                   uint32_t n, uint32_t k, int dtype, int act);
 
+/* out = resid + (x . w + bias), w [k, n] as in sfb_linear; the product is rounded to the element type before the sum, as
+ * by sfb_linear and a separate add (the last line of a pre-LN encoder layer, transformer_inference_part.cpp:239).
+ * resid is [m, n] of x's type and not out itself. */
+int sfb_linear_residual(sfb_stream_t stream, void *out, const void *x, const void *w, const float *bias, const void *resid,
+                        uint32_t m, uint32_t n, uint32_t k, int dtype);
+
 /* out[b, l, :] = table[ids[b, l], :] + pos[l, :]: the front of the encoder stack.  table [vocab, hidden], pos
  * [seq_len, hidden] (may be NULL) and out [batch, seq_len, hidden] are of type dtype; ids are int32 in device memory.
  * An id outside [0, vocab) gives a row of zeros and is counted in *bad_ids (device uint32, may be NULL) instead of

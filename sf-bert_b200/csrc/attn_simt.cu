@@ -47,6 +47,8 @@ __global__ void __launch_bounds__(tile::kThreads, 3) sddmm_nt_kernel(const uint2
     constexpr uint32_t ROWS = PER * BS;                      // staged rows of each operand: 128 or 64
     constexpr uint32_t BUF = 2 * ROWS * kStride;
     extern __shared__ __align__(16) float sm[];              // [2][A rows | B rows]
+    grid_dependency_wait();
+    grid_launch_dependents();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane_row(lane), lc = lane_quad(lane);
     const uint32_t bid0 = blockIdx.x * PER, b = blockIdx.y, h = blockIdx.z;
     const uint32_t nblk = min(PER, p.blocks - bid0);
@@ -226,6 +228,8 @@ __global__ void __launch_bounds__(BS * BS / 8 / SPLIT, (NB > 0 && SPLIT > 1 && B
 {
     typedef typename MaskWord<BS>::type W;
     constexpr int LPR = BS / 8;  // lanes per query row
+    grid_dependency_wait();
+    grid_launch_dependents();
     const uint32_t i = blockIdx.x / SPLIT, b = blockIdx.y, h = blockIdx.z;
     const uint2 *nn = lut + (size_t)h * p.lut_stride;
     const uint2 head = nn[i];
@@ -419,6 +423,8 @@ __global__ void __launch_bounds__(BS * BS / 8 / SPLIT) softmax_grad_kernel(const
                                                                      float scale)
 {
     constexpr int LPR = BS / 8;  // lanes per query row
+    grid_dependency_wait();
+    grid_launch_dependents();
     const uint32_t i = blockIdx.x / SPLIT, b = blockIdx.y, h = blockIdx.z;
     const uint2 *nn = lut + (size_t)h * p.lut_stride;
     const uint2 head = nn[i];
@@ -510,6 +516,8 @@ __global__ void __launch_bounds__(tile::kThreads, 4) spmm_nn_kernel(const uint2 
     constexpr uint32_t PARTS = BS / 32;                                  // chunks per block
     constexpr uint32_t a_stride = TRANS ? BS + 4 : kStride;
     extern __shared__ __align__(16) float sm[];                          // [2][P chunk | V chunk]
+    grid_dependency_wait();
+    grid_launch_dependents();
     const uint32_t nslice = (p.d + DS - 1) / DS;
     const uint32_t i = blockIdx.x / nslice, d0 = (blockIdx.x % nslice) * DS;
     const uint32_t b = blockIdx.y, h = blockIdx.z;
@@ -609,6 +617,8 @@ __global__ void __launch_bounds__(256) fused_sddmm_softmax_kernel(const uint2 *_
     extern __shared__ float smem[];
     float (*Qs)[BS + 1] = (float (*)[BS + 1])smem;
     float (*Ks)[BS + 1] = (float (*)[BS + 1])(smem + DMAX * (BS + 1));
+    grid_dependency_wait();
+    grid_launch_dependents();
     const uint32_t i = blockIdx.x, b = blockIdx.y, h = blockIdx.z;
     const uint2 *nn = lut + (size_t)h * p.lut_stride;
     const uint2 head = nn[i];
@@ -703,9 +713,11 @@ fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q
     typedef typename MaskWord<BS>::type W;
     typedef FaCfg<BS, D> Cfg;
     constexpr int TN = Cfg::TN;
-    constexpr uint32_t G = Cfg::G, NK = Cfg::NK, WC = Cfg::WC, QS = Cfg::q_stride, PS = Cfg::p_stride;
+    constexpr uint32_t G = Cfg::G, WC = Cfg::WC, QS = Cfg::q_stride, PS = Cfg::p_stride;
     extern __shared__ __align__(16) float sm[];
     float *Qs = sm, *bufs = Qs + BS * QS, *Ps = bufs + 2 * Cfg::buf, *red = Ps + BS * PS;
+    grid_dependency_wait();
+    grid_launch_dependents();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane_row(lane), lc = lane_quad(lane);
     // rows are dealt from both ends: the long rows of the layouts at hand sit there and start first
     const uint32_t i = (blockIdx.x & 1u) ? p.nb_a - 1u - (blockIdx.x >> 1) : blockIdx.x >> 1, b = blockIdx.y, h = blockIdx.z;
@@ -883,7 +895,7 @@ int simt_sddmm_nt(cudaStream_t s, const void *lut, const void *a, const void *b,
         const size_t bytes = sizeof(float) * 4 * per * BS * tile::kStride;                                        \
         auto kern = sddmm_nt_kernel<BS, AB, CD>;                                                                  \
         static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                                                      \
-        kern<<<dim3((p.blocks + per - 1) / per, p.B, p.H), tile::kThreads, bytes, s>>>((const uint2 *)lut, a, b, c, p, vec); \
+        launch_overlapped(kern, dim3((p.blocks + per - 1) / per, p.B, p.H), dim3(tile::kThreads), bytes, s, (const uint2 *)lut, a, b, c, p, vec); \
     }
     DISPATCH_BS(bs, DISPATCH_DT(ab_dtype, AB, {
         if (c_dtype == SFB_F32) SD_LAUNCH(SFB_F32) else if (c_dtype == SFB_BF16) SD_LAUNCH(SFB_BF16) else SD_LAUNCH(SFB_F16)
@@ -909,7 +921,7 @@ int simt_softmax(cudaStream_t s, const void *lut, const void *mask, const void *
         nb = (max_lut >= 3 && max_lut <= 4) ? 4 : (max_lut >= 7 && max_lut <= 8) ? 8 : (max_lut >= 14 && max_lut <= 16) ? 16 : 0;
 #define SM_LAUNCH(XD, NBV, SPL)                                                                                        \
     DISPATCH_DT(y_dtype, YD, {                                                                                         \
-        softmax_kernel<BS, XD, YD, NBV, SPL><<<dim3(p.nb_a * SPL, p.B, p.H), BS * BS / 8 / SPL, 0, s>>>(             \
+        launch_overlapped_few(softmax_kernel<BS, XD, YD, NBV, SPL>, dim3(p.nb_a * SPL, p.B, p.H), dim3(BS * BS / 8 / SPL), 0, s, \
             (const uint2 *)lut, (const W *)mask, x, y, p, sl, inplace);                                                \
     })
     DISPATCH_BS(bs, {
@@ -945,11 +957,11 @@ int simt_spmm_nn(cudaStream_t s, const void *lut, const void *a, const void *b, 
         if (trans) {                                                                                              \
             auto kern = spmm_nn_kernel<BS, DSV, AD, BD, true>;                                                    \
             static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                                                  \
-            kern<<<grid, tile::kThreads, bytes, s>>>((const uint2 *)lut, a, b, c, p, avec, vec);                  \
+            launch_overlapped(kern, grid, dim3(tile::kThreads), bytes, s, (const uint2 *)lut, a, b, c, p, avec, vec);                  \
         } else {                                                                                                  \
             auto kern = spmm_nn_kernel<BS, DSV, AD, BD, false>;                                                   \
             static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                                                  \
-            kern<<<grid, tile::kThreads, bytes, s>>>((const uint2 *)lut, a, b, c, p, avec, vec);                  \
+            launch_overlapped(kern, grid, dim3(tile::kThreads), bytes, s, (const uint2 *)lut, a, b, c, p, avec, vec);                  \
         }                                                                                                         \
     }
     DISPATCH_BS(bs, DISPATCH_DT(a_dtype, AD, DISPATCH_DT(bc_dtype, BD, {
@@ -970,7 +982,7 @@ int simt_softmax_grad(cudaStream_t s, const void *lut, const void *dy, const voi
                    : (max_lut >= 17 && max_lut <= 24 && wide) ? 24 : 0;
 #define SG_LAUNCH(NBV, SPL)                                                                                            \
     DISPATCH_DT(dtype, DT, {                                                                                           \
-        softmax_grad_kernel<BS, DT, NBV, SPL><<<dim3(p.nb_a * SPL, p.B, p.H), BS * BS / 8 / SPL, 0, s>>>((const uint2 *)lut, dy, y, dx, p, scale); \
+        launch_overlapped_few(softmax_grad_kernel<BS, DT, NBV, SPL>, dim3(p.nb_a * SPL, p.B, p.H), dim3(BS * BS / 8 / SPL), 0, s, (const uint2 *)lut, dy, y, dx, p, scale); \
     })
     DISPATCH_BS(bs, {
         if (nb == 4) { SG_LAUNCH(4, 1) } else if (nb == 8) { SG_LAUNCH(8, 1) } else if (nb == 12) { SG_LAUNCH(12, 1) }
@@ -992,7 +1004,7 @@ int simt_fused_sddmm_softmax(cudaStream_t s, const void *nn_lut, const void *a, 
         size_t bytes = sizeof(float) * 2 * DMAX * (BS + 1);                                                      \
         auto kern = fused_sddmm_softmax_kernel<BS, DMAX, AB, YD>;                                                \
         static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                                                     \
-        kern<<<grid, 256, bytes, s>>>((const uint2 *)nn_lut, a, b, (const W *)mask, y, p, sl);                   \
+        launch_overlapped(kern, grid, dim3(256), bytes, s, (const uint2 *)nn_lut, a, b, (const W *)mask, y, p, sl);                   \
     }
     DISPATCH_BS(bs, DISPATCH_DT(ab_dtype, AB, DISPATCH_DT(y_dtype, YD, {
         if (p.d <= 64) LAUNCH_FSS(64) else LAUNCH_FSS(128)
@@ -1015,7 +1027,7 @@ int simt_fused_attention(cudaStream_t s, const void *nn_lut, const void *q, cons
         const size_t bytes = sizeof(float) * FaCfg<BS, DV>::floats;                                              \
         auto kern = fused_attention_kernel<BS, DV, DT>;                                                          \
         static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                                                     \
-        kern<<<grid, tile::kThreads, bytes, s>>>((const uint2 *)nn_lut, q, k, v, o, (const W *)mask, p, sl, vec); \
+        launch_overlapped(kern, grid, dim3(tile::kThreads), bytes, s, (const uint2 *)nn_lut, q, k, v, o, (const W *)mask, p, sl, vec); \
     }
     DISPATCH_BS(bs, DISPATCH_DT(dtype, DT, {
         if (p.d <= 32) LAUNCH_FA(32) else if (p.d <= 64) LAUNCH_FA(64) else LAUNCH_FA(128)

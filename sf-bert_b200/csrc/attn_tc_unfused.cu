@@ -114,6 +114,8 @@ sddmm_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant_
         st->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    grid_dependency_wait();
+    grid_launch_dependents();
     if (threadIdx.x >= 64 && threadIdx.x < 64 + T) st->ent[threadIdx.x - 64] = lut[threadIdx.x - 64];
     if (warp == 0) {
         __syncwarp();
@@ -314,6 +316,8 @@ spmm_tc_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
         st->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    grid_dependency_wait();
+    grid_launch_dependents();
     build_union(nn, pair, p.nb, st->entries, st->cand, &st->n_union, &st->abort_flag);
     if (warp == 0) {
         __syncwarp();
@@ -457,6 +461,8 @@ fused_p_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constan
         st->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    grid_dependency_wait();
+    grid_launch_dependents();
     build_union(nn, pair, p.nb, st->entries, st->cand, &st->n_union, &st->abort_flag);
     if (warp == 0) {
         __syncwarp();
@@ -674,7 +680,7 @@ int tc_sddmm(cudaStream_t s, const void *nt_lut, const void *a, const void *b, v
             return fail("sfb_bst_sgemm_nt: cannot reserve %zu bytes of shared memory", kSddmmGradSmem);
         once.mark(dev);
     }
-    sddmm_tc_kernel<false><<<dim3((p.blocks + kChunk - 1) / kChunk, p.B, p.H), 320, kSddmmSmem, s>>>(qm, km, om, om, prm);
+    launch_overlapped(sddmm_tc_kernel<false>, dim3((p.blocks + kChunk - 1) / kChunk, p.B, p.H), dim3(320), kSddmmSmem, s, qm, km, om, om, prm);
     return check_launch("sfb_bst_sgemm_nt");
 }
 
@@ -700,7 +706,7 @@ int tc_sddmm_softmax_grad(cudaStream_t s, const void *nt_lut, const void *dout, 
             return fail("sfb_fused_sddmm_softmax_grad: cannot reserve %zu bytes of shared memory", kSddmmGradSmem);
         once.mark(dev);
     }
-    sddmm_tc_kernel<true><<<dim3((p.blocks + kChunk - 1) / kChunk, p.B, p.H), 320, kSddmmGradSmem, s>>>(qm, km, om, pm, prm);
+    launch_overlapped(sddmm_tc_kernel<true>, dim3((p.blocks + kChunk - 1) / kChunk, p.B, p.H), dim3(320), kSddmmGradSmem, s, qm, km, om, pm, prm);
     return check_launch("sfb_fused_sddmm_softmax_grad");
 }
 
@@ -730,7 +736,7 @@ int tc_fused_p(cudaStream_t s, const void *nn_lut, const void *a, const void *b,
             return fail("sfb_fused_sddmm_softmax: cannot reserve %zu bytes of shared memory", kFpSmem);
         once.mark(dev);
     }
-    fused_p_tc_kernel<<<dim3((p.nb_a + 1) / 2, p.B, p.H), kFpThreads, kFpSmem, s>>>(qm, km, prm);
+    launch_overlapped(fused_p_tc_kernel, dim3((p.nb_a + 1) / 2, p.B, p.H), dim3(kFpThreads), kFpSmem, s, qm, km, prm);
     return check_launch("sfb_fused_sddmm_softmax");
 }
 
@@ -757,7 +763,7 @@ int tc_spmm(cudaStream_t s, const void *nn_lut, const void *a, const void *b, vo
             return fail("sfb_bst_sgemm_xn: cannot reserve %zu bytes of shared memory", kSpmmSmem);
         once.mark(dev);
     }
-    spmm_tc_kernel<<<dim3((p.nb_a + 1) / 2, p.B, p.H), 192, kSpmmSmem, s>>>(pm, vm, prm);
+    launch_overlapped(spmm_tc_kernel, dim3((p.nb_a + 1) / 2, p.B, p.H), dim3(192), kSpmmSmem, s, pm, vm, prm);
     return check_launch("sfb_bst_sgemm_xn");
 }
 

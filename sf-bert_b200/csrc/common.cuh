@@ -81,6 +81,18 @@ static inline cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid,
     return launch_overlapped_cluster(kernel, grid, block, smem, s, 0u, args...);
 }
 
+// The same for kernels of many small CTAs: overlapped while the launch is a few CTAs per SM, where the hand-over counts.
+// Placed one by one behind a draining kernel, the thousands of CTAs of a large softmax cost more than the hand-over saves
+// (a 4096-token sliding-window softmax behind its SDDMM: 262 us overlapped, 249 us not, for the three operators).
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_overlapped_few(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args)
+{
+    if ((uint64_t)grid.x * grid.y * grid.z <= 8ull * (uint64_t)device_sm_count(current_device()))
+        return launch_overlapped(kernel, grid, block, smem, s, args...);
+    kernel<<<grid, block, smem, s>>>(KArgs(args)...);
+    return cudaPeekAtLastError();
+}
+
 // ---- device: element conversion -------------------------------------------------------------
 // fp32 -> bf16 bits the way the reference stores S and P (ew_op_gpu.h:241-253): add half a bf16
 // ulp of the magnitude, round toward zero, keep the upper 16 bits.

@@ -37,6 +37,7 @@ struct GParams {
     int is_bf16, act;
     int w_transposed;   // w is [n, k] row-major (out = x . w^T, the tied-embedding logits): its tile is a K-major B operand
     uint32_t band;      // CTA-pair kernel: column tiles per band of the tile order (tile_coords)
+    const void *resid;  // split kernel: [m, n] of x's type, added to the product (may be out itself), or NULL
 };
 
 // Tile t of the CTA-pair kernel -> (row tile, column tile).  The tiles run band by band, a band being `band` column
@@ -568,7 +569,7 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr)
 }
 
 // eight neighbouring outputs of one row: bias, activation, one 16-byte store
-__device__ __forceinline__ void finish8(const GParams &p, float (&x)[8], const float *bias, uint32_t row, uint32_t col)
+__device__ __forceinline__ void finish8(const GParams &p, float (&x)[8], const float *bias, const uint4 &resid, uint32_t row, uint32_t col)
 {
     if (p.bias) {
         const float4 b0 = *(const float4 *)bias, b1 = *(const float4 *)(bias + 4);
@@ -580,6 +581,17 @@ __device__ __forceinline__ void finish8(const GParams &p, float (&x)[8], const f
         for (int j = 0; j < 8; j++) x[j] = gelu_ref(x[j]);
     }
     uint32_t w[4];
+    if (p.resid) {
+        // the product is rounded to its type before the sum, as two separate operations do
+        const uint32_t r[4] = {resid.x, resid.y, resid.z, resid.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint32_t y = pack2(x[2 * j], x[2 * j + 1], p.is_bf16);
+            const float2 a = unpack2(y, p.is_bf16), b = unpack2(r[j], p.is_bf16);
+            x[2 * j] = a.x + b.x;
+            x[2 * j + 1] = a.y + b.y;
+        }
+    }
 #pragma unroll
     for (int j = 0; j < 4; j++) w[j] = pack2(x[2 * j], x[2 * j + 1], p.is_bf16);
     *(uint4 *)((uint16_t *)p.out + (size_t)row * p.N + col) = make_uint4(w[0], w[1], w[2], w[3]);
@@ -666,9 +678,18 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
     }
     __syncwarp();
     // ===== all eight warps drain the accumulator: 32 rows and half of the columns each =====
+    const uint32_t quarter = warp & 3, ch = warp >> 2, r = quarter * 32 + lane, lane_field = (quarter * 32) << 16;
+    uint4 res[BN / 16];                                    // this thread's residuals, on their way while the products run
+    if (p.resid && split == 1) {
+        const uint32_t row = tm * kGBM + r;
+#pragma unroll
+        for (uint32_t q = 0; q < BN / 16; q++) {
+            const uint32_t col = tn * BN + ch * (BN / 2) + q * 8;
+            if (row < p.M && col < p.N) res[q] = *(const uint4 *)((const uint16_t *)p.resid + (size_t)row * p.N + col);
+        }
+    }
     const bool ok = mbar_wait_warp(&st->acc_full, 0, abort_flag, 63);
     __syncthreads();                                       // the bias is in place
-    const uint32_t quarter = warp & 3, ch = warp >> 2, r = quarter * 32 + lane, lane_field = (quarter * 32) << 16;
     if (ok) {
         tcgen05_fence_after();
 #pragma unroll
@@ -686,7 +707,7 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
                         float x[8];
 #pragma unroll
                         for (int j = 0; j < 8; j++) x[j] = __uint_as_float(v[q * 8 + j]);
-                        finish8(p, x, bias_s + c + q * 8, row, col);
+                        finish8(p, x, bias_s + c + q * 8, res[c0 / 8 + q], row, col);
                     }
                 }
             } else {
@@ -709,6 +730,8 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
             const uint32_t row = tm * kGBM + rr, col = tn * BN + c;
             if (row >= p.M || col >= p.N) continue;
             const uint32_t at = mine + (rr * Cfg::acc_stride + c) * 4;
+            uint4 rs = make_uint4(0u, 0u, 0u, 0u);
+            if (p.resid) rs = *(const uint4 *)((const uint16_t *)p.resid + (size_t)row * p.N + col);
             float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
             for (uint32_t k = 0; k < split; k++) {
@@ -717,7 +740,7 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
                 x[0] += u.x; x[1] += u.y; x[2] += u.z; x[3] += u.w;
                 x[4] += w.x; x[5] += w.y; x[6] += w.z; x[7] += w.w;
             }
-            finish8(p, x, bias_s + c, row, col);
+            finish8(p, x, bias_s + c, rs, row, col);
         }
         __syncwarp();
         cluster_sync_all();                                           // the others have read this CTA's accumulator
@@ -822,8 +845,28 @@ static LinearPlan plan_linear(uint32_t m, uint32_t n, uint32_t k, uint32_t sms)
     return best;
 }
 
-int tc_linear(cudaStream_t s, void *out, const void *x, const void *w, const float *bias, uint32_t m, uint32_t n, uint32_t k,
-              int dtype, int act, bool w_transposed)
+// out += resid, 16 bytes per thread and step (what the kernels with large tiles leave to a pass of its own: read beside the
+// accumulator, a row's residuals cost their epilogues more than the pass does)
+template <bool BF16>
+__global__ void __launch_bounds__(256) add_residual_kernel(void *out, const void *resid, size_t pieces)
+{
+    grid_dependency_wait();
+    grid_launch_dependents();
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < pieces; i += (size_t)gridDim.x * blockDim.x) {
+        const uint4 a = ((const uint4 *)out)[i], b = ((const uint4 *)resid)[i];
+        const uint32_t u[4] = {a.x, a.y, a.z, a.w}, v[4] = {b.x, b.y, b.z, b.w};
+        uint32_t w[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float2 f = tc::unpack2(u[j], BF16), g = tc::unpack2(v[j], BF16);
+            w[j] = tc::pack2(f.x + g.x, f.y + g.y, BF16);
+        }
+        ((uint4 *)out)[i] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+static int linear_product(cudaStream_t s, void *out, const void *x, const void *w, const float *bias, uint32_t m, uint32_t n, uint32_t k,
+                          int dtype, int act, bool w_transposed, const void *resid, bool *added)
 {
     using namespace tc;
     const int is_bf16 = dtype == SFB_BF16;
@@ -834,9 +877,12 @@ int tc_linear(cudaStream_t s, void *out, const void *x, const void *w, const flo
     if (sms <= 0) return fail("sfb_linear: cannot read the SM count");
     const LinearPlan plan = plan_linear(m, n, k, (uint32_t)sms);
     const uint32_t tiles_n = (n + kGBN - 1) / kGBN;
-    GParams prm = {out, bias, m, n, k, 0, tiles_n, is_bf16, act, w_transposed ? 1 : 0, 1};
-    if (plan.kind == 2)
+    GParams prm = {out, bias, m, n, k, 0, tiles_n, is_bf16, act, w_transposed ? 1 : 0, 1, nullptr};
+    if (plan.kind == 2) {
+        prm.resid = resid;
+        *added = true;
         return plan.bn == 64 ? launch_split<64, 8>(s, am, w, prm, plan.split, dev) : launch_split<128, 6>(s, am, w, prm, plan.split, dev);
+    }
     if (plan.kind == 1) {
         CUtensorMap bp;
         if (w_transposed ? make_map_2d(&bp, w, n, k, is_bf16, kGBN / 2) : make_map_2d(&bp, w, k, n, is_bf16, kGBK)) return 1;
@@ -869,6 +915,21 @@ int tc_linear(cudaStream_t s, void *out, const void *x, const void *w, const flo
     const uint32_t grid = tiles < (uint64_t)sms ? (uint32_t)tiles : (uint32_t)sms;
     launch_overlapped(linear_tc_kernel, dim3(grid), dim3(320), kGSmem, s, am, bm, prm);
     return check_launch("sfb_linear");
+}
+
+int tc_linear(cudaStream_t s, void *out, const void *x, const void *w, const float *bias, uint32_t m, uint32_t n, uint32_t k,
+              int dtype, int act, bool w_transposed, const void *resid)
+{
+    bool added = false;
+    if (linear_product(s, out, x, w, bias, m, n, k, dtype, act, w_transposed, resid, &added)) return 1;
+    if (!resid || added) return 0;
+    const size_t pieces = (size_t)m * n / 8;                            // n is a multiple of 16
+    const int sms = device_sm_count(current_device());
+    const size_t want = (pieces + 255) / 256, most = (size_t)(sms > 0 ? sms : 1) * 16;
+    const dim3 grid((unsigned)(want < most ? want : most));
+    if (dtype == SFB_BF16) launch_overlapped(add_residual_kernel<true>, grid, dim3(256), 0, s, out, resid, pieces);
+    else launch_overlapped(add_residual_kernel<false>, grid, dim3(256), 0, s, out, resid, pieces);
+    return check_launch("sfb_linear_residual");
 }
 
 int tc_status_clear_gemm()

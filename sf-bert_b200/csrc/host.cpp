@@ -17,7 +17,7 @@ namespace {
 // ---- the library -----------------------------------------------------------------------------------------------------
 #define SFB_FUNCTIONS(X)                                                                                                 \
     X(sfb_last_error) X(sfb_bst_sgemm_nt) X(sfb_masked_softmax) X(sfb_bst_sgemm_xn) X(sfb_masked_softmax_grad) X(sfb_linear) \
-    X(sfb_linear_nt) X(sfb_embedding) X(sfb_csr_attention) X(sfb_rowdot) X(sfb_fused_sddmm_softmax_grad)                  \
+    X(sfb_linear_nt) X(sfb_linear_residual) X(sfb_embedding) X(sfb_csr_attention) X(sfb_rowdot) X(sfb_fused_sddmm_softmax_grad)                  \
     X(sfb_fused_sddmm_softmax) X(sfb_fused_attention) X(sfb_fused_attention_slice) X(sfb_bias_residual_layernorm)         \
     X(sfb_bias_gelu)
 struct Lib {
@@ -422,9 +422,7 @@ FUNCTION(py_encoder_layer, 6)
         check(L.sfb_linear(s, p_a, p_attn, ptr(wo), nullptr, um, uh, uh, t, SFB_ACT_NONE));
         check(L.sfb_bias_residual_layernorm(s, p_b, p_a, nullptr, nullptr, p_a, bo, ptr(x), g2, be2, um, uh, t));
         check(L.sfb_linear(s, p_ffn, p_b, ptr(w1), b1, um, uf, uh, t, SFB_ACT_GELU));
-        check(L.sfb_linear(s, p_b, p_ffn, ptr(w2), b2, um, uh, uf, t, SFB_ACT_NONE));
-        at::Tensor x1 = ws.narrow(0, m * wide, m * hidden).view({m, hidden}), y = ws.narrow(0, m * (wide + hidden), m * hidden).view({m, hidden});
-        at::add_out(out, x1, y);
+        check(L.sfb_linear_residual(s, ptr(out), p_ffn, ptr(w2), b2, p_a, um, uh, uf, t));
     } else {
         // x1 = LN(x + Attn(x) Wo + bo); out = LN(x1 + GELU(x1 W1 + b1) W2 + b2)
         attention(ptr(x));

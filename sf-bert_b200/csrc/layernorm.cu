@@ -430,6 +430,8 @@ template <int DT>
 __global__ void __launch_bounds__(256) bias_gelu_kernel(void *out, const void *x,
                                                        const float *__restrict__ bias, size_t total, uint32_t n)
 {
+    grid_dependency_wait();
+    grid_launch_dependents();
     constexpr int N = Vec8<DT>::N;
     const size_t stride = (size_t)gridDim.x * blockDim.x * N;
     for (size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * N; i < total; i += stride) {
@@ -458,9 +460,33 @@ __global__ void __launch_bounds__(256) embedding_kernel(void *__restrict__ out, 
                                                        uint32_t per_cta_y, uint32_t seq_len, uint32_t hidden, uint32_t vocab,
                                                        uint32_t *bad_ids)
 {
+    grid_dependency_wait();
+    grid_launch_dependents();
     constexpr int N = Vec8<DT>::N, U = kEmbUnroll;
     constexpr int ESZ = 16 / N;
     const uint32_t per_row = hidden / N;                                   // 16-byte pieces per row
+    if (blockIdx.x == gridDim.x - 1) {
+        // the extra column of CTAs: its first one counts the ids outside the table (nobody has to clear the counter first)
+        if (blockIdx.y || !bad_ids) return;
+        const uint32_t total = batch * seq_len;                            // < 2^31 (checked by the host)
+        uint32_t bad = 0;
+        for (uint32_t t = threadIdx.x; t < total; t += 256 * 8) {
+            int32_t v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) v[u] = t + u * 256 < total ? __ldg(ids + t + u * 256) : 0;
+#pragma unroll
+            for (int u = 0; u < 8; u++) bad += t + u * 256 < total && (v[u] < 0 || (uint32_t)v[u] >= vocab);
+        }
+        __shared__ uint32_t part[8];
+        bad = __reduce_add_sync(0xffffffffu, bad);
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = bad;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < 8; w++) bad += part[w];
+            *bad_ids = bad;
+        }
+        return;
+    }
     const uint32_t piece = blockIdx.x * blockDim.x + threadIdx.x;          // < seq_len * per_row < 2^32 (checked by the host)
     if (piece >= seq_len * per_row) return;
     const uint32_t l = piece / per_row, col = (piece - l * per_row) * N;
@@ -489,7 +515,6 @@ __global__ void __launch_bounds__(256) embedding_kernel(void *__restrict__ out, 
 #pragma unroll
         for (int u = 0; u < U; u++) {
             if (b0 + u < b_end) {
-                if (!ok[u] && col == 0 && bad_ids) atomicAdd(bad_ids, 1u);
                 float v[N];
                 Vec8<DT>::decode(v, tv[u]);
 #pragma unroll
@@ -507,6 +532,8 @@ template <int DT>
 __global__ void __launch_bounds__(256) rowdot_kernel(float *__restrict__ out, const void *__restrict__ a, const void *__restrict__ b,
                                                     size_t rows, uint32_t d)
 {
+    grid_dependency_wait();
+    grid_launch_dependents();
     constexpr int N = Vec8<DT>::N;
     const size_t row = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 8;
     const uint32_t part = threadIdx.x & 7;
@@ -527,9 +554,9 @@ __global__ void __launch_bounds__(256) rowdot_kernel(float *__restrict__ out, co
 int rowdot(cudaStream_t s, float *out, const void *a, const void *b, size_t rows, uint32_t d, int dtype)
 {
     const unsigned ctas = (unsigned)((rows * 8 + 255) / 256);
-    if (dtype == SFB_F32) rowdot_kernel<SFB_F32><<<ctas, 256, 0, s>>>(out, a, b, rows, d);
-    else if (dtype == SFB_BF16) rowdot_kernel<SFB_BF16><<<ctas, 256, 0, s>>>(out, a, b, rows, d);
-    else rowdot_kernel<SFB_F16><<<ctas, 256, 0, s>>>(out, a, b, rows, d);
+    if (dtype == SFB_F32) launch_overlapped(rowdot_kernel<SFB_F32>, dim3(ctas), dim3(256), 0, s, out, a, b, rows, d);
+    else if (dtype == SFB_BF16) launch_overlapped(rowdot_kernel<SFB_BF16>, dim3(ctas), dim3(256), 0, s, out, a, b, rows, d);
+    else launch_overlapped(rowdot_kernel<SFB_F16>, dim3(ctas), dim3(256), 0, s, out, a, b, rows, d);
     return check_launch("sfb_rowdot");
 }
 
@@ -538,7 +565,6 @@ int embedding_lookup(cudaStream_t s, void *out, const void *table, const int32_t
 {
     const int per = dtype == SFB_F32 ? 4 : 8;
     if (hidden % per) return fail("sfb_embedding: hidden=%u must be a multiple of %d for this type", hidden, per);
-    if (bad_ids) cudaMemsetAsync(bad_ids, 0, sizeof(uint32_t), s);
     const size_t pieces = (size_t)seq_len * (hidden / per);                 // one thread per 16-byte piece of a position row
     if (pieces >= (1ull << 32)) return fail("sfb_embedding: seq_len * hidden too large");
     const int sms = device_sm_count(current_device());
@@ -550,10 +576,10 @@ int embedding_lookup(cudaStream_t s, void *out, const void *table, const int32_t
     if (split > 65535u) split = 65535u;
     if (split < 1) split = 1;
     const uint32_t per_y = (batch + split - 1) / split;
-    const dim3 grid((unsigned)ctas_x, (batch + per_y - 1) / per_y);
-    if (dtype == SFB_F32) embedding_kernel<SFB_F32><<<grid, 256, 0, s>>>(out, table, ids, pos, batch, per_y, seq_len, hidden, vocab, bad_ids);
-    else if (dtype == SFB_BF16) embedding_kernel<SFB_BF16><<<grid, 256, 0, s>>>(out, table, ids, pos, batch, per_y, seq_len, hidden, vocab, bad_ids);
-    else embedding_kernel<SFB_F16><<<grid, 256, 0, s>>>(out, table, ids, pos, batch, per_y, seq_len, hidden, vocab, bad_ids);
+    const dim3 grid((unsigned)ctas_x + 1, (batch + per_y - 1) / per_y);
+    if (dtype == SFB_F32) launch_overlapped(embedding_kernel<SFB_F32>, grid, dim3(256), 0, s, out, table, ids, pos, batch, per_y, seq_len, hidden, vocab, bad_ids);
+    else if (dtype == SFB_BF16) launch_overlapped(embedding_kernel<SFB_BF16>, grid, dim3(256), 0, s, out, table, ids, pos, batch, per_y, seq_len, hidden, vocab, bad_ids);
+    else launch_overlapped(embedding_kernel<SFB_F16>, grid, dim3(256), 0, s, out, table, ids, pos, batch, per_y, seq_len, hidden, vocab, bad_ids);
     return check_launch("sfb_embedding");
 }
 
@@ -571,8 +597,8 @@ extern "C" int sfb_bias_gelu(sfb_stream_t stream, void *out, const void *x, cons
     const int per = dtype == SFB_F32 ? 4 : 8;
     size_t ctas = (total / per + 255) / 256;
     if (ctas > 148 * 16) ctas = 148 * 16;
-    if (dtype == SFB_F32) bias_gelu_kernel<SFB_F32><<<(unsigned)ctas, 256, 0, s>>>(out, x, bias, total, n);
-    else if (dtype == SFB_BF16) bias_gelu_kernel<SFB_BF16><<<(unsigned)ctas, 256, 0, s>>>(out, x, bias, total, n);
-    else bias_gelu_kernel<SFB_F16><<<(unsigned)ctas, 256, 0, s>>>(out, x, bias, total, n);
+    if (dtype == SFB_F32) launch_overlapped(bias_gelu_kernel<SFB_F32>, dim3((unsigned)ctas), dim3(256), 0, s, out, x, bias, total, n);
+    else if (dtype == SFB_BF16) launch_overlapped(bias_gelu_kernel<SFB_BF16>, dim3((unsigned)ctas), dim3(256), 0, s, out, x, bias, total, n);
+    else launch_overlapped(bias_gelu_kernel<SFB_F16>, dim3((unsigned)ctas), dim3(256), 0, s, out, x, bias, total, n);
     return check_launch("sfb_bias_gelu");
 }

@@ -150,18 +150,25 @@ extern "C" int sfb_fused_attention_slice(sfb_stream_t stream, const void *nn_lut
 }
 
 static int linear_common(const char *who, sfb_stream_t stream, void *out, const void *x, const void *w, const float *bias, uint32_t m,
-                         uint32_t n, uint32_t k, int dtype, int act, bool w_transposed);
+                         uint32_t n, uint32_t k, int dtype, int act, bool w_transposed, const void *resid);
 
 extern "C" int sfb_linear(sfb_stream_t stream, void *out, const void *x, const void *w, const float *bias, uint32_t m, uint32_t n,
                           uint32_t k, int dtype, int act)
 {
-    return linear_common("sfb_linear", stream, out, x, w, bias, m, n, k, dtype, act, false);
+    return linear_common("sfb_linear", stream, out, x, w, bias, m, n, k, dtype, act, false, nullptr);
 }
 
 extern "C" int sfb_linear_nt(sfb_stream_t stream, void *out, const void *x, const void *wt, const float *bias, uint32_t m, uint32_t n,
                              uint32_t k, int dtype, int act)
 {
-    return linear_common("sfb_linear_nt", stream, out, x, wt, bias, m, n, k, dtype, act, true);
+    return linear_common("sfb_linear_nt", stream, out, x, wt, bias, m, n, k, dtype, act, true, nullptr);
+}
+
+extern "C" int sfb_linear_residual(sfb_stream_t stream, void *out, const void *x, const void *w, const float *bias, const void *resid,
+                                   uint32_t m, uint32_t n, uint32_t k, int dtype)
+{
+    SFB_REQUIRE(resid && resid != out, "sfb_linear_residual: resid is NULL or out itself");
+    return linear_common("sfb_linear_residual", stream, out, x, w, bias, m, n, k, dtype, SFB_ACT_NONE, false, resid);
 }
 
 extern "C" int sfb_embedding(sfb_stream_t stream, void *out, const void *table, const int32_t *ids, const void *pos, uint32_t batch,
@@ -178,7 +185,7 @@ extern "C" int sfb_embedding(sfb_stream_t stream, void *out, const void *table, 
 }
 
 static int linear_common(const char *who, sfb_stream_t stream, void *out, const void *x, const void *w, const float *bias, uint32_t m,
-                         uint32_t n, uint32_t k, int dtype, int act, bool w_transposed)
+                         uint32_t n, uint32_t k, int dtype, int act, bool w_transposed, const void *resid)
 {
     SFB_REQUIRE(out && x && w, "%s: NULL pointer", who);
     SFB_REQUIRE(dtype == SFB_BF16 || dtype == SFB_F16, "%s: x, w and out must be bf16 or fp16 (fp32 products stay with the GEMM library)", who);
@@ -189,7 +196,8 @@ static int linear_common(const char *who, sfb_stream_t stream, void *out, const 
     SFB_REQUIRE((uint64_t)m < (1ull << 31) && (uint64_t)n < (1ull << 31) && (uint64_t)k < (1ull << 31), "%s: dimension too large", who);
     if (m == 0 || n == 0) { clear_error(); return 0; }
     SFB_REQUIRE(k > 0, "%s: k is 0", who);
-    return tc_linear(as_stream(stream), out, x, w, bias, m, n, k, dtype, act, w_transposed);
+    SFB_REQUIRE(aligned16(resid), "%s: resid must be 16-byte aligned", who);
+    return tc_linear(as_stream(stream), out, x, w, bias, m, n, k, dtype, act, w_transposed, resid);
 }
 
 extern "C" int sfb_rowdot(sfb_stream_t stream, float *out, const void *a, const void *b, uint64_t rows, uint32_t d, int dtype)

@@ -300,6 +300,12 @@ __device__ __forceinline__ uint32_t pack2(float a, float b, int is_bf16)
     return *reinterpret_cast<uint32_t *>(&h);
 }
 
+__device__ __forceinline__ float2 unpack2(uint32_t v, int is_bf16)
+{
+    if (is_bf16) return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+    return __half22float2(*reinterpret_cast<const __half2 *>(&v));
+}
+
 #define TMEM_LD_16(r, addr)                                                                                          \
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];" \
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),   \

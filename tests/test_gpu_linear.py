@@ -56,6 +56,18 @@ def test_linear_few_tiles(sfb, oracle, m, n, k, act, transposed):
     assert np.abs(got[rows].float().cpu().numpy() - want).max() <= 2e-2 * np.abs(want).max()
 
 
+@pytest.mark.parametrize("m,n,k", [(129, 80, 72), (64, 192, 520), (2048, 1040, 136), (3000, 2320, 64), (20000, 272, 64)])
+def test_linear_residual(sfb, m, n, k):
+    """The sum in the epilogue (one CTA per tile, several) and as a pass of its own equals the product and a separate add."""
+    g = torch.Generator(device="cuda").manual_seed(7)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.float16)
+    x, w, r, b = rn(m, k), rn(k, n), rn(m, n), torch.randn(n, device="cuda", generator=g)
+    out = torch.empty_like(r)
+    p = lambda t: sfb.C.c_void_p(t.data_ptr())
+    sfb._check(sfb.lib.sfb_linear_residual(sfb._stream(), p(out), p(x), p(w), p(b), p(r), *(sfb.C.c_uint32(v) for v in (m, n, k)), sfb.F16))
+    assert sfb.device_status() == 0 and torch.equal(out, r + sfb.linear(x, w, b))
+
+
 def test_linear_more_tiles_than_sms_and_batched_input(sfb, oracle):
     """A [B, L, hidden] activation (leading dimensions flattened) with enough tiles that every CTA loops."""
     B, L, hidden, n = 2, 4096, 768, 2304
