@@ -43,6 +43,11 @@ int tc_fused_p(cudaStream_t s, const void *nn_lut, const void *a, const void *b,
 int tc_sddmm_softmax_grad(cudaStream_t s, const void *nt_lut, const void *dout, const void *v, const void *pblk, const float *delta,
                           void *ds, int dtype, const AttnDims &p, float scale);
 int rowdot(cudaStream_t s, float *out, const void *a, const void *b, size_t rows, uint32_t d, int dtype);
+bool tc_backward_supported(int dtype, uint32_t bs, const AttnDims &p, uint32_t nn_max, uint32_t tn_max, uint64_t pointers);
+int tc_backward(cudaStream_t s, const void *nn_lut, const void *tn_lut, const void *q, const void *k, const void *v, const void *pblk, const void *o,
+                const void *dout, float *delta, void *dq, void *dk, void *dv, int dtype, const AttnDims &p, float scale);
+int tc_status_backward(uint32_t *out);
+int tc_status_clear_backward();
 int tc_status_unfused(uint32_t *out);
 int tc_status_clear_unfused();
 

@@ -12,8 +12,6 @@ namespace tc {
 
 constexpr int kUStages = 4;
 
-static int make_p_map(CUtensorMap *map, const void *base, uint64_t rows, int is_bf16);
-
 struct UShared {
     uint64_t q_full, in_full[kUStages], in_empty[kUStages], s_full[2], s_empty[2], o_final, drained;
     uint32_t tmem_base, n_union, abort_flag, pad;
@@ -626,22 +624,6 @@ fused_p_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constan
     }
 }
 
-// P viewed as [rows, 64] 16-bit row-major, boxes of 64 x 64, 128-byte swizzle, zero fill outside
-static int make_p_map(CUtensorMap *map, const void *base, uint64_t rows, int is_bf16)
-{
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return fail("cuTensorMapEncodeTiled is not available from this driver");
-    cuuint64_t dims[2] = {64, rows};
-    cuuint64_t strides[1] = {128};
-    cuuint32_t box[2] = {64, 64};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(map, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void *)base, dims,
-                    strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail("cuTensorMapEncodeTiled failed with code %d", (int)r);
-    return 0;
-}
-
 }  // namespace tc
 
 static bool tc_shape_ok(uint32_t bs, const AttnDims &p, uint32_t max_lut)
@@ -669,7 +651,7 @@ int tc_sddmm(cudaStream_t s, const void *nt_lut, const void *a, const void *b, v
     CUtensorMap qm, km, om;
     if (make_map(&qm, a, rows, p.H, is_bf16, 64) || make_map(&km, b, rows, p.H, is_bf16, 64)) return 1;
     // the scores as [B*H*blocks*64 rows, 64] for the TMA stores of 16-bit outputs (unused for fp32 outputs)
-    if (make_p_map(&om, c, (uint64_t)p.B * p.H * p.blocks * 64, c_dtype != SFB_F16)) return 1;
+    if (make_map_2d(&om, c, (uint64_t)p.B * p.H * p.blocks * 64, 64, c_dtype != SFB_F16, 64)) return 1;
     SFB_REQUIRE((uint64_t)p.B * p.H * p.blocks * 64 < (1ull << 31), "sfb_bst_sgemm_nt: too many blocks for one launch");
     UParams prm = {(const uint2 *)nt_lut, c, p.B, p.H, p.nb_a, p.blocks, p.lut_stride, c_dtype, is_bf16, 0};
     static DeviceOnce once;
@@ -695,8 +677,8 @@ int tc_sddmm_softmax_grad(cudaStream_t s, const void *nt_lut, const void *dout, 
     const uint64_t rows = (uint64_t)p.B * p.nb_a * 64, prow = (uint64_t)p.B * p.H * p.blocks * 64;
     SFB_REQUIRE(prow < (1ull << 31), "sfb_fused_sddmm_softmax_grad: too many blocks for one launch");
     CUtensorMap qm, km, om, pm;
-    if (make_map(&qm, dout, rows, p.H, is_bf16, 64) || make_map(&km, v, rows, p.H, is_bf16, 64) || make_p_map(&om, ds, prow, is_bf16) ||
-        make_p_map(&pm, pblk, prow, is_bf16))
+    if (make_map(&qm, dout, rows, p.H, is_bf16, 64) || make_map(&km, v, rows, p.H, is_bf16, 64) || make_map_2d(&om, ds, prow, 64, is_bf16, 64) ||
+        make_map_2d(&pm, pblk, prow, 64, is_bf16, 64))
         return 1;
     UParams prm = {(const uint2 *)nt_lut, ds, p.B, p.H, p.nb_a, p.blocks, p.lut_stride, dtype, is_bf16, 0, 0, delta, scale};
     static DeviceOnce once;
@@ -754,7 +736,7 @@ int tc_spmm(cudaStream_t s, const void *nn_lut, const void *a, const void *b, vo
     const int is_bf16 = dtype == SFB_BF16;
     const uint64_t prow = (uint64_t)p.B * p.H * p.blocks * 64;
     CUtensorMap pm, vm;
-    if (make_p_map(&pm, a, prow, is_bf16) || make_map(&vm, b, (uint64_t)p.B * p.nb_b * 64, p.H, is_bf16, 64)) return 1;
+    if (make_map_2d(&pm, a, prow, 64, is_bf16, 64) || make_map(&vm, b, (uint64_t)p.B * p.nb_b * 64, p.H, is_bf16, 64)) return 1;
     UParams prm = {(const uint2 *)nn_lut, c, p.B, p.H, p.nb_a, p.blocks, p.lut_stride, dtype, is_bf16, (uint32_t)prow, trans ? 1 : 0};
     static DeviceOnce once;
     const int dev = current_device();

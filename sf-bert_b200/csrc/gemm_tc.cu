@@ -766,22 +766,6 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
     }
 }
 
-// [rows, cols] 16-bit row-major tensor, boxes of box_rows x 64 elements, 128-byte swizzle
-static int make_map_2d(CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols, int is_bf16, uint32_t box_rows)
-{
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return fail("cuTensorMapEncodeTiled is not available from this driver");
-    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-    cuuint32_t box[2] = {64, box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(map, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void *)base, dims,
-                    strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail("cuTensorMapEncodeTiled failed with code %d", (int)r);
-    return 0;
-}
-
 }  // namespace tc
 
 template <int BN, int ST>

@@ -19,7 +19,7 @@ namespace {
     X(sfb_last_error) X(sfb_bst_sgemm_nt) X(sfb_masked_softmax) X(sfb_bst_sgemm_xn) X(sfb_masked_softmax_grad) X(sfb_linear) \
     X(sfb_linear_nt) X(sfb_linear_residual) X(sfb_embedding) X(sfb_csr_attention) X(sfb_rowdot) X(sfb_fused_sddmm_softmax_grad)                  \
     X(sfb_fused_sddmm_softmax) X(sfb_fused_attention) X(sfb_fused_attention_slice) X(sfb_bias_residual_layernorm)         \
-    X(sfb_bias_gelu)
+    X(sfb_bias_gelu) X(sfb_attention_backward)
 struct Lib {
 #define DECL(f) decltype(&::f) f = nullptr;
     SFB_FUNCTIONS(DECL)
@@ -441,6 +441,23 @@ FUNCTION(py_attention_backward_fused, 8)
     const at::Tensor &dout = tensor(a[0]), &q = tensor(a[1]), &k = tensor(a[2]), &v = tensor(a[3]), &p = tensor(a[4]), &o = tensor(a[5]);
     const Lay lay(a[6]);
     const float scale = (float)number(a[7]);
+    const Dims n(q, lay);
+    const int t = tag(q);
+    void *tn = lay.get(n_tn_lut);
+    const uint32_t tn_max = attr_u32(lay.o, n_tn_max);
+    // dS on chip where the library has the kernels for it, otherwise operator by operator
+    auto tidy = [](const at::Tensor &x) { return x.is_contiguous() && ((uintptr_t)ptr(x) & 15) == 0; };
+    if (t != SFB_F32 && lay.bs == 64 && n.d == 64 && lay.blocks && lay.nn_max && lay.nn_max <= 256 && tn_max && tn_max <= 256 && tag(k) == t &&
+        tag(v) == t && tag(p) == t && tag(o) == t && tag(dout) == t && tidy(q) && tidy(k) && tidy(v) && tidy(p) && tidy(o) && tidy(dout) &&
+        (int64_t)n.B * n.H * lay.blocks * 64 < (1ll << 31) - 64 && (int64_t)n.B * n.L < (1ll << 31)) {
+        require(o.sizes() == dout.sizes() && dout.sizes() == q.sizes(), "q, o and dO differ in shape");
+        at::Tensor delta = empty({n.B, n.H, n.L}, at::kFloat, q), dq = alike(q), dk = alike(k), dv = alike(v);
+        check(L.sfb_attention_backward(stream(), lay.get(n_nn_lut), tn, ptr(q), ptr(k), ptr(v), ptr(p), ptr(o), ptr(dout), (float *)ptr(delta), ptr(dq),
+                                       ptr(dk), ptr(dv), t, lay.bs, lay.blocks, n.B, lay.nb, n.H, n.d, lay.heads, lay.blocks + lay.nb, lay.nn_max,
+                                       tn_max, scale));
+        Ref x(wrap(dq)), y(wrap(dk)), z(wrap(dv));
+        return PyTuple_Pack(3, x.o, y.o, z.o);
+    }
     at::Tensor dv = bst_sgemm(p, dout, lay, true);
     at::Tensor ds = fused_sddmm_softmax_grad(dout, v, p, rowdot(dout, o), lay, scale);
     at::Tensor dk = bst_sgemm(ds, q, lay, true), dq = bst_sgemm(ds, k, lay, false);

@@ -229,9 +229,27 @@ extern "C" int sfb_fused_sddmm_softmax_grad(sfb_stream_t stream, const void *nt_
     return tc_sddmm_softmax_grad(as_stream(stream), nt_lut, dout, v, p_blocks, delta, ds, dtype, p, scale);
 }
 
+extern "C" int sfb_attention_backward(sfb_stream_t stream, const void *nn_lut, const void *tn_lut, const void *q, const void *k, const void *v,
+                                      const void *p_blocks, const void *o, const void *dout, float *delta, void *dq, void *dk, void *dv,
+                                      int dtype, uint32_t block_size, uint32_t blocks, uint32_t batch_dim, uint32_t ctx_blks, uint32_t head_dim,
+                                      uint32_t state_dim, uint32_t lut_heads, uint32_t lut_dim, uint32_t nn_max, uint32_t tn_max, float scale)
+{
+    const char *who = "sfb_attention_backward";
+    SFB_REQUIRE(nn_lut && tn_lut && q && k && v && p_blocks && o && dout && delta && dq && dk && dv, "%s: NULL pointer", who);
+    if (check_common(who, block_size, batch_dim, head_dim, state_dim, lut_heads)) return 1;
+    SFB_REQUIRE(lut_heads == 1 || lut_dim >= blocks + ctx_blks, "%s: lut_dim %u smaller than blocks+ctx_blks", who, lut_dim);
+    if (ctx_blks == 0) { clear_error(); return 0; }
+    AttnDims p = {batch_dim, head_dim, state_dim, ctx_blks, ctx_blks, blocks, lut_heads > 1 ? lut_dim : 0, 0};
+    const uint64_t pointers = (uint64_t)((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)p_blocks | (uintptr_t)o | (uintptr_t)dout |
+                                         (uintptr_t)delta | (uintptr_t)dq | (uintptr_t)dk | (uintptr_t)dv);
+    SFB_REQUIRE(tc_backward_supported(dtype, block_size, p, nn_max, tn_max, pointers),
+                "%s: needs 16-bit operands, 64x64 blocks, 64-wide heads, 16-byte aligned pointers and rows and columns of 1 to 256 blocks", who);
+    return tc_backward(as_stream(stream), nn_lut, tn_lut, q, k, v, p_blocks, o, dout, delta, dq, dk, dv, dtype, p, scale);
+}
+
 extern "C" int sfb_device_status_clear(void)
 {
-    if (tc_status_clear_fused() || tc_status_clear_unfused() || tc_status_clear_gemm()) return 1;
+    if (tc_status_clear_backward() || tc_status_clear_fused() || tc_status_clear_unfused() || tc_status_clear_gemm()) return 1;
     clear_error();
     return 0;
 }
@@ -239,9 +257,9 @@ extern "C" int sfb_device_status_clear(void)
 extern "C" int sfb_device_status(uint32_t *status)
 {
     SFB_REQUIRE(status, "sfb_device_status: NULL pointer");
-    uint32_t a = 0, b = 0, c = 0;
-    if (tc_status_fused(&a) || tc_status_unfused(&b) || tc_status_gemm(&c)) return 1;
-    *status = a ? a : b ? b : c;
+    uint32_t a = 0, b = 0, c = 0, d = 0;
+    if (tc_status_fused(&a) || tc_status_unfused(&b) || tc_status_gemm(&c) || tc_status_backward(&d)) return 1;
+    *status = a ? a : b ? b : c ? c : d;
     clear_error();
     return 0;
 }
