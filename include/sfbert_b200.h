@@ -161,11 +161,11 @@ int sfb_fused_sddmm_softmax_grad(sfb_stream_t stream, const void *nt_lut, const 
                                  uint32_t state_dim, uint32_t lut_heads, uint32_t lut_dim, float scale);
 
 /* The whole backward from the saved probabilities, dS kept on chip:
- *   delta = scale * rowsum(dO * O) (float [B, H, L], written), dS = P * (dO.V^T * scale - delta),
+ *   delta = -scale * rowsum(dO * O) (float [B, H, L], written), dS = P * (dO.V^T * scale + delta),
  *   dQ = dS.K, dK = dS^T.Q, dV = P^T.dO     (transformer_attention_optimize.cu:924-964).
- * 16-bit operands of one type, 64x64 blocks, 64-wide heads, rows and columns of 1 to 256 blocks (nn_max, tn_max: the longest),
- * all pointers 16-byte aligned; anything else is rejected (the separate operators take it).  lut_dim is the per-head
- * stride of both LUTs (blocks + ctx_blks). */
+ * 16-bit operands of one type, 64x64 blocks, 64-wide heads, at most 256 blocks per side of the block grid or rows and
+ * columns of at most 128 blocks (nn_max, tn_max: the longest, not 0), all pointers 32-byte aligned; anything else is
+ * rejected (the separate operators take it).  lut_dim is the per-head stride of both LUTs (blocks + ctx_blks). */
 int sfb_attention_backward(sfb_stream_t stream, const void *nn_lut, const void *tn_lut, const void *q, const void *k, const void *v,
                            const void *p_blocks, const void *o, const void *dout, float *delta, void *dq, void *dk, void *dv,
                            int dtype, uint32_t block_size, uint32_t blocks, uint32_t batch_dim, uint32_t ctx_blks, uint32_t head_dim,

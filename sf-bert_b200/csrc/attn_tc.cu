@@ -127,35 +127,13 @@ __device__ __forceinline__ void give_up(volatile uint32_t *abort_flag, uint32_t 
     atomicCAS(&g_status, 0u, (code << 24) | (blockIdx.x & 0xffffffu));
 }
 
-#ifndef SFB_TC_HINT_NS
-#define SFB_TC_HINT_NS 2000
-#endif
-constexpr uint32_t kSleepPolls = kWaitLimit >> 8;    // polls of up to SFB_TC_HINT_NS each before a wait gives up
-
-// bounded wait that sleeps in the barrier unit between polls
-__device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity, volatile uint32_t *abort_flag, uint32_t code)
-{
-    if (mbar_try_wait(bar, parity)) return true;
-    for (uint32_t i = 0; i < kSleepPolls; i++) {
-        if (mbar_try_wait_sleep(bar, parity, SFB_TC_HINT_NS)) return true;
-        if ((i & 15u) == 15u && *abort_flag) return false;
-    }
-    give_up(abort_flag, code);
-    return false;
-}
-__device__ __forceinline__ bool bar_wait_warp(uint64_t *bar, uint32_t parity, volatile uint32_t *abort_flag, uint32_t code)
-{
-    const bool ok = bar_wait(bar, parity, abort_flag, code);
-    return __all_sync(0xffffffffu, ok);
-}
-
 // bounded wait on two barriers at once (one dependent chain instead of two)
 __device__ __forceinline__ bool mbar_wait2(uint64_t *bar_a, uint32_t par_a, uint64_t *bar_b, uint32_t par_b, volatile uint32_t *abort_flag,
                                            uint32_t code)
 {
     const bool a = mbar_try_wait(bar_a, par_a), b = mbar_try_wait(bar_b, par_b);
     if (a && b) return true;
-    return (a || bar_wait(bar_a, par_a, abort_flag, code)) && (b || bar_wait(bar_b, par_b, abort_flag, code));
+    return (a || mbar_wait(bar_a, par_a, abort_flag, code)) && (b || mbar_wait(bar_b, par_b, abort_flag, code));
 }
 
 // The union of the key blocks of block-rows 2*pair and 2*pair+1, built by ONE warp: the upper row's blocks in LUT
@@ -398,7 +376,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
                 const uint32_t id = item_id(k, s, p);
                 if (id >= p.n_items) break;
                 const uint32_t slot = k & 1;
-                if (k >= 2 && !bar_wait_warp(&st->list_free[slot], ((k >> 1) - 1) & 1, abort_flag, 20)) break;
+                if (k >= 2 && !mbar_wait_warp(&st->list_free[slot], ((k >> 1) - 1) & 1, abort_flag, 20)) break;
                 const Item it = decode_item(id, p);
                 uint32_t n = plan_union(p.nn_lut + (size_t)it.h * p.lut_stride, it.pair, p.nb, lists + (s * 2 + slot) * kMaxU, lane);
                 if (n == 0xffffffffu) {
@@ -432,7 +410,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
                 const uint32_t b2 = gg & 1;
                 // S(gg) overlaps half of S(gg-1): that one must be in the softmax threads' registers
                 if (gg >= 1 ? !mbar_wait2(&st->s_free, (gg - 1) & 1, &st->k_full[b2], (gg >> 1) & 1, abort_flag, 4)
-                            : !bar_wait(&st->k_full[b2], (gg >> 1) & 1, abort_flag, 3))
+                            : !mbar_wait(&st->k_full[b2], (gg >> 1) & 1, abort_flag, 3))
                     return false;
                 tcgen05_fence_after();
                 const uint64_t k_desc = smem_desc_sw128(smem_u32(smem + kOffK + (s * 2 + b2) * kTileBytes));
@@ -445,10 +423,10 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
             for (uint32_t k = 0; alive; k++) {
                 const uint32_t id = item_id(k, s, p);
                 if (id >= p.n_items) break;
-                if (!bar_wait(&st->list_ready[k & 1], (k >> 1) & 1, abort_flag, 8)) break;
+                if (!mbar_wait(&st->list_ready[k & 1], (k >> 1) & 1, abort_flag, 8)) break;
                 const uint32_t T = st->list_n[k & 1];
                 if (T > 0) {
-                    if (!bar_wait(&st->q_full, kq & 1, abort_flag, 2)) break;
+                    if (!mbar_wait(&st->q_full, kq & 1, abort_flag, 2)) break;
                     alive = issue_qk(g);
                     if (alive && T == 1) umma_commit(&st->q_free);
                     for (uint32_t t = 0; alive && t < T; t++) {
@@ -458,7 +436,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
                             if (t + 2 == T) umma_commit(&st->q_free);
                         }
                         // the accumulator still holds the previous item's O until its epilogue has read it
-                        if (t == 0 && kq >= 1 && !bar_wait(&st->o_free, (kq - 1) & 1, abort_flag, 11)) { alive = false; break; }
+                        if (t == 0 && kq >= 1 && !mbar_wait(&st->o_free, (kq - 1) & 1, abort_flag, 11)) { alive = false; break; }
                         if (!mbar_wait2(&st->p_full[b2], (gg >> 1) & 1, &st->v_full[b2], (gg >> 1) & 1, abort_flag, 5)) { alive = false; break; }
                         tcgen05_fence_after();
                         const uint64_t v_desc = smem_desc_sw128(smem_u32(smem + kOffV + (s * 2 + b2) * kTileBytes));
@@ -500,7 +478,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
             const bool has_row1 = e_pair * 2 + 1 < p.nb;
             float inv = 0.f;
             if (has_data) {
-                if (!bar_wait_warp(&st->o_final, kq & 1, abort_flag, 10)) return false;
+                if (!mbar_wait_warp(&st->o_final, kq & 1, abort_flag, 10)) return false;
                 tcgen05_fence_after();
                 float a0, a1, a2, a3;
                 up64(l0, a0, a1);
@@ -509,7 +487,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
                 inv = lsum > 0.f ? 1.f / lsum : 0.f;
             }
             // the previous store out of the staging tile has been read out of shared memory
-            if (n_epi >= 1 && !bar_wait_warp(&st->stage_free, (n_epi - 1) & 1, abort_flag, 13)) return false;
+            if (n_epi >= 1 && !mbar_wait_warp(&st->stage_free, (n_epi - 1) & 1, abort_flag, 13)) return false;
             uint8_t *orow = ostage + r * 128;
             uint16_t *dst = (uint16_t *)p.O + ((size_t)e_b * L + (size_t)e_pair * 128 + r) * (size_t)p.o_pitch + (size_t)e_h * 64;
 #pragma unroll
@@ -555,7 +533,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
         for (uint32_t k = 0; alive; k++) {
             const uint32_t id = item_id(k, s, p);
             if (id >= p.n_items) break;
-            if (!bar_wait_warp(&st->list_ready[k & 1], (k >> 1) & 1, abort_flag, 8)) break;
+            if (!mbar_wait_warp(&st->list_ready[k & 1], (k >> 1) & 1, abort_flag, 8)) break;
             const uint32_t T = st->list_n[k & 1];
             const UEntry *list = lists + (s * 2 + (k & 1)) * kMaxU;
             const uint32_t item_h = HAS_MASK ? decode_item(id, p).h : 0u;
@@ -564,7 +542,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
             for (uint32_t t = 0; t < T; t++) {
                 const uint32_t gg = g + t, b2 = gg & 1;
                 const uint32_t t_s = tbase + 32 * b2, t_p = tbase + 64 * b2;
-                if (!bar_wait_warp(&st->qk_done[b2], (gg >> 1) & 1, abort_flag, 6)) { alive = false; break; }
+                if (!mbar_wait_warp(&st->qk_done[b2], (gg >> 1) & 1, abort_flag, 6)) { alive = false; break; }
                 tcgen05_fence_after();
                 TMEM_LD_32((sr), t_s);
                 TMEM_LD_32((sr + 32), t_s + 32);
@@ -604,7 +582,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
                         }
                         if (t > 0 && __any_sync(0xffffffffu, fix_o)) {
                             // O must be complete before it is rescaled, and P(t) is only handed over afterwards
-                            if (!bar_wait_warp(&st->pv_done[(gg - 1) & 1], ((gg - 1) >> 1) & 1, abort_flag, 7)) { alive = false; break; }
+                            if (!mbar_wait_warp(&st->pv_done[(gg - 1) & 1], ((gg - 1) >> 1) & 1, abort_flag, 7)) { alive = false; break; }
                             tcgen05_fence_after();
 #pragma unroll
                             for (int c0 = 0; c0 < 64; c0 += 16) {

@@ -446,8 +446,8 @@ FUNCTION(py_attention_backward_fused, 8)
     void *tn = lay.get(n_tn_lut);
     const uint32_t tn_max = attr_u32(lay.o, n_tn_max);
     // dS on chip where the library has the kernels for it, otherwise operator by operator
-    auto tidy = [](const at::Tensor &x) { return x.is_contiguous() && ((uintptr_t)ptr(x) & 15) == 0; };
-    if (t != SFB_F32 && lay.bs == 64 && n.d == 64 && lay.blocks && lay.nn_max && lay.nn_max <= 256 && tn_max && tn_max <= 256 && tag(k) == t &&
+    auto tidy = [](const at::Tensor &x) { return x.is_contiguous() && ((uintptr_t)ptr(x) & 31) == 0; };
+    if (t != SFB_F32 && lay.bs == 64 && n.d == 64 && lay.blocks && lay.nn_max && tn_max && (lay.nb <= 256 || (lay.nn_max <= 128 && tn_max <= 128)) && tag(k) == t &&
         tag(v) == t && tag(p) == t && tag(o) == t && tag(dout) == t && tidy(q) && tidy(k) && tidy(v) && tidy(p) && tidy(o) && tidy(dout) &&
         (int64_t)n.B * n.H * lay.blocks * 64 < (1ll << 31) - 64 && (int64_t)n.B * n.L < (1ll << 31)) {
         require(o.sizes() == dout.sizes() && dout.sizes() == q.sizes(), "q, o and dO differ in shape");

@@ -243,7 +243,7 @@ extern "C" int sfb_attention_backward(sfb_stream_t stream, const void *nn_lut, c
     const uint64_t pointers = (uint64_t)((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)p_blocks | (uintptr_t)o | (uintptr_t)dout |
                                          (uintptr_t)delta | (uintptr_t)dq | (uintptr_t)dk | (uintptr_t)dv);
     SFB_REQUIRE(tc_backward_supported(dtype, block_size, p, nn_max, tn_max, pointers),
-                "%s: needs 16-bit operands, 64x64 blocks, 64-wide heads, 16-byte aligned pointers and rows and columns of 1 to 256 blocks", who);
+                "%s: needs 16-bit operands, 64x64 blocks, 64-wide heads, 32-byte aligned pointers and unions of two rows or columns of at most 256 blocks", who);
     return tc_backward(as_stream(stream), nn_lut, tn_lut, q, k, v, p_blocks, o, dout, delta, dq, dk, dv, dtype, p, scale);
 }
 

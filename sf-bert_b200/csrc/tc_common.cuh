@@ -92,12 +92,16 @@ __device__ __forceinline__ bool mbar_try_wait_sleep(uint64_t *bar, uint32_t pari
         : "memory");
     return ok != 0;
 }
-// bounded wait: false when the limit ran out or another role already gave up
+// bounded wait: false when the limit ran out or another role already gave up.  Between polls the thread sleeps in the barrier
+// unit: polling flat out, the one-thread roles of a CTA took a good part of the issue slots from the warps that compute
+constexpr uint32_t kSleepNs = 2000;
+constexpr uint32_t kSleepPolls = kWaitLimit >> 8;            // polls of up to kSleepNs each before a wait gives up
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile uint32_t *abort_flag, uint32_t code)
 {
-    for (uint32_t i = 0; i < kWaitLimit; i++) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((i & 255u) == 255u && *abort_flag) return false;
+    if (mbar_try_wait(bar, parity)) return true;
+    for (uint32_t i = 0; i < kSleepPolls; i++) {
+        if (mbar_try_wait_sleep(bar, parity, kSleepNs)) return true;
+        if ((i & 15u) == 15u && *abort_flag) return false;
     }
     *abort_flag = 1;
     atomicCAS(&g_status, 0u, (code << 24) | (blockIdx.x & 0xffffffu));
@@ -110,6 +114,13 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, v
 {
     const bool ok = mbar_wait(bar, parity, abort_flag, code);
     return __all_sync(0xffffffffu, ok);
+}
+
+// one arrival for a warp whose lanes have all done what the barrier stands for (32 arrivals of one warp are taken one by one)
+__device__ __forceinline__ void mbar_arrive_warp(uint64_t *bar, uint32_t lane)
+{
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
 }
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint64_t *bar, int32_t x, int32_t y)

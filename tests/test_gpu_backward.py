@@ -229,3 +229,33 @@ def test_fused_sddmm_softmax_grad(sfb, oracle, dtype, H_lut, nb, kind, kw, dev):
     for a, b in ((dq1, dq0), (dk1, dk0), (dv1, dv0)):
         assert float((a.float() - b.float()).abs().max()) <= 5e-2 * float(b.float().abs().max())
 
+
+
+@pytest.mark.parametrize("nb,heads,case", [(1, 1, "all"), (2, 1, "sparse"), (3, 2, "sparse"), (17, 3, "sparse"), (33, 1, "global"), (64, 2, "empty"),
+                                           (257, 1, "sparse")])
+def test_backward_with_ds_on_chip(sfb, nb, heads, case):
+    """Rows and columns of very different length, empty ones, an odd last one and per-head tables: the one-call backward against
+    the separate operators (which the other tests hold against the oracle)."""
+    B, d, bs = 2, 64, 64
+    g = torch.Generator(device="cuda").manual_seed(nb)
+    lay8 = torch.zeros(heads, nb, nb, dtype=torch.uint8, device="cuda")
+    n = nb * nb if case == "all" else max(1, 4 * nb if nb < 100 else 3 * nb)
+    for h in range(heads):                                   # every head keeps the same number of blocks
+        if case == "global":
+            lay8[h, 3] = 1
+            lay8[h, :, 7] = 1
+        lay8[h].view(-1)[torch.randperm(nb * nb, device="cuda", generator=g)[:min(n, nb * nb // 2 + 1 if case != "all" else n)]] = 1
+        if case == "empty":
+            lay8[h].zero_()
+            for r in range(5, nb, 3):
+                lay8[h, r, (r * 7 + h) % 9] = 1
+    lay = sfb.BlockLayout(lay8, bs)
+    q, k, v, do = (torch.randn(B, nb * bs, heads, d, device="cuda", generator=g).to(torch.bfloat16) for _ in range(4))
+    p = sfb.fused_sddmm_softmax(q, k, lay, 0.125, torch.bfloat16)
+    o = sfb.bst_sgemm_xn(p, v, lay)
+    got = sfb.attention_backward_fused(q, k, v, p, o, do, lay, 0.125)
+    want = sfb.attention_backward(q, k, v, p, do, lay, 0.125)
+    assert sfb.device_status() == 0
+    for a, b in zip(got, want):
+        assert float((a.float() - b.float()).abs().max()) <= 5e-2 * float(b.float().abs().max())
+        assert torch.equal(a.float().abs().amax(-1) == 0, b.float().abs().amax(-1) == 0)      # what has no blocks is zero, nothing else is
