@@ -290,6 +290,14 @@ int sfb_csr_attention(sfb_stream_t stream, const int32_t *rowptr, const int32_t 
                       const void *v, void *o, int dtype, uint32_t batch_dim, uint32_t seq_len, uint32_t head_dim,
                       uint32_t state_dim, float scale, uint32_t *bad_columns);
 
+/* The same with a workspace of sfb_csr_workspace(nnz, seq_len) bytes (16-byte aligned; 0: the sequence is too long for it):
+ * the pattern is first laid out by tiles of 32 query rows, whose keys are then fetched once per tile instead of once per
+ * row.  nnz = elements of colidx.  bad_columns counts as above (it may be NULL). */
+uint64_t sfb_csr_workspace(uint32_t nnz, uint32_t seq_len);
+int sfb_csr_attention_planned(sfb_stream_t stream, const int32_t *rowptr, const int32_t *colidx, uint32_t nnz, const void *q,
+                              const void *k, const void *v, void *o, int dtype, uint32_t batch_dim, uint32_t seq_len,
+                              uint32_t head_dim, uint32_t state_dim, float scale, uint32_t *bad_columns, void *workspace);
+
 #ifdef __cplusplus
 }
 #endif

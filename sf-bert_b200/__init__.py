@@ -27,7 +27,8 @@ SYMBOLS = [
     "sfb_fused_attention", "sfb_bias_residual_layernorm", "sfb_device_status", "sfb_bias_gelu", "sfb_lut_build_tn",
     "sfb_masked_softmax_grad", "sfb_linear", "sfb_linear_nt", "sfb_embedding", "sfb_csr_from_layout",
     "sfb_csr_attention", "sfb_rowdot", "sfb_fused_sddmm_softmax_grad", "sfb_fused_attention_slice", "sfb_device_status_clear",
-    "sfb_linear_residual", "sfb_attention_backward",
+    "sfb_linear_residual", "sfb_attention_backward", "sfb_csr_workspace",
+    "sfb_csr_attention_planned",
 ]
 
 if not os.path.exists(LIB_PATH):

@@ -6,6 +6,7 @@
 // rows ty+16m and columns tx+16n of a tile, so the 16 lanes of a half-warp own one set of rows
 // and row reductions are four shuffles.
 #include "simt_tile.cuh"
+#include "csr.cuh"
 #include <float.h>
 #include <math.h>
 
@@ -856,6 +857,156 @@ fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q
 }
 
 // ------------------------------------------------------------------------------------------------
+// Element-sparse attention of one tile of 32 query rows on fp32 operands (csr.cu makes the tile's list of columns and
+// row masks): the kernel above on keys gathered by column, 128 of them per step, a 32x32 score tile per warp.
+template <int ROWS, int COLS>
+__device__ __forceinline__ void stage_gather(float *dst, uint32_t stride, const float *src, const CsrTileArgs &a, uint32_t base, uint32_t top,
+                                             uint32_t distinct, uint32_t first, uint32_t n, size_t pitch)
+{
+    using namespace tile;
+    constexpr int P = COLS / 4, STEP = (int)kThreads / P;
+    const uint32_t r0 = threadIdx.x / P, c = (threadIdx.x % P) * 4;
+#pragma unroll
+    for (int i = 0; i < ROWS / STEP; i++) {
+        const uint32_t r = r0 + i * STEP;
+        const bool in = first + r < n;                                   // rows behind the list arrive as zeros
+        const uint32_t col = in ? csr_entry(a.entries, base, top, distinct, first + r).x : 0u;
+        cp_async16(dst + r * stride + c, src + (size_t)col * pitch + c, in ? 16u : 0u);
+    }
+}
+template <int D>
+__global__ void __launch_bounds__(tile::kThreads, 3) csr_tile_f32_kernel(const CsrTileArgs a)
+{
+    using namespace tile;
+    typedef FaCfg<32, D> Cfg;
+    constexpr int TN = Cfg::TN;
+    constexpr uint32_t NK = Cfg::NK, QS = Cfg::q_stride, PS = Cfg::p_stride, kchunks = D / kChunk;
+    extern __shared__ __align__(16) float sm[];
+    float *Qs = sm, *bufs = Qs + 32 * QS, *Ps = bufs + 2 * Cfg::buf, *red = Ps + 32 * PS;
+    grid_dependency_wait();
+    grid_launch_dependents();
+    csr_write_bad(a);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane_row(lane), lc = lane_quad(lane);
+    const uint32_t tl = a.tiles - 1u - blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+    const uint32_t distinct = a.counts[4 * tl], base = a.counts[4 * tl + 2], top = a.counts[4 * tl + 3], n = distinct + a.counts[4 * tl + 1];
+    const size_t HD = (size_t)a.H * D, head = (size_t)b * a.L * HD + (size_t)h * D;
+    const float *K = (const float *)a.K + head, *V = (const float *)a.V + head;
+    const uint32_t n0 = warp * (D / 4);
+
+    uint32_t is_e = 0, is_k = 0, is_n = 0;                               // next chunk to issue: step's first key, index in the step, overall
+    auto issue = [&]() {
+        float *buf = bufs + (is_n & 1) * Cfg::buf;
+        if (is_k < kchunks) stage_gather<(int)NK, (int)kChunk>(buf, kStride, K + is_k * kChunk, a, base, top, distinct, is_e, n, HD);
+        else stage_gather<32, D>(buf, D + 4, V, a, base, top, distinct, is_e + (is_k - kchunks) * 32, n, HD);
+        cp_commit();
+        is_n++;
+        if (++is_k == kchunks + (min(NK, n - is_e) + 31) / 32) {
+            is_k = 0;
+            is_e += NK;
+        }
+    };
+    if (n) {
+        const uint32_t rows = min(32u, a.L - tl * 32);                   // rows behind the sequence: the last one again, not written
+        constexpr int P = D / 4, STEP = (int)kThreads / P;
+#pragma unroll
+        for (int i = 0; i < 32 / STEP; i++) {
+            const uint32_t r = threadIdx.x / P + i * STEP, c = (threadIdx.x % P) * 4;
+            cp_async16(Qs + r * QS + c, (const float *)a.Q + head + (size_t)(tl * 32 + min(r, rows - 1)) * HD + c, 16u);
+        }
+        issue();
+    }
+    float mx[4], sum[4];
+    uint64_t acc[4][TN / 2];
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+        mx[m] = -INFINITY;
+        sum[m] = 0.f;
+#pragma unroll
+        for (int j = 0; j < TN / 2; j++) acc[m][j] = 0;
+    }
+    uint32_t c = 0;
+    for (uint32_t e = 0; e < n; e += NK) {
+        const uint32_t left = min(NK, n - e);
+        const bool live = 32 * warp < left;
+        uint64_t s2[4][8];
+#pragma unroll
+        for (int m = 0; m < 4; m++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) s2[m][j] = 0;
+        uint32_t mk[8];                                                  // the rows of this thread's eight columns
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const uint32_t col = 32 * warp + lc + 4 * j;
+            mk[j] = col < left ? csr_entry(a.entries, base, top, distinct, e + col).y : 0u;
+        }
+        for (uint32_t kc = 0; kc < kchunks; kc++, c++) {
+            cp_wait_all();
+            __syncthreads();
+            issue();                                                     // a value chunk follows every key chunk of a step
+            if (live) mma_nt(s2, Qs + lr * QS + kc * kChunk, QS, bufs + (c & 1) * Cfg::buf + (32 * warp + lc) * kStride, kStride);
+        }
+        float s[4][8], bm[4];
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            bm[m] = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                s[m][j] = (mk[j] >> (lr + 8 * m)) & 1u ? half_sum(s2[m][j]) * a.scale_log2e : -INFINITY;
+                bm[m] = fmaxf(bm[m], s[m][j]);
+            }
+            bm[m] = fmaxf(bm[m], __shfl_xor_sync(0xffffffffu, bm[m], 1));
+            bm[m] = fmaxf(bm[m], __shfl_xor_sync(0xffffffffu, bm[m], 4));
+            if (lc == 0) red[warp * 32 + lr + 8 * m] = bm[m];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            const uint32_t r = lr + 8 * m;
+            float mn = mx[m];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) mn = fmaxf(mn, red[k * 32 + r]);
+            const float alpha = mn > mx[m] ? exp2f(mx[m] - mn) : 1.f;
+            mx[m] = mn;
+            float ps = 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const float pv = mn > -INFINITY ? exp2f(s[m][j] - mn) : 0.f;
+                Ps[r * PS + 32 * warp + lc + 4 * j] = pv;
+                ps += pv;
+            }
+            sum[m] = fmaf(sum[m], alpha, ps);                            // this thread's columns only; the shares meet at the end
+            const uint64_t a2 = pair(alpha, alpha);
+#pragma unroll
+            for (int j = 0; j < TN / 2; j++) acc[m][j] = fma2(acc[m][j], a2, 0ull);
+        }
+        const uint32_t vchunks = (left + 31) / 32;
+        for (uint32_t vc = 0; vc < vchunks; vc++, c++) {
+            cp_wait_all();
+            __syncthreads();
+            if (vc + 1 < vchunks || e + NK < n) issue();
+            mma_nn<TN>(acc, Ps + lr * PS + vc * 32, PS, bufs + (c & 1) * Cfg::buf + n0 + lane_col<TN>(lc), D + 4);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+        sum[m] += __shfl_xor_sync(0xffffffffu, sum[m], 1);
+        sum[m] += __shfl_xor_sync(0xffffffffu, sum[m], 4);
+        if (lc == 0) red[warp * 32 + lr + 8 * m] = sum[m];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+        const uint32_t r = lr + 8 * m;
+        float l = 0.f;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) l += red[k * 32 + r];
+        const float inv = l > 0.f ? 1.f / (l + 1e-6f) : 0.f;             // the reference's denominator (ewops.h:93, cuda_kernels.h:1022)
+        if (tl * 32 + r < a.L) store_cols<SFB_F32, TN>(a.O, head + (size_t)(tl * 32 + r) * HD + n0, lc, acc[m], inv, D / 4, true);
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
 // host-side dispatch
 #define DISPATCH_BS(bs, ...)            \
     if (bs == 32) { constexpr int BS = 32; __VA_ARGS__ } else { constexpr int BS = 64; __VA_ARGS__ }
@@ -1034,6 +1185,20 @@ int simt_fused_attention(cudaStream_t s, const void *nn_lut, const void *q, cons
     }))
 #undef LAUNCH_FA
     return check_launch("sfb_fused_attention");
+}
+
+int csr_tile_f32(cudaStream_t s, const CsrTileArgs &a, uint32_t B, uint32_t d)
+{
+#define LAUNCH_CT(DV)                                                                                            \
+    {                                                                                                            \
+        const size_t bytes = sizeof(float) * FaCfg<32, DV>::floats;                                              \
+        auto kern = csr_tile_f32_kernel<DV>;                                                                     \
+        static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                       \
+        launch_overlapped(kern, dim3(a.tiles, a.H, B), dim3(tile::kThreads), bytes, s, a);                       \
+    }
+    if (d == 32) LAUNCH_CT(32) else if (d == 64) LAUNCH_CT(64) else LAUNCH_CT(128)
+#undef LAUNCH_CT
+    return check_launch("sfb_csr_attention");
 }
 
 }  // namespace sfb

@@ -3,16 +3,18 @@
 // One CSR pattern (rowptr [L+1], colidx [nnz], int32) is shared by every (batch, head).
 //
 //   csr_from_layout_kernel   block layout -> the CSR pattern of all elements of its kept blocks
-//   csr_attention_*_kernel   O_i = sum_j softmax_j(q_i . k_j) v_j over the row's columns, one WARP per query row.
-//                            In use: four lanes per key, each with a quarter of q_i and of the accumulators in
-//                            registers (eight keys per warp and step, partial scores joined by two shuffles, K and V
-//                            pieces requested together); every group of four runs its own online softmax, merged by
-//                            shuffles at the end.  Measured on the BERT-base stride pattern: 5.7 ms, against 9.0 ms with
-//                            two lanes per key, 17.7 ms with one (whole q_i per lane, 8 resident warps per SM), 6.8 ms with eight,
-//                            7.0 ms with four and two keys per group and step.
-// The format has no reuse of K/V between query rows (every row gathers its own keys through L2), which is why the
-// block-sparse path exists; these kernels are the correct, coalesced-per-key version of the prototype, not a fast path.
+//   csr_plan_kernel          the pattern by tiles of 32 query rows: the columns any of them has, in ascending order, each with
+//                            a 32-bit mask of the rows that have it
+//   csr_tile_kernel          O for one tile and (batch, head) over those columns, 16-bit operands, on warp MMAs
+//   csr_tile_f32_kernel      (attn_simt.cu) the same on the CUDA cores, for fp32 operands
+//   csr_attention_split_kernel   one warp per query row, four lanes per key: callers without a workspace for the plan, and
+//                            sequences whose columns do not fit the plan's shared memory
+// Row by row every query gathers its own keys through L2 (294 keys, 75 KB, per row of a 256-token window with strided and
+// random columns): 626 us at B 2, H 12, L 4096, d 64, with the FMA pipes half idle.  32 neighbouring rows mostly want the
+// same keys, so a tile fetches each column once and masks the rows that do not have it: a ninth of the bytes, and the
+// products are contractions again.  The plan is made once per call and shared by the batch's heads.
 #include "attn.cuh"
+#include "csr.cuh"
 
 namespace sfb {
 
@@ -43,109 +45,6 @@ __global__ void csr_from_layout_kernel(const uint8_t *__restrict__ layout, uint3
     }
 }
 
-template <int DT> struct Row;   // loads D consecutive elements of a [.., d] row as floats, 16 bytes at a time
-template <> struct Row<SFB_F32> {
-    template <int D> static __device__ __forceinline__ void load(float (&v)[D], const void *p, size_t off)
-    {
-        const float4 *s = (const float4 *)((const float *)p + off);
-#pragma unroll
-        for (int i = 0; i < D / 4; i++) { const float4 t = __ldg(s + i); v[4 * i] = t.x; v[4 * i + 1] = t.y; v[4 * i + 2] = t.z; v[4 * i + 3] = t.w; }
-    }
-};
-template <> struct Row<SFB_BF16> {
-    template <int D> static __device__ __forceinline__ void load(float (&v)[D], const void *p, size_t off)
-    {
-        const uint4 *s = (const uint4 *)((const uint16_t *)p + off);
-#pragma unroll
-        for (int i = 0; i < D / 8; i++) {
-            const uint4 t = __ldg(s + i);
-            const uint32_t w[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-            for (int j = 0; j < 4; j++) { v[8 * i + 2 * j] = __uint_as_float(w[j] << 16); v[8 * i + 2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u); }
-        }
-    }
-};
-template <> struct Row<SFB_F16> {
-    template <int D> static __device__ __forceinline__ void load(float (&v)[D], const void *p, size_t off)
-    {
-        const uint4 *s = (const uint4 *)((const uint16_t *)p + off);
-#pragma unroll
-        for (int i = 0; i < D / 8; i++) {
-            const uint4 t = __ldg(s + i);
-            const uint32_t w[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-            for (int j = 0; j < 4; j++) { const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[j])); v[8 * i + 2 * j] = f.x; v[8 * i + 2 * j + 1] = f.y; }
-        }
-    }
-};
-
-// D = head size rounded up to 32/64/128 by the dispatcher only when it is exactly that value
-template <int DT, int D>
-__global__ void __launch_bounds__(128) csr_attention_kernel(const int32_t *__restrict__ rowptr, const int32_t *__restrict__ colidx,
-                                                           const void *__restrict__ Q, const void *__restrict__ K,
-                                                           const void *__restrict__ V, void *__restrict__ O, uint32_t L, uint32_t H,
-                                                           float scale_log2e, uint32_t *bad)
-{
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t i = blockIdx.x * 4 + (threadIdx.x >> 5), b = blockIdx.y, h = blockIdx.z;
-    if (i >= L) return;
-    const size_t HD = (size_t)H * D;
-    const size_t row_off = ((size_t)b * L + i) * HD + (size_t)h * D;
-    const int32_t lo = rowptr[i], hi = rowptr[i + 1];
-    float q[D], acc[D];
-    Row<DT>::template load<D>(q, Q, row_off);
-#pragma unroll
-    for (int x = 0; x < D; x++) acc[x] = 0.f;
-    float m = -INFINITY, l = 0.f;          // m: running max of the unscaled scores of this lane's keys
-    for (int32_t e = lo + (int32_t)lane; e < hi; e += 32) {
-        const int32_t j = __ldg(colidx + e);
-        if (j < 0 || (uint32_t)j >= L) {   // a column outside the sequence: counted, not read
-            if (bad) atomicAdd(bad, 1u);
-            continue;
-        }
-        const size_t key_off = ((size_t)b * L + (uint32_t)j) * HD + (size_t)h * D;
-        float t[D];
-        Row<DT>::template load<D>(t, K, key_off);
-        float s = 0.f;
-#pragma unroll
-        for (int x = 0; x < D; x++) s = fmaf(q[x], t[x], s);
-        if (s > m) {
-            const float f = exp2f((m - s) * scale_log2e);   // 0 on the first key
-            l *= f;
-#pragma unroll
-            for (int x = 0; x < D; x++) acc[x] *= f;
-            m = s;
-        }
-        const float p = exp2f((s - m) * scale_log2e);
-        l += p;
-        Row<DT>::template load<D>(t, V, key_off);
-#pragma unroll
-        for (int x = 0; x < D; x++) acc[x] = fmaf(p, t[x], acc[x]);
-    }
-    // merge the 32 lanes' softmaxes
-    float M = m;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-    const float f = m > -INFINITY ? exp2f((m - M) * scale_log2e) : 0.f;
-    l *= f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    const float inv = l > 0.f ? 1.f / (l + 1e-6f) : 0.f;   // the reference's denominator (ewops.h:93, cuda_kernels.h:1022)
-    // transpose-reduce: after step k lane holds sums over lane groups; finally lane x owns elements x, x+32, ...
-#pragma unroll
-    for (int x = 0; x < D; x++) {
-        float a = acc[x] * f;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        acc[x] = a * inv;
-    }
-    // every lane holds the whole row now; each writes its share
-#pragma unroll
-    for (int x = 0; x < D; x++)
-        if ((x & 31) == (int)lane) Elem<DT>::store(O, row_off + x, acc[x]);
-}
-
-
 // 16-byte pieces -> floats, by element type
 template <int DT> struct Piece;
 template <> struct Piece<SFB_F32> {
@@ -174,10 +73,9 @@ template <> struct Piece<SFB_F16> {
     }
 };
 
-// The same attention with TWO lanes per key, each owning half of the head dimension: half the registers per lane
-// (q and the accumulators are D/2 wide), so twice the warps are resident, and the key's K and V pieces are all
-// requested before the first is used (one memory round trip per key instead of two).  The two lanes exchange their
-// partial scores with one shuffle; both then carry the same running max and sum.
+// One warp per query row with LPK lanes per key, each owning a share of the head dimension; the key's K and V pieces are all
+// requested before the first is used.  The lanes of a key join their partial scores by shuffles and carry the same running
+// max and sum; the groups' softmaxes are merged at the end.
 template <int DT, int D, int LPK>
 __global__ void __launch_bounds__(128) csr_attention_split_kernel(const int32_t *__restrict__ rowptr, const int32_t *__restrict__ colidx,
                                                                  const void *__restrict__ Q, const void *__restrict__ K,
@@ -274,6 +172,397 @@ __global__ void __launch_bounds__(128) csr_attention_split_kernel(const int32_t 
     }
 }
 
+// ---- the plan -------------------------------------------------------------------------------------------------
+// One CTA per tile of 32 query rows.  Every element sets its row's bit in its column's mask in shared memory; what is set
+// is written out column by column.  A column that a row names twice counts twice, as it does row by row: the second one
+// becomes an entry of its own at the end.  The tile's entries start at its first row's offset in colidx: there are never
+// more of them than elements.  Columns outside the sequence are counted and dropped.
+constexpr uint32_t kPlanThreads = 512;
+constexpr uint32_t kPlanMaxL = 48 * 1024;                    // columns whose masks fit shared memory
+__global__ void __launch_bounds__(kPlanThreads) csr_plan_kernel(const int32_t *__restrict__ rowptr, const int32_t *__restrict__ colidx, uint32_t L,
+                                                                uint32_t nnz, uint2 *__restrict__ entries, uint32_t *__restrict__ counts,
+                                                                uint32_t *__restrict__ bad)
+{
+    extern __shared__ uint32_t mask[];                       // [L]
+    __shared__ uint32_t warp_count[kPlanThreads / 32], n_twice, n_bad;
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const uint32_t tile = blockIdx.x, row0 = tile * 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rows = min(32u, L - row0);
+    const uint32_t base = min((uint32_t)max(rowptr[row0], 0), nnz), top = min((uint32_t)max(rowptr[row0 + rows], 0), nnz);
+    if (threadIdx.x == 0) n_twice = n_bad = 0;
+    for (uint32_t j = threadIdx.x; j < L; j += kPlanThreads) mask[j] = 0;
+    __syncthreads();
+    for (uint32_t r = warp; r < rows; r += kPlanThreads / 32) {
+        const int32_t lo = max(rowptr[row0 + r], 0), hi = (int32_t)min((uint32_t)max(rowptr[row0 + r + 1], 0), nnz);
+        for (int32_t e = lo + (int32_t)lane; e < hi; e += 32) {
+            const int32_t j = __ldg(colidx + e);
+            if (j < 0 || (uint32_t)j >= L) { atomicAdd(&n_bad, 1u); continue; }
+            if (atomicOr(&mask[j], 1u << r) & (1u << r)) {
+                const uint32_t at = top - 1u - atomicAdd(&n_twice, 1u);      // from the end of the tile's share backwards
+                if (at >= base && at < nnz) entries[at] = make_uint2((uint32_t)j, 1u << r);
+            }
+        }
+    }
+    __syncthreads();
+    // every warp takes a run of columns: count, prefix over the warps, write
+    const uint32_t per = ((L + kPlanThreads / 32 - 1) / (kPlanThreads / 32) + 31) & ~31u;
+    const uint32_t from = min(warp * per, L), to = min(from + per, L);
+    uint32_t c = 0;
+    for (uint32_t j0 = from; j0 < to; j0 += 32) c += __popc(__ballot_sync(0xffffffffu, j0 + lane < to && mask[j0 + lane] != 0));
+    if (lane == 0) warp_count[warp] = c;
+    __syncthreads();
+    uint32_t at = base, total = 0;
+    for (uint32_t w = 0; w < kPlanThreads / 32; w++) {
+        if (w < warp) at += warp_count[w];
+        total += warp_count[w];
+    }
+    for (uint32_t j0 = from; j0 < to; j0 += 32) {
+        const uint32_t m = j0 + lane < to ? mask[j0 + lane] : 0;
+        const uint32_t votes = __ballot_sync(0xffffffffu, m != 0);
+        const uint32_t dst = at + __popc(votes & ((1u << lane) - 1u));
+        if (m && dst < nnz) entries[dst] = make_uint2(j0 + lane, m);
+        at += __popc(votes);
+    }
+    if (threadIdx.x == 0) {
+        counts[4 * tile] = min(total, nnz - base);
+        counts[4 * tile + 1] = min(n_twice, top - min(base, top));
+        counts[4 * tile + 2] = base;
+        counts[4 * tile + 3] = top;
+        bad[tile] = n_bad;
+    }
+}
+
+// ---- one tile of 32 query rows x one (batch, head), 16-bit operands ------------------------------------------------
+// Four warps share the tile's columns, a chunk of KC of them at a time each (two warps share a chunk when D is 128: 16 rows
+// each), with no barrier between them: a warp fetches its chunk's K and V rows into its own two buffers (cp.async, one
+// chunk ahead), multiplies on warp MMAs (m16n8k16), and keeps its own running maximum, sum and output; the four meet at
+// the end.  Warp MMAs rather than tcgen05: the columns of a tile are rows scattered over K and V, and 32 rows is where
+// neighbouring queries still share them; the kernel is bound by the gather and the exponentials.
+// P enters P.V as two 16-bit terms (the rounded value and what the rounding left), so the product keeps the fp32
+// probabilities to 16 bits (bf16) and 22 bits (fp16).
+template <int D> struct CsrCfg {
+    static constexpr int MT = D == 128 ? 1 : 2;              // 16-row tiles per warp
+    static constexpr int SPLITS = D == 128 ? 2 : 4;          // warps that take different chunks
+    static constexpr int KC = D == 128 ? 16 : 32;            // columns per chunk
+    static constexpr uint32_t tile_bytes = KC * D * 2;
+    static constexpr uint32_t warp_bytes = 4 * tile_bytes;   // K and V, two buffers
+    static constexpr uint32_t o_stride = D + 4;              // floats; the outputs take the buffers' place at the end
+    static constexpr size_t smem = 4 * warp_bytes;
+    static_assert(MT * 16 * o_stride * 4 <= warp_bytes, "the output fits the buffers");
+};
+__device__ __forceinline__ void ldsm(uint32_t (&r)[4], uint32_t addr)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm_trans(uint32_t (&r)[4], uint32_t addr)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+template <bool BF16>
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+{
+    if (BF16)
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    else
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <bool BF16>
+__device__ __forceinline__ uint32_t pack16(float a, float b)
+{
+    uint32_t y;
+    if (BF16) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(y) : "f"(b), "f"(a));
+    else asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(y) : "f"(b), "f"(a));
+    return y;
+}
+template <bool BF16>
+__device__ __forceinline__ float2 unpack16(uint32_t v)
+{
+    if (BF16) return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+    return __half22float2(*reinterpret_cast<const __half2 *>(&v));
+}
+__device__ __forceinline__ float ex2f(float x)
+{
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+template <bool BF16, int D>
+__global__ void __launch_bounds__(128, D == 128 ? 2 : 3) csr_tile_kernel(const CsrTileArgs a)
+{
+    typedef CsrCfg<D> Cfg;
+    constexpr int MT = Cfg::MT, KC = Cfg::KC, NT = KC / 8, CH = D / 8, DN = D / 8;
+    extern __shared__ __align__(128) uint8_t sm[];
+    __shared__ __align__(8) uint32_t masks[4][2][KC];
+    __shared__ float2 ml[4][MT * 16];
+    grid_dependency_wait();
+    grid_launch_dependents();
+    csr_write_bad(a);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane >> 2, tq = lane & 3;
+    const uint32_t tile = a.tiles - 1u - blockIdx.x, h = blockIdx.y, b = blockIdx.z;     // causal patterns: the long rows first
+    const uint32_t distinct = a.counts[4 * tile], twice = a.counts[4 * tile + 1], base = a.counts[4 * tile + 2], top = a.counts[4 * tile + 3];
+    const uint32_t n = distinct + twice, chunks = (n + KC - 1) / KC;
+    const uint32_t split = MT == 2 ? warp : warp >> 1, rg = MT == 2 ? 0 : warp & 1;        // this warp's chunks and 16-row tile
+    const size_t HD = (size_t)a.H * D;
+    const uint16_t *K = (const uint16_t *)a.K + (size_t)b * a.L * HD + (size_t)h * D, *V = (const uint16_t *)a.V + (size_t)b * a.L * HD + (size_t)h * D;
+    uint8_t *buf = sm + warp * Cfg::warp_bytes;
+
+    // Q as A fragments, straight from memory (once)
+    uint32_t q[MT][D / 16][4];
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const uint32_t row = tile * 32 + rg * 16 + mt * 16 + quad + 8 * e;
+            const uint32_t *src = (const uint32_t *)((const uint16_t *)a.Q + ((size_t)b * a.L + row) * HD + (size_t)h * D) + tq;
+#pragma unroll
+            for (int kk = 0; kk < D / 16; kk++) {
+                q[mt][kk][e] = row < a.L ? __ldg(src + kk * 8) : 0u;
+                q[mt][kk][2 + e] = row < a.L ? __ldg(src + kk * 8 + 4) : 0u;
+            }
+        }
+    float o[MT][DN][4], m[MT][2], l[MT][2];
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++) {
+        m[mt][0] = m[mt][1] = -INFINITY;
+        l[mt][0] = l[mt][1] = 0.f;
+#pragma unroll
+        for (int d = 0; d < DN; d++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) o[mt][d][j] = 0.f;
+    }
+    auto entry = [&](uint32_t c) {
+        const uint32_t i = c * KC + lane;
+        return (KC == 32 || lane < KC) && i < n ? csr_entry(a.entries, base, top, distinct, i) : make_uint2(0u, 0u);
+    };
+    // 16-byte chunk c of row r of a tile sits at chunk c ^ (r % 8) (64-byte rows: c ^ (r / 2 % 4)): no bank twice in a ldmatrix
+    auto place = [](uint32_t r, uint32_t c) { return r * (D * 2) + ((c ^ (D == 32 ? (r >> 1) & 3u : r & 7u)) << 4); };
+    auto issue = [&](const uint2 &e, uint32_t s) {
+        const uint32_t kt = (uint32_t)__cvta_generic_to_shared(buf + s * 2 * Cfg::tile_bytes), vt = kt + Cfg::tile_bytes;
+#pragma unroll
+        for (int i = 0; i < KC * CH / 32; i++) {
+            const uint32_t t = i * 32 + lane, r = t / CH, c = t % CH;
+            const size_t at = (size_t)__shfl_sync(0xffffffffu, e.x, r) * HD + c * 8;
+            const uint32_t off = place(r, c);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(kt + off), "l"(K + at) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(vt + off), "l"(V + at) : "memory");
+        }
+        if (KC == 32 || lane < KC) masks[warp][s][lane % KC] = e.y;
+    };
+    uint2 e_next = make_uint2(0u, 0u);
+    if (split < chunks) {
+        issue(entry(split), 0);
+        if (split + Cfg::SPLITS < chunks) e_next = entry(split + Cfg::SPLITS);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    uint32_t s = 0;
+    for (uint32_t c = split; c < chunks; c += Cfg::SPLITS, s ^= 1) {
+        if (c + Cfg::SPLITS < chunks) {
+            issue(e_next, s ^ 1);
+            if (c + 2 * Cfg::SPLITS < chunks) e_next = entry(c + 2 * Cfg::SPLITS);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        const uint32_t kt = (uint32_t)__cvta_generic_to_shared(buf + s * 2 * Cfg::tile_bytes), vt = kt + Cfg::tile_bytes;
+        // S = Q . K^T
+        float sc[MT][NT][4];
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+            for (int t = 0; t < NT; t++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) sc[mt][t][j] = 0.f;
+#pragma unroll
+        for (int t = 0; t < NT; t += 2)
+#pragma unroll
+            for (int kk = 0; kk < D / 16; kk++) {
+                uint32_t f[4];
+                ldsm(f, kt + place(t * 8 + (lane & 7) + ((lane >> 4) << 3), 2 * kk + ((lane >> 3) & 1)));
+#pragma unroll
+                for (int mt = 0; mt < MT; mt++) {
+                    mma16816<BF16>(sc[mt][t], q[mt][kk], f[0], f[1]);
+                    mma16816<BF16>(sc[mt][t + 1], q[mt][kk], f[2], f[3]);
+                }
+            }
+        // mask: bit `row` of a column's word
+        uint2 mk[NT];
+        uint32_t all = 0xffffffffu;
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+            mk[t] = *(const uint2 *)&masks[warp][s][t * 8 + 2 * tq];
+            all &= mk[t].x & mk[t].y;
+        }
+        if (__any_sync(0xffffffffu, all != 0xffffffffu)) {
+#pragma unroll
+            for (int t = 0; t < NT; t++) {
+                const uint32_t x = mk[t].x >> (rg * 16 + quad), y = mk[t].y >> (rg * 16 + quad);
+#pragma unroll
+                for (int mt = 0; mt < MT; mt++) {
+                    sc[mt][t][0] = (x >> (16 * mt)) & 1u ? sc[mt][t][0] : -INFINITY;
+                    sc[mt][t][1] = (y >> (16 * mt)) & 1u ? sc[mt][t][1] : -INFINITY;
+                    sc[mt][t][2] = (x >> (16 * mt + 8)) & 1u ? sc[mt][t][2] : -INFINITY;
+                    sc[mt][t][3] = (y >> (16 * mt + 8)) & 1u ? sc[mt][t][3] : -INFINITY;
+                }
+            }
+        }
+        // running maximum of every row over its quad of lanes, in units of log2 after the scale
+        float nm[MT][2];
+        bool grow = false;
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                float x = fmaxf(sc[mt][0][2 * e], sc[mt][0][2 * e + 1]);
+#pragma unroll
+                for (int t = 1; t < NT; t++) x = fmaxf(x, fmaxf(sc[mt][t][2 * e], sc[mt][t][2 * e + 1]));
+                x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
+                x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
+                nm[mt][e] = fmaxf(m[mt][e], x * a.scale_log2e);
+                grow |= nm[mt][e] > m[mt][e];
+            }
+        if (__any_sync(0xffffffffu, grow)) {
+#pragma unroll
+            for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const float f = m[mt][e] > -INFINITY ? ex2f(m[mt][e] - nm[mt][e]) : 0.f;
+                    m[mt][e] = nm[mt][e];
+                    l[mt][e] *= f;
+#pragma unroll
+                    for (int d = 0; d < DN; d++) {
+                        o[mt][d][2 * e] *= f;
+                        o[mt][d][2 * e + 1] *= f;
+                    }
+                }
+        }
+        float neg[MT][2];
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+            for (int e = 0; e < 2; e++) neg[mt][e] = m[mt][e] > -INFINITY ? -m[mt][e] : 0.f;
+        // P.V, 16 columns at a time
+#pragma unroll
+        for (int j = 0; j < NT / 2; j++) {
+            uint32_t hi[MT][4], lo[MT][4];
+#pragma unroll
+            for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+                for (int t = 0; t < 2; t++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        const float p0 = ex2f(fmaf(sc[mt][2 * j + t][2 * e], a.scale_log2e, neg[mt][e]));
+                        const float p1 = ex2f(fmaf(sc[mt][2 * j + t][2 * e + 1], a.scale_log2e, neg[mt][e]));
+                        l[mt][e] += p0 + p1;
+                        const uint32_t w = pack16<BF16>(p0, p1);
+                        const float2 r = unpack16<BF16>(w);
+                        hi[mt][2 * t + e] = w;
+                        lo[mt][2 * t + e] = pack16<BF16>(p0 - r.x, p1 - r.y);
+                    }
+#pragma unroll
+            for (int d = 0; d < DN; d += 2) {
+                uint32_t f[4];
+                ldsm_trans(f, vt + place(j * 16 + (lane & 7) + (((lane >> 3) & 1) << 3), d + (lane >> 4)));
+#pragma unroll
+                for (int mt = 0; mt < MT; mt++) {
+                    mma16816<BF16>(o[mt][d], hi[mt], f[0], f[1]);
+                    mma16816<BF16>(o[mt][d + 1], hi[mt], f[2], f[3]);
+                    mma16816<BF16>(o[mt][d], lo[mt], f[0], f[1]);
+                    mma16816<BF16>(o[mt][d + 1], lo[mt], f[2], f[3]);
+                }
+            }
+        }
+        __syncwarp();                                        // the buffer may be filled again
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+    // the warps' outputs, maxima and sums meet in shared memory
+    float *ow = (float *)buf;
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            float sum = l[mt][e];
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            const uint32_t r = mt * 16 + quad + 8 * e;
+            if (tq == 0) ml[warp][r] = make_float2(m[mt][e], sum);
+#pragma unroll
+            for (int d = 0; d < DN; d++) *(float2 *)(ow + r * Cfg::o_stride + d * 8 + 2 * tq) = make_float2(o[mt][d][2 * e], o[mt][d][2 * e + 1]);
+        }
+    __syncthreads();
+    const uint32_t r = threadIdx.x >> 2, row = tile * 32 + r, d0 = (threadIdx.x & 3) * (D / 4);
+    if (row >= a.L) return;
+    const uint32_t w0 = MT == 2 ? 0 : r >> 4, wr = MT == 2 ? r : r & 15;                  // the warps that hold this row
+    constexpr uint32_t WS = MT == 2 ? 1 : 2;
+    float M = -INFINITY, sum = 0.f, f[Cfg::SPLITS];
+#pragma unroll
+    for (int k = 0; k < Cfg::SPLITS; k++) M = fmaxf(M, ml[w0 + k * WS][wr].x);
+#pragma unroll
+    for (int k = 0; k < Cfg::SPLITS; k++) {
+        const float2 x = ml[w0 + k * WS][wr];
+        f[k] = x.x > -INFINITY ? ex2f(x.x - M) : 0.f;
+        sum = fmaf(x.y, f[k], sum);
+    }
+    const float inv = sum > 0.f ? 1.f / (sum + 1e-6f) : 0.f;   // the reference's denominator (ewops.h:93, cuda_kernels.h:1022)
+    uint16_t *dst = (uint16_t *)a.O + ((size_t)b * a.L + row) * HD + (size_t)h * D + d0;
+#pragma unroll
+    for (int c = 0; c < D / 4; c += 8) {
+        float y[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int k = 0; k < Cfg::SPLITS; k++) {
+            const float *src = (const float *)(sm + (w0 + k * WS) * Cfg::warp_bytes) + wr * Cfg::o_stride + d0 + c;
+#pragma unroll
+            for (int j = 0; j < 8; j++) y[j] = fmaf(src[j], f[k], y[j]);
+        }
+        *(uint4 *)(dst + c) = make_uint4(pack16<BF16>(y[0] * inv, y[1] * inv), pack16<BF16>(y[2] * inv, y[3] * inv),
+                                         pack16<BF16>(y[4] * inv, y[5] * inv), pack16<BF16>(y[6] * inv, y[7] * inv));
+    }
+}
+
+template <bool BF16, int D>
+static int launch_csr_tile(cudaStream_t s, const CsrTileArgs &a, uint32_t B)
+{
+    static DeviceOnce once;
+    const int dev = current_device();
+    if (!once.done(dev)) {
+        if (cudaFuncSetAttribute(csr_tile_kernel<BF16, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CsrCfg<D>::smem) != cudaSuccess)
+            return fail("sfb_csr_attention: cannot reserve %zu bytes of shared memory", CsrCfg<D>::smem);
+        once.mark(dev);
+    }
+    launch_overlapped(csr_tile_kernel<BF16, D>, dim3(a.tiles, a.H, B), dim3(128), CsrCfg<D>::smem, s, a);
+    return check_launch("sfb_csr_attention");
+}
+
+// entries of 8 bytes, one per element, then four counts and a bad-column count per tile of 32 rows
+static size_t csr_workspace(uint64_t nnz, uint32_t L) { return nnz * 8 + (size_t)((L + 31) / 32) * 5 * sizeof(uint32_t); }
+
+static int csr_attention_planned(cudaStream_t s, const int32_t *rowptr, const int32_t *colidx, uint32_t nnz, const void *q, const void *k,
+                                 const void *v, void *o, int dtype, uint32_t B, uint32_t L, uint32_t H, uint32_t d, float scale, uint32_t *bad,
+                                 void *workspace)
+{
+    const uint32_t tiles = (L + 31) / 32;
+    uint2 *entries = (uint2 *)workspace;
+    uint32_t *counts = (uint32_t *)(entries + nnz);
+    static DeviceOnce once;
+    const int dev = current_device();
+    if (!once.done(dev)) {
+        if (cudaFuncSetAttribute(csr_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kPlanMaxL * sizeof(uint32_t))) != cudaSuccess)
+            return fail("sfb_csr_attention: cannot reserve %u bytes of shared memory", kPlanMaxL * 4u);
+        once.mark(dev);
+    }
+    launch_overlapped(csr_plan_kernel, dim3(tiles), dim3(kPlanThreads), L * sizeof(uint32_t), s, rowptr, colidx, L, nnz, entries, counts, counts + 4 * tiles);
+    const CsrTileArgs a = {entries, counts, counts + 4 * tiles, q, k, v, o, L, H, tiles, B * H, scale * 1.4426950408889634f, bad};
+    if (dtype == SFB_F32) return csr_tile_f32(s, a, B, d);
+#define CSR_TILE(BF) return d == 32 ? launch_csr_tile<BF, 32>(s, a, B) : d == 64 ? launch_csr_tile<BF, 64>(s, a, B) : launch_csr_tile<BF, 128>(s, a, B)
+    if (dtype == SFB_BF16) CSR_TILE(true);
+    CSR_TILE(false);
+#undef CSR_TILE
+}
+
 int csr_from_layout(cudaStream_t s, const uint8_t *layout, uint32_t nb, uint32_t bs, int32_t *rowptr, int32_t *colidx)
 {
     csr_from_layout_kernel<<<nb, 256, nb * sizeof(uint32_t), s>>>(layout, nb, bs, rowptr, colidx);
@@ -286,17 +575,16 @@ int csr_attention(cudaStream_t s, const int32_t *rowptr, const int32_t *colidx, 
     if (bad) cudaMemsetAsync(bad, 0, sizeof(uint32_t), s);
     const dim3 grid((L + 3) / 4, B, H);
     const float sl = scale * 1.4426950408889634f;
-    const int lanes = 4;   // lanes per key; the one- and two-lane kernels are kept for comparison
-#define CSR_LAUNCH(DTV, DV)                                                                                            \
-    do {                                                                                                               \
-        if (lanes == 4) csr_attention_split_kernel<DTV, DV, 4><<<grid, 128, 0, s>>>(rowptr, colidx, q, k, v, o, L, H, sl, bad); \
-        else if (lanes == 2) csr_attention_split_kernel<DTV, DV, 2><<<grid, 128, 0, s>>>(rowptr, colidx, q, k, v, o, L, H, sl, bad); \
-        else csr_attention_kernel<DTV, DV><<<grid, 128, 0, s>>>(rowptr, colidx, q, k, v, o, L, H, sl, bad);             \
+#define CSR_BY_D(DTV)                                                                                                               \
+    do {                                                                                                                            \
+        if (d == 32) csr_attention_split_kernel<DTV, 32, 4><<<grid, 128, 0, s>>>(rowptr, colidx, q, k, v, o, L, H, sl, bad);         \
+        else if (d == 64) csr_attention_split_kernel<DTV, 64, 4><<<grid, 128, 0, s>>>(rowptr, colidx, q, k, v, o, L, H, sl, bad);    \
+        else csr_attention_split_kernel<DTV, 128, 4><<<grid, 128, 0, s>>>(rowptr, colidx, q, k, v, o, L, H, sl, bad);                \
     } while (0)
-#define CSR_BY_D(DTV) if (d == 32) CSR_LAUNCH(DTV, 32); else if (d == 64) CSR_LAUNCH(DTV, 64); else CSR_LAUNCH(DTV, 128)
-    if (dtype == SFB_F32) { CSR_BY_D(SFB_F32); } else if (dtype == SFB_BF16) { CSR_BY_D(SFB_BF16); } else { CSR_BY_D(SFB_F16); }
+    if (dtype == SFB_F32) CSR_BY_D(SFB_F32);
+    else if (dtype == SFB_BF16) CSR_BY_D(SFB_BF16);
+    else CSR_BY_D(SFB_F16);
 #undef CSR_BY_D
-#undef CSR_LAUNCH
     return check_launch("sfb_csr_attention");
 }
 
@@ -311,17 +599,42 @@ extern "C" int sfb_csr_from_layout(sfb_stream_t stream, const uint8_t *layout, u
     return sfb::csr_from_layout((cudaStream_t)stream, layout, nb, block_size, rowptr, colidx);
 }
 
-extern "C" int sfb_csr_attention(sfb_stream_t stream, const int32_t *rowptr, const int32_t *colidx, const void *q, const void *k,
-                                 const void *v, void *o, int dtype, uint32_t batch_dim, uint32_t seq_len, uint32_t head_dim,
-                                 uint32_t state_dim, float scale, uint32_t *bad_columns)
+static int csr_check(const char *who, const int32_t *rowptr, const int32_t *colidx, const void *q, const void *k, const void *v, void *o,
+                     int dtype, uint32_t batch_dim, uint32_t head_dim, uint32_t state_dim)
 {
-    const char *who = "sfb_csr_attention";
     SFB_REQUIRE(rowptr && colidx && q && k && v && o, "%s: NULL pointer", who);
     SFB_REQUIRE(dtype == SFB_F32 || dtype == SFB_BF16 || dtype == SFB_F16, "%s: unknown dtype", who);
     SFB_REQUIRE(state_dim == 32 || state_dim == 64 || state_dim == 128, "%s: state_dim %u not supported (32, 64 or 128)", who, state_dim);
     SFB_REQUIRE(batch_dim >= 1 && batch_dim <= 65535 && head_dim >= 1 && head_dim <= 65535, "%s: bad batch_dim=%u head_dim=%u", who, batch_dim, head_dim);
     SFB_REQUIRE((((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)o) & 15) == 0, "%s: q, k, v, o must be 16-byte aligned", who);
+    return 0;
+}
+
+extern "C" int sfb_csr_attention(sfb_stream_t stream, const int32_t *rowptr, const int32_t *colidx, const void *q, const void *k,
+                                 const void *v, void *o, int dtype, uint32_t batch_dim, uint32_t seq_len, uint32_t head_dim,
+                                 uint32_t state_dim, float scale, uint32_t *bad_columns)
+{
+    if (csr_check("sfb_csr_attention", rowptr, colidx, q, k, v, o, dtype, batch_dim, head_dim, state_dim)) return 1;
     if (seq_len == 0) { sfb::clear_error(); return 0; }
     return sfb::csr_attention((cudaStream_t)stream, rowptr, colidx, q, k, v, o, dtype, batch_dim, seq_len, head_dim, state_dim, scale,
                               bad_columns);
+}
+
+extern "C" uint64_t sfb_csr_workspace(uint32_t nnz, uint32_t seq_len)
+{
+    return seq_len <= sfb::kPlanMaxL ? (uint64_t)sfb::csr_workspace(nnz, seq_len) : 0;
+}
+
+extern "C" int sfb_csr_attention_planned(sfb_stream_t stream, const int32_t *rowptr, const int32_t *colidx, uint32_t nnz, const void *q,
+                                         const void *k, const void *v, void *o, int dtype, uint32_t batch_dim, uint32_t seq_len,
+                                         uint32_t head_dim, uint32_t state_dim, float scale, uint32_t *bad_columns, void *workspace)
+{
+    const char *who = "sfb_csr_attention_planned";
+    if (csr_check(who, rowptr, colidx, q, k, v, o, dtype, batch_dim, head_dim, state_dim)) return 1;
+    SFB_REQUIRE(workspace && ((uintptr_t)workspace & 15) == 0, "%s: workspace is NULL or not 16-byte aligned", who);
+    SFB_REQUIRE(seq_len <= sfb::kPlanMaxL, "%s: seq_len %u > %u", who, seq_len, sfb::kPlanMaxL);
+    SFB_REQUIRE(nnz < (1u << 31), "%s: too many elements", who);
+    if (seq_len == 0) { sfb::clear_error(); return 0; }
+    return sfb::csr_attention_planned((cudaStream_t)stream, rowptr, colidx, nnz, q, k, v, o, dtype, batch_dim, seq_len, head_dim, state_dim, scale,
+                                      bad_columns, workspace);
 }

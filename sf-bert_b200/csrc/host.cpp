@@ -17,7 +17,7 @@ namespace {
 // ---- the library -----------------------------------------------------------------------------------------------------
 #define SFB_FUNCTIONS(X)                                                                                                 \
     X(sfb_last_error) X(sfb_bst_sgemm_nt) X(sfb_masked_softmax) X(sfb_bst_sgemm_xn) X(sfb_masked_softmax_grad) X(sfb_linear) \
-    X(sfb_linear_nt) X(sfb_linear_residual) X(sfb_embedding) X(sfb_csr_attention) X(sfb_rowdot) X(sfb_fused_sddmm_softmax_grad)                  \
+    X(sfb_linear_nt) X(sfb_linear_residual) X(sfb_embedding) X(sfb_csr_attention) X(sfb_csr_attention_planned) X(sfb_csr_workspace) X(sfb_rowdot) X(sfb_fused_sddmm_softmax_grad)                  \
     X(sfb_fused_sddmm_softmax) X(sfb_fused_attention) X(sfb_fused_attention_slice) X(sfb_bias_residual_layernorm)         \
     X(sfb_bias_gelu) X(sfb_attention_backward)
 struct Lib {
@@ -303,6 +303,16 @@ FUNCTION(py_csr_attention, 6)
     require(rowptr.scalar_type() == at::kInt && colidx.scalar_type() == at::kInt && rowptr.numel() == q.size(1) + 1,
             "rowptr and colidx must be int32, rowptr of L + 1 elements");
     at::Tensor o = alike(q), bad = empty({1}, at::kInt, q);
+    const int64_t nnz = colidx.numel();
+    const uint64_t bytes = nnz < (1ll << 31) ? L.sfb_csr_workspace((uint32_t)nnz, (uint32_t)q.size(1)) : 0;
+    if (bytes) {
+        at::Tensor ws = empty({(int64_t)bytes}, at::kByte, q);
+        check(L.sfb_csr_attention_planned(stream(), (const int32_t *)ptr(rowptr), (const int32_t *)ptr(colidx), (uint32_t)nnz, ptr(q),
+                                          ptr(tensor(a[1])), ptr(tensor(a[2])), ptr(o), tag(q), (uint32_t)q.size(0), (uint32_t)q.size(1),
+                                          (uint32_t)q.size(2), (uint32_t)q.size(3), (float)number(a[5]), (uint32_t *)ptr(bad), ptr(ws)));
+        Ref r(wrap(o)), n(wrap(bad));
+        return PyTuple_Pack(2, r.o, n.o);
+    }
     check(L.sfb_csr_attention(stream(), (const int32_t *)ptr(rowptr), (const int32_t *)ptr(colidx), ptr(q), ptr(tensor(a[1])), ptr(tensor(a[2])),
                               ptr(o), tag(q), (uint32_t)q.size(0), (uint32_t)q.size(1), (uint32_t)q.size(2), (uint32_t)q.size(3),
                               (float)number(a[5]), (uint32_t *)ptr(bad)));

@@ -64,3 +64,45 @@ def test_csr_columns_outside_the_sequence_are_counted_not_read(sfb):
     o, bad = sfb.csr_attention(q, q, q, rowptr, colidx, 1.0)
     assert int(bad.item()) == 2
     assert torch.allclose(o, torch.ones_like(o), atol=1e-4)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("L,d", [(1, 64), (31, 32), (33, 128), (64, 64), (517, 64), (530, 128), (545, 32)])
+def test_csr_tiles_against_oracle(sfb, oracle, dtype, L, d):
+    """Tiles of 32 rows: a single row, ragged last tiles, lists shorter and longer than a chunk, rows that name a column
+    twice (it counts twice), an empty tile, and the call without a workspace."""
+    B, H = 2, 2
+    rng = np.random.RandomState(L)
+    rows = []
+    for i in range(L):
+        n = 0 if 96 <= i < 128 else int(rng.randint(0, min(L, 300) + 1))
+        r = rng.choice(L, size=n, replace=False)
+        if n and i % 4 == 0:
+            r = np.r_[r, r[:3]]
+        rows.append(r.astype(np.int32))
+    rows[0] = np.array([0], np.int32)
+    rowptr = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+    colidx = np.concatenate(rows).astype(np.int32)
+    q, k, v = (torch.from_numpy(oracle.fill_normal((B, L, H, d), 530 + i)).cuda().to(TD[dtype]) for i in range(3))
+    rp, ci = torch.from_numpy(rowptr).cuda(), torch.from_numpy(colidx).cuda()
+    o, bad = sfb.csr_attention(q, k, v, rp, ci, 0.125)
+    assert int(bad.item()) == 0
+    plain = torch.empty_like(q)
+    p = lambda t: sfb.C.c_void_p(t.data_ptr())
+    sfb._check(sfb.lib.sfb_csr_attention(sfb._stream(), p(rp), p(ci), p(q), p(k), p(v), p(plain), sfb.dtype_tag(q), B, L, H, d, 0.125, p(bad)))
+    want = oracle.csr_attention(q.float().cpu().numpy(), k.float().cpu().numpy(), v.float().cpu().numpy(), rowptr, colidx, np.float32(0.125))
+    for got in (o, plain):
+        assert np.abs(got.float().cpu().numpy() - want).max() <= (1e-5 if dtype == "f32" else 2e-2 * np.abs(want).max())
+    if dtype != "f32":   # 16-bit outputs of the two agree to their last bit nearly everywhere: nothing between them is rounded more
+        assert float((o != plain).float().mean()) < 0.02
+
+
+def test_csr_bad_columns_are_counted_per_batch_and_head(sfb):
+    L, d = 70, 64
+    q = torch.ones(2, L, 3, d, device="cuda", dtype=torch.bfloat16)
+    rowptr = torch.arange(0, 2 * L + 1, 2, dtype=torch.int32, device="cuda")
+    colidx = torch.tensor([0, 1] * L, dtype=torch.int32, device="cuda")
+    colidx[3], colidx[100], colidx[139] = -5, L, 1 << 30
+    o, bad = sfb.csr_attention(q, q, q, rowptr, colidx, 1.0)
+    assert int(bad.item()) == 3 * 2 * 3
+    assert torch.equal(o, q)
