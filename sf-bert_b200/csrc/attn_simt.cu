@@ -231,7 +231,8 @@ __global__ void __launch_bounds__(BS * BS / 8 / SPLIT, (NB > 0 && SPLIT > 1 && B
     constexpr int LPR = BS / 8;  // lanes per query row
     grid_dependency_wait();
     grid_launch_dependents();
-    const uint32_t i = blockIdx.x / SPLIT, b = blockIdx.y, h = blockIdx.z;
+    // last (batch, head) first: the scores were written in ascending order, and the last of them are still in L2
+    const uint32_t i = blockIdx.x / SPLIT, b = gridDim.y - 1 - blockIdx.y, h = gridDim.z - 1 - blockIdx.z;
     const uint2 *nn = lut + (size_t)h * p.lut_stride;
     const uint2 head = nn[i];
     const uint32_t off = head.x, cnt = head.y;
@@ -426,7 +427,8 @@ __global__ void __launch_bounds__(BS * BS / 8 / SPLIT) softmax_grad_kernel(const
     constexpr int LPR = BS / 8;  // lanes per query row
     grid_dependency_wait();
     grid_launch_dependents();
-    const uint32_t i = blockIdx.x / SPLIT, b = blockIdx.y, h = blockIdx.z;
+    // last (batch, head) first, as the softmax: dy was written in ascending order
+    const uint32_t i = blockIdx.x / SPLIT, b = gridDim.y - 1 - blockIdx.y, h = gridDim.z - 1 - blockIdx.z;
     const uint2 *nn = lut + (size_t)h * p.lut_stride;
     const uint2 head = nn[i];
     const uint32_t off = head.x, cnt = head.y;

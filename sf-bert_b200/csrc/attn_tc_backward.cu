@@ -267,9 +267,14 @@ backward_tc_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_consta
             if (id != kNoItem) {
                 const bool first = id < first_items;
                 const uint32_t rest = first ? id : id - first_items, per = first ? first_pairs : p.npairs - first_pairs;
-                bh = rest / per;
-                const uint32_t pair = rest - bh * per + (first ? 0 : first_pairs);
-                const uint2 *lut = p.lut + (size_t)(bh % p.H) * p.lut_stride;
+                // head by head as the product before this call walks P; the row kernel backwards, the column kernel forwards again,
+                // so that each starts with the blocks the kernel before it left in L2
+                uint32_t at = rest / per;
+                const uint32_t pair = rest - at * per + (first ? 0 : first_pairs);
+                if (!COL) at = p.B * p.H - 1 - at;
+                const uint32_t h = at / p.B, b = at - h * p.B;
+                bh = b * p.H + h;
+                const uint2 *lut = p.lut + (size_t)h * p.lut_stride;
                 pick_pair(lut, pair, p.nb, p.blocks, lane, own);
                 n = warp_union(lut, own, st->lists[slot], lane);
                 if (n == kNoItem) {                           // more blocks than the caller's maximum: recorded, zeros written

@@ -442,7 +442,8 @@ fused_p_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constan
     float2 *comb = (float2 *)(st + 1);         // [column half][row]: (max, sum) after sweep 1
 
     const uint32_t warp = uniform_warp(), lane = threadIdx.x & 31;
-    const uint32_t pair = blockIdx.x, b = blockIdx.y, h = blockIdx.z;
+    // last (batch, head) first: the product that reads the probabilities next starts with the ones still in L2
+    const uint32_t pair = blockIdx.x, b = gridDim.y - 1 - blockIdx.y, h = gridDim.z - 1 - blockIdx.z;
     const uint32_t L = p.nb * 64;
     const uint2 *nn = p.nn_lut + (size_t)h * p.lut_stride;
     volatile uint32_t *abort_flag = &st->abort_flag;

@@ -195,12 +195,19 @@ __global__ void __launch_bounds__(kPlanThreads) csr_plan_kernel(const int32_t *_
     __syncthreads();
     for (uint32_t r = warp; r < rows; r += kPlanThreads / 32) {
         const int32_t lo = max(rowptr[row0 + r], 0), hi = (int32_t)min((uint32_t)max(rowptr[row0 + r + 1], 0), nnz);
-        for (int32_t e = lo + (int32_t)lane; e < hi; e += 32) {
-            const int32_t j = __ldg(colidx + e);
-            if (j < 0 || (uint32_t)j >= L) { atomicAdd(&n_bad, 1u); continue; }
-            if (atomicOr(&mask[j], 1u << r) & (1u << r)) {
-                const uint32_t at = top - 1u - atomicAdd(&n_twice, 1u);      // from the end of the tile's share backwards
-                if (at >= base && at < nnz) entries[at] = make_uint2((uint32_t)j, 1u << r);
+        for (int32_t e0 = lo + (int32_t)lane; e0 < hi; e0 += 32 * 8) {
+            int32_t col[8];                                  // eight reads on their way at once
+#pragma unroll
+            for (int u = 0; u < 8; u++) col[u] = e0 + 32 * u < hi ? __ldg(colidx + e0 + 32 * u) : 0;
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                if (e0 + 32 * u >= hi) break;
+                const int32_t j = col[u];
+                if (j < 0 || (uint32_t)j >= L) { atomicAdd(&n_bad, 1u); continue; }
+                if (atomicOr(&mask[j], 1u << r) & (1u << r)) {
+                    const uint32_t at = top - 1u - atomicAdd(&n_twice, 1u);      // from the end of the tile's share backwards
+                    if (at >= base && at < nnz) entries[at] = make_uint2((uint32_t)j, 1u << r);
+                }
             }
         }
     }
