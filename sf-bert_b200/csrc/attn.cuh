@@ -29,7 +29,7 @@ int simt_fused_attention(cudaStream_t s, const void *nn_lut, const void *q, cons
 // tcgen05 kernels (attn_tc.cu)
 bool tc_fused_attention_supported(int dtype, uint32_t bs, const AttnDims &p, float scale, uint32_t max_lut);
 int tc_fused_attention(cudaStream_t s, const void *nn_lut, const void *q, const void *k, const void *v, void *o,
-                       const void *mask, int dtype, const AttnDims &p, float scale);
+                       const void *mask, int dtype, const AttnDims &p, float scale, uint32_t max_lut);
 int tc_status_fused(uint32_t *out);
 int tc_status_clear_fused();
 bool tc_sddmm_supported(int ab_dtype, uint32_t bs, const AttnDims &p, const void *a, const void *b, const void *c);

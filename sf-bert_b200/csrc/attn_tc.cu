@@ -57,11 +57,14 @@ struct StreamState {
     uint64_t list_ready[2], list_free[2];
     uint64_t stage_full, stage_free;
     uint32_t list_n[2];
+    uint64_t part_ready, part_free;     // split items: this stream's share is complete / has been taken over
+    uint32_t part_steps;
     int32_t store_x, store_y;   // where the staged output tile goes (y < 0: the rows were written directly)
 };
 
 struct SharedState {
     StreamState st[kStreams];
+    float2 part[kStreams][128];         // split items: (reference maximum, sum) of every row
     uint64_t drained[kStreams];
     uint32_t tmem_base, abort_flag;
 };
@@ -81,7 +84,7 @@ struct Params {
     void *O;
     uint32_t B, H, nb, npairs, n_items, lut_stride, mask_stride;
     uint32_t o_pitch;      // elements between consecutive rows of O
-    uint32_t cta_first;    // order in which a round's items are dealt to the CTAs' streams (item_id)
+    uint32_t deal;         // how items are dealt to the CTAs' streams (item_id): kDealNear, kDealSpread, kDealSplit
     float scale_log2e;
 };
 
@@ -102,15 +105,18 @@ __device__ __forceinline__ Item decode_item(uint32_t id, const Params &p)
     it.h = bh % p.H;
     return it;
 }
-// round k, stream s of this CTA.  Long launches: a CTA's three streams take neighbouring items (neighbouring row pairs
-// of one head).  Launches of only a few rounds (p.cta_first): within a round the items go to stream 0 of every CTA
+enum { kDealNear = 0, kDealSpread = 1, kDealSplit = 2 };
+// round k, stream s of this CTA.  Split (launches with hardly more items than SMs, long rows): the three streams share every
+// item of their CTA, each walking every third entry of its union, and meet in the epilogue of stream 0.  Long launches: a CTA's three streams take neighbouring items (neighbouring row pairs
+// of one head).  Launches of only a few rounds (kDealSpread): within a round the items go to stream 0 of every CTA
 // first, then to stream 1, ...: in the last, partial round a CTA then runs fewer streams at once instead of some CTAs
 // running three and others none, and a stream with the SM to itself finishes its item sooner (the 24-layer stack with
 // 512 items per launch: 973 -> 1036 sequences/s).  On long launches with items of very different length (BigBird)
 // that order measured 8 % slower, so it is kept to the launches that are all tail.
 __device__ __forceinline__ uint32_t item_id(uint32_t k, uint32_t s, const Params &p)
 {
-    return p.cta_first ? (k * kStreams + s) * gridDim.x + blockIdx.x : (k * gridDim.x + blockIdx.x) * kStreams + s;
+    if (p.deal == kDealSplit) return k * gridDim.x + blockIdx.x;
+    return p.deal == kDealSpread ? (k * kStreams + s) * gridDim.x + blockIdx.x : (k * gridDim.x + blockIdx.x) * kStreams + s;
 }
 
 template <bool BF16>
@@ -345,6 +351,8 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
             mbar_init(&st->o_free, 128);
             mbar_init(&st->stage_full, 128);
             mbar_init(&st->stage_free, 1);
+            mbar_init(&st->part_ready, 4);
+            mbar_init(&st->part_free, 4);
             mbar_init(&sh->drained[s], 1);
         }
         sh->abort_flag = 0;
@@ -383,6 +391,20 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
                     // a row pair that is too long for this kernel: recorded, and the pair's rows are written as zeros
                     if (lane == 0) atomicCAS(&g_status, 0u, (9u << 24) | (blockIdx.x & 0xffffffu));
                     n = 0;
+                }
+                if (p.deal == kDealSplit) {
+                    // this stream's share: entries s, s + 3, ... moved to the front (a group of 32 reads before it writes, and what
+                    // it writes lies before what the groups after it read)
+                    UEntry *ent = lists + (s * 2 + slot) * kMaxU;
+                    const uint32_t share = n > s ? (n - s + kStreams - 1) / kStreams : 0;
+                    for (uint32_t i = 0; i < share; i += 32) {
+                        UEntry e = {};
+                        if (i + lane < share) e = ent[(i + lane) * kStreams + s];
+                        __syncwarp();
+                        if (i + lane < share) ent[i + lane] = e;
+                        __syncwarp();
+                    }
+                    n = share;
                 }
                 if (lane == 0) {
                     st->list_n[slot] = n;
@@ -472,57 +494,109 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
         // The epilogue of an item: O / row sum -> the stream's staging tile -> (value producer) one TMA store per row pair,
         // 16 accumulator columns at a time.  (Running it behind the next item's first softmax step, so that nothing waits
         // for the item's last O product, was built and measured: slower.)
-        auto epilogue = [&](bool has_data, uint32_t e_id, uint64_t l0, uint64_t l1) -> bool {
+        auto epilogue = [&](uint32_t k, uint32_t T, uint32_t e_id, float m_used, uint64_t l0, uint64_t l1) -> bool {
             const Item e_it = decode_item(e_id, p);
             const uint32_t e_pair = e_it.pair, e_b = e_it.b, e_h = e_it.h;
             const bool has_row1 = e_pair * 2 + 1 < p.nb;
-            float inv = 0.f;
-            if (has_data) {
+            float a0, a1, a2, a3;
+            up64(l0, a0, a1);
+            up64(l1, a2, a3);
+            float lsum = (a0 + a1) + (a2 + a3);
+            const bool split = p.deal == kDealSplit, mine = !split || s == 0;
+            float fac[kStreams] = {1.f, 0.f, 0.f};         // what the streams' accumulators are multiplied by, and their steps
+            uint32_t steps[kStreams] = {T, 0, 0};
+            if (T > 0) {
                 if (!mbar_wait_warp(&st->o_final, kq & 1, abort_flag, 10)) return false;
                 tcgen05_fence_after();
-                float a0, a1, a2, a3;
-                up64(l0, a0, a1);
-                up64(l1, a2, a3);
-                const float lsum = (a0 + a1) + (a2 + a3);
-                inv = lsum > 0.f ? 1.f / lsum : 0.f;
+                kq++;
+            }
+            if (!mine) {
+                // hand this share to stream 0, whose warps read the accumulator straight out of TMEM
+                if (k >= 1 && !mbar_wait_warp(&st->part_free, (k - 1) & 1, abort_flag, 16)) return false;
+                sh->part[s][r] = make_float2(m_used, lsum);
+                if (r == 0) st->part_steps = T;
+                tcgen05_fence_before();
+                mbar_arrive_warp(&st->part_ready, lane);
+            } else {
+                if (split) {
+                    float M = m_used;
+                    float2 part[kStreams];
+#pragma unroll
+                    for (int j = 1; j < kStreams; j++) {
+                        if (!mbar_wait_warp(&sh->st[j].part_ready, k & 1, abort_flag, 17)) return false;
+                        part[j] = sh->part[j][r];
+                        steps[j] = sh->st[j].part_steps;
+                        M = fmaxf(M, part[j].x);
+                    }
+                    tcgen05_fence_after();
+                    fac[0] = m_used > -INFINITY ? ex2_approx(m_used - M) : 0.f;
+                    lsum *= fac[0];
+#pragma unroll
+                    for (int j = 1; j < kStreams; j++) {
+                        fac[j] = part[j].x > -INFINITY ? ex2_approx(part[j].x - M) : 0.f;
+                        lsum = fmaf(part[j].y, fac[j], lsum);
+                    }
+                }
+                const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
+#pragma unroll
+                for (int j = 0; j < kStreams; j++) fac[j] *= inv;
             }
             // the previous store out of the staging tile has been read out of shared memory
             if (n_epi >= 1 && !mbar_wait_warp(&st->stage_free, (n_epi - 1) & 1, abort_flag, 13)) return false;
-            uint8_t *orow = ostage + r * 128;
-            uint16_t *dst = (uint16_t *)p.O + ((size_t)e_b * L + (size_t)e_pair * 128 + r) * (size_t)p.o_pitch + (size_t)e_h * 64;
+            if (mine) {
+                uint8_t *orow = ostage + r * 128;
+                uint16_t *dst = (uint16_t *)p.O + ((size_t)e_b * L + (size_t)e_pair * 128 + r) * (size_t)p.o_pitch + (size_t)e_h * 64;
 #pragma unroll
-            for (int c0 = 0; c0 < 64; c0 += 16) {
-                uint32_t oc[16];
-                if (has_data) {
-                    TMEM_LD_16((oc), t_o + c0);
-                    tmem_wait_ld();
-                } else {
+                for (int c0 = 0; c0 < 64; c0 += 16) {
+                    uint32_t oc[16];
+                    if (T > 0) {
+                        TMEM_LD_16((oc), t_o + c0);
+                        tmem_wait_ld();
 #pragma unroll
-                    for (int c = 0; c < 16; c++) oc[c] = 0u;      // a row pair without key blocks gives zeros (blocksparse.h:949-962)
+                        for (int c = 0; c < 16; c++) oc[c] = __float_as_uint(__uint_as_float(oc[c]) * fac[0]);
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 16; c++) oc[c] = 0u;  // a row pair without key blocks gives zeros (blocksparse.h:949-962)
+                    }
+                    if (split) {
+#pragma unroll
+                        for (int j = 1; j < kStreams; j++)
+                            if (steps[j]) {
+                                uint32_t od[16];
+                                TMEM_LD_16((od), t_o + j * kStreamCols + c0);
+                                tmem_wait_ld();
+#pragma unroll
+                                for (int c = 0; c < 16; c++) oc[c] = __float_as_uint(fmaf(__uint_as_float(od[c]), fac[j], __uint_as_float(oc[c])));
+                            }
+                    }
+                    uint32_t w[8];
+#pragma unroll
+                    for (int j = 0; j < 8; j++) w[j] = pack_pair<BF16>(__uint_as_float(oc[2 * j]), __uint_as_float(oc[2 * j + 1]));
+                    if (has_row1) {
+                        // 16-byte chunk c of row r sits at chunk c ^ (r % 8): the tensor map's 128-byte swizzle
+                        const int ch = c0 >> 3;
+                        *(uint4 *)(orow + (((ch) ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+                        *(uint4 *)(orow + (((ch + 1) ^ (r & 7)) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
+                    } else if (half == 0) {
+                        // an odd number of block-rows: the last pair has 64 rows only, written directly
+                        *(uint4 *)(dst + c0) = make_uint4(w[0], w[1], w[2], w[3]);
+                        *(uint4 *)(dst + c0 + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+                    }
                 }
-                uint32_t w[8];
-#pragma unroll
-                for (int j = 0; j < 8; j++) w[j] = pack_pair<BF16>(__uint_as_float(oc[2 * j]) * inv, __uint_as_float(oc[2 * j + 1]) * inv);
-                if (has_row1) {
-                    // 16-byte chunk c of row r sits at chunk c ^ (r % 8): the tensor map's 128-byte swizzle
-                    const int ch = c0 >> 3;
-                    *(uint4 *)(orow + (((ch) ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-                    *(uint4 *)(orow + (((ch + 1) ^ (r & 7)) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
-                } else if (half == 0) {
-                    // an odd number of block-rows: the last pair has 64 rows only, written directly
-                    *(uint4 *)(dst + c0) = make_uint4(w[0], w[1], w[2], w[3]);
-                    *(uint4 *)(dst + c0 + 8) = make_uint4(w[4], w[5], w[6], w[7]);
-                }
-            }
-            if (has_data) {
                 tcgen05_fence_before();
-                mbar_arrive(&st->o_free);              // the next item's first O product may overwrite the accumulator
-                kq++;
+                if (T > 0) mbar_arrive(&st->o_free);       // the next item's first O product may overwrite the accumulator
+                if (split) {
+#pragma unroll
+                    for (int j = 1; j < kStreams; j++) {
+                        if (steps[j]) mbar_arrive(&sh->st[j].o_free);
+                        mbar_arrive_warp(&sh->st[j].part_free, lane);
+                    }
+                }
+                if (has_row1) fence_proxy_async();
             }
-            if (has_row1) fence_proxy_async();
             if (r == 0) {
                 st->store_x = (int32_t)(e_h * 64);
-                st->store_y = has_row1 ? (int32_t)(e_b * L + e_pair * 128) : -1;
+                st->store_y = mine && has_row1 ? (int32_t)(e_b * L + e_pair * 128) : -1;
             }
             mbar_arrive(&st->stage_full);      // the value producer issues the store and hands the tile back
             n_epi++;
@@ -539,9 +613,16 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
             const uint32_t item_h = HAS_MASK ? decode_item(id, p).h : 0u;
             float m_used = -INFINITY;
             uint64_t lacc0 = 0, lacc1 = 0;                 // four partial row sums (two packed pairs)
+            // the element mask of this row in block t: fetched a step ahead (its latency was part of every step)
+            auto mask_word = [&](uint32_t t) -> uint64_t {
+                return (list[t].col_flags >> (30 + half)) & 1 ? __ldg(p.mask + (size_t)item_h * p.mask_stride + (size_t)list[t].blk[half] * 64 + (r & 63)) : ~0ull;
+            };
+            uint64_t mw_next = HAS_MASK && T > 0 ? mask_word(0) : ~0ull;
             for (uint32_t t = 0; t < T; t++) {
                 const uint32_t gg = g + t, b2 = gg & 1;
                 const uint32_t t_s = tbase + 32 * b2, t_p = tbase + 64 * b2;
+                const uint64_t mw = mw_next;
+                if (HAS_MASK && t + 1 < T) mw_next = mask_word(t + 1);
                 if (!mbar_wait_warp(&st->qk_done[b2], (gg >> 1) & 1, abort_flag, 6)) { alive = false; break; }
                 tcgen05_fence_after();
                 TMEM_LD_32((sr), t_s);
@@ -552,10 +633,11 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
                 const bool mine = (list[t].col_flags >> (30 + half)) & 1;     // the same for the whole warp
                 if (mine) {
                     if (HAS_MASK) {
-                        const uint64_t mw = p.mask[(size_t)item_h * p.mask_stride + (size_t)list[t].blk[half] * 64 + (r & 63)];
+                        if (!__all_sync(0xffffffffu, mw == ~0ull)) {
 #pragma unroll
-                        for (int c = 0; c < 64; c++)
-                            if (!((mw >> c) & 1)) sr[c] = 0xff800000u;
+                            for (int c = 0; c < 64; c++)
+                                if (!((mw >> c) & 1)) sr[c] = 0xff800000u;
+                        }
                     }
                     float m4[4];
 #pragma unroll
@@ -632,7 +714,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
             }
             if (!alive) break;
             g += T;
-            if (!epilogue(T > 0, id, lacc0, lacc1)) break;
+            if (!epilogue(k, T, id, m_used, lacc0, lacc1)) break;
             __syncwarp();
             if (lane == 0) mbar_arrive(&st->list_free[k & 1]);
         }
@@ -670,8 +752,26 @@ bool tc_fused_attention_supported(int dtype, uint32_t bs, const AttnDims &p, flo
            longest <= (uint64_t)tc::kMaxU && (uint64_t)p.B * p.nb_a * 64 < (1ull << 31) && p.nb_a < (1u << 30);
 }
 
+// How a launch deals its items.  From four rounds of items up: near.  From one to four: spread.  Within one round the split
+// deal may finish sooner, estimated in microseconds: a step takes a stream that has its SM to itself 0.77, two streams 1.06
+// and three 1.45; split, a third of a CTA's items' steps at the rate of three streams plus 1.2 per item for the shares'
+// meeting, one item after the other.  Rows longer than the mean finish last either way.  Measured (bf16, launches in
+// sequence), spread against split: 128 items of 16 steps 19.4 / 16.2 us, 64 of 32 31.9 / 23.3, BigBird's 128 (11 steps on
+// average, 64 at most) 56.8 / 35.1; 252 of 7 on average 17.5 / 18.1 and 384 of 16 29.8 / 37.6, which stay spread.
+static uint32_t choose_deal(uint32_t n_items, double mean, uint32_t longest, uint32_t sms)
+{
+    using namespace tc;
+    if (n_items >= 4u * kStreams * sms) return kDealNear;
+    if (n_items > kStreams * sms) return kDealSpread;
+    const double most = longest > mean ? (double)longest : mean;
+    const uint32_t rounds = (n_items + sms - 1) / sms;                     // 1 to 3: streams per CTA, or items one after the other
+    const double chain = most * 0.8, level = mean * (rounds == 1 ? 0.77 : rounds == 2 ? 1.06 : 1.45);
+    const double spread = chain > level ? chain : level, split = rounds * (mean * 0.483 + 1.2) + (most - mean) * 0.483;
+    return split < spread ? kDealSplit : kDealSpread;
+}
+
 int tc_fused_attention(cudaStream_t s, const void *nn_lut, const void *q, const void *k, const void *v, void *o,
-                       const void *mask, int dtype, const AttnDims &p, float scale)
+                       const void *mask, int dtype, const AttnDims &p, float scale, uint32_t max_lut)
 {
     using namespace tc;
     const int is_bf16 = dtype == SFB_BF16;
@@ -687,7 +787,7 @@ int tc_fused_attention(cudaStream_t s, const void *nn_lut, const void *q, const 
                   p.mask_stride, (uint32_t)(p.out_pitch ? p.out_pitch : (uint64_t)p.H * 64), 0u, scale * 1.4426950408889634f};
     const int dev = current_device();
     const int sms = device_sm_count(dev);
-    prm.cta_first = sms > 0 && n_items < 4ull * kStreams * (uint64_t)sms ? 1u : 0u;     // fewer than four rounds
+    prm.deal = sms > 0 ? choose_deal((uint32_t)n_items, (double)p.blocks / p.nb_a, max_lut, (uint32_t)sms) : kDealNear;
     if (sms <= 0) return fail("sfb_fused_attention: cannot read the SM count");
     static DeviceOnce once;
     if (!once.done(dev)) {
@@ -699,7 +799,7 @@ int tc_fused_attention(cudaStream_t s, const void *nn_lut, const void *q, const 
         once.mark(dev);
     }
     // one CTA per SM, three streams each; fewer CTAs only when there are fewer items than SMs (few rounds) or than streams
-    const uint64_t want = prm.cta_first ? n_items : (n_items + kStreams - 1) / kStreams;
+    const uint64_t want = prm.deal != kDealNear ? n_items : (n_items + kStreams - 1) / kStreams;
     const dim3 grid((unsigned)(want < (uint64_t)sms ? want : (uint64_t)sms));
     const dim3 block(kThreads);
     if (mask && is_bf16) launch_overlapped(fused_attention_tc_kernel<true, true, SFB_TC_POLY>, grid, block, kSmemBytes, s, qm, km, vm, om, prm);

@@ -126,7 +126,7 @@ static int fused_attention_common(const char *who, sfb_stream_t stream, const vo
     // (16-byte aligned bases and row pitches); everything else runs on the CUDA cores
     const bool tma_ok = ((((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)o) & 15) == 0) && in_pitch % 8 == 0 && out_pitch % 8 == 0;
     if (tma_ok && tc_fused_attention_supported(dtype, block_size, p, scale, max_lut))
-        return tc_fused_attention(as_stream(stream), nn_lut, q, k, v, o, mask, dtype, p, scale);
+        return tc_fused_attention(as_stream(stream), nn_lut, q, k, v, o, mask, dtype, p, scale, max_lut);
     return simt_fused_attention(as_stream(stream), nn_lut, q, k, v, o, mask, dtype, block_size, p, scale);
 }
 

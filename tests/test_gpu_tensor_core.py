@@ -327,3 +327,31 @@ def test_host_pipeline_matches_resident_call(sfb):
         pipe(hq, hk, hv, ho, 0.125)
         torch.cuda.synchronize()
         assert torch.equal(ho, want.cpu())
+
+
+@pytest.mark.parametrize("B,H,nb,kind", [(1, 1, 1, "full"), (1, 2, 2, "full"), (2, 3, 5, "full"), (1, 4, 7, "causal"), (1, 2, 8, "full"), (3, 5, 16, "causal"),
+                                         (1, 3, 33, "sparse"), (2, 4, 64, "global"), (1, 1, 256, "sparse")])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_few_items_shared_by_the_streams(sfb, B, H, nb, kind, dtype):
+    """Launches of hardly more row pairs than SMs, whose key blocks the three streams of a CTA share: fewer blocks than
+    streams, an odd last block-row, rows without blocks, one row far longer than the rest, element masks; against the
+    CUDA-core kernel on the same values in fp32."""
+    g = torch.Generator(device="cuda").manual_seed(nb)
+    lay8 = torch.ones(1, nb, nb, dtype=torch.uint8, device="cuda")
+    if kind == "causal":
+        lay8 = lay8.tril()
+    elif kind != "full":
+        lay8 = (torch.rand(1, nb, nb, device="cuda", generator=g) < 6.0 / nb).to(torch.uint8)
+        lay8[:, 2] = 0                                       # a row without blocks, and a whole pair
+        lay8[:, 4:6] = 0
+        if kind == "global":
+            lay8[:, 9] = 1
+    lay = sfb.BlockLayout(lay8, 64)
+    if kind == "causal":
+        lay.pack_mask(sfb.MASK_CAUSAL_DIAG)
+    q, k, v = (torch.randn(B, nb * 64, H, 64, device="cuda", generator=g).to(dtype) for _ in range(3))
+    got = sfb.fused_attention(q, k, v, lay, 0.125, use_mask=kind == "causal")
+    assert sfb.device_status() == 0
+    want = sfb.fused_attention(q.float(), k.float(), v.float(), lay, 0.125, use_mask=kind == "causal")
+    assert float((got.float() - want).abs().max()) <= 2e-2 * float(want.abs().max())
+    assert torch.equal(got.float().abs().amax(-1) == 0, want.abs().amax(-1) == 0)
