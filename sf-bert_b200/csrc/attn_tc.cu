@@ -25,12 +25,6 @@
 // Every wait is bounded; on a timeout the CTA records a status word and leaves through the common teardown.
 #include "tc_common.cuh"
 
-// every SFB_TC_POLY-th pair of exponentials runs as a cubic on the FMA pipe (0 = all on the MUFU, the default: with
-// every fourth pair moved the kernel was no faster, the MUFU is not what holds it back)
-#ifndef SFB_TC_POLY
-#define SFB_TC_POLY 0
-#endif
-
 namespace sfb {
 
 namespace tc {
@@ -113,9 +107,10 @@ enum { kDealNear = 0, kDealSpread = 1, kDealSplit = 2 };
 // running three and others none, and a stream with the SM to itself finishes its item sooner (the 24-layer stack with
 // 512 items per launch: 973 -> 1036 sequences/s).  On long launches with items of very different length (BigBird)
 // that order measured 8 % slower, so it is kept to the launches that are all tail.
+template <bool SPLIT>
 __device__ __forceinline__ uint32_t item_id(uint32_t k, uint32_t s, const Params &p)
 {
-    if (p.deal == kDealSplit) return k * gridDim.x + blockIdx.x;
+    if (SPLIT) return k * gridDim.x + blockIdx.x;
     return p.deal == kDealSpread ? (k * kStreams + s) * gridDim.x + blockIdx.x : (k * gridDim.x + blockIdx.x) * kStreams + s;
 }
 
@@ -194,7 +189,7 @@ __device__ __forceinline__ uint32_t plan_union(const uint2 *nn, uint32_t pair, u
 // registers and advance side by side (a single thread walking three cursors kept them in local or shared memory and
 // needed thousands of cycles per round, measured).  Nothing here suspends the thread, so one slow stream never
 // holds up another for longer than a divergent branch.
-template <bool IS_K>
+template <bool IS_K, bool SPLIT>
 __device__ __forceinline__ void tma_producer(uint32_t s, uint8_t *smem, SharedState *sh, const UEntry *lists, const CUtensorMap &qmap,
                                              const CUtensorMap &tmap, const Params &p, uint32_t L, volatile uint32_t *abort_flag)
 {
@@ -234,7 +229,7 @@ __device__ __forceinline__ void tma_producer(uint32_t s, uint8_t *smem, SharedSt
         while (again) {
             again = false;
             if (stage == 0) {
-                const uint32_t id = item_id(k, s, p);
+                const uint32_t id = item_id<SPLIT>(k, s, p);
                 if (id >= p.n_items) {
                     if (IS_K) done = true;
                     else stage = 4;            // loads done; the stores of the last items are still to come
@@ -311,8 +306,8 @@ __device__ __forceinline__ void tma_producer(uint32_t s, uint8_t *smem, SharedSt
 }
 
 // ---- the kernel ---------------------------------------------------------------------------------
-// POLY: every POLY-th pair of exponentials runs on the FMA pipe (0 = none)
-template <bool HAS_MASK, bool BF16, int POLY>
+// SPLIT: the streams of a CTA share its items (a kernel of its own: the merge in the epilogue cost the others 3 %)
+template <bool HAS_MASK, bool BF16, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
                           const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap omap, const Params p)
@@ -376,12 +371,12 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
         asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
         // ===== planner of stream s: the unions of the coming items, up to two ahead =====
         if (warp == 16) {
-            if (lane < (uint32_t)kStreams) tma_producer<false>(lane, smem, sh, lists, omap, vmap, p, L, abort_flag);
+            if (lane < (uint32_t)kStreams) tma_producer<false, SPLIT>(lane, smem, sh, lists, omap, vmap, p, L, abort_flag);
         } else {
             const uint32_t s = warp - 17;
             StreamState *st = &sh->st[s];
             for (uint32_t k = 0;; k++) {
-                const uint32_t id = item_id(k, s, p);
+                const uint32_t id = item_id<SPLIT>(k, s, p);
                 if (id >= p.n_items) break;
                 const uint32_t slot = k & 1;
                 if (k >= 2 && !mbar_wait_warp(&st->list_free[slot], ((k >> 1) - 1) & 1, abort_flag, 20)) break;
@@ -392,7 +387,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
                     if (lane == 0) atomicCAS(&g_status, 0u, (9u << 24) | (blockIdx.x & 0xffffffu));
                     n = 0;
                 }
-                if (p.deal == kDealSplit) {
+                if (SPLIT) {
                     // this stream's share: entries s, s + 3, ... moved to the front (a group of 32 reads before it writes, and what
                     // it writes lies before what the groups after it read)
                     UEntry *ent = lists + (s * 2 + slot) * kMaxU;
@@ -415,7 +410,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
     } else if (warp >= 12) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
         if (warp == 15) {
-            if (lane < (uint32_t)kStreams) tma_producer<true>(lane, smem, sh, lists, qmap, kmap, p, L, abort_flag);
+            if (lane < (uint32_t)kStreams) tma_producer<true, SPLIT>(lane, smem, sh, lists, qmap, kmap, p, L, abort_flag);
         } else {
         // ===== MMA issuer of stream s:  S(0) | S(1) O(0) | S(2) O(1) | ...  =====
         const uint32_t s = warp - 12;
@@ -443,7 +438,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
                 return true;
             };
             for (uint32_t k = 0; alive; k++) {
-                const uint32_t id = item_id(k, s, p);
+                const uint32_t id = item_id<SPLIT>(k, s, p);
                 if (id >= p.n_items) break;
                 if (!mbar_wait(&st->list_ready[k & 1], (k >> 1) & 1, abort_flag, 8)) break;
                 const uint32_t T = st->list_n[k & 1];
@@ -502,7 +497,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
             up64(l0, a0, a1);
             up64(l1, a2, a3);
             float lsum = (a0 + a1) + (a2 + a3);
-            const bool split = p.deal == kDealSplit, mine = !split || s == 0;
+            const bool mine = !SPLIT || s == 0;
             float fac[kStreams] = {1.f, 0.f, 0.f};         // what the streams' accumulators are multiplied by, and their steps
             uint32_t steps[kStreams] = {T, 0, 0};
             if (T > 0) {
@@ -518,7 +513,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
                 tcgen05_fence_before();
                 mbar_arrive_warp(&st->part_ready, lane);
             } else {
-                if (split) {
+                if (SPLIT) {
                     float M = m_used;
                     float2 part[kStreams];
 #pragma unroll
@@ -558,7 +553,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
 #pragma unroll
                         for (int c = 0; c < 16; c++) oc[c] = 0u;  // a row pair without key blocks gives zeros (blocksparse.h:949-962)
                     }
-                    if (split) {
+                    if (SPLIT) {
 #pragma unroll
                         for (int j = 1; j < kStreams; j++)
                             if (steps[j]) {
@@ -585,7 +580,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
                 }
                 tcgen05_fence_before();
                 if (T > 0) mbar_arrive(&st->o_free);       // the next item's first O product may overwrite the accumulator
-                if (split) {
+                if (SPLIT) {
 #pragma unroll
                     for (int j = 1; j < kStreams; j++) {
                         if (steps[j]) mbar_arrive(&sh->st[j].o_free);
@@ -605,7 +600,7 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
 
         uint32_t sr[64];                                   // this row of S(t), fp32 bits
         for (uint32_t k = 0; alive; k++) {
-            const uint32_t id = item_id(k, s, p);
+            const uint32_t id = item_id<SPLIT>(k, s, p);
             if (id >= p.n_items) break;
             if (!mbar_wait_warp(&st->list_ready[k & 1], (k >> 1) & 1, abort_flag, 8)) break;
             const uint32_t T = st->list_n[k & 1];
@@ -686,15 +681,9 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
                         for (int j = 0; j < 16; j++) {
                             const int c = hh * 32 + 2 * j;
                             const uint64_t x = fma2p(pk64(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])), sl2, nm2);
-                            float e0, e1;
-                            if (POLY > 0 && (j % (POLY > 0 ? POLY : 1)) == (POLY > 0 ? POLY : 1) - 1) {
-                                exp2_fma_pair(x, e0, e1);
-                            } else {
-                                float x0, x1;
-                                up64(x, x0, x1);
-                                e0 = ex2_approx(x0);
-                                e1 = ex2_approx(x1);
-                            }
+                            float x0, x1;
+                            up64(x, x0, x1);
+                            const float e0 = ex2_approx(x0), e1 = ex2_approx(x1);
                             if (j & 1) lacc1 = add2p(lacc1, pk64(e0, e1));
                             else lacc0 = add2p(lacc0, pk64(e0, e1));
                             pk[j] = pack_pair<BF16>(e0, e1);
@@ -752,6 +741,21 @@ bool tc_fused_attention_supported(int dtype, uint32_t bs, const AttnDims &p, flo
            longest <= (uint64_t)tc::kMaxU && (uint64_t)p.B * p.nb_a * 64 < (1ull << 31) && p.nb_a < (1u << 30);
 }
 
+template <bool HAS_MASK, bool BF16, bool SPLIT>
+static int launch_fused(cudaStream_t s, dim3 grid, const CUtensorMap &qm, const CUtensorMap &km, const CUtensorMap &vm, const CUtensorMap &om,
+                        const tc::Params &prm, int dev)
+{
+    using namespace tc;
+    static DeviceOnce once;
+    if (!once.done(dev)) {
+        if (cudaFuncSetAttribute(fused_attention_tc_kernel<HAS_MASK, BF16, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) != cudaSuccess)
+            return fail("sfb_fused_attention: cannot reserve %zu bytes of shared memory", kSmemBytes);
+        once.mark(dev);
+    }
+    launch_overlapped(fused_attention_tc_kernel<HAS_MASK, BF16, SPLIT>, grid, dim3(kThreads), kSmemBytes, s, qm, km, vm, om, prm);
+    return check_launch("sfb_fused_attention");
+}
+
 // How a launch deals its items.  From four rounds of items up: near.  From one to four: spread.  Within one round the split
 // deal may finish sooner, estimated in microseconds: a step takes a stream that has its SM to itself 0.77, two streams 1.06
 // and three 1.45; split, a third of a CTA's items' steps at the rate of three streams plus 1.2 per item for the shares'
@@ -789,24 +793,16 @@ int tc_fused_attention(cudaStream_t s, const void *nn_lut, const void *q, const 
     const int sms = device_sm_count(dev);
     prm.deal = sms > 0 ? choose_deal((uint32_t)n_items, (double)p.blocks / p.nb_a, max_lut, (uint32_t)sms) : kDealNear;
     if (sms <= 0) return fail("sfb_fused_attention: cannot read the SM count");
-    static DeviceOnce once;
-    if (!once.done(dev)) {
-        cudaError_t e = cudaFuncSetAttribute(fused_attention_tc_kernel<false, false, SFB_TC_POLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(fused_attention_tc_kernel<false, true, SFB_TC_POLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(fused_attention_tc_kernel<true, false, SFB_TC_POLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(fused_attention_tc_kernel<true, true, SFB_TC_POLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-        if (e != cudaSuccess) return fail("sfb_fused_attention: cannot reserve %zu bytes of shared memory", kSmemBytes);
-        once.mark(dev);
-    }
     // one CTA per SM, three streams each; fewer CTAs only when there are fewer items than SMs (few rounds) or than streams
     const uint64_t want = prm.deal != kDealNear ? n_items : (n_items + kStreams - 1) / kStreams;
     const dim3 grid((unsigned)(want < (uint64_t)sms ? want : (uint64_t)sms));
-    const dim3 block(kThreads);
-    if (mask && is_bf16) launch_overlapped(fused_attention_tc_kernel<true, true, SFB_TC_POLY>, grid, block, kSmemBytes, s, qm, km, vm, om, prm);
-    else if (mask) launch_overlapped(fused_attention_tc_kernel<true, false, SFB_TC_POLY>, grid, block, kSmemBytes, s, qm, km, vm, om, prm);
-    else if (is_bf16) launch_overlapped(fused_attention_tc_kernel<false, true, SFB_TC_POLY>, grid, block, kSmemBytes, s, qm, km, vm, om, prm);
-    else launch_overlapped(fused_attention_tc_kernel<false, false, SFB_TC_POLY>, grid, block, kSmemBytes, s, qm, km, vm, om, prm);
-    return check_launch("sfb_fused_attention");
+    const int variant = (mask ? 4 : 0) | (is_bf16 ? 2 : 0) | (prm.deal == kDealSplit ? 1 : 0);
+#define FA_CASE(V, M, BF, SP) case V: return launch_fused<M, BF, SP>(s, grid, qm, km, vm, om, prm, dev)
+    switch (variant) {
+        FA_CASE(0, false, false, false); FA_CASE(1, false, false, true); FA_CASE(2, false, true, false); FA_CASE(3, false, true, true);
+        FA_CASE(4, true, false, false); FA_CASE(5, true, false, true); FA_CASE(6, true, true, false); default: FA_CASE(7, true, true, true);
+    }
+#undef FA_CASE
 }
 
 int tc_status_clear_fused()
