@@ -697,28 +697,30 @@ __global__ void __launch_bounds__(256) fused_sddmm_softmax_kernel(const uint2 *_
 // chunks of 32 of d, the softmax in registers (row maxima meet in shared memory), P to shared memory, then O += P . V in
 // chunks of 32 keys, each warp on its share of O's columns (and, for 64 rows, of its rows).  Keys and values flow through
 // the same two buffers as one sequence of chunks.  Score and O rows of a thread are the same, so O is rescaled in place.
-template <int BS, int D> struct FaCfg {
+// ST chunk buffers: two let three CTAs share an SM; four keep three chunks on their way, for launches that do not fill the SMs
+// anyway and wait for L2 chunk by chunk.
+template <int BS, int D, int ST = 2> struct FaCfg {
     static constexpr uint32_t G = BS == 32 ? 4 : 1;                      // key blocks per step
     static constexpr uint32_t NK = G * BS;                               // keys per step
     static constexpr uint32_t WC = BS == 32 ? 4 : 2;                     // warps side by side (score columns, O columns)
     static constexpr int TN = D / (int)WC / 4;
     static constexpr uint32_t kbuf = NK * tile::kStride, vbuf = 32 * (D + 4), buf = kbuf > vbuf ? kbuf : vbuf;
     static constexpr uint32_t p_stride = NK + 4, q_stride = D + 4;
-    static constexpr uint32_t floats = BS * q_stride + 2 * buf + BS * p_stride + WC * BS;
-    static constexpr int ctas = BS == 64 && D == 128 ? 2 : 3;            // what registers and shared memory allow per SM
+    static constexpr uint32_t floats = BS * q_stride + ST * buf + BS * p_stride + WC * BS;
+    static constexpr int ctas = ST > 2 || (BS == 64 && D == 128) ? 2 : 3;            // what registers and shared memory allow per SM
 };
-template <int BS, int D, int DT>
-__global__ void __launch_bounds__(tile::kThreads, (FaCfg<BS, D>::ctas))
+template <int BS, int D, int DT, int ST>
+__global__ void __launch_bounds__(tile::kThreads, (FaCfg<BS, D, ST>::ctas))
 fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q, const void *__restrict__ K, const void *__restrict__ V,
                        void *__restrict__ O, const typename MaskWord<BS>::type *__restrict__ mask, AttnDims p, float scale_log2e, bool vec)
 {
     using namespace tile;
     typedef typename MaskWord<BS>::type W;
-    typedef FaCfg<BS, D> Cfg;
+    typedef FaCfg<BS, D, ST> Cfg;
     constexpr int TN = Cfg::TN;
     constexpr uint32_t G = Cfg::G, WC = Cfg::WC, QS = Cfg::q_stride, PS = Cfg::p_stride;
     extern __shared__ __align__(16) float sm[];
-    float *Qs = sm, *bufs = Qs + BS * QS, *Ps = bufs + 2 * Cfg::buf, *red = Ps + BS * PS;
+    float *Qs = sm, *bufs = Qs + BS * QS, *Ps = bufs + ST * Cfg::buf, *red = Ps + BS * PS;
     grid_dependency_wait();
     grid_launch_dependents();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane_row(lane), lc = lane_quad(lane);
@@ -738,13 +740,17 @@ fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q
     uint32_t is_e = 0, is_k = 0, is_n = 0;                               // next chunk to issue: step's first entry, index in the step, overall
     size_t koff[G];
     auto issue = [&]() {
+        if (is_e >= cnt) {                                               // nothing left: an empty group keeps the count
+            cp_commit();
+            return;
+        }
         const uint32_t nblk = min(G, cnt - is_e);
         if (is_k == 0) {
 #pragma unroll
             for (uint32_t g = 0; g < G; g++)
                 koff[g] = ((size_t)b * p.nb_b + nn[head.x + is_e + (g < nblk ? g : 0)].y) * BS * HD + (size_t)h * p.d;
         }
-        float *buf = bufs + (is_n & 1) * Cfg::buf;
+        float *buf = bufs + (is_n % ST) * Cfg::buf;
         if (is_k < kchunks) {
             const uint32_t k0 = is_k * kChunk;
 #pragma unroll
@@ -765,7 +771,8 @@ fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q
 
     if (cnt) {
         stage<DT, BS, D>(Qs, QS, Q, ((size_t)b * p.nb_a + i) * BS * HD + (size_t)h * p.d, HD, p.d, vec);
-        issue();
+#pragma unroll
+        for (int i = 0; i < ST - 1; i++) issue();
     }
     float mx[4], sum[4];
     uint64_t acc[4][TN / 2];
@@ -786,10 +793,10 @@ fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q
 #pragma unroll
             for (int n = 0; n < 8; n++) s2[m][n] = 0;
         for (uint32_t kc = 0; kc < kchunks; kc++, c++) {
-            cp_wait_all();
+            cp_wait<ST - 2>();
             __syncthreads();
-            issue();                                                     // a value chunk follows every key chunk of a step
-            const float *buf = bufs + (c & 1) * Cfg::buf;
+            issue();
+            const float *buf = bufs + (c % ST) * Cfg::buf;
             if (live) mma_nt(s2, Qs + (r0 + lr) * QS + kc * kChunk, QS, buf + (32 * wc + lc) * kStride, kStride);
         }
         const uint32_t blk = nn[head.x + e + (G > 1 && live ? warp : 0)].x;
@@ -831,10 +838,10 @@ fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q
         }
         const uint32_t vchunks = nblk * (BS / 32);
         for (uint32_t vc = 0; vc < vchunks; vc++, c++) {
-            cp_wait_all();
+            cp_wait<ST - 2>();
             __syncthreads();
-            if (vc + 1 < vchunks || e + G < cnt) issue();
-            const float *buf = bufs + (c & 1) * Cfg::buf;
+            issue();
+            const float *buf = bufs + (c % ST) * Cfg::buf;
             mma_nn<TN>(acc, Ps + (r0 + lr) * PS + vc * 32, PS, buf + n0 + lane_col<TN>(lc), D + 4);
         }
     }
@@ -1174,17 +1181,23 @@ int simt_fused_attention(cudaStream_t s, const void *nn_lut, const void *q, cons
     const float sl = scale * LOG2E_F;
     const uint64_t HD = (uint64_t)p.H * p.d, in = p.in_pitch ? p.in_pitch : HD, on = p.out_pitch ? p.out_pitch : HD;
     const bool vec = rows_vec(q, dtype, in, p.d) && rows_vec(k, dtype, in, p.d) && rows_vec(v, dtype, in, p.d) && rows_vec(o, dtype, on, p.d);
-#define LAUNCH_FA(DV)                                                                                            \
+    // a launch that two CTAs per SM hold at once waits for its chunks one after another: more of them on their way
+    // (B 1, H 4, L 512, d 64: 64 CTAs)
+    const int sms = device_sm_count(current_device());
+    const bool few = (uint64_t)p.nb_a * p.B * p.H <= 2ull * (uint64_t)(sms > 0 ? sms : 0);
+#define LAUNCH_FA_ST(DV, STV)                                                                                    \
     {                                                                                                            \
         typedef typename MaskWord<BS>::type W;                                                                   \
-        const size_t bytes = sizeof(float) * FaCfg<BS, DV>::floats;                                              \
-        auto kern = fused_attention_kernel<BS, DV, DT>;                                                          \
-        static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                                                     \
+        const size_t bytes = sizeof(float) * FaCfg<BS, DV, STV>::floats;                                         \
+        auto kern = fused_attention_kernel<BS, DV, DT, STV>;                                                     \
+        static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                       \
         launch_overlapped(kern, grid, dim3(tile::kThreads), bytes, s, (const uint2 *)nn_lut, q, k, v, o, (const W *)mask, p, sl, vec); \
     }
+#define LAUNCH_FA(DV) { if (few) LAUNCH_FA_ST(DV, 4) else LAUNCH_FA_ST(DV, 2) }
     DISPATCH_BS(bs, DISPATCH_DT(dtype, DT, {
         if (p.d <= 32) LAUNCH_FA(32) else if (p.d <= 64) LAUNCH_FA(64) else LAUNCH_FA(128)
     }))
+#undef LAUNCH_FA_ST
 #undef LAUNCH_FA
     return check_launch("sfb_fused_attention");
 }
