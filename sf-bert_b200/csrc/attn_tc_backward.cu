@@ -36,7 +36,6 @@ constexpr uint32_t kBwStages = 3;
 constexpr uint32_t kBwStageBytes = 4 * kTileBytes;              // two blocks of P, Y, Z
 constexpr uint32_t kBwThreads = 12 * 32;
 constexpr uint32_t kBwMaxUnion = 256;
-constexpr uint32_t kNoItem = 0xffffffffu;
 
 struct BwShared {
     uint64_t in_full[kBwStages], in_empty[kBwStages], x_ready, s_full, s_free, ds_full, ds_free, o_final, o_free;
@@ -95,104 +94,6 @@ __device__ __forceinline__ uint32_t ds_pair(uint32_t v0, uint32_t v1, uint32_t p
     return pack2(e0, e1, BF16);
 }
 
-// Which two rows (columns) of the LUT make pair `pair`: in the order long ones first, then the rest, each by index; long is
-// more than twice the mean.  Neighbours share most of their blocks in the layouts at hand, except where one of them is a
-// global row or a strided column: next to a row of four blocks, its 64 steps are all half empty.  Paired with each other the
-// long ones fill their steps, and they start first.  One warp; own[1] = kNoItem when the last row is alone.
-__device__ __forceinline__ void pick_pair(const uint2 *lut, uint32_t pair, uint32_t nb, uint32_t blocks, uint32_t lane, uint32_t (&own)[2])
-{
-    uint32_t n_long = 0;
-    for (uint32_t base = 0; base < nb; base += 32) {
-        const uint32_t i = base + lane;
-        n_long += __popc(__ballot_sync(0xffffffffu, i < nb && (uint64_t)lut[i].y * nb > 2ull * blocks));
-    }
-    own[0] = own[1] = kNoItem;
-    uint32_t seen_long = 0, seen_rest = n_long;               // places in the order taken so far by each kind
-    for (uint32_t base = 0; base < nb; base += 32) {
-        const uint32_t i = base + lane;
-        const bool in = i < nb, is_long = in && (uint64_t)lut[i].y * nb > 2ull * blocks;
-        const uint32_t longs = __ballot_sync(0xffffffffu, is_long), rest = __ballot_sync(0xffffffffu, in && !is_long);
-        const uint32_t below = (1u << lane) - 1u;
-        const uint32_t place = is_long ? seen_long + __popc(longs & below) : seen_rest + __popc(rest & below);
-#pragma unroll
-        for (int o = 0; o < 2; o++) {
-            const uint32_t hit = __ballot_sync(0xffffffffu, in && place == 2 * pair + o);
-            if (hit) own[o] = base + __ffs(hit) - 1;
-        }
-        seen_long += __popc(longs);
-        seen_rest += __popc(rest);
-    }
-}
-
-// The union of the blocks of rows (columns) own[0] and own[1], built by ONE warp: the first one's in LUT order, then those
-// only the second has.  At most kBwMaxUnion entries (checked by the host); kNoItem when the LUT says otherwise.
-__device__ __forceinline__ uint32_t warp_union(const uint2 *lut, const uint32_t (&own)[2], UnionEntry *ent, uint32_t lane)
-{
-    const uint2 head0 = lut[own[0]];
-    const uint2 head1 = own[1] != kNoItem ? lut[own[1]] : make_uint2(0, 0);
-    const uint32_t n0 = head0.y, n1 = head1.y;
-    if (n0 > kBwMaxUnion || n1 > kBwMaxUnion) return kNoItem;
-    uint2 next = lane < n1 ? lut[head1.x + lane] : make_uint2(0, 0);      // on its way while the first list is written
-    for (uint32_t i = lane; i < n0; i += 32) {
-        const uint2 e = lut[head0.x + i];
-        ent[i].col = e.y;
-        ent[i].flags = 1;
-        ent[i].blk[0] = e.x;
-        ent[i].blk[1] = 0;
-    }
-    __syncwarp();
-    uint32_t n = n0;
-    for (uint32_t base = 0; base < n1; base += 32) {
-        const uint2 e = next;
-        const bool valid = base + lane < n1;
-        if (base + 32 + lane < n1) next = lut[head1.x + base + 32 + lane];
-        bool fresh = valid;
-        if (valid)
-            for (uint32_t u = 0; u < n0; u++)
-                if (ent[u].col == e.y) {
-                    ent[u].flags |= 2;
-                    ent[u].blk[1] = e.x;
-                    fresh = false;
-                    break;
-                }
-        const uint32_t votes = __ballot_sync(0xffffffffu, fresh);
-        const uint32_t at = n + __popc(votes & ((1u << lane) - 1u));
-        if (n + __popc(votes) > kBwMaxUnion) return kNoItem;
-        if (fresh) {
-            ent[at].col = e.y;
-            ent[at].flags = 2;
-            ent[at].blk[0] = 0;
-            ent[at].blk[1] = e.x;
-        }
-        n += __popc(votes);
-    }
-    __syncwarp();
-    return n;
-}
-
-// asks for the next item that no CTA has started; the answer arrives on bar with 16 bytes
-__device__ __forceinline__ void clc_request(uint32_t *response, uint64_t *bar)
-{
-    mbar_expect_tx(bar, 16);
-    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(response)),
-                 "r"(smem_u32(bar))
-                 : "memory");
-}
-__device__ __forceinline__ uint32_t clc_item(const uint32_t *response)
-{
-    uint32_t ok, x = 0;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b128 r;\n\t"
-        "ld.shared.b128 r, [%2];\n\t"
-        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, _, _, _}, r;\n\t}"
-        : "=r"(ok), "+r"(x)
-        : "r"(smem_u32(response))
-        : "memory");
-    return ok ? x : kNoItem;
-}
-
 template <bool COL, bool BF16>
 __global__ void __launch_bounds__(kBwThreads, 2)
 backward_tc_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__ CUtensorMap ymap, const __grid_constant__ CUtensorMap zmap,
@@ -246,15 +147,7 @@ backward_tc_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_consta
     if (warp == 11) {
         // ===== planner: the coming items and their unions, up to two ahead =====
         uint32_t id = blockIdx.x;
-        // one LUT for all heads: the items of the long pairs of all (batch, head)s come before the rest, so that none of them
-        // is left for the end; otherwise (batch, head) by (batch, head)
-        uint32_t first_pairs = 0;
-        if (p.lut_stride == 0) {
-            uint32_t n_long = 0;
-            for (uint32_t base = 0; base < p.nb; base += 32)
-                n_long += __popc(__ballot_sync(0xffffffffu, base + lane < p.nb && (uint64_t)p.lut[base + lane].y * p.nb > 2ull * p.blocks));
-            first_pairs = (n_long + 1) / 2;
-        }
+        const uint32_t first_pairs = p.lut_stride == 0 ? long_pairs(p.lut, p.nb, p.blocks, lane) : 0;
         const uint32_t first_items = first_pairs * p.B * p.H;
         for (uint32_t k = 0;; k++) {
             const uint32_t slot = k & 1;
@@ -276,7 +169,7 @@ backward_tc_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_consta
                 bh = b * p.H + h;
                 const uint2 *lut = p.lut + (size_t)h * p.lut_stride;
                 pick_pair(lut, pair, p.nb, p.blocks, lane, own);
-                n = warp_union(lut, own, st->lists[slot], lane);
+                n = warp_union(lut, own, st->lists[slot], kBwMaxUnion, lane);
                 if (n == kNoItem) {                           // more blocks than the caller's maximum: recorded, zeros written
                     if (lane == 0) atomicCAS(&g_status, 0u, (9u << 24) | (blockIdx.x & 0xffffffu));
                     n = 0;

@@ -1,8 +1,9 @@
 // The unfused operators on the tensor cores (tcgen05) for 16-bit operands, block_size 64, head size 64:
 //   sddmm_tc_kernel   S(block) = Q_i . K_j^T for every kept block          (bst_sgemm_nt,  blocksparse.h:425)
 //   spmm_tc_kernel    O_i = sum over the row's blocks of P(block) . V_j     (bst_sgemm_xn,  blocksparse.h:965)
-// Same tiling as the fused kernel: a CTA owns a pair of adjacent block-rows (128 queries, one M=128 MMA
-// tile) and walks the union of their key blocks; operands arrive by TMA into 128-byte-swizzled shared
+// Same tiling as the fused kernel: a CTA owns a pair of adjacent block-rows (128 queries, one M=128 MMA tile; the fused
+// probabilities pair long rows with each other, see locate_item: BigBird 327 -> 290 us; SpMM, whose half-empty steps cost
+// no memory traffic, lost 3 % to the search) and walks the union of their key blocks; operands arrive by TMA into 128-byte-swizzled shared
 // memory, accumulators live in TMEM.  Both operators are HBM-bound (8 KB of S or P per 1 MFLOP), so the
 // point of the tensor cores here is to get the arithmetic out of the way of the memory system.
 #include "tc_common.cuh"
@@ -316,7 +317,8 @@ spmm_tc_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
     }
     grid_dependency_wait();
     grid_launch_dependents();
-    build_union(nn, pair, p.nb, st->entries, st->cand, &st->n_union, &st->abort_flag);
+    const uint32_t own[2] = {pair * 2, has_row1 ? pair * 2 + 1 : kNoItem};
+    build_union(nn, own, st->entries, st->cand, &st->n_union, &st->abort_flag);
     if (warp == 0) {
         __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&st->tmem_base)), "r"(64u) : "memory");
@@ -442,10 +444,7 @@ fused_p_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constan
     float2 *comb = (float2 *)(st + 1);         // [column half][row]: (max, sum) after sweep 1
 
     const uint32_t warp = uniform_warp(), lane = threadIdx.x & 31;
-    // last (batch, head) first: the product that reads the probabilities next starts with the ones still in L2
-    const uint32_t pair = blockIdx.x, b = gridDim.y - 1 - blockIdx.y, h = gridDim.z - 1 - blockIdx.z;
     const uint32_t L = p.nb * 64;
-    const uint2 *nn = p.nn_lut + (size_t)h * p.lut_stride;
     volatile uint32_t *abort_flag = &st->abort_flag;
     const uint32_t fmt = p.is_bf16 ? 1u : 0u;
 
@@ -462,7 +461,10 @@ fused_p_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constan
     }
     grid_dependency_wait();
     grid_launch_dependents();
-    build_union(nn, pair, p.nb, st->entries, st->cand, &st->n_union, &st->abort_flag);
+    // last (batch, head) first: the product that reads the probabilities next starts with the ones still in L2
+    const ItemAt it = locate_item(p.nn_lut, p.lut_stride, p.B, p.H, p.nb, p.blocks, blockIdx.x, lane, true);
+    const uint32_t b = it.b, h = it.h;
+    build_union(p.nn_lut + (size_t)h * p.lut_stride, it.own, st->entries, st->cand, &st->n_union, &st->abort_flag);
     if (warp == 0) {
         __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&st->tmem_base)), "r"(128u) : "memory");
@@ -480,7 +482,10 @@ fused_p_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constan
     if (warp == 0) {
         if (T > 0 && elect_one()) {
             mbar_expect_tx(&st->q_full, kQBytes);
-            tma_load_2d(smem_u32(q_tile), &qmap, &st->q_full, xq, (int32_t)(b * L + pair * 128));
+#pragma unroll
+            for (uint32_t o = 0; o < 2; o++)      // a row that does not exist: beyond the tensor, zeros
+                tma_load_2d(smem_u32(q_tile + o * kTileBytes), &qmap, &st->q_full, xq,
+                            it.own[o] != kNoItem ? (int32_t)(b * L + it.own[o] * 64) : (int32_t)(p.B * L));
             for (uint32_t t = 0; t < T2; t++) {
                 const uint32_t s = t % kUStages;
                 if (t >= kUStages && !mbar_wait(&st->in_empty[s], ((t / kUStages) - 1) & 1, abort_flag, 41)) break;
@@ -709,7 +714,7 @@ int tc_fused_p(cudaStream_t s, const void *nn_lut, const void *a, const void *b,
     const int is_bf16 = ab_dtype == SFB_BF16;
     const uint64_t rows = (uint64_t)p.B * p.nb_a * 64;
     CUtensorMap qm, km;
-    if (make_map(&qm, a, rows, p.H, is_bf16, 128) || make_map(&km, b, rows, p.H, is_bf16, 64)) return 1;
+    if (make_map(&qm, a, rows, p.H, is_bf16, 64) || make_map(&km, b, rows, p.H, is_bf16, 64)) return 1;
     FpParams prm = {(const uint2 *)nn_lut, (const uint64_t *)mask, y, p.B, p.H, p.nb_a, p.blocks, p.lut_stride, p.mask_stride,
                     scale * 1.4426950408889634f, y_dtype, is_bf16};
     static DeviceOnce once;
@@ -719,7 +724,7 @@ int tc_fused_p(cudaStream_t s, const void *nn_lut, const void *a, const void *b,
             return fail("sfb_fused_sddmm_softmax: cannot reserve %zu bytes of shared memory", kFpSmem);
         once.mark(dev);
     }
-    launch_overlapped(fused_p_tc_kernel, dim3((p.nb_a + 1) / 2, p.B, p.H), dim3(kFpThreads), kFpSmem, s, qm, km, prm);
+    launch_overlapped(fused_p_tc_kernel, dim3((p.nb_a + 1) / 2 * p.B * p.H), dim3(kFpThreads), kFpSmem, s, qm, km, prm);
     return check_launch("sfb_fused_sddmm_softmax");
 }
 

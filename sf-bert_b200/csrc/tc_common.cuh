@@ -329,17 +329,16 @@ __device__ __forceinline__ float2 unpack2(uint32_t v, int is_bf16)
                    "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])      \
                  : "memory")
 
-// Builds the union of the key blocks of block-rows 2*pair and 2*pair+1 in shared memory: the upper row's
+// Builds the union of the key blocks of block-rows own[0] and own[1] (0xffffffff: none) in shared memory: the upper row's
 // blocks in LUT order, then the blocks only the lower row has.  All threads of the CTA call it (it contains
 // __syncthreads); the result is complete after the caller's next __syncthreads.  cand is kMaxUnion words of
 // scratch.  Returns through *n_out; 0 with *abort_flag set if a row does not fit.  Two dependent global reads
 // deep (row headers, then both rows' entries at once); everything after that works from shared memory.
-__device__ __forceinline__ void build_union(const uint2 *nn, uint32_t pair, uint32_t nb, UnionEntry *entries,
+__device__ __forceinline__ void build_union(const uint2 *nn, const uint32_t (&own)[2], UnionEntry *entries,
                                             uint2 *cand, uint32_t *n_out, uint32_t *abort_flag)
 {
-    const uint32_t row0 = pair * 2, row1 = pair * 2 + 1;
-    const uint2 head0 = nn[row0];
-    const uint2 head1 = row1 < nb ? nn[row1] : make_uint2(0, 0);
+    const uint2 head0 = nn[own[0]];
+    const uint2 head1 = own[1] != 0xffffffffu ? nn[own[1]] : make_uint2(0, 0);
     const uint32_t n0 = head0.y, n1 = head1.y;
     const bool fits = n0 <= kMaxUnion && n1 <= kMaxUnion;
     if (fits) {
@@ -398,6 +397,144 @@ __device__ __forceinline__ void build_union(const uint2 *nn, uint32_t pair, uint
             *n_out = n;
         }
     }
+}
+
+// ---- items of the persistent kernels: pairs of block-rows (block-columns) -------------------------------------------
+constexpr uint32_t kNoItem = 0xffffffffu;
+
+// Which two rows (columns) of the LUT make pair `pair`: in the order long ones first, then the rest, each by index; long is
+// more than twice the mean.  Neighbours share most of their blocks in the layouts at hand, except where one of them is a
+// global row or a strided column: next to a row of four blocks, its 64 steps are all half empty.  Paired with each other the
+// long ones fill their steps, and they start first.  One warp; own[1] = kNoItem when the last row is alone.
+__device__ __forceinline__ void pick_pair(const uint2 *lut, uint32_t pair, uint32_t nb, uint32_t blocks, uint32_t lane, uint32_t (&own)[2])
+{
+    uint32_t n_long = 0;
+    for (uint32_t base = 0; base < nb; base += 32) {
+        const uint32_t i = base + lane;
+        n_long += __popc(__ballot_sync(0xffffffffu, i < nb && (uint64_t)lut[i].y * nb > 2ull * blocks));
+    }
+    own[0] = own[1] = kNoItem;
+    uint32_t seen_long = 0, seen_rest = n_long;               // places in the order taken so far by each kind
+    for (uint32_t base = 0; base < nb; base += 32) {
+        const uint32_t i = base + lane;
+        const bool in = i < nb, is_long = in && (uint64_t)lut[i].y * nb > 2ull * blocks;
+        const uint32_t longs = __ballot_sync(0xffffffffu, is_long), rest = __ballot_sync(0xffffffffu, in && !is_long);
+        const uint32_t below = (1u << lane) - 1u;
+        const uint32_t place = is_long ? seen_long + __popc(longs & below) : seen_rest + __popc(rest & below);
+#pragma unroll
+        for (int o = 0; o < 2; o++) {
+            const uint32_t hit = __ballot_sync(0xffffffffu, in && place == 2 * pair + o);
+            if (hit) own[o] = base + __ffs(hit) - 1;
+        }
+        seen_long += __popc(longs);
+        seen_rest += __popc(rest);
+    }
+}
+
+// The union of the blocks of rows (columns) own[0] and own[1], built by ONE warp: the first one's in LUT order, then those
+// only the second has.  At most `most` entries (checked by the host); kNoItem when the LUT says otherwise.
+__device__ __forceinline__ uint32_t warp_union(const uint2 *lut, const uint32_t (&own)[2], UnionEntry *ent, uint32_t most, uint32_t lane)
+{
+    const uint2 head0 = lut[own[0]];
+    const uint2 head1 = own[1] != kNoItem ? lut[own[1]] : make_uint2(0, 0);
+    const uint32_t n0 = head0.y, n1 = head1.y;
+    if (n0 > most || n1 > most) return kNoItem;
+    uint2 next = lane < n1 ? lut[head1.x + lane] : make_uint2(0, 0);      // on its way while the first list is written
+    for (uint32_t i = lane; i < n0; i += 32) {
+        const uint2 e = lut[head0.x + i];
+        ent[i].col = e.y;
+        ent[i].flags = 1;
+        ent[i].blk[0] = e.x;
+        ent[i].blk[1] = 0;
+    }
+    __syncwarp();
+    uint32_t n = n0;
+    for (uint32_t base = 0; base < n1; base += 32) {
+        const uint2 e = next;
+        const bool valid = base + lane < n1;
+        if (base + 32 + lane < n1) next = lut[head1.x + base + 32 + lane];
+        bool fresh = valid;
+        if (valid)
+            for (uint32_t u = 0; u < n0; u++)
+                if (ent[u].col == e.y) {
+                    ent[u].flags |= 2;
+                    ent[u].blk[1] = e.x;
+                    fresh = false;
+                    break;
+                }
+        const uint32_t votes = __ballot_sync(0xffffffffu, fresh);
+        const uint32_t at = n + __popc(votes & ((1u << lane) - 1u));
+        if (n + __popc(votes) > most) return kNoItem;
+        if (fresh) {
+            ent[at].col = e.y;
+            ent[at].flags = 2;
+            ent[at].blk[0] = 0;
+            ent[at].blk[1] = e.x;
+        }
+        n += __popc(votes);
+    }
+    __syncwarp();
+    return n;
+}
+
+// asks for the next item that no CTA has started; the answer arrives on bar with 16 bytes
+__device__ __forceinline__ void clc_request(uint32_t *response, uint64_t *bar)
+{
+    mbar_expect_tx(bar, 16);
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(response)),
+                 "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ uint32_t clc_item(const uint32_t *response)
+{
+    uint32_t ok, x = 0;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b128 r;\n\t"
+        "ld.shared.b128 r, [%2];\n\t"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, _, _, _}, r;\n\t}"
+        : "=r"(ok), "+r"(x)
+        : "r"(smem_u32(response))
+        : "memory");
+    return ok ? x : kNoItem;
+}
+
+// How many pairs the long rows of a head make.  With one LUT for all heads the items of these pairs of all (batch, head)s
+// come before the rest, so that none of them is left for the end; otherwise (batch, head) by (batch, head).
+__device__ __forceinline__ uint32_t long_pairs(const uint2 *lut, uint32_t nb, uint32_t blocks, uint32_t lane)
+{
+    uint32_t n_long = 0;
+    for (uint32_t base = 0; base < nb; base += 32)
+        n_long += __popc(__ballot_sync(0xffffffffu, base + lane < nb && (uint64_t)lut[base + lane].y * nb > 2ull * blocks));
+    return (n_long + 1) / 2;
+}
+
+// Item `id` of a launch over the row pairs of all (batch, head)s, one CTA each: the long pairs of all of them first (with one
+// LUT for all heads), then the rest, head by head; `back`: from the last (batch, head).  Every warp calls it.
+struct ItemAt {
+    uint32_t b, h, own[2];
+};
+__device__ __forceinline__ ItemAt locate_item(const uint2 *lut, uint32_t lut_stride, uint32_t B, uint32_t H, uint32_t nb, uint32_t blocks,
+                                              uint32_t id, uint32_t lane, bool back)
+{
+    const uint32_t npairs = (nb + 1) / 2;
+    const uint32_t first_pairs = lut_stride == 0 ? long_pairs(lut, nb, blocks, lane) : 0, first_items = first_pairs * B * H;
+    const bool first = id < first_items;
+    const uint32_t rest = first ? id : id - first_items, per = first ? first_pairs : npairs - first_pairs;
+    uint32_t at = rest / per;
+    const uint32_t pair = rest - at * per + (first ? 0 : first_pairs);
+    if (back) at = B * H - 1 - at;
+    ItemAt it;
+    it.h = at / B;
+    it.b = at - it.h * B;
+    if (lut_stride == 0 && first_pairs == 0) {                // no long rows: neighbours
+        it.own[0] = 2 * pair;
+        it.own[1] = 2 * pair + 1 < nb ? 2 * pair + 1 : kNoItem;
+    } else {
+        pick_pair(lut + (size_t)it.h * lut_stride, pair, nb, blocks, lane, it.own);
+    }
+    return it;
 }
 
 // ---- host side ------------------------------------------------------------------------------------
