@@ -30,10 +30,11 @@ struct UParams {
     int trans;                 // spmm: 1 = the blocks are used transposed and the LUT walks block columns (TN_OP)
     const float *delta;        // sddmm, gradient mode: [B, L, H] row sums of dO * O
     float scale;               // sddmm, gradient mode
+    uint32_t chunk;            // sddmm: consecutive LUT entries one CTA takes
 };
 
 constexpr int kSdStagesMax = 5;                 // key stages: five without the P tile, four with it (shared memory per CTA)
-constexpr uint32_t kChunk = 32;                 // consecutive LUT entries one CTA takes
+constexpr uint32_t kChunk = 32;                 // consecutive LUT entries one CTA takes at most
 struct SdShared {
     uint64_t in_full[kSdStagesMax], in_empty[kSdStagesMax], s_full[2], s_empty[2], drained, q_full[2], q_empty[2];
     uint32_t tmem_base, abort_flag;
@@ -93,8 +94,8 @@ sddmm_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant_
 
     const uint32_t warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t b = blockIdx.y, h = blockIdx.z;
-    const uint32_t k0 = blockIdx.x * kChunk;
-    const uint32_t T = min(kChunk, p.blocks - k0);
+    const uint32_t k0 = blockIdx.x * p.chunk;
+    const uint32_t T = min(p.chunk, p.blocks - k0);
     const uint32_t L = p.nb * 64;
     const uint2 *lut = p.nn_lut + (size_t)h * p.lut_stride + k0;   // here: the nt_lut
     volatile uint32_t *abort_flag = &st->abort_flag;
@@ -647,6 +648,19 @@ bool tc_sddmm_supported(int ab_dtype, uint32_t bs, const AttnDims &p, const void
            (uint64_t)p.B * (p.nb_a > p.nb_b ? p.nb_a : p.nb_b) * 64 < (1ull << 31);
 }
 
+// Blocks per CTA: the fewest with which the launch is still one wave of two CTAs per SM, which is what shared memory admits,
+// and kChunk for what is longer.  A launch of 544 blocks was CTAs of 32 blocks one after the other: 17.0 us, 6.6 now.  At
+// least 4, under which a CTA is all set-up.  A few CTAs beyond the wave cost more than the shorter ones save: 8576 blocks
+// in 288 CTAs take 20.5 us, in 320 of them 24.1.
+static uint32_t sddmm_chunk(const AttnDims &p)
+{
+    const int sms = device_sm_count(current_device());
+    const uint64_t bh = (uint64_t)p.B * p.H, slots = 2ull * (uint64_t)(sms > 0 ? sms : 1);
+    uint32_t chunk = 4;
+    while (chunk < tc::kChunk && (p.blocks + chunk - 1) / chunk * bh > slots) chunk++;
+    return chunk;
+}
+
 int tc_sddmm(cudaStream_t s, const void *nt_lut, const void *a, const void *b, void *c, int ab_dtype, int c_dtype, const AttnDims &p)
 {
     using namespace tc;
@@ -659,7 +673,7 @@ int tc_sddmm(cudaStream_t s, const void *nt_lut, const void *a, const void *b, v
     // the scores as [B*H*blocks*64 rows, 64] for the TMA stores of 16-bit outputs (unused for fp32 outputs)
     if (make_map_2d(&om, c, (uint64_t)p.B * p.H * p.blocks * 64, 64, c_dtype != SFB_F16, 64)) return 1;
     SFB_REQUIRE((uint64_t)p.B * p.H * p.blocks * 64 < (1ull << 31), "sfb_bst_sgemm_nt: too many blocks for one launch");
-    UParams prm = {(const uint2 *)nt_lut, c, p.B, p.H, p.nb_a, p.blocks, p.lut_stride, c_dtype, is_bf16, 0};
+    UParams prm = {(const uint2 *)nt_lut, c, p.B, p.H, p.nb_a, p.blocks, p.lut_stride, c_dtype, is_bf16, 0, 0, nullptr, 0.f, sddmm_chunk(p)};
     static DeviceOnce once;
     const int dev = current_device();
     if (!once.done(dev)) {
@@ -668,7 +682,7 @@ int tc_sddmm(cudaStream_t s, const void *nt_lut, const void *a, const void *b, v
             return fail("sfb_bst_sgemm_nt: cannot reserve %zu bytes of shared memory", kSddmmGradSmem);
         once.mark(dev);
     }
-    launch_overlapped(sddmm_tc_kernel<false>, dim3((p.blocks + kChunk - 1) / kChunk, p.B, p.H), dim3(320), kSddmmSmem, s, qm, km, om, om, prm);
+    launch_overlapped(sddmm_tc_kernel<false>, dim3((p.blocks + prm.chunk - 1) / prm.chunk, p.B, p.H), dim3(320), kSddmmSmem, s, qm, km, om, om, prm);
     return check_launch("sfb_bst_sgemm_nt");
 }
 
@@ -686,7 +700,7 @@ int tc_sddmm_softmax_grad(cudaStream_t s, const void *nt_lut, const void *dout, 
     if (make_map(&qm, dout, rows, p.H, is_bf16, 64) || make_map(&km, v, rows, p.H, is_bf16, 64) || make_map_2d(&om, ds, prow, 64, is_bf16, 64) ||
         make_map_2d(&pm, pblk, prow, 64, is_bf16, 64))
         return 1;
-    UParams prm = {(const uint2 *)nt_lut, ds, p.B, p.H, p.nb_a, p.blocks, p.lut_stride, dtype, is_bf16, 0, 0, delta, scale};
+    UParams prm = {(const uint2 *)nt_lut, ds, p.B, p.H, p.nb_a, p.blocks, p.lut_stride, dtype, is_bf16, 0, 0, delta, scale, sddmm_chunk(p)};
     static DeviceOnce once;
     const int dev = current_device();
     if (!once.done(dev)) {
@@ -694,7 +708,7 @@ int tc_sddmm_softmax_grad(cudaStream_t s, const void *nt_lut, const void *dout, 
             return fail("sfb_fused_sddmm_softmax_grad: cannot reserve %zu bytes of shared memory", kSddmmGradSmem);
         once.mark(dev);
     }
-    launch_overlapped(sddmm_tc_kernel<true>, dim3((p.blocks + kChunk - 1) / kChunk, p.B, p.H), dim3(320), kSddmmGradSmem, s, qm, km, om, pm, prm);
+    launch_overlapped(sddmm_tc_kernel<true>, dim3((p.blocks + prm.chunk - 1) / prm.chunk, p.B, p.H), dim3(320), kSddmmGradSmem, s, qm, km, om, pm, prm);
     return check_launch("sfb_fused_sddmm_softmax_grad");
 }
 
