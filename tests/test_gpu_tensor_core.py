@@ -355,3 +355,24 @@ def test_few_items_shared_by_the_streams(sfb, B, H, nb, kind, dtype):
     want = sfb.fused_attention(q.float(), k.float(), v.float(), lay, 0.125, use_mask=kind == "causal")
     assert float((got.float() - want).abs().max()) <= 2e-2 * float(want.abs().max())
     assert torch.equal(got.float().abs().amax(-1) == 0, want.abs().amax(-1) == 0)
+
+
+@pytest.mark.parametrize("B,H,nb", [(1, 1, 1), (1, 3, 3), (1, 16, 9), (2, 16, 9), (2, 15, 17), (2, 16, 17)])
+def test_sddmm_blocks_per_cta(sfb, B, H, nb):
+    """Launches of the fewest blocks per CTA, of some in between with a remainder, of the most that one wave takes and of
+    more than one wave; scores and their gradient against fp32."""
+    g = torch.Generator(device="cuda").manual_seed(nb)
+    lay8 = torch.ones(1, nb, nb, dtype=torch.uint8, device="cuda")
+    lay = sfb.BlockLayout(lay8, 64)
+    q, k = (torch.randn(B, nb * 64, H, 64, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    want = torch.einsum("bihd,bjhd->bhij", q.float(), k.float())
+    want = want.reshape(B, H, nb, 64, nb, 64).permute(0, 1, 2, 4, 3, 5).reshape(B, H, lay.blocks, 64, 64)
+    s = sfb.bst_sgemm_nt(q, k, lay, torch.float32)
+    assert float((s - want).abs().max()) <= 1e-3 * 8
+    p = torch.rand(B, H, lay.blocks, 64, 64, device="cuda", generator=g).to(torch.bfloat16)
+    delta = torch.randn(B, nb * 64, H, device="cuda", generator=g)
+    ds = sfb.fused_sddmm_softmax_grad(q, k, p, delta, lay, 0.125).float()
+    rows = delta.permute(0, 2, 1).reshape(B, H, nb, 1, 64, 1).expand(-1, -1, -1, nb, -1, -1).reshape(B, H, lay.blocks, 64, 1)
+    want = p.float() * (want - rows) * 0.125
+    assert sfb.device_status() == 0
+    assert float((ds - want).abs().max()) <= 2.0 ** -7 * float(want.abs().max())
