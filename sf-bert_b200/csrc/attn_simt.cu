@@ -897,7 +897,8 @@ __global__ void __launch_bounds__(tile::kThreads, 3) csr_tile_f32_kernel(const C
     csr_write_bad(a);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane_row(lane), lc = lane_quad(lane);
     const uint32_t tl = a.tiles - 1u - blockIdx.x, h = blockIdx.y, b = blockIdx.z;
-    const uint32_t distinct = a.counts[4 * tl], base = a.counts[4 * tl + 2], top = a.counts[4 * tl + 3], n = distinct + a.counts[4 * tl + 1];
+    const uint32_t *cnt = a.counts + kCsrCounts * tl;
+    const uint32_t distinct = cnt[0], base = cnt[2], top = cnt[3], n = distinct + cnt[1];
     const size_t HD = (size_t)a.H * D, head = (size_t)b * a.L * HD + (size_t)h * D;
     const float *K = (const float *)a.K + head, *V = (const float *)a.V + head;
     const uint32_t n0 = warp * (D / 4);

@@ -177,14 +177,19 @@ __global__ void __launch_bounds__(128) csr_attention_split_kernel(const int32_t 
 // is written out column by column.  A column that a row names twice counts twice, as it does row by row: the second one
 // becomes an entry of its own at the end.  The tile's entries start at its first row's offset in colidx: there are never
 // more of them than elements.  Columns outside the sequence are counted and dropped.
+// HALVES: the distinct columns come in three groups: those that only the tile's first 16 rows have, those of both halves,
+// those of the last 16 rows alone.  Scattered columns mostly belong to one row; the kernels whose warps work for 16 rows
+// (D 128) leave out the group of the other half.
 constexpr uint32_t kPlanThreads = 512;
 constexpr uint32_t kPlanMaxL = 48 * 1024;                    // columns whose masks fit shared memory
+template <bool HALVES>
 __global__ void __launch_bounds__(kPlanThreads) csr_plan_kernel(const int32_t *__restrict__ rowptr, const int32_t *__restrict__ colidx, uint32_t L,
                                                                 uint32_t nnz, uint2 *__restrict__ entries, uint32_t *__restrict__ counts,
                                                                 uint32_t *__restrict__ bad)
 {
     extern __shared__ uint32_t mask[];                       // [L]
-    __shared__ uint32_t warp_count[kPlanThreads / 32], n_twice, n_bad;
+    constexpr uint32_t NG = HALVES ? 3 : 1;                  // groups of columns
+    __shared__ uint32_t warp_count[NG][kPlanThreads / 32], n_twice, n_bad;
     grid_dependency_wait();
     grid_launch_dependents();
     const uint32_t tile = blockIdx.x, row0 = tile * 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -212,30 +217,47 @@ __global__ void __launch_bounds__(kPlanThreads) csr_plan_kernel(const int32_t *_
         }
     }
     __syncthreads();
-    // every warp takes a run of columns: count, prefix over the warps, write
+    // every warp takes a run of columns: count by group, prefix over the groups and warps, write
+    auto group = [](uint32_t m) { return !m ? NG : !HALVES || !(m >> 16) ? 0u : m & 0xffffu ? 1u : 2u; };
     const uint32_t per = ((L + kPlanThreads / 32 - 1) / (kPlanThreads / 32) + 31) & ~31u;
     const uint32_t from = min(warp * per, L), to = min(from + per, L);
-    uint32_t c = 0;
-    for (uint32_t j0 = from; j0 < to; j0 += 32) c += __popc(__ballot_sync(0xffffffffu, j0 + lane < to && mask[j0 + lane] != 0));
-    if (lane == 0) warp_count[warp] = c;
+    uint32_t at[NG] = {}, all[NG] = {};
+    for (uint32_t j0 = from; j0 < to; j0 += 32) {
+        const uint32_t g = group(j0 + lane < to ? mask[j0 + lane] : 0);
+#pragma unroll
+        for (uint32_t k = 0; k < NG; k++) at[k] += __popc(__ballot_sync(0xffffffffu, g == k));
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < NG; k++)
+        if (lane == k) warp_count[k][warp] = at[k];
     __syncthreads();
-    uint32_t at = base, total = 0;
-    for (uint32_t w = 0; w < kPlanThreads / 32; w++) {
-        if (w < warp) at += warp_count[w];
-        total += warp_count[w];
+    uint32_t total = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < NG; k++) {
+        const uint32_t c = lane < kPlanThreads / 32 ? warp_count[k][lane] : 0;
+        at[k] = base + total + __reduce_add_sync(0xffffffffu, lane < warp ? c : 0);
+        all[k] = __reduce_add_sync(0xffffffffu, c);
+        total += all[k];
     }
     for (uint32_t j0 = from; j0 < to; j0 += 32) {
-        const uint32_t m = j0 + lane < to ? mask[j0 + lane] : 0;
-        const uint32_t votes = __ballot_sync(0xffffffffu, m != 0);
-        const uint32_t dst = at + __popc(votes & ((1u << lane) - 1u));
-        if (m && dst < nnz) entries[dst] = make_uint2(j0 + lane, m);
-        at += __popc(votes);
+        const uint32_t m = j0 + lane < to ? mask[j0 + lane] : 0, g = group(m);
+#pragma unroll
+        for (uint32_t k = 0; k < NG; k++) {
+            const uint32_t votes = __ballot_sync(0xffffffffu, g == k), dst = at[k] + __popc(votes & ((1u << lane) - 1u));
+            if (g == k && dst < nnz) entries[dst] = make_uint2(j0 + lane, m);
+            at[k] += __popc(votes);
+        }
     }
     if (threadIdx.x == 0) {
-        counts[4 * tile] = min(total, nnz - base);
-        counts[4 * tile + 1] = min(n_twice, top - min(base, top));
-        counts[4 * tile + 2] = base;
-        counts[4 * tile + 3] = top;
+        uint32_t *c = counts + kCsrCounts * tile;
+        c[0] = min(total, nnz - base);
+        c[1] = min(n_twice, top - min(base, top));
+        c[2] = base;
+        c[3] = top;
+        if (HALVES) {
+            c[4] = all[0];
+            c[5] = all[NG - 1];
+        }
         bad[tile] = n_bad;
     }
 }
@@ -245,18 +267,23 @@ __global__ void __launch_bounds__(kPlanThreads) csr_plan_kernel(const int32_t *_
 // each), with no barrier between them: a warp fetches its chunk's K and V rows into its own two buffers (cp.async, one
 // chunk ahead), multiplies on warp MMAs (m16n8k16), and keeps its own running maximum, sum and output; the four meet at
 // the end.  Warp MMAs rather than tcgen05: the columns of a tile are rows scattered over K and V, and 32 rows is where
-// neighbouring queries still share them; the kernel is bound by the gather and the exponentials.
+// neighbouring queries still share them.
+// The queries are read from shared memory as they are needed and the chunks are small: what bounds the kernel is latency
+// (42 % of the issue slots, L2 16 %), so the registers go to more CTAs (D 128: two per SM became three, 226 -> 170 us for
+// the window pattern at B 2, H 12, L 4096) or keep the accumulators out of local memory (D 64: 114.4 -> 105.8, at four CTAs
+// per SM 119).
 // P enters P.V as two 16-bit terms (the rounded value and what the rounding left), so the product keeps the fp32
 // probabilities to 16 bits (bf16) and 22 bits (fp16).
 template <int D> struct CsrCfg {
     static constexpr int MT = D == 128 ? 1 : 2;              // 16-row tiles per warp
     static constexpr int SPLITS = D == 128 ? 2 : 4;          // warps that take different chunks
-    static constexpr int KC = D == 128 ? 16 : 32;            // columns per chunk
+    static constexpr int KC = D >= 64 ? 16 : 32;             // columns per chunk
     static constexpr uint32_t tile_bytes = KC * D * 2;
-    static constexpr uint32_t warp_bytes = 4 * tile_bytes;   // K and V, two buffers
+    static constexpr int CTAS = D >= 64 ? 3 : 4;             // per SM: what their registers admit
     static constexpr uint32_t o_stride = D + 4;              // floats; the outputs take the buffers' place at the end
-    static constexpr size_t smem = 4 * warp_bytes;
-    static_assert(MT * 16 * o_stride * 4 <= warp_bytes, "the output fits the buffers");
+    static constexpr uint32_t o_bytes = MT * 16 * o_stride * 4, kv_bytes = 4 * tile_bytes;       // K and V, two buffers
+    static constexpr uint32_t warp_bytes = o_bytes > kv_bytes ? o_bytes : kv_bytes;
+    static constexpr size_t smem = 4 * warp_bytes + 32 * D * 2;      // the tile's queries behind the warps' buffers
 };
 __device__ __forceinline__ void ldsm(uint32_t (&r)[4], uint32_t addr)
 {
@@ -270,11 +297,11 @@ template <bool BF16>
 __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
     if (BF16)
-        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
     else
-        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 template <bool BF16>
 __device__ __forceinline__ uint32_t pack16(float a, float b)
@@ -298,7 +325,7 @@ __device__ __forceinline__ float ex2f(float x)
 }
 
 template <bool BF16, int D>
-__global__ void __launch_bounds__(128, D == 128 ? 2 : 3) csr_tile_kernel(const CsrTileArgs a)
+__global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const CsrTileArgs a)
 {
     typedef CsrCfg<D> Cfg;
     constexpr int MT = Cfg::MT, KC = Cfg::KC, NT = KC / 8, CH = D / 8, DN = D / 8;
@@ -310,27 +337,24 @@ __global__ void __launch_bounds__(128, D == 128 ? 2 : 3) csr_tile_kernel(const C
     csr_write_bad(a);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane >> 2, tq = lane & 3;
     const uint32_t tile = a.tiles - 1u - blockIdx.x, h = blockIdx.y, b = blockIdx.z;     // causal patterns: the long rows first
-    const uint32_t distinct = a.counts[4 * tile], twice = a.counts[4 * tile + 1], base = a.counts[4 * tile + 2], top = a.counts[4 * tile + 3];
-    const uint32_t n = distinct + twice, chunks = (n + KC - 1) / KC;
+    const uint32_t *cnt = a.counts + kCsrCounts * tile;
+    const uint32_t distinct = cnt[0], twice = cnt[1], base = cnt[2], top = cnt[3];
     const uint32_t split = MT == 2 ? warp : warp >> 1, rg = MT == 2 ? 0 : warp & 1;        // this warp's chunks and 16-row tile
+    // with 16 rows per warp: not the other half's columns (entries of columns named twice are behind all of them)
+    const uint32_t first = MT == 1 && rg == 1 ? min(cnt[4], distinct) : 0;
+    const uint32_t n = MT == 1 && rg == 0 && twice == 0 ? distinct - min(cnt[5], distinct) : distinct + twice;
+    const uint32_t chunks = (n - first + KC - 1) / KC;
     const size_t HD = (size_t)a.H * D;
     const uint16_t *K = (const uint16_t *)a.K + (size_t)b * a.L * HD + (size_t)h * D, *V = (const uint16_t *)a.V + (size_t)b * a.L * HD + (size_t)h * D;
     uint8_t *buf = sm + warp * Cfg::warp_bytes;
 
-    // Q as A fragments, straight from memory (once)
-    uint32_t q[MT][D / 16][4];
+    uint4 q_piece[CH / 4];                                   // this thread's share of the queries, on its way to shared memory
 #pragma unroll
-    for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-            const uint32_t row = tile * 32 + rg * 16 + mt * 16 + quad + 8 * e;
-            const uint32_t *src = (const uint32_t *)((const uint16_t *)a.Q + ((size_t)b * a.L + row) * HD + (size_t)h * D) + tq;
-#pragma unroll
-            for (int kk = 0; kk < D / 16; kk++) {
-                q[mt][kk][e] = row < a.L ? __ldg(src + kk * 8) : 0u;
-                q[mt][kk][2 + e] = row < a.L ? __ldg(src + kk * 8 + 4) : 0u;
-            }
-        }
+    for (int i = 0; i < CH / 4; i++) {
+        const uint32_t t = i * 128 + threadIdx.x, row = tile * 32 + t / CH;
+        const uint16_t *src = (const uint16_t *)a.Q + ((size_t)b * a.L + row) * HD + (size_t)h * D + t % CH * 8;
+        q_piece[i] = row < a.L ? __ldg((const uint4 *)src) : make_uint4(0u, 0u, 0u, 0u);
+    }
     float o[MT][DN][4], m[MT][2], l[MT][2];
 #pragma unroll
     for (int mt = 0; mt < MT; mt++) {
@@ -342,7 +366,7 @@ __global__ void __launch_bounds__(128, D == 128 ? 2 : 3) csr_tile_kernel(const C
             for (int j = 0; j < 4; j++) o[mt][d][j] = 0.f;
     }
     auto entry = [&](uint32_t c) {
-        const uint32_t i = c * KC + lane;
+        const uint32_t i = first + c * KC + lane;
         return (KC == 32 || lane < KC) && i < n ? csr_entry(a.entries, base, top, distinct, i) : make_uint2(0u, 0u);
     };
     // 16-byte chunk c of row r of a tile sits at chunk c ^ (r % 8) (64-byte rows: c ^ (r / 2 % 4)): no bank twice in a ldmatrix
@@ -359,12 +383,19 @@ __global__ void __launch_bounds__(128, D == 128 ? 2 : 3) csr_tile_kernel(const C
         }
         if (KC == 32 || lane < KC) masks[warp][s][lane % KC] = e.y;
     };
+    const uint32_t qt = (uint32_t)__cvta_generic_to_shared(sm + 4 * Cfg::warp_bytes);
     uint2 e_next = make_uint2(0u, 0u);
     if (split < chunks) {
         issue(entry(split), 0);
         if (split + Cfg::SPLITS < chunks) e_next = entry(split + Cfg::SPLITS);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < CH / 4; i++) {
+        const uint32_t t = i * 128 + threadIdx.x;
+        *(uint4 *)(sm + 4 * Cfg::warp_bytes + place(t / CH, t % CH)) = q_piece[i];
+    }
+    __syncthreads();
     uint32_t s = 0;
     for (uint32_t c = split; c < chunks; c += Cfg::SPLITS, s ^= 1) {
         if (c + Cfg::SPLITS < chunks) {
@@ -384,17 +415,17 @@ __global__ void __launch_bounds__(128, D == 128 ? 2 : 3) csr_tile_kernel(const C
 #pragma unroll
                 for (int j = 0; j < 4; j++) sc[mt][t][j] = 0.f;
 #pragma unroll
-        for (int t = 0; t < NT; t += 2)
+        for (int kk = 0; kk < D / 16; kk++) {
+            uint32_t q[MT][4], f[NT / 2][4];
 #pragma unroll
-            for (int kk = 0; kk < D / 16; kk++) {
-                uint32_t f[4];
-                ldsm(f, kt + place(t * 8 + (lane & 7) + ((lane >> 4) << 3), 2 * kk + ((lane >> 3) & 1)));
+            for (int mt = 0; mt < MT; mt++) ldsm(q[mt], qt + place((rg + mt) * 16 + (lane & 15), 2 * kk + (lane >> 4)));
 #pragma unroll
-                for (int mt = 0; mt < MT; mt++) {
-                    mma16816<BF16>(sc[mt][t], q[mt][kk], f[0], f[1]);
-                    mma16816<BF16>(sc[mt][t + 1], q[mt][kk], f[2], f[3]);
-                }
-            }
+            for (int t = 0; t < NT; t += 2) ldsm(f[t / 2], kt + place(t * 8 + (lane & 7) + ((lane >> 4) << 3), 2 * kk + ((lane >> 3) & 1)));
+#pragma unroll
+            for (int t = 0; t < NT; t++)
+#pragma unroll
+                for (int mt = 0; mt < MT; mt++) mma16816<BF16>(sc[mt][t], q[mt], f[t / 2][2 * (t & 1)], f[t / 2][2 * (t & 1) + 1]);
+        }
         // mask: bit `row` of a column's word
         uint2 mk[NT];
         uint32_t all = 0xffffffffu;
@@ -469,18 +500,15 @@ __global__ void __launch_bounds__(128, D == 128 ? 2 : 3) csr_tile_kernel(const C
                         hi[mt][2 * t + e] = w;
                         lo[mt][2 * t + e] = pack16<BF16>(p0 - r.x, p1 - r.y);
                     }
+            uint32_t f[DN / 2][4];
 #pragma unroll
-            for (int d = 0; d < DN; d += 2) {
-                uint32_t f[4];
-                ldsm_trans(f, vt + place(j * 16 + (lane & 7) + (((lane >> 3) & 1) << 3), d + (lane >> 4)));
+            for (int d = 0; d < DN; d += 2) ldsm_trans(f[d / 2], vt + place(j * 16 + (lane & 7) + (((lane >> 3) & 1) << 3), d + (lane >> 4)));
 #pragma unroll
-                for (int mt = 0; mt < MT; mt++) {
-                    mma16816<BF16>(o[mt][d], hi[mt], f[0], f[1]);
-                    mma16816<BF16>(o[mt][d + 1], hi[mt], f[2], f[3]);
-                    mma16816<BF16>(o[mt][d], lo[mt], f[0], f[1]);
-                    mma16816<BF16>(o[mt][d + 1], lo[mt], f[2], f[3]);
-                }
-            }
+            for (int term = 0; term < 2; term++)
+#pragma unroll
+                for (int d = 0; d < DN; d++)
+#pragma unroll
+                    for (int mt = 0; mt < MT; mt++) mma16816<BF16>(o[mt][d], term ? lo[mt] : hi[mt], f[d / 2][2 * (d & 1)], f[d / 2][2 * (d & 1) + 1]);
         }
         __syncwarp();                                        // the buffer may be filled again
     }
@@ -544,8 +572,8 @@ static int launch_csr_tile(cudaStream_t s, const CsrTileArgs &a, uint32_t B)
     return check_launch("sfb_csr_attention");
 }
 
-// entries of 8 bytes, one per element, then four counts and a bad-column count per tile of 32 rows
-static size_t csr_workspace(uint64_t nnz, uint32_t L) { return nnz * 8 + (size_t)((L + 31) / 32) * 5 * sizeof(uint32_t); }
+// entries of 8 bytes, one per element, then the counts and a bad-column count per tile of 32 rows
+static size_t csr_workspace(uint64_t nnz, uint32_t L) { return nnz * 8 + (size_t)((L + 31) / 32) * (kCsrCounts + 1) * sizeof(uint32_t); }
 
 static int csr_attention_planned(cudaStream_t s, const int32_t *rowptr, const int32_t *colidx, uint32_t nnz, const void *q, const void *k,
                                  const void *v, void *o, int dtype, uint32_t B, uint32_t L, uint32_t H, uint32_t d, float scale, uint32_t *bad,
@@ -557,12 +585,13 @@ static int csr_attention_planned(cudaStream_t s, const int32_t *rowptr, const in
     static DeviceOnce once;
     const int dev = current_device();
     if (!once.done(dev)) {
-        if (cudaFuncSetAttribute(csr_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kPlanMaxL * sizeof(uint32_t))) != cudaSuccess)
+        if (cudaFuncSetAttribute(csr_plan_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kPlanMaxL * sizeof(uint32_t))) != cudaSuccess ||
+            cudaFuncSetAttribute(csr_plan_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kPlanMaxL * sizeof(uint32_t))) != cudaSuccess)
             return fail("sfb_csr_attention: cannot reserve %u bytes of shared memory", kPlanMaxL * 4u);
         once.mark(dev);
     }
-    launch_overlapped(csr_plan_kernel, dim3(tiles), dim3(kPlanThreads), L * sizeof(uint32_t), s, rowptr, colidx, L, nnz, entries, counts, counts + 4 * tiles);
-    const CsrTileArgs a = {entries, counts, counts + 4 * tiles, q, k, v, o, L, H, tiles, B * H, scale * 1.4426950408889634f, bad};
+    launch_overlapped(dtype != SFB_F32 && d == 128 ? csr_plan_kernel<true> : csr_plan_kernel<false>, dim3(tiles), dim3(kPlanThreads), L * sizeof(uint32_t), s, rowptr, colidx, L, nnz, entries, counts, counts + kCsrCounts * tiles);
+    const CsrTileArgs a = {entries, counts, counts + kCsrCounts * tiles, q, k, v, o, L, H, tiles, B * H, scale * 1.4426950408889634f, bad};
     if (dtype == SFB_F32) return csr_tile_f32(s, a, B, d);
 #define CSR_TILE(BF) return d == 32 ? launch_csr_tile<BF, 32>(s, a, B) : d == 64 ? launch_csr_tile<BF, 64>(s, a, B) : launch_csr_tile<BF, 128>(s, a, B)
     if (dtype == SFB_BF16) CSR_TILE(true);

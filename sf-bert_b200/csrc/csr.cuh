@@ -4,9 +4,12 @@
 
 namespace sfb {
 
+constexpr uint32_t kCsrCounts = 6;
 struct CsrTileArgs {
     const uint2 *entries;            // (column, mask of the tile's rows that have it)
-    const uint32_t *counts, *bad;    // per tile: [distinct columns, entries of columns named twice, first entry, behind the last], bad columns
+    // per tile: [distinct columns, entries of columns named twice, first entry, behind the last; for 16-bit operands with
+    // d 128: distinct columns of the first 16 rows alone, of the last 16 alone], bad columns
+    const uint32_t *counts, *bad;
     const void *Q, *K, *V;
     void *O;
     uint32_t L, H, tiles, BH;

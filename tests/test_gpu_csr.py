@@ -106,3 +106,27 @@ def test_csr_bad_columns_are_counted_per_batch_and_head(sfb):
     o, bad = sfb.csr_attention(q, q, q, rowptr, colidx, 1.0)
     assert int(bad.item()) == 3 * 2 * 3
     assert torch.equal(o, q)
+
+
+@pytest.mark.parametrize("upper,lower,both", [(0, 0, 40), (37, 0, 0), (0, 5, 0), (16, 16, 16), (3, 70, 1), (50, 1, 33)])
+@pytest.mark.parametrize("twice", [False, True])
+def test_csr_columns_of_half_a_tile(sfb, oracle, upper, lower, both, twice):
+    """Tiles whose columns belong to the first 16 rows, to the last 16, or to both, in any proportion, with and without
+    columns named twice, at the head width whose warps work for half a tile each."""
+    L, d = 128, 128
+    rng = np.random.RandomState(upper + lower)
+    rows = []
+    for t in range(L // 32):
+        cols = rng.permutation(L)[:upper + lower + both]
+        u, w, b = np.split(cols, [upper, upper + lower])
+        for r in range(32):
+            c = np.r_[u if r < 16 else w, b]
+            c = c[rng.rand(len(c)) < (1.0 if r % 16 == 3 else 0.3)]
+            rows.append(np.r_[c, c[:1] if twice and r % 8 == 3 else []].astype(np.int32))
+    rowptr = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+    colidx = np.concatenate(rows).astype(np.int32)
+    q, k, v = (torch.from_numpy(oracle.fill_normal((1, L, 2, d), 640 + i)).cuda().to(torch.bfloat16) for i in range(3))
+    o, bad = sfb.csr_attention(q, k, v, torch.from_numpy(rowptr).cuda(), torch.from_numpy(colidx).cuda(), 0.125)
+    want = oracle.csr_attention(q.float().cpu().numpy(), k.float().cpu().numpy(), v.float().cpu().numpy(), rowptr, colidx, np.float32(0.125))
+    assert int(bad.item()) == 0
+    assert np.abs(o.float().cpu().numpy() - want).max() <= 2e-2 * np.abs(want).max()
