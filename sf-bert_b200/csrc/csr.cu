@@ -180,7 +180,10 @@ __global__ void __launch_bounds__(128) csr_attention_split_kernel(const int32_t 
 // HALVES: the distinct columns come in three groups: those that only the tile's first 16 rows have, those of both halves,
 // those of the last 16 rows alone.  Scattered columns mostly belong to one row; the kernels whose warps work for 16 rows
 // (D 128) leave out the group of the other half.
-constexpr uint32_t kPlanThreads = 512;
+// A warp per row, whose elements are on their way at once (102.4 us with the tiles at B 2, H 12, L 4096 against 106 with
+// two rows per warp).  The tiles' launch is not let in early: their CTAs would crowd the SMs that the plan left free and stay
+// there (128 tiles, B 1, H 1: 24.4 us, 17.4 like this).
+constexpr uint32_t kPlanThreads = 1024;
 constexpr uint32_t kPlanMaxL = 48 * 1024;                    // columns whose masks fit shared memory
 template <bool HALVES>
 __global__ void __launch_bounds__(kPlanThreads) csr_plan_kernel(const int32_t *__restrict__ rowptr, const int32_t *__restrict__ colidx, uint32_t L,
@@ -191,7 +194,6 @@ __global__ void __launch_bounds__(kPlanThreads) csr_plan_kernel(const int32_t *_
     constexpr uint32_t NG = HALVES ? 3 : 1;                  // groups of columns
     __shared__ uint32_t warp_count[NG][kPlanThreads / 32], n_twice, n_bad;
     grid_dependency_wait();
-    grid_launch_dependents();
     const uint32_t tile = blockIdx.x, row0 = tile * 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rows = min(32u, L - row0);
     const uint32_t base = min((uint32_t)max(rowptr[row0], 0), nnz), top = min((uint32_t)max(rowptr[row0 + rows], 0), nnz);
