@@ -56,7 +56,9 @@ __device__ __forceinline__ void tile_coords(const GParams &p, uint32_t t, uint32
 // Four of the bias values of the 128 columns from n0 on, for this lane.  The epilogue reads them from shared memory: from
 // global memory they cost it a trip to the cache per 16 columns, one after another.  Each epilogue warp keeps the values
 // of its tile (fetched a tile ahead) in the slot of its column half and the tile's accumulator; the four warps that
-// share a slot write the same values, and none is more than one tile ahead of another, so two slots are enough.
+// share a slot write the same values.  A warp writes the slot of tile i only once tile i's accumulator is full: that
+// accumulator was emptied by every warp at tile i - 2, so none still reads the slot's earlier values.  (Written before that
+// wait, a warp whose rows lie beyond the output, and which therefore stores nothing, could be two tiles ahead.)
 __device__ __forceinline__ float4 fetch_bias(const GParams &p, uint32_t n0, uint32_t lane)
 {
     return p.bias && n0 + lane * 4 < p.N ? __ldg((const float4 *)(p.bias + n0 + lane * 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -274,10 +276,10 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
             const uint32_t buf = i % kGBufs;
             const uint32_t n0 = (t / p.tiles_m) * kGBN + chalf * 128;
             float *bias = bias_s + ((i & 1) * 2 + chalf) * 128;
+            if (!mbar_wait_warp(&st->acc_full[buf], (i / kGBufs) & 1, abort_flag, 44)) break;
             *(float4 *)(bias + lane * 4) = next;
             __syncwarp();
             if (t + gridDim.x < n_tiles) next = fetch_bias(p, ((t + gridDim.x) / p.tiles_m) * kGBN + chalf * 128, lane);
-            if (!mbar_wait_warp(&st->acc_full[buf], (i / kGBufs) & 1, abort_flag, 44)) break;
             tcgen05_fence_after();
             drain_rows(p, tmem + buf * kGBN + chalf * 128 + lane_field, bias, (t % p.tiles_m) * kGBM + r, n0);
             tcgen05_fence_before();
@@ -500,13 +502,13 @@ linear_tc_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_con
             const uint32_t n0 = tn * kGBN + chalf * 128;
             const uint32_t m0 = tm * 256 + rank * kGBM;
             float *bias = bias_s + (buf * 2 + chalf) * 128;
+            if (!mbar_wait_warp(&st->acc_full[buf], (i >> 1) & 1, abort_flag, 54)) break;
             *(float4 *)(bias + lane * 4) = next;
             __syncwarp();
             if (t + pairs < n_tiles) {
                 tile_coords(p, t + pairs, tm, tn);
                 next = fetch_bias(p, tn * kGBN + chalf * 128, lane);
             }
-            if (!mbar_wait_warp(&st->acc_full[buf], (i >> 1) & 1, abort_flag, 54)) break;
             tcgen05_fence_after();
             drain_rows_staged(p, &omap, tmem + buf * kGBN + chalf * 128 + lane_field, staging + (warp - 2) * 4096, bias, m0 + quarter * 32, n0, lane);
             tcgen05_fence_before();

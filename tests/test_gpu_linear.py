@@ -109,6 +109,26 @@ def test_linear_on_cta_pairs(sfb, dtype, m, n, k, act, transposed):
     assert float((got.float() - want).abs().max()) <= 2e-2 * float(want.abs().max())
 
 
+@pytest.mark.parametrize("m,n,k", [
+    (20, 592 * 256, 64),             # one-CTA tiles: only the first of the four epilogue warps of a column half has rows to store
+    (160, 592 * 256, 256),           # CTA pairs: the odd CTA has 32 rows
+    (20, 600 * 256 - 112, 64),       # the last column tile is ragged too
+])
+def test_linear_bias_over_many_tiles_of_few_rows(sfb, m, n, k):
+    """Several tiles per CTA, one or two k-blocks each, and epilogue warps without rows: those run ahead of the others as far
+    as the accumulators let them, and must not replace the bias of a tile that is still being written.  The bias steps by 8
+    from one column tile to the next, far above the rounding of the result."""
+    gen = torch.Generator(device="cuda").manual_seed(78)
+    x = torch.randn(m, k, device="cuda", generator=gen).to(torch.bfloat16)
+    w = (0.01 * torch.randn(k, n, device="cuda", generator=gen)).to(torch.bfloat16)
+    b = (torch.arange(n, device="cuda") // 256 % 7 * 8).float()
+    want = x.float() @ w.float() + b
+    for _ in range(5):
+        got = sfb.linear(x, w, b)
+        assert float((got.float() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max()) + 1e-3
+    assert sfb.device_status() == 0
+
+
 def test_linear_rejects_what_it_cannot_do(sfb):
     x = torch.zeros(16, 64, device="cuda")
     w = torch.zeros(64, 64, device="cuda")
