@@ -95,6 +95,12 @@ inline long integer(PyObject *o)
     if (x == -1 && PyErr_Occurred()) throw Raised();
     return x;
 }
+// a size that something is divided by: 0 is Python's ZeroDivisionError, and never reaches the division (which would kill the process)
+inline int64_t divisor(int64_t n)
+{
+    if (n == 0) raise(PyExc_ZeroDivisionError, "division by a size that is 0");
+    return n;
+}
 inline at::ScalarType scalar_type(int tag)
 {
     return tag == SFB_F32 ? at::kFloat : tag == SFB_BF16 ? at::kBFloat16 : at::kHalf;
@@ -180,7 +186,7 @@ at::Tensor rowdot(const at::Tensor &a, const at::Tensor &b)
 {
     require(a.sizes() == b.sizes() && a.scalar_type() == b.scalar_type() && a.is_contiguous() && b.is_contiguous(),
             "a and b must be contiguous and alike");
-    const int64_t d = a.size(-1);
+    const int64_t d = divisor(a.size(-1));
     at::Tensor out = empty(a.sizes().slice(0, a.dim() - 1), at::kFloat, a);
     check(L.sfb_rowdot(stream(), (float *)ptr(out), ptr(a), ptr(b), (uint64_t)(a.numel() / d), (uint32_t)d, tag(a)));
     return out;
@@ -211,6 +217,7 @@ at::Tensor fused_sddmm_softmax(const at::Tensor &q, const at::Tensor &k, const L
 void linear_into(const at::Tensor &x, const at::Tensor &w, const void *bias, int act, bool nt, const at::Tensor &out)
 {
     const int64_t k = w.size(nt ? 1 : 0), n = w.size(nt ? 0 : 1);
+    divisor(k);
     require(x.size(-1) == k && x.scalar_type() == w.scalar_type() && x.is_contiguous() && w.is_contiguous(),
             "x and w must be contiguous, of one type and of matching sizes");
     auto f = nt ? L.sfb_linear_nt : L.sfb_linear;
@@ -220,6 +227,7 @@ void linear_into(const at::Tensor &x, const at::Tensor &w, const void *bias, int
 at::Tensor linear(const at::Tensor &x, const at::Tensor &w, const void *bias, int act, bool nt)
 {
     const int64_t n = w.size(nt ? 0 : 1);
+    divisor(w.size(nt ? 1 : 0));
     at::Tensor out;
     if (x.dim() == 2) {
         out = empty({x.size(0), n}, x.scalar_type(), x);
@@ -319,7 +327,7 @@ FUNCTION(py_csr_attention, 6)
     Ref r(wrap(o)), n(wrap(bad));
     return PyTuple_Pack(2, r.o, n.o);
 }
-inline float scale_or(PyObject *o, uint32_t d) { return o == Py_None ? (float)(1.0 / std::sqrt((double)d)) : (float)number(o); }
+inline float scale_or(PyObject *o, uint32_t d) { return o == Py_None ? (float)(1.0 / std::sqrt((double)divisor(d))) : (float)number(o); }
 // (q, k, v, lay, scale, use_mask, out)
 FUNCTION(py_fused_attention, 7)
 {
@@ -390,10 +398,11 @@ FUNCTION(py_encoder_layer, 6)
     const at::Tensor &x = tensor(a[0]);
     PyObject *w = a[1];
     const Lay lay(a[2]);
-    const int64_t heads = integer(a[3]), m = x.size(0), hidden = x.size(1), d = hidden / heads, len = (int64_t)lay.nb * lay.bs;
+    require(x.dim() == 2, "expected an [m, hidden] tensor");
+    const int64_t heads = divisor(integer(a[3])), m = x.size(0), hidden = x.size(1), d = hidden / heads, len = divisor((int64_t)lay.nb * lay.bs);
     const bool pre = truth(a[4]);
     const float scale = (float)number(a[5]);
-    require(x.is_contiguous() && hidden % heads == 0 && m % len == 0, "x must be contiguous, whole sequences of whole heads");
+    require(x.is_contiguous() && heads > 0 && hidden % heads == 0 && m % len == 0, "x must be contiguous, whole sequences of whole heads");
     const int64_t B = m / len;
     require(lay.heads == 1 || lay.heads == heads, "the layout's heads are neither 1 nor the tensor's");
     Ref qkv(PyObject_CallMethodNoArgs(w, names[n_fused_qkv]));
