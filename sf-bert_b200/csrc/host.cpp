@@ -214,10 +214,17 @@ at::Tensor fused_sddmm_softmax(const at::Tensor &q, const at::Tensor &k, const L
     return y;
 }
 
+// the two dimensions of a weight: k and n
+inline void weight_dims(const at::Tensor &w, bool nt, int64_t &k, int64_t &n)
+{
+    require(w.dim() == 2, "the weight must have two dimensions");
+    k = divisor(w.size(nt ? 1 : 0));
+    n = w.size(nt ? 0 : 1);
+}
 void linear_into(const at::Tensor &x, const at::Tensor &w, const void *bias, int act, bool nt, const at::Tensor &out)
 {
-    const int64_t k = w.size(nt ? 1 : 0), n = w.size(nt ? 0 : 1);
-    divisor(k);
+    int64_t k, n;
+    weight_dims(w, nt, k, n);
     require(x.size(-1) == k && x.scalar_type() == w.scalar_type() && x.is_contiguous() && w.is_contiguous(),
             "x and w must be contiguous, of one type and of matching sizes");
     auto f = nt ? L.sfb_linear_nt : L.sfb_linear;
@@ -226,8 +233,8 @@ void linear_into(const at::Tensor &x, const at::Tensor &w, const void *bias, int
 
 at::Tensor linear(const at::Tensor &x, const at::Tensor &w, const void *bias, int act, bool nt)
 {
-    const int64_t n = w.size(nt ? 0 : 1);
-    divisor(w.size(nt ? 1 : 0));
+    int64_t k, n;
+    weight_dims(w, nt, k, n);
     at::Tensor out;
     if (x.dim() == 2) {
         out = empty({x.size(0), n}, x.scalar_type(), x);

@@ -24,6 +24,9 @@ REFUSE = [
     "sfb.encoder_layer_tensor(torch.zeros(256, 64), w, lay(), 3, 'post', 0.125)",
     "sfb.encoder_layer_tensor(torch.zeros(255, 64), w, lay(), 1, 'post', 0.125)",
     "sfb.encoder_layer_tensor(torch.zeros(1, 256, 64), w, lay(), 1, 'post', 0.125)",
+    "sfb.linear(torch.zeros(2, 64), torch.zeros(64, 32, 1))",
+    "sfb.linear(torch.zeros(2, 64), torch.zeros(64))",
+    "sfb.linear_nt(torch.zeros(2, 64), torch.zeros(32, 64, 1))",
 ]
 
 # one child that loads the package once and forks for every call
@@ -67,5 +70,5 @@ def test_sizes_of_zero_that_something_is_divided_by(said, call):
 
 
 @pytest.mark.parametrize("call", REFUSE)
-def test_encoder_layer_shapes_that_do_not_fit(said, call):
+def test_shapes_that_do_not_fit(said, call):
     assert said[call] == "AssertionError"
