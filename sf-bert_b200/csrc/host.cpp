@@ -420,6 +420,7 @@ FUNCTION(py_encoder_layer, 6)
     const float *bo = (const float *)attr_ptr(w, n_bo), *b1 = (const float *)attr_ptr(w, n_b1), *b2 = (const float *)attr_ptr(w, n_b2),
                 *g1 = (const float *)attr_ptr(w, n_g1), *be1 = (const float *)attr_ptr(w, n_be1), *g2 = (const float *)attr_ptr(w, n_g2),
                 *be2 = (const float *)attr_ptr(w, n_be2);
+    require(wqkv.dim() == 2 && wo.dim() == 2 && w1.dim() == 2 && w2.dim() == 2, "a weight of the layer does not have two dimensions");
     const int64_t ffn = w1.size(1);
     require(wqkv.size(0) == hidden && wqkv.size(1) == 3 * hidden && wo.size(0) == hidden && wo.size(1) == hidden && w1.size(0) == hidden &&
                 w2.size(0) == ffn && w2.size(1) == hidden && wqkv.is_contiguous() && wo.is_contiguous() && w1.is_contiguous() && w2.is_contiguous(),

@@ -24,6 +24,9 @@ REFUSE = [
     "sfb.encoder_layer_tensor(torch.zeros(256, 64), w, lay(), 3, 'post', 0.125)",
     "sfb.encoder_layer_tensor(torch.zeros(255, 64), w, lay(), 1, 'post', 0.125)",
     "sfb.encoder_layer_tensor(torch.zeros(1, 256, 64), w, lay(), 1, 'post', 0.125)",
+    "sfb.encoder_layer_tensor(torch.zeros(256, 64), layer(w1=torch.zeros(64, 128, 1)), lay(), 1, 'post', 0.125)",
+    "sfb.encoder_layer_tensor(torch.zeros(256, 64), layer(wo=torch.zeros(64, 64, 1)), lay(), 1, 'post', 0.125)",
+    "sfb.encoder_layer_tensor(torch.zeros(256, 64), layer(w2=torch.zeros(128)), lay(), 1, 'post', 0.125)",
     "sfb.linear(torch.zeros(2, 64), torch.zeros(64, 32, 1))",
     "sfb.linear(torch.zeros(2, 64), torch.zeros(64))",
     "sfb.linear_nt(torch.zeros(2, 64), torch.zeros(32, 64, 1))",
@@ -38,6 +41,12 @@ import __graft_entry__ as ge
 sfb = ge.load_package()
 def lay(nb=4, bs=64):
     return types.SimpleNamespace(heads=1, nb=nb, block_size=bs, blocks=nb, nn_max=1, nn_lut=None, mask_np=None)
+def layer(**changed):
+    z = torch.zeros
+    w = dict(fused_qkv=lambda: (z(64, 192), z(192)), wo=z(64, 64), w1=z(64, 128), w2=z(128, 64), b1=z(128))
+    w.update({n: z(64) for n in ("bo", "b2", "g1", "g2", "be1", "be2")})
+    w.update(changed)
+    return types.SimpleNamespace(**w)
 w = types.SimpleNamespace()
 for call in json.load(sys.stdin):
     r, wr = os.pipe()
