@@ -770,8 +770,9 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
 
 }  // namespace tc
 
+// *refused: the device or partition cannot place the clusters, nothing was launched
 template <int BN, int ST>
-static int launch_split(cudaStream_t s, const CUtensorMap &am, const void *w, const tc::GParams &g, uint32_t split, int dev)
+static int launch_split(cudaStream_t s, const CUtensorMap &am, const void *w, const tc::GParams &g, uint32_t split, int dev, bool *refused)
 {
     using namespace tc;
     static DeviceOnce once;
@@ -785,8 +786,10 @@ static int launch_split(cudaStream_t s, const CUtensorMap &am, const void *w, co
     GParams prm = g;
     prm.tiles_m = (g.M + kGBM - 1) / kGBM;
     prm.tiles_n = (g.N + BN - 1) / BN;
-    launch_overlapped_cluster(linear_tc_split_kernel<BN, ST>, dim3(prm.tiles_m * prm.tiles_n * split), dim3(256), SCfg<BN, ST>::smem, s, split, am, bm,
-                              prm, split);
+    const cudaError_t e = launch_overlapped_cluster(linear_tc_split_kernel<BN, ST>, dim3(prm.tiles_m * prm.tiles_n * split), dim3(256),
+                                                    SCfg<BN, ST>::smem, s, split, am, bm, prm, split);
+    *refused = split > 1 && e != cudaSuccess;
+    if (*refused) { (void)cudaGetLastError(); return 0; }
     return check_launch("sfb_linear");
 }
 
@@ -864,10 +867,13 @@ static int linear_product(cudaStream_t s, void *out, const void *x, const void *
     const LinearPlan plan = plan_linear(m, n, k, (uint32_t)sms);
     const uint32_t tiles_n = (n + kGBN - 1) / kGBN;
     GParams prm = {out, bias, m, n, k, 0, tiles_n, is_bf16, act, w_transposed ? 1 : 0, 1, nullptr};
+    // a device or a partition that cannot place clusters refuses their launch: the single-CTA kernel at the end takes over
     if (plan.kind == 2) {
-        prm.resid = resid;
-        *added = true;
-        return plan.bn == 64 ? launch_split<64, 8>(s, am, w, prm, plan.split, dev) : launch_split<128, 6>(s, am, w, prm, plan.split, dev);
+        GParams few = prm;
+        few.resid = resid;
+        bool refused = false;
+        const int rc = plan.bn == 64 ? launch_split<64, 8>(s, am, w, few, plan.split, dev, &refused) : launch_split<128, 6>(s, am, w, few, plan.split, dev, &refused);
+        if (!refused) { *added = true; return rc; }
     }
     if (plan.kind == 1) {
         CUtensorMap bp;
@@ -884,9 +890,9 @@ static int linear_product(cudaStream_t s, void *out, const void *x, const void *
         prm.band = tiles_n < kPBand ? tiles_n : kPBand;
         const uint64_t pair_tiles = (uint64_t)prm.tiles_m * tiles_n;
         const uint32_t pairs = pair_tiles < (uint64_t)(sms / 2) ? (uint32_t)pair_tiles : (uint32_t)(sms / 2);
-        launch_overlapped(linear_tc_pair_kernel, dim3(2 * pairs), dim3(320), kPSmem, s, am, bp, om, prm);
-        // a device or a partition that cannot place the clusters refuses the launch: the single-CTA kernel takes over
-        if (cudaGetLastError() == cudaSuccess) { clear_error(); return 0; }
+        if (launch_overlapped(linear_tc_pair_kernel, dim3(2 * pairs), dim3(320), kPSmem, s, am, bp, om, prm) == cudaSuccess)
+            return check_launch("sfb_linear");
+        (void)cudaGetLastError();
     }
     if (w_transposed ? make_map_2d(&bm, w, n, k, is_bf16, kGBN) : make_map_2d(&bm, w, k, n, is_bf16, kGBK)) return 1;
     static DeviceOnce once;

@@ -1,5 +1,9 @@
 """GPU parity of the tcgen05 dense projection (sfb_linear, sfb_linear_nt) and of the embedding front end against the CPU oracle.  Tolerance: 16-bit operands with
 fp32 accumulation, 2e-2 relative to the largest reference value (the output itself is rounded to 16 bits)."""
+import ctypes
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -39,7 +43,8 @@ def test_linear_against_oracle(sfb, oracle, dtype, m, n, k, act, with_bias):
 @pytest.mark.parametrize("m,n,k,act", [
     (1, 16, 8, 0),                   # the smallest: one row, one column group, an eighth of a k-block
     (129, 80, 72, 1),                # one row and 16 columns into the second tiles
-    (64, 192, 520, 1),               # nine k-blocks over four CTAs per tile
+    (64, 192, 520, 1),               # nine k-blocks in one CTA per tile
+    (64, 192, 2056, 1),              # 33 k-blocks over four CTAs per tile, one of them with nine
     (320, 768, 3072, 0),             # two CTAs per 128 x 64 tile
     (640, 1040, 4096, 1),            # two CTAs per 128 x 128 tile, the last one 16 columns wide
     (2048, 1024, 1032, 0),           # 128 x 128 tiles, eight elements into the last k-block
@@ -127,6 +132,42 @@ def test_linear_bias_over_many_tiles_of_few_rows(sfb, m, n, k):
         got = sfb.linear(x, w, b)
         assert float((got.float() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max()) + 1e-3
     assert sfb.device_status() == 0
+
+
+@pytest.fixture(scope="module")
+def refusing(tmp_path_factory):
+    """The projections built so that every launch of a cluster is refused (refused_clusters.cu)."""
+    out = str(tmp_path_factory.mktemp("refused") / "refused.so")
+    here = os.path.dirname(os.path.abspath(__file__))
+    subprocess.run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-shared", "-Xcompiler", "-fPIC",
+                    os.path.join(here, "refused_clusters.cu"), "-o", out], check=True)
+    lib = ctypes.CDLL(out)
+    lib.linear_refused.argtypes = [ctypes.c_void_p] * 6 + [ctypes.c_uint] * 3 + [ctypes.c_int] * 2 + [ctypes.POINTER(ctypes.c_int)]
+    return lib
+
+
+@pytest.mark.parametrize("m,n,k,act,transposed,residual", [
+    (320, 768, 3072, 0, False, False),       # clusters of two on 128 x 64 tiles
+    (320, 768, 3072, 0, False, True),        # their residual, which the kernel that takes over leaves to a pass of its own
+    (64, 192, 2056, 1, True, False),         # clusters of four
+    (640, 1040, 4096, 0, True, False),       # clusters of two on 128 x 128 tiles
+    (8192, 752, 1032, 1, False, False),      # CTA pairs
+])
+def test_linear_where_clusters_are_refused(sfb, refusing, m, n, k, act, transposed, residual):
+    gen = torch.Generator(device="cuda").manual_seed(79)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen).to(torch.bfloat16)
+    x, w, b = rn(m, k), rn(*((n, k) if transposed else (k, n))), torch.randn(n, device="cuda", generator=gen)
+    r, out, n_refused = rn(m, n) if residual else None, torch.empty(m, n, device="cuda", dtype=torch.bfloat16), ctypes.c_int(0)
+    p = lambda t: None if t is None else t.data_ptr()
+    rc = refusing.linear_refused(torch.cuda.current_stream().cuda_stream, p(out), p(x), p(w), p(b), p(r), m, n, k, act, int(transposed), ctypes.byref(n_refused))
+    assert rc == 0 and n_refused.value > 0
+    t = x.float() @ (w.t() if transposed else w).float() + b
+    want = t * torch.sigmoid(1.702 * t) if act else t
+    if residual:
+        want = want + r.float()
+    assert float((out.float() - want).abs().max()) <= 2e-2 * float(want.abs().max())
+    status = ctypes.c_uint(1)
+    assert refusing.linear_status(ctypes.byref(status)) == 0 and status.value == 0
 
 
 def test_linear_rejects_what_it_cannot_do(sfb):
