@@ -454,20 +454,29 @@ __global__ void __launch_bounds__(256) bias_gelu_kernel(void *out, const void *x
 // in flight per step, their ids requested one step ahead.  A warp covers 512 contiguous bytes of a row.  An id outside
 // [0, vocab) gives a row of zeros (plus pos) and is counted in *bad_ids -- no out-of-bounds read.
 constexpr int kEmbUnroll = 4;
+constexpr uint32_t kNoColumn = 0xffffffffu;
+// Who counts the ids outside the table.  Up to this many ids: one CTA beside the others, which reads them all and writes the
+// count, so that nothing has to clear it first.  It reads 2048 ids per trip of about half a microsecond, one after the other,
+// so beyond that the threads that read the ids anyway add to a counter cleared by a memset in front of the kernel, which costs
+// the overlap with the kernel before.  Measured (bf16, hidden 8 / 64 / 768, calls back to back), one CTA against memset: 4096
+// ids 2.1 / 2.1 / 4.2 against 5.4 / 4.5 / 8.2 us, 16384 5.3 / 5.5 / 7.1 against 5.6 / 6.2 / 10.3, 32768 9.6 / 10.1 / 17.3
+// against 5.7 / 6.2 / 14.4, a million at hidden 8 / 64 271 / 275 against 11 / 27.
+constexpr uint64_t kEmbOneCtaIds = 16384;
 template <int DT>
 __global__ void __launch_bounds__(256) embedding_kernel(void *__restrict__ out, const void *__restrict__ table,
                                                        const int32_t *__restrict__ ids, const void *__restrict__ pos, uint32_t batch,
                                                        uint32_t per_cta_y, uint32_t seq_len, uint32_t hidden, uint32_t vocab,
-                                                       uint32_t *bad_ids)
+                                                       uint32_t *bad_ids, uint32_t count_column)
 {
     grid_dependency_wait();
     grid_launch_dependents();
     constexpr int N = Vec8<DT>::N, U = kEmbUnroll;
     constexpr int ESZ = 16 / N;
     const uint32_t per_row = hidden / N;                                   // 16-byte pieces per row
-    if (blockIdx.x == gridDim.x - 1) {
+    const bool count_here = bad_ids && count_column == kNoColumn;          // the counter has been cleared on the stream
+    if (blockIdx.x == count_column) {
         // the extra column of CTAs: its first one counts the ids outside the table (nobody has to clear the counter first)
-        if (blockIdx.y || !bad_ids) return;
+        if (blockIdx.y) return;
         const uint32_t total = batch * seq_len;                            // < 2^31 (checked by the host)
         uint32_t bad = 0;
         for (uint32_t t = threadIdx.x; t < total; t += 256 * 8) {
@@ -501,6 +510,7 @@ __global__ void __launch_bounds__(256) embedding_kernel(void *__restrict__ out, 
         for (int u = 0; u < U; u++) id[u] = b0 + u < b_end ? __ldg(ids + (size_t)(b0 + u) * seq_len + l) : -1;
     };
     int32_t id[U], id_next[U];
+    uint32_t bad = 0;
     if (b_begin < b_end) fetch_ids(b_begin, id);
     for (uint32_t b0 = b_begin; b0 < b_end; b0 += U) {
         uint4 tv[U];
@@ -515,6 +525,7 @@ __global__ void __launch_bounds__(256) embedding_kernel(void *__restrict__ out, 
 #pragma unroll
         for (int u = 0; u < U; u++) {
             if (b0 + u < b_end) {
+                bad += !ok[u];
                 float v[N];
                 Vec8<DT>::decode(v, tv[u]);
 #pragma unroll
@@ -524,6 +535,7 @@ __global__ void __launch_bounds__(256) embedding_kernel(void *__restrict__ out, 
             id[u] = id_next[u];
         }
     }
+    if (count_here && col == 0 && bad) atomicAdd(bad_ids, bad);            // one thread per token position counts
 }
 
 // out[row] = sum over the row of a * b: rows of d elements, 8 lanes per row (16-byte accesses, shuffle reduction).
@@ -576,10 +588,16 @@ int embedding_lookup(cudaStream_t s, void *out, const void *table, const int32_t
     if (split > 65535u) split = 65535u;
     if (split < 1) split = 1;
     const uint32_t per_y = (batch + split - 1) / split;
-    const dim3 grid((unsigned)ctas_x + 1, (batch + per_y - 1) / per_y);
-    if (dtype == SFB_F32) launch_overlapped(embedding_kernel<SFB_F32>, grid, dim3(256), 0, s, out, table, ids, pos, batch, per_y, seq_len, hidden, vocab, bad_ids);
-    else if (dtype == SFB_BF16) launch_overlapped(embedding_kernel<SFB_BF16>, grid, dim3(256), 0, s, out, table, ids, pos, batch, per_y, seq_len, hidden, vocab, bad_ids);
-    else launch_overlapped(embedding_kernel<SFB_F16>, grid, dim3(256), 0, s, out, table, ids, pos, batch, per_y, seq_len, hidden, vocab, bad_ids);
+    const bool one_cta = bad_ids && (uint64_t)batch * seq_len <= kEmbOneCtaIds;
+    const uint32_t column = one_cta ? (uint32_t)ctas_x : kNoColumn;
+    if (bad_ids && !one_cta) {
+        const cudaError_t e = cudaMemsetAsync(bad_ids, 0, sizeof(uint32_t), s);
+        if (e != cudaSuccess) return fail("sfb_embedding: %s", cudaGetErrorString(e));
+    }
+    const dim3 grid((unsigned)ctas_x + one_cta, (batch + per_y - 1) / per_y);
+    if (dtype == SFB_F32) launch_overlapped(embedding_kernel<SFB_F32>, grid, dim3(256), 0, s, out, table, ids, pos, batch, per_y, seq_len, hidden, vocab, bad_ids, column);
+    else if (dtype == SFB_BF16) launch_overlapped(embedding_kernel<SFB_BF16>, grid, dim3(256), 0, s, out, table, ids, pos, batch, per_y, seq_len, hidden, vocab, bad_ids, column);
+    else launch_overlapped(embedding_kernel<SFB_F16>, grid, dim3(256), 0, s, out, table, ids, pos, batch, per_y, seq_len, hidden, vocab, bad_ids, column);
     return check_launch("sfb_embedding");
 }
 

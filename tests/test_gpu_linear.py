@@ -234,6 +234,49 @@ def test_embedding_batch_runs(sfb, B, L, hidden):
     assert torch.equal(out, want)
 
 
+@pytest.mark.parametrize("dtype,B,L,hidden", [("bf16", 4, 4096, 8), ("bf16", 5, 4096, 64), ("f32", 1, 16385, 8), ("f16", 3001, 7, 40), ("bf16", 1, 70001, 16)])
+def test_embedding_counts_bad_ids_on_both_sides_of_the_line(sfb, dtype, B, L, hidden):
+    """Up to 16384 ids one CTA counts, beyond that every reader: first and last ids of the sequence and the batch among the bad."""
+    td = {"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}[dtype]
+    gen = torch.Generator(device="cuda").manual_seed(32)
+    table = torch.randn(500, hidden, device="cuda", generator=gen).to(td)
+    ids = torch.randint(-50, 550, (B, L), device="cuda", generator=gen, dtype=torch.int32)
+    ids[0, 0], ids[-1, -1], ids[0, -1], ids[-1, 0] = -1, 500, 1 << 30, -(1 << 31)
+    ok = (ids >= 0) & (ids < 500)
+    for _ in range(2):                       # the second call starts from the first one's count
+        out, bad = sfb.embedding(table, ids)
+        assert int(bad.item()) == int((~ok).sum())
+        assert torch.equal(out, table[ids.clamp(0, 499).long()] * ok.unsqueeze(-1))
+    none = torch.zeros_like(ids)
+    assert int(sfb.embedding(table, none)[1].item()) == 0
+
+
+def test_embedding_count_does_not_set_the_time_of_a_long_lookup(sfb):
+    """A million ids on narrow rows: with the count at most three times the time without it (one CTA reading all ids took 28
+    times as long)."""
+    B, L, hidden = 256, 4096, 8
+    table = torch.ones(1000, hidden, device="cuda", dtype=torch.bfloat16)
+    ids = torch.zeros(B, L, device="cuda", dtype=torch.int32)
+    out, bad = sfb.embedding(table, ids)
+    p = lambda t: ctypes.c_void_p(None if t is None else t.data_ptr())
+
+    def us(count):
+        times = []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(20):
+                sfb._check(sfb.lib.sfb_embedding(sfb._stream(), p(out), p(table), p(ids), None, *(ctypes.c_uint32(v) for v in (B, L, hidden, 1000)),
+                                                 sfb.BF16, p(count)))
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    us(bad)
+    assert us(bad) <= 3 * us(None)
+
+
 def test_embedding_ids_outside_the_table_are_counted_not_read(sfb):
     table = torch.ones(10, 16, device="cuda", dtype=torch.bfloat16)
     ids = torch.tensor([[0, 9, 10, -1, 5]], dtype=torch.int32, device="cuda")
