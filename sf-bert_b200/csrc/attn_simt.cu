@@ -977,10 +977,11 @@ __global__ void __launch_bounds__(tile::kThreads, 3) csr_tile_f32_kernel(const C
             for (uint32_t k = 0; k < 4; k++) mn = fmaxf(mn, red[k * 32 + r]);
             const float alpha = mn > mx[m] ? exp2f(mx[m] - mn) : 1.f;
             mx[m] = mn;
+            const float off = mn > -INFINITY ? mn : 0.f;                 // nothing kept so far: exp2(-inf) = 0, and NaN stays NaN
             float ps = 0.f;
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-                const float pv = mn > -INFINITY ? exp2f(s[m][j] - mn) : 0.f;
+                const float pv = exp2f(s[m][j] - off);
                 Ps[r * PS + 32 * warp + lc + 4 * j] = pv;
                 ps += pv;
             }

@@ -130,3 +130,24 @@ def test_csr_columns_of_half_a_tile(sfb, oracle, upper, lower, both, twice):
     want = oracle.csr_attention(q.float().cpu().numpy(), k.float().cpu().numpy(), v.float().cpu().numpy(), rowptr, colidx, np.float32(0.125))
     assert int(bad.item()) == 0
     assert np.abs(o.float().cpu().numpy() - want).max() <= 2e-2 * np.abs(want).max()
+
+
+def _random_rows(L, seed, most=60):
+    rng = np.random.RandomState(seed)
+    rows = [rng.choice(L, size=0 if 32 <= i < 40 else int(rng.randint(1, min(L, most) + 1)), replace=False).astype(np.int32) for i in range(L)]
+    return rows, np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32), np.concatenate(rows).astype(np.int32)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("d", [32, 64, 128])
+def test_csr_nan_query_gives_nan(sfb, dtype, d):
+    """A query with a NaN has a NaN for every output, and no other row has one."""
+    L, bad_row = 100, 70
+    _, rowptr, colidx = _random_rows(L, 9)
+    gen = torch.Generator(device="cuda").manual_seed(90)
+    q, k, v = (torch.randn(1, L, 1, d, device="cuda", generator=gen).to(TD[dtype]) for _ in range(3))
+    q[0, bad_row, 0, 5] = float("nan")
+    o, _ = sfb.csr_attention(q, k, v, torch.from_numpy(rowptr).cuda(), torch.from_numpy(colidx).cuda(), 0.125)
+    want = torch.zeros(L, d, dtype=torch.bool)
+    want[bad_row] = True
+    assert torch.equal(torch.isnan(o[0, :, 0]).cpu(), want)
