@@ -884,7 +884,7 @@ __device__ __forceinline__ void stage_gather(float *dst, uint32_t stride, const 
     }
 }
 template <int D>
-__global__ void __launch_bounds__(tile::kThreads, 3) csr_tile_f32_kernel(const CsrTileArgs a)
+__global__ void __launch_bounds__(tile::kThreads, 3) csr_tile_f32_kernel(const __grid_constant__ CsrTileArgs a)
 {
     using namespace tile;
     typedef FaCfg<32, D> Cfg;
@@ -1006,6 +1006,7 @@ __global__ void __launch_bounds__(tile::kThreads, 3) csr_tile_f32_kernel(const C
         if (lc == 0) red[warp * 32 + lr + 8 * m] = sum[m];
     }
     __syncthreads();
+    uint32_t odd = 0;                                                    // this thread's rows with an output that is not finite
 #pragma unroll
     for (int m = 0; m < 4; m++) {
         const uint32_t r = lr + 8 * m;
@@ -1014,7 +1015,24 @@ __global__ void __launch_bounds__(tile::kThreads, 3) csr_tile_f32_kernel(const C
         for (uint32_t k = 0; k < 4; k++) l += red[k * 32 + r];
         const float inv = l > 0.f ? 1.f / (l + 1e-6f) : 0.f;             // the reference's denominator (ewops.h:93, cuda_kernels.h:1022)
         if (tl * 32 + r < a.L) store_cols<SFB_F32, TN>(a.O, head + (size_t)(tl * 32 + r) * HD + n0, lc, acc[m], inv, D / 4, true);
+        float zero = 0.f;                                                // stays 0 as long as every output is finite
+#pragma unroll
+        for (int j = 0; j < TN / 2; j++) {
+            const float2 f = unpair(acc[m][j]);
+            zero = fmaf(f.x, 0.f, fmaf(f.y, 0.f, zero));
+        }
+        if (!(zero == 0.f) && tl * 32 + r < a.L) odd |= 1u << r;
     }
+    if (!__syncthreads_or(odd != 0)) return;
+    // rows that are not finite are made again (csr_row_again), once every warp has written its columns of them
+    uint32_t *again = (uint32_t *)red;
+    if (threadIdx.x == 0) *again = 0;
+    __syncthreads();
+    if (odd) atomicOr(again, odd);
+    __syncthreads();
+    const uint32_t rows = *again;
+    for (uint32_t r = warp; r < 32; r += 4)
+        if ((rows >> r) & 1u) csr_row_again<SFB_F32, D>(a, b, h, tl * 32 + r);
 }
 
 // ------------------------------------------------------------------------------------------------

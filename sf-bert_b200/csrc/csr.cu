@@ -45,131 +45,15 @@ __global__ void csr_from_layout_kernel(const uint8_t *__restrict__ layout, uint3
     }
 }
 
-// 16-byte pieces -> floats, by element type
-template <int DT> struct Piece;
-template <> struct Piece<SFB_F32> {
-    static constexpr int N = 4;
-    static __device__ __forceinline__ void unpack(float *v, const uint4 &t)
-    {
-        v[0] = __uint_as_float(t.x); v[1] = __uint_as_float(t.y); v[2] = __uint_as_float(t.z); v[3] = __uint_as_float(t.w);
-    }
-};
-template <> struct Piece<SFB_BF16> {
-    static constexpr int N = 8;
-    static __device__ __forceinline__ void unpack(float *v, const uint4 &t)
-    {
-        const uint32_t w[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-        for (int j = 0; j < 4; j++) { v[2 * j] = __uint_as_float(w[j] << 16); v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u); }
-    }
-};
-template <> struct Piece<SFB_F16> {
-    static constexpr int N = 8;
-    static __device__ __forceinline__ void unpack(float *v, const uint4 &t)
-    {
-        const uint32_t w[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-        for (int j = 0; j < 4; j++) { const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[j])); v[2 * j] = f.x; v[2 * j + 1] = f.y; }
-    }
-};
-
-// One warp per query row with LPK lanes per key, each owning a share of the head dimension; the key's K and V pieces are all
-// requested before the first is used.  The lanes of a key join their partial scores by shuffles and carry the same running
-// max and sum; the groups' softmaxes are merged at the end.
+// One warp per query row.
 template <int DT, int D, int LPK>
 __global__ void __launch_bounds__(128) csr_attention_split_kernel(const int32_t *__restrict__ rowptr, const int32_t *__restrict__ colidx,
                                                                  const void *__restrict__ Q, const void *__restrict__ K,
                                                                  const void *__restrict__ V, void *__restrict__ O, uint32_t L,
                                                                  uint32_t H, float scale_log2e, uint32_t *bad)
 {
-    constexpr int HD2 = D / LPK;                     // elements per lane
-    constexpr int KPI = 32 / LPK;                    // keys per warp and step
-    constexpr int NP = HD2 / Piece<DT>::N;           // 16-byte pieces per lane and operand
-    constexpr int ESZ = 16 / Piece<DT>::N;
-    const uint32_t lane = threadIdx.x & 31, hp = lane % LPK, pi = lane / LPK;
-    const uint32_t i = blockIdx.x * 4 + (threadIdx.x >> 5), b = blockIdx.y, h = blockIdx.z;
-    if (i >= L) return;
-    const size_t HD = (size_t)H * D;
-    const size_t row_off = ((size_t)b * L + i) * HD + (size_t)h * D + hp * HD2;
-    const int32_t lo = rowptr[i], hi = rowptr[i + 1];
-    float q[HD2], acc[HD2];
-    {
-        const uint4 *src = (const uint4 *)((const uint8_t *)Q + row_off * ESZ);
-#pragma unroll
-        for (int n = 0; n < NP; n++) Piece<DT>::unpack(q + n * Piece<DT>::N, __ldg(src + n));
-    }
-#pragma unroll
-    for (int x = 0; x < HD2; x++) acc[x] = 0.f;
-    float m = -INFINITY, l = 0.f;
-    for (int32_t base = lo; base < hi; base += KPI) {          // the same trip count for every lane: the shuffle below is full-warp
-        const int32_t e = base + (int32_t)pi;
-        bool valid = e < hi;
-        int32_t j = 0;
-        if (valid) {
-            j = __ldg(colidx + e);
-            if (j < 0 || (uint32_t)j >= L) {                   // a column outside the sequence: counted once, not read
-                if (bad && hp == 0) atomicAdd(bad, 1u);
-                valid = false;
-            }
-        }
-        uint4 kr[NP], vr[NP];
-        if (valid) {
-            const size_t key_off = (((size_t)b * L + (uint32_t)j) * HD + (size_t)h * D + hp * HD2) * ESZ;
-            const uint4 *ks = (const uint4 *)((const uint8_t *)K + key_off), *vs = (const uint4 *)((const uint8_t *)V + key_off);
-#pragma unroll
-            for (int n = 0; n < NP; n++) kr[n] = __ldg(ks + n);
-#pragma unroll
-            for (int n = 0; n < NP; n++) vr[n] = __ldg(vs + n);
-        }
-        float part = 0.f;
-        if (valid) {
-#pragma unroll
-            for (int n = 0; n < NP; n++) {
-                float t[Piece<DT>::N];
-                Piece<DT>::unpack(t, kr[n]);
-#pragma unroll
-                for (int x = 0; x < Piece<DT>::N; x++) part = fmaf(q[n * Piece<DT>::N + x], t[x], part);
-            }
-        }
-        float sc = part;
-#pragma unroll
-        for (int o = 1; o < LPK; o <<= 1) sc += __shfl_xor_sync(0xffffffffu, sc, o);
-        if (valid) {
-            if (sc > m) {
-                const float f = exp2f((m - sc) * scale_log2e);   // 0 on the first key
-                l *= f;
-#pragma unroll
-                for (int x = 0; x < HD2; x++) acc[x] *= f;
-                m = sc;
-            }
-            const float p = exp2f((sc - m) * scale_log2e);
-            l += p;
-#pragma unroll
-            for (int n = 0; n < NP; n++) {
-                float t[Piece<DT>::N];
-                Piece<DT>::unpack(t, vr[n]);
-#pragma unroll
-                for (int x = 0; x < Piece<DT>::N; x++) acc[n * Piece<DT>::N + x] = fmaf(p, t[x], acc[n * Piece<DT>::N + x]);
-            }
-        }
-    }
-    // merge the 16 pairs' softmaxes (the two lanes of a pair hold the same max and sum: offsets 16..2 only)
-    float M = m;
-#pragma unroll
-    for (int o = 16; o >= LPK; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-    const float f = m > -INFINITY ? exp2f((m - M) * scale_log2e) : 0.f;
-    l *= f;
-#pragma unroll
-    for (int o = 16; o >= LPK; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    const float inv = l > 0.f ? 1.f / (l + 1e-6f) : 0.f;   // the reference's denominator (ewops.h:93, cuda_kernels.h:1022)
-#pragma unroll
-    for (int x = 0; x < HD2; x++) {
-        float a = acc[x] * f;
-#pragma unroll
-        for (int o = 16; o >= LPK; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        // every lane of this parity holds the element now; pair x % 16 writes it
-        if ((x % KPI) == (int)pi) Elem<DT>::store(O, row_off + x, a * inv);
-    }
+    const uint32_t i = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (i < L) csr_row<DT, D, LPK>(colidx, rowptr[i], rowptr[i + 1], Q, K, V, O, L, H, blockIdx.y, blockIdx.z, i, scale_log2e, bad);
 }
 
 // ---- the plan -------------------------------------------------------------------------------------------------
@@ -327,7 +211,7 @@ __device__ __forceinline__ float ex2f(float x)
 }
 
 template <bool BF16, int D>
-__global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const CsrTileArgs a)
+__global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const __grid_constant__ CsrTileArgs a)
 {
     typedef CsrCfg<D> Cfg;
     constexpr int MT = Cfg::MT, KC = Cfg::KC, NT = KC / 8, CH = D / 8, DN = D / 8;
@@ -532,7 +416,6 @@ __global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const Cs
         }
     __syncthreads();
     const uint32_t r = threadIdx.x >> 2, row = tile * 32 + r, d0 = (threadIdx.x & 3) * (D / 4);
-    if (row >= a.L) return;
     const uint32_t w0 = MT == 2 ? 0 : r >> 4, wr = MT == 2 ? r : r & 15;                  // the warps that hold this row
     constexpr uint32_t WS = MT == 2 ? 1 : 2;
     float M = -INFINITY, sum = 0.f, f[Cfg::SPLITS];
@@ -546,6 +429,7 @@ __global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const Cs
     }
     const float inv = sum > 0.f ? 1.f / (sum + 1e-6f) : 0.f;   // the reference's denominator (ewops.h:93, cuda_kernels.h:1022)
     uint16_t *dst = (uint16_t *)a.O + ((size_t)b * a.L + row) * HD + (size_t)h * D + d0;
+    float zero = 0.f;                                          // stays 0 as long as every output is finite
 #pragma unroll
     for (int c = 0; c < D / 4; c += 8) {
         float y[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -555,8 +439,18 @@ __global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const Cs
 #pragma unroll
             for (int j = 0; j < 8; j++) y[j] = fmaf(src[j], f[k], y[j]);
         }
-        *(uint4 *)(dst + c) = make_uint4(pack16<BF16>(y[0] * inv, y[1] * inv), pack16<BF16>(y[2] * inv, y[3] * inv),
-                                         pack16<BF16>(y[4] * inv, y[5] * inv), pack16<BF16>(y[6] * inv, y[7] * inv));
+#pragma unroll
+        for (int j = 0; j < 8; j++) zero = fmaf(y[j], 0.f, zero);
+        if (row < a.L)
+            *(uint4 *)(dst + c) = make_uint4(pack16<BF16>(y[0] * inv, y[1] * inv), pack16<BF16>(y[2] * inv, y[3] * inv),
+                                             pack16<BF16>(y[4] * inv, y[5] * inv), pack16<BF16>(y[6] * inv, y[7] * inv));
+    }
+    // a warp has written rows of its own, four lanes each: it makes those that are not finite again (csr_row_again)
+    uint32_t odd = __ballot_sync(0xffffffffu, row < a.L && !(zero == 0.f));
+    while (odd) {
+        const uint32_t first_lane = __ffs(odd) - 1u, rr = (warp * 32 + first_lane) >> 2;
+        odd &= ~(0xfu << (first_lane & ~3u));
+        csr_row_again<BF16 ? SFB_BF16 : SFB_F16, D>(a, b, h, tile * 32 + rr);
     }
 }
 
@@ -593,7 +487,7 @@ static int csr_attention_planned(cudaStream_t s, const int32_t *rowptr, const in
         once.mark(dev);
     }
     launch_overlapped(dtype != SFB_F32 && d == 128 ? csr_plan_kernel<true> : csr_plan_kernel<false>, dim3(tiles), dim3(kPlanThreads), L * sizeof(uint32_t), s, rowptr, colidx, L, nnz, entries, counts, counts + kCsrCounts * tiles);
-    const CsrTileArgs a = {entries, counts, counts + kCsrCounts * tiles, q, k, v, o, L, H, tiles, B * H, scale * 1.4426950408889634f, bad};
+    const CsrTileArgs a = {entries, counts, counts + kCsrCounts * tiles, rowptr, colidx, nnz, q, k, v, o, L, H, tiles, B * H, scale * 1.4426950408889634f, bad};
     if (dtype == SFB_F32) return csr_tile_f32(s, a, B, d);
 #define CSR_TILE(BF) return d == 32 ? launch_csr_tile<BF, 32>(s, a, B) : d == 64 ? launch_csr_tile<BF, 64>(s, a, B) : launch_csr_tile<BF, 128>(s, a, B)
     if (dtype == SFB_BF16) CSR_TILE(true);

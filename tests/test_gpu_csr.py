@@ -151,3 +151,31 @@ def test_csr_nan_query_gives_nan(sfb, dtype, d):
     want = torch.zeros(L, d, dtype=torch.bool)
     want[bad_row] = True
     assert torch.equal(torch.isnan(o[0, :, 0]).cpu(), want)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("value", ["nan", "inf", "-inf"])
+def test_csr_values_that_are_not_finite_stay_in_the_rows_that_have_them(sfb, oracle, dtype, d, value):
+    """An infinity or a NaN among the values of a column reaches the rows that have the column, in that element, and no other:
+    rows of the same tile are as they are without it.  Also in a column of its own that nobody has, in tiles of one row and
+    in rows without elements."""
+    B, L, H = 2, 193, 2                                      # the last tile has one row
+    rows, rowptr, colidx = _random_rows(L, 11)
+    cols = [3, 77, 192]
+    nobody = [c for c in range(L) if not any(c in r for r in rows)]
+    q, k, v = (torch.from_numpy(oracle.fill_normal((B, L, H, d), 700 + i)).cuda().to(TD[dtype]) for i in range(3))
+    rp, ci = torch.from_numpy(rowptr).cuda(), torch.from_numpy(colidx).cuda()
+    clean = sfb.csr_attention(q, k, v, rp, ci, 0.125)[0].float().cpu().numpy()
+    dirty = v.clone()
+    for n, c in enumerate(cols + nobody[:2]):
+        dirty[:, c, :, (5 * n) % d] = float(value)
+    got = sfb.csr_attention(q, k, dirty, rp, ci, 0.125)[0].float().cpu().numpy()
+    has = np.zeros((L, d), bool)                             # elements of the output that one of the values belongs to
+    for n, c in enumerate(cols):
+        for i, r in enumerate(rows):
+            has[i, (5 * n) % d] |= c in r
+    assert has.any() and np.array_equal(~np.isfinite(got), np.broadcast_to(has[None, :, None], got.shape))
+    keep = ~np.broadcast_to(has[None, :, None], got.shape)
+    # two sums in a different order, rounded to the type of the output
+    assert np.abs(got - clean)[keep].max() <= (1e-5 if dtype == "f32" else 2.0 ** -7) * np.abs(clean).max()
