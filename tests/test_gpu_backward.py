@@ -259,3 +259,33 @@ def test_backward_with_ds_on_chip(sfb, nb, heads, case):
     for a, b in zip(got, want):
         assert float((a.float() - b.float()).abs().max()) <= 5e-2 * float(b.float().abs().max())
         assert torch.equal(a.float().abs().amax(-1) == 0, b.float().abs().amax(-1) == 0)      # what has no blocks is zero, nothing else is
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("which", ["v", "do", "o"])
+@pytest.mark.parametrize("value", ["nan", "inf"])
+def test_backward_with_ds_on_chip_keeps_what_is_not_finite_where_it_belongs(sfb, dtype, which, value):
+    """One element of V, dO or O that is not finite: dQ is finite in every block-row that does not keep the element's block,
+    dK in every block-column that the element's block-row does not keep, as dS of the separate operators is."""
+    B, H, d, bs, nb = 1, 2, 64, 64, 7
+    layout = np.zeros((1, nb, nb), np.uint8)
+    layout[0, np.arange(nb), np.arange(nb)] = 1
+    layout[0, 2, :] = 1                                      # one long row, one long column: each paired with a short one
+    layout[0, :, 5] = 1
+    layout[0, 3, 0] = 1
+    lay = sfb.BlockLayout(torch.from_numpy(layout).cuda(), bs)
+    g = torch.Generator(device="cuda").manual_seed(91)
+    q, k, v, do = (torch.randn(B, nb * bs, H, d, device="cuda", generator=g).to(TD[dtype]) for _ in range(4))
+    p = sfb.fused_sddmm_softmax(q, k, lay, 0.125, TD[dtype])
+    o = sfb.bst_sgemm_xn(p, v, lay)
+    for at in range(nb):
+        x = {"v": v, "do": do, "o": o}
+        x[which] = x[which].clone()
+        x[which][0, at * bs + 11, 1, 7] = float(value)
+        dq, dk, _ = sfb.attention_backward_fused(q, k, x["v"], p, x["o"], x["do"], lay, 0.125)
+        assert sfb.device_status() == 0
+        rows = layout[0, :, at] != 0 if which == "v" else np.arange(nb) == at          # block-rows whose dS it reaches
+        cols = np.arange(nb) == at if which == "v" else layout[0, at] != 0             # block-columns
+        for got, reached in ((dq, rows), (dk, cols)):
+            finite = torch.isfinite(got).view(nb, bs, H, d).permute(2, 0, 1, 3).flatten(2).all(-1).cpu().numpy()     # [H, block-row]
+            assert finite[0].all() and finite[1][~reached].all()
