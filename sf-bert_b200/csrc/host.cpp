@@ -43,6 +43,24 @@ inline void check(int rc)
 {
     if (rc != 0) raise(error_type, L.sfb_last_error());
 }
+// While this exists other Python threads run: a launch waits when the stream's queue is full, for as long as the GPU is behind.
+struct Unlocked {
+    PyThreadState *state = PyEval_SaveThread();
+    Unlocked() {}
+    Unlocked(const Unlocked &) = delete;
+    ~Unlocked() { PyEval_RestoreThread(state); }
+};
+// One call of the library.  Its arguments are evaluated before other threads are let in.
+template <typename... P, typename... A>
+inline void call(int (*f)(P...), A... a)
+{
+    int rc;
+    {
+        Unlocked others;
+        rc = f(a...);
+    }
+    check(rc);                           // the library's message is the thread's own
+}
 
 // ---- Python objects ----------------------------------------------------------------------------------------------------
 struct Ref {                         // an owned reference
@@ -148,8 +166,8 @@ at::Tensor bst_sgemm_nt(const at::Tensor &q, const at::Tensor &k, const Lay &lay
 {
     const Dims n(q, lay);
     at::Tensor s = empty({n.B, n.H, lay.blocks, lay.bs, lay.bs}, scalar_type(out_tag), q);
-    check(L.sfb_bst_sgemm_nt(stream(), lay.get(n_nt_lut), ptr(q), ptr(k), ptr(s), tag(q), out_tag, lay.bs, lay.blocks, n.B, lay.nb, lay.nb, n.H,
-                             n.d, lay.heads, lay.blocks));
+    call(L.sfb_bst_sgemm_nt, stream(), lay.get(n_nt_lut), ptr(q), ptr(k), ptr(s), tag(q), out_tag, lay.bs, lay.blocks, n.B, lay.nb, lay.nb, n.H,
+                             n.d, lay.heads, lay.blocks);
     return s;
 }
 
@@ -157,9 +175,9 @@ at::Tensor bst_sgemm(const at::Tensor &p, const at::Tensor &v, const Lay &lay, b
 {
     const Dims n(v, lay);
     at::Tensor o = alike(v);
-    check(L.sfb_bst_sgemm_xn(stream(), lay.get(trans ? n_tn_lut : n_nn_lut), ptr(p), ptr(v), ptr(o), tag(p), tag(v), lay.bs, lay.blocks, n.B,
+    call(L.sfb_bst_sgemm_xn, stream(), lay.get(trans ? n_tn_lut : n_nn_lut), ptr(p), ptr(v), ptr(o), tag(p), tag(v), lay.bs, lay.blocks, n.B,
                              lay.nb, lay.nb, n.H, n.d, lay.heads, lay.blocks + lay.nb, trans ? SFB_TN_OP : SFB_NN_OP, 0, 0,
-                             trans ? attr_u32(lay.o, n_tn_max) : lay.nn_max));
+                             trans ? attr_u32(lay.o, n_tn_max) : lay.nn_max);
     return o;
 }
 
@@ -167,9 +185,9 @@ at::Tensor masked_softmax(const at::Tensor &s, const Lay &lay, float scale, int 
 {
     require(s.dim() >= 2, "expected a [B, H, blocks, bs, bs] tensor");
     at::Tensor y = empty(s.sizes(), scalar_type(out_tag), s);
-    check(L.sfb_masked_softmax(stream(), lay.get(n_nn_lut), use_mask ? lay.get(n_mask_t) : nullptr, ptr(s), ptr(y), tag(s), out_tag, lay.bs,
+    call(L.sfb_masked_softmax, stream(), lay.get(n_nn_lut), use_mask ? lay.get(n_mask_t) : nullptr, ptr(s), ptr(y), tag(s), out_tag, lay.bs,
                                lay.blocks, (uint32_t)s.size(0), (uint32_t)s.size(1), lay.nb, lay.heads, lay.blocks + lay.nb, lay.nn_max, lay.heads,
-                               scale));
+                               scale);
     return y;
 }
 
@@ -177,8 +195,8 @@ at::Tensor masked_softmax_grad(const at::Tensor &dy, const at::Tensor &y, const 
 {
     require(dy.scalar_type() == y.scalar_type() && dy.sizes() == y.sizes(), "dy and y differ in type or shape");
     at::Tensor dx = alike(y);
-    check(L.sfb_masked_softmax_grad(stream(), lay.get(n_nn_lut), ptr(dy), ptr(y), ptr(dx), tag(y), lay.bs, lay.blocks, (uint32_t)y.size(0),
-                                    (uint32_t)y.size(1), lay.nb, lay.heads, lay.blocks + lay.nb, lay.nn_max, scale));
+    call(L.sfb_masked_softmax_grad, stream(), lay.get(n_nn_lut), ptr(dy), ptr(y), ptr(dx), tag(y), lay.bs, lay.blocks, (uint32_t)y.size(0),
+                                    (uint32_t)y.size(1), lay.nb, lay.heads, lay.blocks + lay.nb, lay.nn_max, scale);
     return dx;
 }
 
@@ -188,7 +206,7 @@ at::Tensor rowdot(const at::Tensor &a, const at::Tensor &b)
             "a and b must be contiguous and alike");
     const int64_t d = divisor(a.size(-1));
     at::Tensor out = empty(a.sizes().slice(0, a.dim() - 1), at::kFloat, a);
-    check(L.sfb_rowdot(stream(), (float *)ptr(out), ptr(a), ptr(b), (uint64_t)(a.numel() / d), (uint32_t)d, tag(a)));
+    call(L.sfb_rowdot, stream(), (float *)ptr(out), ptr(a), ptr(b), (uint64_t)(a.numel() / d), (uint32_t)d, tag(a));
     return out;
 }
 
@@ -200,8 +218,8 @@ at::Tensor fused_sddmm_softmax_grad(const at::Tensor &dout, const at::Tensor &v,
     require(delta.scalar_type() == at::kFloat && delta.dim() == 3 && delta.size(0) == n.B && delta.size(1) == n.L && delta.size(2) == n.H,
             "delta is not a float [B, L, H] tensor");
     at::Tensor ds = alike(p);
-    check(L.sfb_fused_sddmm_softmax_grad(stream(), lay.get(n_nt_lut), ptr(dout), ptr(v), ptr(p), (const float *)ptr(delta), ptr(ds), tag(p), lay.bs,
-                                         lay.blocks, n.B, lay.nb, n.H, n.d, lay.heads, lay.blocks, scale));
+    call(L.sfb_fused_sddmm_softmax_grad, stream(), lay.get(n_nt_lut), ptr(dout), ptr(v), ptr(p), (const float *)ptr(delta), ptr(ds), tag(p), lay.bs,
+                                         lay.blocks, n.B, lay.nb, n.H, n.d, lay.heads, lay.blocks, scale);
     return ds;
 }
 
@@ -209,8 +227,8 @@ at::Tensor fused_sddmm_softmax(const at::Tensor &q, const at::Tensor &k, const L
 {
     const Dims n(q, lay);
     at::Tensor y = empty({n.B, n.H, lay.blocks, lay.bs, lay.bs}, scalar_type(out_tag), q);
-    check(L.sfb_fused_sddmm_softmax(stream(), lay.get(n_nn_lut), ptr(q), ptr(k), use_mask ? lay.get(n_mask_np) : nullptr, ptr(y), tag(q), out_tag,
-                                    lay.bs, lay.blocks, n.B, lay.nb, lay.nb, n.H, n.d, lay.heads, lay.blocks, lay.heads, scale));
+    call(L.sfb_fused_sddmm_softmax, stream(), lay.get(n_nn_lut), ptr(q), ptr(k), use_mask ? lay.get(n_mask_np) : nullptr, ptr(y), tag(q), out_tag,
+                                    lay.bs, lay.blocks, n.B, lay.nb, lay.nb, n.H, n.d, lay.heads, lay.blocks, lay.heads, scale);
     return y;
 }
 
@@ -228,7 +246,7 @@ void linear_into(const at::Tensor &x, const at::Tensor &w, const void *bias, int
     require(x.size(-1) == k && x.scalar_type() == w.scalar_type() && x.is_contiguous() && w.is_contiguous(),
             "x and w must be contiguous, of one type and of matching sizes");
     auto f = nt ? L.sfb_linear_nt : L.sfb_linear;
-    check(f(stream(), ptr(out), ptr(x), ptr(w), (const float *)bias, (uint32_t)(x.numel() / k), (uint32_t)n, (uint32_t)k, tag(x), act));
+    call(f, stream(), ptr(out), ptr(x), ptr(w), (const float *)bias, (uint32_t)(x.numel() / k), (uint32_t)n, (uint32_t)k, tag(x), act);
 }
 
 at::Tensor linear(const at::Tensor &x, const at::Tensor &w, const void *bias, int act, bool nt)
@@ -305,8 +323,8 @@ FUNCTION(py_embedding, 3)
     require(ids.scalar_type() == at::kInt && ids.is_contiguous() && table.is_contiguous(), "ids must be int32 and contiguous, like the table");
     const int64_t B = ids.size(0), len = ids.size(1), vocab = table.size(0), hidden = table.size(1);
     at::Tensor out = empty({B, len, hidden}, table.scalar_type(), table), bad = empty({1}, at::kInt, table);
-    check(L.sfb_embedding(stream(), ptr(out), ptr(table), (const int32_t *)ptr(ids), ptr_or_null(a[2]), (uint32_t)B, (uint32_t)len,
-                          (uint32_t)hidden, (uint32_t)vocab, tag(table), (uint32_t *)ptr(bad)));
+    call(L.sfb_embedding, stream(), ptr(out), ptr(table), (const int32_t *)ptr(ids), ptr_or_null(a[2]), (uint32_t)B, (uint32_t)len,
+                          (uint32_t)hidden, (uint32_t)vocab, tag(table), (uint32_t *)ptr(bad));
     Ref o(wrap(out)), n(wrap(bad));
     return PyTuple_Pack(2, o.o, n.o);
 }
@@ -322,15 +340,15 @@ FUNCTION(py_csr_attention, 6)
     const uint64_t bytes = nnz < (1ll << 31) ? L.sfb_csr_workspace((uint32_t)nnz, (uint32_t)q.size(1)) : 0;
     if (bytes) {
         at::Tensor ws = empty({(int64_t)bytes}, at::kByte, q);
-        check(L.sfb_csr_attention_planned(stream(), (const int32_t *)ptr(rowptr), (const int32_t *)ptr(colidx), (uint32_t)nnz, ptr(q),
+        call(L.sfb_csr_attention_planned, stream(), (const int32_t *)ptr(rowptr), (const int32_t *)ptr(colidx), (uint32_t)nnz, ptr(q),
                                           ptr(tensor(a[1])), ptr(tensor(a[2])), ptr(o), tag(q), (uint32_t)q.size(0), (uint32_t)q.size(1),
-                                          (uint32_t)q.size(2), (uint32_t)q.size(3), (float)number(a[5]), (uint32_t *)ptr(bad), ptr(ws)));
+                                          (uint32_t)q.size(2), (uint32_t)q.size(3), (float)number(a[5]), (uint32_t *)ptr(bad), ptr(ws));
         Ref r(wrap(o)), n(wrap(bad));
         return PyTuple_Pack(2, r.o, n.o);
     }
-    check(L.sfb_csr_attention(stream(), (const int32_t *)ptr(rowptr), (const int32_t *)ptr(colidx), ptr(q), ptr(tensor(a[1])), ptr(tensor(a[2])),
+    call(L.sfb_csr_attention, stream(), (const int32_t *)ptr(rowptr), (const int32_t *)ptr(colidx), ptr(q), ptr(tensor(a[1])), ptr(tensor(a[2])),
                               ptr(o), tag(q), (uint32_t)q.size(0), (uint32_t)q.size(1), (uint32_t)q.size(2), (uint32_t)q.size(3),
-                              (float)number(a[5]), (uint32_t *)ptr(bad)));
+                              (float)number(a[5]), (uint32_t *)ptr(bad));
     Ref r(wrap(o)), n(wrap(bad));
     return PyTuple_Pack(2, r.o, n.o);
 }
@@ -342,9 +360,9 @@ FUNCTION(py_fused_attention, 7)
     const Lay lay(a[3]);
     const Dims n(q, lay);
     at::Tensor o = out_or(a[6], q);
-    check(L.sfb_fused_attention(stream(), lay.get(n_nn_lut), ptr(q), ptr(tensor(a[1])), ptr(tensor(a[2])), ptr(o),
+    call(L.sfb_fused_attention, stream(), lay.get(n_nn_lut), ptr(q), ptr(tensor(a[1])), ptr(tensor(a[2])), ptr(o),
                                 truth(a[5]) ? lay.get(n_mask_np) : nullptr, tag(q), lay.bs, lay.blocks, n.B, lay.nb, n.H, n.d, lay.heads, lay.blocks,
-                                lay.heads, scale_or(a[4], n.d), lay.nn_max));
+                                lay.heads, scale_or(a[4], n.d), lay.nn_max);
     return wrap(o);
 }
 // Row pitch (elements) of a [B, L, H, d] view whose heads are a slice of a wider tensor: rows of one batch element and
@@ -365,9 +383,9 @@ FUNCTION(py_fused_attention_slice, 7)
     at::Tensor o = a[6] == Py_None ? empty(q.sizes(), q.scalar_type(), q) : tensor(a[6]);
     const uint64_t pitch = row_pitch(q);
     require(row_pitch(k) == pitch && row_pitch(v) == pitch, "q, k and v have different row pitches");
-    check(L.sfb_fused_attention_slice(stream(), lay.get(n_nn_lut), ptr(q), ptr(k), ptr(v), ptr(o), truth(a[5]) ? lay.get(n_mask_np) : nullptr,
+    call(L.sfb_fused_attention_slice, stream(), lay.get(n_nn_lut), ptr(q), ptr(k), ptr(v), ptr(o), truth(a[5]) ? lay.get(n_mask_np) : nullptr,
                                       tag(q), lay.bs, lay.blocks, n.B, lay.nb, n.H, n.d, lay.heads, lay.blocks, lay.heads, scale_or(a[4], n.d),
-                                      lay.nn_max, pitch, row_pitch(o)));
+                                      lay.nn_max, pitch, row_pitch(o));
     return wrap(o);
 }
 // (x, bias, resid, gain, beta, want_sum, out)
@@ -378,9 +396,9 @@ FUNCTION(py_bias_residual_layernorm, 7)
     const int64_t m = x.size(0), hidden = x.size(1);
     at::Tensor out = out_or(a[6], x), sum, mean = empty({m}, at::kFloat, x), rstd = empty({m}, at::kFloat, x);
     if (truth(a[5])) sum = alike(x);
-    check(L.sfb_bias_residual_layernorm(stream(), ptr(out), sum.defined() ? ptr(sum) : nullptr, (float *)ptr(mean), (float *)ptr(rstd), ptr(x),
+    call(L.sfb_bias_residual_layernorm, stream(), ptr(out), sum.defined() ? ptr(sum) : nullptr, (float *)ptr(mean), (float *)ptr(rstd), ptr(x),
                                         (const float *)ptr_or_null(a[1]), ptr_or_null(a[2]), (const float *)ptr(tensor(a[3])),
-                                        (const float *)ptr(tensor(a[4])), (uint32_t)m, (uint32_t)hidden, tag(x)));
+                                        (const float *)ptr(tensor(a[4])), (uint32_t)m, (uint32_t)hidden, tag(x));
     Ref o(wrap(out)), mu(wrap(mean)), rs(wrap(rstd));
     if (!sum.defined()) return PyTuple_Pack(4, o.o, Py_None, mu.o, rs.o);
     Ref s(wrap(sum));
@@ -392,7 +410,7 @@ FUNCTION(py_bias_gelu, 3)
     const at::Tensor &x = tensor(a[0]);
     require(x.dim() == 2, "expected an [m, n] tensor");
     at::Tensor out = out_or(a[2], x);
-    check(L.sfb_bias_gelu(stream(), ptr(out), ptr(x), (const float *)ptr_or_null(a[1]), (uint32_t)x.size(0), (uint32_t)x.size(1), tag(x)));
+    call(L.sfb_bias_gelu, stream(), ptr(out), ptr(x), (const float *)ptr_or_null(a[1]), (uint32_t)x.size(0), (uint32_t)x.size(1), tag(x));
     return wrap(out);
 }
 
@@ -434,31 +452,39 @@ FUNCTION(py_encoder_layer, 6)
     char *p_qkv = base, *p_attn = base + row * 3 * hidden, *p_ffn = base, *p_a = base + row * wide, *p_b = p_a + row * hidden;
     const sfb_stream_t s = stream();
     const uint32_t um = (uint32_t)m, uh = (uint32_t)hidden, uf = (uint32_t)ffn;
+    const void *lut = lay.get(n_nn_lut), *px = ptr(x), *pwqkv = ptr(wqkv), *pwo = ptr(wo), *pw1 = ptr(w1), *pw2 = ptr(w2);
+    void *pout = ptr(out);
+    int rc = 0;
+    auto done = [&](int r) { return (rc = r) == 0; };
     auto attention = [&](const void *h) {
-        check(L.sfb_linear(s, p_qkv, h, ptr(wqkv), (const float *)bqkv, um, 3 * uh, uh, t, SFB_ACT_NONE));
         // Q, K and V are column slices of the [m, 3 * hidden] result
         const int64_t col = hidden * x.element_size();
-        check(L.sfb_fused_attention_slice(s, lay.get(n_nn_lut), p_qkv, p_qkv + col, p_qkv + 2 * col, p_attn, nullptr, t, lay.bs, lay.blocks,
-                                          (uint32_t)B, lay.nb, (uint32_t)heads, (uint32_t)d, lay.heads, lay.blocks, lay.heads, scale, lay.nn_max,
-                                          3 * hidden, hidden));
+        return done(L.sfb_linear(s, p_qkv, h, pwqkv, (const float *)bqkv, um, 3 * uh, uh, t, SFB_ACT_NONE)) &&
+               done(L.sfb_fused_attention_slice(s, lut, p_qkv, p_qkv + col, p_qkv + 2 * col, p_attn, nullptr, t, lay.bs, lay.blocks, (uint32_t)B,
+                                                lay.nb, (uint32_t)heads, (uint32_t)d, lay.heads, lay.blocks, lay.heads, scale, lay.nn_max, 3 * hidden,
+                                                hidden));
     };
-    if (pre) {
-        // h = LN(x); a = Attn(h) Wo; h2, x1 = LN(x + a + bo) and the sum; out = x1 + GELU(h2 W1 + b1) W2 + b2
-        check(L.sfb_bias_residual_layernorm(s, p_b, nullptr, nullptr, nullptr, ptr(x), nullptr, nullptr, g1, be1, um, uh, t));
-        attention(p_b);
-        check(L.sfb_linear(s, p_a, p_attn, ptr(wo), nullptr, um, uh, uh, t, SFB_ACT_NONE));
-        check(L.sfb_bias_residual_layernorm(s, p_b, p_a, nullptr, nullptr, p_a, bo, ptr(x), g2, be2, um, uh, t));
-        check(L.sfb_linear(s, p_ffn, p_b, ptr(w1), b1, um, uf, uh, t, SFB_ACT_GELU));
-        check(L.sfb_linear_residual(s, ptr(out), p_ffn, ptr(w2), b2, p_a, um, uh, uf, t));
-    } else {
-        // x1 = LN(x + Attn(x) Wo + bo); out = LN(x1 + GELU(x1 W1 + b1) W2 + b2)
-        attention(ptr(x));
-        check(L.sfb_linear(s, p_a, p_attn, ptr(wo), nullptr, um, uh, uh, t, SFB_ACT_NONE));
-        check(L.sfb_bias_residual_layernorm(s, p_b, nullptr, nullptr, nullptr, p_a, bo, ptr(x), g1, be1, um, uh, t));
-        check(L.sfb_linear(s, p_ffn, p_b, ptr(w1), b1, um, uf, uh, t, SFB_ACT_GELU));
-        check(L.sfb_linear(s, p_a, p_ffn, ptr(w2), nullptr, um, uh, uf, t, SFB_ACT_NONE));
-        check(L.sfb_bias_residual_layernorm(s, ptr(out), nullptr, nullptr, nullptr, p_a, b2, p_b, g2, be2, um, uh, t));
+    {
+        Unlocked others;                     // once for all launches of the layer
+        if (pre) {
+            // h = LN(x); a = Attn(h) Wo; h2, x1 = LN(x + a + bo) and the sum; out = x1 + GELU(h2 W1 + b1) W2 + b2
+            (void)(done(L.sfb_bias_residual_layernorm(s, p_b, nullptr, nullptr, nullptr, px, nullptr, nullptr, g1, be1, um, uh, t)) &&
+                   attention(p_b) &&
+                   done(L.sfb_linear(s, p_a, p_attn, pwo, nullptr, um, uh, uh, t, SFB_ACT_NONE)) &&
+                   done(L.sfb_bias_residual_layernorm(s, p_b, p_a, nullptr, nullptr, p_a, bo, px, g2, be2, um, uh, t)) &&
+                   done(L.sfb_linear(s, p_ffn, p_b, pw1, b1, um, uf, uh, t, SFB_ACT_GELU)) &&
+                   done(L.sfb_linear_residual(s, pout, p_ffn, pw2, b2, p_a, um, uh, uf, t)));
+        } else {
+            // x1 = LN(x + Attn(x) Wo + bo); out = LN(x1 + GELU(x1 W1 + b1) W2 + b2)
+            (void)(attention(px) &&
+                   done(L.sfb_linear(s, p_a, p_attn, pwo, nullptr, um, uh, uh, t, SFB_ACT_NONE)) &&
+                   done(L.sfb_bias_residual_layernorm(s, p_b, nullptr, nullptr, nullptr, p_a, bo, px, g1, be1, um, uh, t)) &&
+                   done(L.sfb_linear(s, p_ffn, p_b, pw1, b1, um, uf, uh, t, SFB_ACT_GELU)) &&
+                   done(L.sfb_linear(s, p_a, p_ffn, pw2, nullptr, um, uh, uf, t, SFB_ACT_NONE)) &&
+                   done(L.sfb_bias_residual_layernorm(s, pout, nullptr, nullptr, nullptr, p_a, b2, p_b, g2, be2, um, uh, t)));
+        }
     }
+    check(rc);
     return wrap(out);
 }
 
@@ -479,9 +505,9 @@ FUNCTION(py_attention_backward_fused, 8)
         (int64_t)n.B * n.H * lay.blocks * 64 < (1ll << 31) - 64 && (int64_t)n.B * n.L < (1ll << 31)) {
         require(o.sizes() == dout.sizes() && dout.sizes() == q.sizes(), "q, o and dO differ in shape");
         at::Tensor delta = empty({n.B, n.H, n.L}, at::kFloat, q), dq = alike(q), dk = alike(k), dv = alike(v);
-        check(L.sfb_attention_backward(stream(), lay.get(n_nn_lut), tn, ptr(q), ptr(k), ptr(v), ptr(p), ptr(o), ptr(dout), (float *)ptr(delta), ptr(dq),
+        call(L.sfb_attention_backward, stream(), lay.get(n_nn_lut), tn, ptr(q), ptr(k), ptr(v), ptr(p), ptr(o), ptr(dout), (float *)ptr(delta), ptr(dq),
                                        ptr(dk), ptr(dv), t, lay.bs, lay.blocks, n.B, lay.nb, n.H, n.d, lay.heads, lay.blocks + lay.nb, lay.nn_max,
-                                       tn_max, scale));
+                                       tn_max, scale);
         Ref x(wrap(dq)), y(wrap(dk)), z(wrap(dv));
         return PyTuple_Pack(3, x.o, y.o, z.o);
     }
