@@ -45,6 +45,8 @@ from . import _host  # noqa: E402
 _host.bind({n: C.cast(getattr(lib, n), C.c_void_p).value for n in _host.wanted().split()})
 SfbError = _host.SfbError
 
+# The signatures of the C ABI, for programs that call `lib` themselves: without them ctypes would pass a pointer given as a
+# plain integer as 32 bits.  The operators below go through _host and need them only where they call `lib`.
 _u32, _i32, _u64, _f32, _vp = C.c_uint32, C.c_int, C.c_uint64, C.c_float, C.c_void_p
 lib.sfb_layout_generate.argtypes = [_vp, _vp, _u32, _u32, _i32, _u32, _u32, _u32, _u32, _i32, _u64]
 lib.sfb_lut_count.argtypes = [_vp, _vp, _u32, _u32, _vp]
@@ -68,10 +70,13 @@ lib.sfb_fused_sddmm_softmax.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32
 lib.sfb_fused_attention.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32] + [_u32] * 9 + [_f32, _u32]
 lib.sfb_fused_attention_slice.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32] + [_u32] * 9 + [_f32, _u32, _u64, _u64]
 lib.sfb_bias_residual_layernorm.argtypes = [_vp] * 10 + [_u32, _u32, _i32]
-
-
 lib.sfb_device_status.argtypes = [C.POINTER(_u32)]
 lib.sfb_bias_gelu.argtypes = [_vp, _vp, _vp, _vp, _u32, _u32, _i32]
+lib.sfb_linear_residual.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp, _u32, _u32, _u32, _i32]
+lib.sfb_attention_backward.argtypes = [_vp] * 13 + [_i32] + [_u32] * 10 + [_f32]
+lib.sfb_csr_workspace.argtypes = [_u32, _u32]
+lib.sfb_csr_workspace.restype = _u64
+lib.sfb_csr_attention_planned.argtypes = [_vp, _vp, _vp, _u32, _vp, _vp, _vp, _vp, _i32, _u32, _u32, _u32, _u32, _f32, _vp, _vp]
 
 
 def device_status():

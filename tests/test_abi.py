@@ -39,6 +39,32 @@ def test_package_symbol_list_matches_header():
         assert '"%s"' % n in src, n
 
 
+C_TYPES = {"int": C.c_int, "uint32_t": C.c_uint32, "uint64_t": C.c_uint64, "float": C.c_float}
+
+
+def test_ctypes_signatures_match_header():
+    """`sfb.lib` takes every declared function with the header's own arguments: a pointer passed as a plain integer must not
+    be cut to 32 bits, whichever of them a program calls."""
+    import __graft_entry__ as ge
+    sfb = ge.load_package()
+    text = re.sub(r"/\*.*?\*/", "", open(os.path.join(ROOT, "include", "sfbert_b200.h")).read(), flags=re.S)
+    found = re.findall(r"([a-z0-9_ ]+?[ *]+)(sfb_[a-z0-9_]+)\s*\(([^)]*)\)\s*;", text)
+    assert sorted(n for _, n, _ in found) == _declared_symbols()
+    for ret, name, params in found:
+        fn = getattr(sfb.lib, name)
+        params = [p.strip() for p in params.split(",") if p.strip() not in ("", "void")]
+        if params:
+            assert fn.argtypes is not None and len(fn.argtypes) == len(params), name
+        for got, p in zip(fn.argtypes or [], params):
+            words = p.replace("*", " * ").split()
+            if "*" in words or words[0] == "sfb_stream_t":
+                assert got is C.c_void_p or issubclass(got, C._Pointer), (name, p)
+            else:
+                assert got is C_TYPES[words[-2]], (name, p)
+        if ret.split() == ["uint64_t"]:
+            assert fn.restype is C.c_uint64, name
+
+
 def test_version_and_magic(lib, oracle):
     assert lib.sfb_version() >= 100
     for d in (1, 2, 3, 4, 5, 6, 7, 8, 12, 100):
