@@ -289,3 +289,71 @@ def test_backward_with_ds_on_chip_keeps_what_is_not_finite_where_it_belongs(sfb,
         for got, reached in ((dq, rows), (dk, cols)):
             finite = torch.isfinite(got).view(nb, bs, H, d).permute(2, 0, 1, 3).flatten(2).all(-1).cpu().numpy()     # [H, block-row]
             assert finite[0].all() and finite[1][~reached].all()
+
+
+def _uneven_layout(case):
+    """uint8 [heads, nb, nb] with rows and columns of very different length."""
+    rng = np.random.RandomState(7)
+    if case == "global":                                     # two long rows, three long columns, paired with each other
+        lay = np.zeros((1, 33, 33), np.uint8)
+        lay[0, np.arange(33), np.arange(33)] = 1
+        lay[0, [3, 20]] = 1
+        lay[0][:, [0, 7, 30]] = 1
+        return lay
+    if case == "one_long":                                   # one long row and one long column, each next to a short one
+        lay = np.zeros((1, 18, 18), np.uint8)
+        lay[0, np.arange(18), (np.arange(18) * 5) % 18] = 1
+        lay[0, 4] = 1
+        lay[0][:, 9] = 1
+        return lay
+    if case == "per_head":
+        lay = np.zeros((3, 9, 9), np.uint8)
+        for h in range(3):
+            lay[h].reshape(-1)[rng.choice(81, size=25, replace=False)] = 1
+        return lay
+    lay = np.zeros((1, 12, 12), np.uint8)                    # rows and columns without blocks
+    lay[0, [1, 2, 6, 9], [0, 3, 3, 11]] = 1
+    return lay
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("case", ["global", "one_long", "per_head", "empty"])
+def test_backward_with_ds_on_chip_against_oracle(sfb, oracle, dtype, case):
+    """The one-call backward against the oracle's products in fp32, element by element.  The bound: dS is rounded once to the
+    16-bit type (unit roundoff u) and every output once; the sums are fp32 (a relative 2^-24 per term and addition); in fp16
+    a dS below the normal range is off by half of the smallest subnormal, 2^-25."""
+    layout = _uneven_layout(case)
+    heads, nb = layout.shape[:2]
+    B, H, d, bs, scale = 2, 3, 64, 64, np.float32(0.125)
+    lay = sfb.BlockLayout(torch.from_numpy(layout).cuda(), bs)
+    luts, tn = oracle.lut_build(layout), oracle.lut_build_tn(layout)["tn"]
+    (q, qn), (k, kn), (v, vn), (do, don) = (_blocks(oracle, (B, nb * bs, H, d), 380 + i, dtype) for i in range(4))
+    p = sfb.fused_sddmm_softmax(q, k, lay, float(scale), TD[dtype])
+    o = sfb.bst_sgemm_xn(p, v, lay)
+    got = sfb.attention_backward_fused(q, k, v, p, o, do, lay, float(scale))
+    assert sfb.device_status() == 0
+    pn, on = p.float().cpu().numpy(), o.float().cpu().numpy()
+    u, eps = (2.0 ** -8, 2.0 ** -24) if dtype == "bf16" else (2.0 ** -11, 2.0 ** -24)
+    tiny = 0.0 if dtype == "bf16" else 2.0 ** -25
+    row_of = luts["nt"][..., 0].astype(np.int64)             # block-row of every block, per head of the layout
+
+    def per_block(x):                                        # [B, L, H] -> [B, H, blocks, bs, 1]: a row's value at its block's rows
+        x = x.reshape(B, nb, bs, H).transpose(0, 3, 1, 2)
+        return np.stack([x[:, h, row_of[h if heads > 1 else 0]] for h in range(H)], axis=1)[..., None]
+
+    scores = lambda a, b: oracle.attention(a, b, b, luts, bs, scale, want=("s",))["s"]
+    dp = scores(don, vn)
+    ds = pn * (dp - per_block((don * on).sum(-1))) * scale
+    # what dP and delta may be off by: 64 terms each, and the handful of operations after them
+    e_x = 80 * eps * (scores(np.abs(don), np.abs(vn)) + per_block((np.abs(don) * np.abs(on)).sum(-1)))
+    e_ds = u * np.abs(ds) + tiny + (1 + u) * pn * e_x * scale
+    longest = bs * max(luts["nn_max"], int(tn[..., :nb, 1].max()))
+    e_sum = (longest + 8) * eps
+    products = {
+        "dq": (oracle.spmm_nn(ds, kn, luts["nn"], bs), oracle.spmm_nn(e_ds + e_sum * np.abs(ds), np.abs(kn), luts["nn"], bs)),
+        "dk": (oracle.spmm_tn(ds, qn, tn, bs), oracle.spmm_tn(e_ds + e_sum * np.abs(ds), np.abs(qn), tn, bs)),
+        "dv": (oracle.spmm_tn(pn, don, tn, bs), oracle.spmm_tn(e_sum * np.abs(pn), np.abs(don), tn, bs)),
+    }
+    for t, (name, (want, bound)) in zip(got, products.items()):
+        err = np.abs(t.float().cpu().numpy() - want)
+        assert (err <= (bound + u * (np.abs(want) + bound) + tiny) * 1.001).all(), name

@@ -98,10 +98,17 @@ def test_linear_more_tiles_than_sms_and_batched_input(sfb, oracle):
     (129, 19200, 128, 0, True),      # a single row into the second CTA's half
     (8192, 768, 256, 0, True),
     (8192, 752, 200, 1, True),       # ragged n (the last tile's second half has 112 of its 128 columns) and k
+    # from here on the estimated times send the product to the CTA pairs; the shapes above go to 128 x 256 tiles
+    (400000, 256, 64, 0, False),     # one k-block, one column tile, 22 rounds of tiles
+    (8100, 752, 1032, 1, False),     # ragged in m (last 256-row tile: 164 rows), n (the last tile's second half: 112 columns) and k
+    (8192, 752, 1032, 1, True),      # the same with w as [n, k]
+    (4096, 3968, 520, 1, True),      # the odd CTA's half of the last column tile lies beyond n
+    (385, 19200, 1024, 0, True),     # a single row into the second CTA's half of the last row tile
+    (8192, 768, 3072, 0, False),     # 48 k-blocks: the stage ring wraps eight times per tile
 ])
 def test_linear_on_cta_pairs(sfb, dtype, m, n, k, act, transposed):
-    """Shapes with at least one 256 x 256 tile per pair of SMs take the two-CTA kernel: against a float32 product on
-    the device (the oracle checks the same entry point on small shapes above)."""
+    """Persistent kernels, on shapes with about one tile per SM and more: against a float32 product on the device (the oracle
+    checks the same entry point on small shapes above)."""
     gen = torch.Generator(device="cuda").manual_seed(77)
     x = torch.randn(m, k, device="cuda", generator=gen).to(TD[dtype])
     w = (0.05 * torch.randn(k, n, device="cuda", generator=gen)).to(TD[dtype])
