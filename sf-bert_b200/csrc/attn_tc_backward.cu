@@ -53,7 +53,7 @@ struct BwParams {
     const uint2 *lut;          // nn_lut (rows) or tn_lut (columns)
     float *delta;              // [B, H, L] -scale * rowsum(dO * O): written by the row kernel, read by the column kernel
     void *out1, *out2;         // dQ, - or dK, dV
-    uint32_t B, H, nb, npairs, blocks, lut_stride, p_rows;
+    uint32_t B, H, nb, blocks, lut_stride, p_rows;
     float scale;
 };
 
@@ -148,7 +148,6 @@ backward_tc_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_consta
         // ===== planner: the coming items and their unions, up to two ahead =====
         uint32_t id = blockIdx.x;
         const uint32_t first_pairs = p.lut_stride == 0 ? long_pairs(p.lut, p.nb, p.blocks, lane) : 0;
-        const uint32_t first_items = first_pairs * p.B * p.H;
         for (uint32_t k = 0;; k++) {
             const uint32_t slot = k & 1;
             if (id != kNoItem && lane == 0) {
@@ -158,18 +157,13 @@ backward_tc_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_consta
             if (k >= 2 && !mbar_wait_warp(&st->list_free[slot], ((k >> 1) - 1) & 1, abort_flag, 70)) break;
             uint32_t n = 0, bh = kNoItem, own[2] = {kNoItem, kNoItem};
             if (id != kNoItem) {
-                const bool first = id < first_items;
-                const uint32_t rest = first ? id : id - first_items, per = first ? first_pairs : p.npairs - first_pairs;
                 // head by head as the product before this call walks P; the row kernel backwards, the column kernel forwards again,
                 // so that each starts with the blocks the kernel before it left in L2
-                uint32_t at = rest / per;
-                const uint32_t pair = rest - at * per + (first ? 0 : first_pairs);
-                if (!COL) at = p.B * p.H - 1 - at;
-                const uint32_t h = at / p.B, b = at - h * p.B;
-                bh = b * p.H + h;
-                const uint2 *lut = p.lut + (size_t)h * p.lut_stride;
-                pick_pair(lut, pair, p.nb, p.blocks, lane, own);
-                n = warp_union(lut, own, st->lists[slot], kBwMaxUnion, lane);
+                const ItemAt it = locate_item(p.lut, p.lut_stride, p.B, p.H, p.nb, p.blocks, first_pairs, id, lane, !COL);
+                bh = it.b * p.H + it.h;
+                own[0] = it.own[0];
+                own[1] = it.own[1];
+                n = warp_union(p.lut + (size_t)it.h * p.lut_stride, own, st->lists[slot], kBwMaxUnion, lane);
                 if (n == kNoItem) {                           // more blocks than the caller's maximum: recorded, zeros written
                     if (lane == 0) atomicCAS(&g_status, 0u, (9u << 24) | (blockIdx.x & 0xffffffu));
                     n = 0;
@@ -526,8 +520,8 @@ static int launch_backward(cudaStream_t s, const void *nn_lut, const void *tn_lu
     }
     const uint32_t npairs = (p.nb_a + 1) / 2;
     const dim3 grid(npairs * p.B * p.H);
-    const BwParams row = {(const uint2 *)nn_lut, delta, dq, nullptr, p.B, p.H, p.nb_a, npairs, p.blocks, p.lut_stride, (uint32_t)prow, scale};
-    const BwParams col = {(const uint2 *)tn_lut, delta, dk, dv, p.B, p.H, p.nb_a, npairs, p.blocks, p.lut_stride, (uint32_t)prow, scale};
+    const BwParams row = {(const uint2 *)nn_lut, delta, dq, nullptr, p.B, p.H, p.nb_a, p.blocks, p.lut_stride, (uint32_t)prow, scale};
+    const BwParams col = {(const uint2 *)tn_lut, delta, dk, dv, p.B, p.H, p.nb_a, p.blocks, p.lut_stride, (uint32_t)prow, scale};
     launch_overlapped(backward_tc_kernel<false, BF16>, grid, dim3(kBwThreads), kBwSmem, s, pm, vm, km, dm, om, row);
     launch_overlapped(backward_tc_kernel<true, BF16>, grid, dim3(kBwThreads), kBwSmem, s, pm, dm, qm, vm, vm, col);
     return check_launch("sfb_attention_backward");

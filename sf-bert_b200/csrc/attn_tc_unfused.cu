@@ -463,7 +463,8 @@ fused_p_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constan
     grid_dependency_wait();
     grid_launch_dependents();
     // last (batch, head) first: the product that reads the probabilities next starts with the ones still in L2
-    const ItemAt it = locate_item(p.nn_lut, p.lut_stride, p.B, p.H, p.nb, p.blocks, blockIdx.x, lane, true);
+    const uint32_t first_pairs = p.lut_stride == 0 ? long_pairs(p.nn_lut, p.nb, p.blocks, lane) : 0;
+    const ItemAt it = locate_item(p.nn_lut, p.lut_stride, p.B, p.H, p.nb, p.blocks, first_pairs, blockIdx.x, lane, true);
     const uint32_t b = it.b, h = it.h;
     build_union(p.nn_lut + (size_t)h * p.lut_stride, it.own, st->entries, st->cand, &st->n_union, &st->abort_flag);
     if (warp == 0) {

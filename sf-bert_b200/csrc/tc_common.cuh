@@ -510,16 +510,15 @@ __device__ __forceinline__ uint32_t long_pairs(const uint2 *lut, uint32_t nb, ui
     return (n_long + 1) / 2;
 }
 
-// Item `id` of a launch over the row pairs of all (batch, head)s, one CTA each: the long pairs of all of them first (with one
-// LUT for all heads), then the rest, head by head; `back`: from the last (batch, head).  Every warp calls it.
+// Item `id` of a launch over the row pairs of all (batch, head)s: the long pairs of all of them first (first_pairs of each, see
+// long_pairs; 0 with a LUT per head), then the rest, head by head; `back`: from the last (batch, head).  A warp calls it.
 struct ItemAt {
     uint32_t b, h, own[2];
 };
 __device__ __forceinline__ ItemAt locate_item(const uint2 *lut, uint32_t lut_stride, uint32_t B, uint32_t H, uint32_t nb, uint32_t blocks,
-                                              uint32_t id, uint32_t lane, bool back)
+                                              uint32_t first_pairs, uint32_t id, uint32_t lane, bool back)
 {
-    const uint32_t npairs = (nb + 1) / 2;
-    const uint32_t first_pairs = lut_stride == 0 ? long_pairs(lut, nb, blocks, lane) : 0, first_items = first_pairs * B * H;
+    const uint32_t npairs = (nb + 1) / 2, first_items = first_pairs * B * H;
     const bool first = id < first_items;
     const uint32_t rest = first ? id : id - first_items, per = first ? first_pairs : npairs - first_pairs;
     uint32_t at = rest / per;
