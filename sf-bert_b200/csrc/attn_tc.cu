@@ -36,10 +36,24 @@ constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kStreamCols = 160;
 constexpr float kRescaleThreshold = 8.0f;       // log2 units: P stays below 2^8
 
+// a UnionEntry with column and flags in one word: the softmax warps read one word per step (apart, stride and BigBird 1 % slower)
 struct UEntry {
     uint32_t col_flags;   // key block column | bit 30: upper block-row has it | bit 31: lower block-row has it
     uint32_t blk[2];      // block ids (for the element masks)
     uint32_t pad;
+    __device__ __forceinline__ void put(uint32_t col, uint32_t row, uint32_t block)
+    {
+        col_flags = (col & 0x3fffffffu) | (1u << (30 + row));
+        blk[0] = row ? 0u : block;
+        blk[1] = row ? block : 0u;
+    }
+    __device__ __forceinline__ bool take(uint32_t col, uint32_t block)
+    {
+        if (((col_flags ^ col) & 0x3fffffffu) != 0) return false;
+        col_flags |= 1u << 31;
+        blk[1] = block;
+        return true;
+    }
 };
 
 struct StreamState {
@@ -135,51 +149,6 @@ __device__ __forceinline__ bool mbar_wait2(uint64_t *bar_a, uint32_t par_a, uint
     const bool a = mbar_try_wait(bar_a, par_a), b = mbar_try_wait(bar_b, par_b);
     if (a && b) return true;
     return (a || mbar_wait(bar_a, par_a, abort_flag, code)) && (b || mbar_wait(bar_b, par_b, abort_flag, code));
-}
-
-// The union of the key blocks of block-rows 2*pair and 2*pair+1, built by ONE warp: the upper row's blocks in LUT
-// order, then the blocks only the lower row has.  Returns the number of entries, or 0xffffffff when a row or the
-// union does not fit kMaxU.
-__device__ __forceinline__ uint32_t plan_union(const uint2 *nn, uint32_t pair, uint32_t nb, UEntry *ent, uint32_t lane)
-{
-    const uint32_t row0 = pair * 2, row1 = pair * 2 + 1;
-    const uint2 head0 = nn[row0];
-    const uint2 head1 = row1 < nb ? nn[row1] : make_uint2(0, 0);
-    const uint32_t n0 = head0.y, n1 = head1.y;
-    if (n0 > (uint32_t)kMaxU || n1 > (uint32_t)kMaxU) return 0xffffffffu;
-    for (uint32_t i = lane; i < n0; i += 32) {
-        const uint2 e = nn[head0.x + i];
-        ent[i].col_flags = (e.y & 0x3fffffffu) | (1u << 30);
-        ent[i].blk[0] = e.x;
-        ent[i].blk[1] = 0;
-    }
-    __syncwarp();
-    uint32_t n = n0;
-    for (uint32_t base = 0; base < n1; base += 32) {
-        const uint32_t i = base + lane;
-        const bool valid = i < n1;
-        const uint2 e = valid ? nn[head1.x + i] : make_uint2(0, 0);
-        bool fresh = valid;
-        if (valid)
-            for (uint32_t u = 0; u < n0; u++)
-                if ((ent[u].col_flags & 0x3fffffffu) == (e.y & 0x3fffffffu)) {
-                    ent[u].col_flags |= 1u << 31;
-                    ent[u].blk[1] = e.x;
-                    fresh = false;
-                    break;
-                }
-        const uint32_t votes = __ballot_sync(0xffffffffu, fresh);
-        const uint32_t at = n + __popc(votes & ((1u << lane) - 1u));
-        if (n + __popc(votes) > (uint32_t)kMaxU) return 0xffffffffu;
-        if (fresh) {
-            ent[at].col_flags = (e.y & 0x3fffffffu) | (1u << 31);
-            ent[at].blk[0] = 0;
-            ent[at].blk[1] = e.x;
-        }
-        n += __popc(votes);
-    }
-    __syncwarp();
-    return n;
 }
 
 // A TMA producer: IS_K = true loads every item's query tile and key tiles, IS_K = false its value tiles (the two run
@@ -381,8 +350,9 @@ fused_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
                 const uint32_t slot = k & 1;
                 if (k >= 2 && !mbar_wait_warp(&st->list_free[slot], ((k >> 1) - 1) & 1, abort_flag, 20)) break;
                 const Item it = decode_item(id, p);
-                uint32_t n = plan_union(p.nn_lut + (size_t)it.h * p.lut_stride, it.pair, p.nb, lists + (s * 2 + slot) * kMaxU, lane);
-                if (n == 0xffffffffu) {
+                const uint32_t own[2] = {it.pair * 2, it.pair * 2 + 1 < p.nb ? it.pair * 2 + 1 : kNoItem};
+                uint32_t n = warp_union(p.nn_lut + (size_t)it.h * p.lut_stride, own, lists + (s * 2 + slot) * kMaxU, (uint32_t)kMaxU, lane);
+                if (n == kNoItem) {
                     // a row pair that is too long for this kernel: recorded, and the pair's rows are written as zeros
                     if (lane == 0) atomicCAS(&g_status, 0u, (9u << 24) | (blockIdx.x & 0xffffffu));
                     n = 0;

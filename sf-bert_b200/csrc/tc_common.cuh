@@ -20,6 +20,20 @@ struct UnionEntry {
     uint32_t col;      // key block column
     uint32_t flags;    // bit 0: upper block-row has it, bit 1: lower block-row has it
     uint32_t blk[2];   // block ids
+    __device__ __forceinline__ void put(uint32_t c, uint32_t row, uint32_t block)      // a block that row 0 or 1 has
+    {
+        col = c;
+        flags = 1u << row;
+        blk[0] = row ? 0u : block;
+        blk[1] = row ? block : 0u;
+    }
+    __device__ __forceinline__ bool take(uint32_t c, uint32_t block)                  // the lower row has it too
+    {
+        if (col != c) return false;
+        flags |= 2;
+        blk[1] = block;
+        return true;
+    }
 };
 
 // 0 = ok; otherwise (code << 24 | CTA index) of the first CTA that gave up on a bounded wait.  One copy per
@@ -433,7 +447,8 @@ __device__ __forceinline__ void pick_pair(const uint2 *lut, uint32_t pair, uint3
 
 // The union of the blocks of rows (columns) own[0] and own[1], built by ONE warp: the first one's in LUT order, then those
 // only the second has.  At most `most` entries (checked by the host); kNoItem when the LUT says otherwise.
-__device__ __forceinline__ uint32_t warp_union(const uint2 *lut, const uint32_t (&own)[2], UnionEntry *ent, uint32_t most, uint32_t lane)
+template <typename Entry>
+__device__ __forceinline__ uint32_t warp_union(const uint2 *lut, const uint32_t (&own)[2], Entry *ent, uint32_t most, uint32_t lane)
 {
     const uint2 head0 = lut[own[0]];
     const uint2 head1 = own[1] != kNoItem ? lut[own[1]] : make_uint2(0, 0);
@@ -442,10 +457,7 @@ __device__ __forceinline__ uint32_t warp_union(const uint2 *lut, const uint32_t 
     uint2 next = lane < n1 ? lut[head1.x + lane] : make_uint2(0, 0);      // on its way while the first list is written
     for (uint32_t i = lane; i < n0; i += 32) {
         const uint2 e = lut[head0.x + i];
-        ent[i].col = e.y;
-        ent[i].flags = 1;
-        ent[i].blk[0] = e.x;
-        ent[i].blk[1] = 0;
+        ent[i].put(e.y, 0, e.x);
     }
     __syncwarp();
     uint32_t n = n0;
@@ -456,21 +468,14 @@ __device__ __forceinline__ uint32_t warp_union(const uint2 *lut, const uint32_t 
         bool fresh = valid;
         if (valid)
             for (uint32_t u = 0; u < n0; u++)
-                if (ent[u].col == e.y) {
-                    ent[u].flags |= 2;
-                    ent[u].blk[1] = e.x;
+                if (ent[u].take(e.y, e.x)) {
                     fresh = false;
                     break;
                 }
         const uint32_t votes = __ballot_sync(0xffffffffu, fresh);
         const uint32_t at = n + __popc(votes & ((1u << lane) - 1u));
         if (n + __popc(votes) > most) return kNoItem;
-        if (fresh) {
-            ent[at].col = e.y;
-            ent[at].flags = 2;
-            ent[at].blk[0] = 0;
-            ent[at].blk[1] = e.x;
-        }
+        if (fresh) ent[at].put(e.y, 1, e.x);
         n += __popc(votes);
     }
     __syncwarp();
