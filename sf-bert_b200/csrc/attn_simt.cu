@@ -884,7 +884,7 @@ __device__ __forceinline__ void stage_gather(float *dst, uint32_t stride, const 
     }
 }
 template <int D>
-__global__ void __launch_bounds__(tile::kThreads, 3) csr_tile_f32_kernel(const __grid_constant__ CsrTileArgs a)
+__global__ void __launch_bounds__(tile::kThreads, 3) csr_tile_f32_kernel(const CsrTileArgs a)
 {
     using namespace tile;
     typedef FaCfg<32, D> Cfg;
@@ -1032,7 +1032,7 @@ __global__ void __launch_bounds__(tile::kThreads, 3) csr_tile_f32_kernel(const _
     __syncthreads();
     const uint32_t rows = *again;
     for (uint32_t r = warp; r < 32; r += 4)
-        if ((rows >> r) & 1u) csr_row_again<SFB_F32, D>(a, b, h, tl * 32 + r);
+        if ((rows >> r) & 1u) csr_row_again<SFB_F32, D>(a.rowptr, a.colidx, a.nnz, a.Q, a.K, a.V, a.O, a.L, a.H, b, h, tl * 32 + r, a.scale_log2e);
 }
 
 // ------------------------------------------------------------------------------------------------

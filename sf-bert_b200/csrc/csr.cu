@@ -211,7 +211,7 @@ __device__ __forceinline__ float ex2f(float x)
 }
 
 template <bool BF16, int D>
-__global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const __grid_constant__ CsrTileArgs a)
+__global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const CsrTileArgs a)
 {
     typedef CsrCfg<D> Cfg;
     constexpr int MT = Cfg::MT, KC = Cfg::KC, NT = KC / 8, CH = D / 8, DN = D / 8;
@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const __
     while (odd) {
         const uint32_t first_lane = __ffs(odd) - 1u, rr = (warp * 32 + first_lane) >> 2;
         odd &= ~(0xfu << (first_lane & ~3u));
-        csr_row_again<BF16 ? SFB_BF16 : SFB_F16, D>(a, b, h, tile * 32 + rr);
+        csr_row_again<BF16 ? SFB_BF16 : SFB_F16, D>(a.rowptr, a.colidx, a.nnz, a.Q, a.K, a.V, a.O, a.L, a.H, b, h, tile * 32 + rr, a.scale_log2e);
     }
 }
 
