@@ -639,9 +639,18 @@ def run_bandwidth_kernel(args):
         rowptr, colidx = sfb.csr_from_layout(lay)
         q, k, v = (torch.randn(B, L, H, d, device="cuda").to(tdt) for _ in range(3))
         fn = lambda: sfb.csr_attention(q, k, v, rowptr, colidx, 0.125)
-        # what the format makes every query row gather: its keys' K and V rows (through L2), plus Q in and O out
-        nbytes = int(colidx.numel()) * B * H * 2 * d * q.element_size() + 2 * q.numel() * q.element_size()
-        name, unit_name = "csr_attention_split_kernel", "K and V rows gathered per query row (L2 traffic, not HBM) + Q read + O written"
+        if sfb.lib.sfb_csr_workspace(colidx.numel(), L):
+            # every tile of 32 query rows gathers the K and V rows of the columns that any of them has, once per (batch, head), and
+            # reads its list of them (8 bytes each); the plan reads the pattern and writes the lists; plus Q in and O out
+            rows = torch.repeat_interleave(torch.arange(L, device="cuda"), rowptr.diff().long())
+            columns = torch.unique(rows // 32 * L + colidx.long()).numel()
+            nbytes = columns * (B * H * (2 * d * q.element_size() + 8) + 8) + 4 * colidx.numel() + 2 * q.numel() * q.element_size()
+            name = "csr_plan_kernel + " + ("csr_tile_f32_kernel" if tdt == torch.float32 else "csr_tile_kernel")
+            unit_name = "pattern and column lists + K and V rows gathered per tile of 32 query rows (L2 traffic, not HBM) + Q read + O written"
+        else:
+            # a warp per query row: it gathers the K and V rows of its own keys
+            nbytes = int(colidx.numel()) * B * H * 2 * d * q.element_size() + 2 * q.numel() * q.element_size()
+            name, unit_name = "csr_attention_split_kernel", "K and V rows gathered per query row (L2 traffic, not HBM) + Q read + O written"
     elif args.kernel == "embedding":
         tdt = {"f16": torch.float16, "bf16": torch.bfloat16, "f32": torch.float32}[cfg["dtype"]]
         vocab, hidden = 30522, H * d
@@ -677,9 +686,9 @@ def run_bandwidth_kernel(args):
         if args.fused_grad:
             o = sfb.bst_sgemm_xn(pblk, v, lay)
             fn = lambda: sfb.attention_backward_fused(q, k, v, pblk, o, do, lay, 0.125)
-            # dV: P in; dS: P in, dS out; dK, dQ: dS in
-            nbytes = 5 * blk_bytes + 10 * q.numel() * 2
-            name, unit_name = "spmm_tc_kernel x3 + sddmm_tc_kernel<GRAD> + rowdot_kernel", "5 passes over the block tensors + the dense operands"
+            # P in for dQ and again for dK and dV, dS on chip; O, dO, Q, K, V in, dQ, dK, dV out, V and dO in for both
+            nbytes = 2 * blk_bytes + 10 * q.numel() * 2
+            name, unit_name = "backward_tc_kernel (rows) + backward_tc_kernel (columns)", "2 passes over P + the dense operands"
         else:
             fn = lambda: sfb.attention_backward(q, k, v, pblk, do, lay, 0.125)
             # dV: P in; dP: out; dS: dP, P in, dS out; dK, dQ: dS in -- plus each [B,L,H,d] operand once per call
@@ -770,7 +779,8 @@ def run_bandwidth_kernel(args):
                      "copy_of_same_bytes": {"gbs": round(copy_gbs, 1), "ms": round(copy_ms, 5),
                                             "frac_of_it": round(gbs / copy_gbs, 4)},
                      "fill_gbs": round(fill_gbs, 1)},
-        "gpu_launches": args.steps * (5 if args.kernel == "attention_backward" else 1), "clocks": clocks}), flush=True)
+        "gpu_launches": args.steps * (2 if name.startswith(("backward_tc_kernel", "csr_plan_kernel")) else 5 if args.kernel == "attention_backward" else 1),
+        "clocks": clocks}), flush=True)
 
 
 def run_linear(args, sfb, cfg, pk, flush):
@@ -1139,7 +1149,7 @@ if __name__ == "__main__":
                     help="fused = the headline fused attention; softmax / layernorm = the bandwidth kernels (N=1)")
     ap.add_argument("--projections", default="tensor", choices=["tensor", "library"],
                     help="--kernel encoder_layer: the layer's GEMMs on this library's tcgen05 kernel or on the GEMM library")
-    ap.add_argument("--fused-grad", action="store_true", help="--kernel attention_backward: dP and dS in one launch (sfb_fused_sddmm_softmax_grad)")
+    ap.add_argument("--fused-grad", action="store_true", help="--kernel attention_backward: the one-call backward with dS on chip (sfb_attention_backward)")
     ap.add_argument("--l2-flush", default="write_read", choices=["write_read", "write"],
                     help="what runs between timed steps: 256 MB written and 256 MB read (cold, clean L2), or the write alone")
     ap.add_argument("--layers", type=int, default=24, help="--kernel encoder_stack: number of encoder layers")

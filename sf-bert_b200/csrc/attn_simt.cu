@@ -2,9 +2,10 @@
 // SpMM and the two block-row-owned fusions.  They serve fp32 operands (1e-5 parity with the CPU
 // reference cannot be met on tensor cores) and every shape the tcgen05 kernels do not cover.
 //
-// Thread layout shared by all matmul kernels: 256 threads as a 16x16 grid; thread (ty,tx) owns
-// rows ty+16m and columns tx+16n of a tile, so the 16 lanes of a half-warp own one set of rows
-// and row reductions are four shuffles.
+// SDDMM, SpMM, the fused attention and the fp32 element-sparse tiles are made of warp tiles of 4 x 8
+// outputs per thread (simt_tile.cuh).  The fused SDDMM + softmax (fused_sddmm_softmax_kernel) has 256
+// threads as a 16x16 grid; thread (ty,tx) owns rows ty+16m and columns tx+16n of a tile, so the 16
+// lanes of a half-warp own one set of rows and row reductions are four shuffles.
 #include "simt_tile.cuh"
 #include "csr.cuh"
 #include <float.h>

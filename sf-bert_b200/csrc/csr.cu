@@ -64,8 +64,8 @@ __global__ void __launch_bounds__(128) csr_attention_split_kernel(const int32_t 
 // HALVES: the distinct columns come in three groups: those that only the tile's first 16 rows have, those of both halves,
 // those of the last 16 rows alone.  Scattered columns mostly belong to one row; the kernels whose warps work for 16 rows
 // (D 128) leave out the group of the other half.
-// A warp per row, whose elements are on their way at once (102.4 us with the tiles at B 2, H 12, L 4096 against 106 with
-// two rows per warp).  The tiles' launch is not let in early: their CTAs would crowd the SMs that the plan left free and stay
+// A warp per row, whose elements are on their way at once (plan and tiles of the window pattern, B 2, H 12, L 4096, d 64:
+// 105.8 us against 108.7 with two rows per warp).  The tiles' launch is not let in early: their CTAs would crowd the SMs that the plan left free and stay
 // there (128 tiles, B 1, H 1: 24.4 us, 17.4 like this).
 constexpr uint32_t kPlanThreads = 1024;
 constexpr uint32_t kPlanMaxL = 48 * 1024;                    // columns whose masks fit shared memory

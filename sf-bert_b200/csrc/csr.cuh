@@ -137,7 +137,7 @@ __device__ __forceinline__ void csr_row(const int32_t *__restrict__ colidx, int3
             }
         }
     }
-    // merge the 16 pairs' softmaxes (the two lanes of a pair hold the same max and sum: offsets 16..2 only)
+    // merge the groups' softmaxes (the LPK lanes of a group hold the same max and sum: offsets from LPK on)
     float M = m;
 #pragma unroll
     for (int o = 16; o >= LPK; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
@@ -151,7 +151,7 @@ __device__ __forceinline__ void csr_row(const int32_t *__restrict__ colidx, int3
         float a = acc[x] * f;
 #pragma unroll
         for (int o = 16; o >= LPK; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        // every lane of this parity holds the element now; pair x % 16 writes it
+        // every lane with this share of the head holds the element now; group x % KPI writes it
         if ((x % KPI) == (int)pi) Elem<DT>::store(O, row_off + x, a * inv);
     }
 }

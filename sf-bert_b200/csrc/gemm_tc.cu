@@ -37,7 +37,7 @@ struct GParams {
     int is_bf16, act;
     int w_transposed;   // w is [n, k] row-major (out = x . w^T, the tied-embedding logits): its tile is a K-major B operand
     uint32_t band;      // CTA-pair kernel: column tiles per band of the tile order (tile_coords)
-    const void *resid;  // split kernel: [m, n] of x's type, added to the product (may be out itself), or NULL
+    const void *resid;  // split kernel: [m, n] of x's type, added to the product (not out itself), or NULL
 };
 
 // Tile t of the CTA-pair kernel -> (row tile, column tile).  The tiles run band by band, a band being `band` column
@@ -724,7 +724,7 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
     if (split > 1) {
         // every CTA of the cluster reaches both barriers, also after a timeout (the status word then says that the sums are not to be used)
         cluster_sync_all();
-        const uint32_t rows = kGBM / split, first = rank * rows;      // split is 2, 4 or 8
+        const uint32_t rows = kGBM / split, first = rank * rows;      // split is 2 or 4
         const uint32_t mine = smem_u32(acc_s);
         constexpr uint32_t PIECES = BN / 8;
         for (uint32_t t = threadIdx.x; t < rows * PIECES; t += 256) {
