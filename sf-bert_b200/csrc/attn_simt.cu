@@ -1,10 +1,10 @@
-// FP32-arithmetic (CUDA-core) kernels of the block-sparse attention path: SDDMM, masked softmax,
-// SpMM and the two block-row-owned fusions.  They serve fp32 operands (1e-5 parity with the CPU
-// reference cannot be met on tensor cores) and every shape the tcgen05 kernels do not cover.
+// Kernels of the block-sparse attention path that serve fp32 operands (1e-5 parity with the CPU reference, more than one
+// 16-bit or tf32 product gives) and every shape the tcgen05 kernels do not cover: SDDMM, masked softmax, SpMM and the two
+// block-row-owned fusions.
 //
-// SDDMM, SpMM, the fused attention and the fp32 element-sparse tiles are made of warp tiles of 4 x 8
-// outputs per thread (simt_tile.cuh).  The fused SDDMM + softmax (fused_sddmm_softmax_kernel) has 256
-// threads as a 16x16 grid; thread (ty,tx) owns rows ty+16m and columns tx+16n of a tile, so the 16
+// SDDMM, SpMM, the fused attention and the fp32 element-sparse tiles take their products from warp-level tensor-core
+// instructions on operands split into bf16 terms (simt_tile.cuh).  The fused SDDMM + softmax (fused_sddmm_softmax_kernel) is on the
+// FMA pipe: 256 threads as a 16x16 grid; thread (ty,tx) owns rows ty+16m and columns tx+16n of a tile, so the 16
 // lanes of a half-warp own one set of rows and row reductions are four shuffles.
 #include "simt_tile.cuh"
 #include "csr.cuh"
@@ -36,102 +36,125 @@ __device__ __forceinline__ void load_tile_kmajor(float (*dst)[BS + 1], const voi
 }
 
 // ------------------------------------------------------------------------------------------------
+// A score that is not finite, made again by plain FMAs (simt_tile.cuh says why).
+template <int DT>
+__device__ __noinline__ float dot_again(const void *A, const void *B, size_t a, size_t b, uint32_t d)
+{
+    float s = 0.f;
+    for (uint32_t k = 0; k < d; k++) s = fmaf(Elem<DT>::load(A, a + k), Elem<DT>::load(B, b + k), s);
+    return s;
+}
+
 // SDDMM.  A CTA (four warps) makes one 64x64 block, a 32x32 quarter per warp, or four consecutive 32x32 blocks of the LUT,
-// one per warp.  Consecutive blocks mostly share their block-row (the LUT is in row-major scan order): its query rows
-// are then staged once for the four.  Both operands come chunk by chunk (32 of d) through two buffers; the scores leave
-// through shared memory, eight per lane, so that a row is written in whole pieces of 16 or 32 bytes.
+// one per warp.  The keys come chunk by chunk (32 of d) through a ring of the warps that use them; the query rows go straight to
+// fragments, a chunk ahead in registers: consecutive blocks mostly share their block-row (the LUT is in row-major scan
+// order), so three of the four warps find them in L1.  No warp waits for another one that does not share its keys.  A thread
+// holds eight neighbouring scores of a row, so that they leave in whole pieces of 16 or 32 bytes.
+template <int BS> struct SddmmCfg {
+    static constexpr int TEAMS = BS == 32 ? 4 : 2, TT = 128 / TEAMS;      // teams that stage keys of their own
+    static constexpr uint32_t buf = 32 * tile::kStride;
+};
 template <int BS, int AB_DT, int C_DT>
 __global__ void __launch_bounds__(tile::kThreads, 3) sddmm_nt_kernel(const uint2 *__restrict__ lut, const void *__restrict__ A,
                                                                    const void *__restrict__ Bm, void *__restrict__ C, AttnDims p, bool vec)
 {
     using namespace tile;
+    typedef SddmmCfg<BS> Cfg;
     constexpr uint32_t PER = BS == 32 ? 4 : 1;               // blocks per CTA
-    constexpr uint32_t ROWS = PER * BS;                      // staged rows of each operand: 128 or 64
-    constexpr uint32_t BUF = 2 * ROWS * kStride;
-    extern __shared__ __align__(16) float sm[];              // [2][A rows | B rows]
+    constexpr int T = kTerms<AB_DT>, TT = Cfg::TT;
+    extern __shared__ __align__(16) float sm[];              // [team][2][32 keys]
     grid_dependency_wait();
     grid_launch_dependents();
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane_row(lane), lc = lane_quad(lane);
-    const uint32_t bid0 = blockIdx.x * PER, b = blockIdx.y, h = blockIdx.z;
-    const uint32_t nblk = min(PER, p.blocks - bid0);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const uint32_t b = blockIdx.y, h = blockIdx.z;
+    const uint32_t bid = blockIdx.x * PER + (BS == 32 ? warp : 0);
+    if (bid >= p.blocks) return;
+    const uint32_t r0 = BS == 64 ? 32 * (warp >> 1) : 0, team = BS == 64 ? warp & 1 : warp, c0 = BS == 64 ? 32 * team : 0;
+    const uint32_t rank = BS == 64 ? 32 * (warp >> 1) + lane : lane;
     const size_t HD = (size_t)p.H * p.d;
-    const size_t head = (size_t)h * p.d;
-    size_t offA[PER], offB[PER];
-    bool shared_rows = true;
-    {
-        const uint2 *e = lut + (size_t)h * p.lut_stride + bid0;
-        const uint32_t x0 = e[0].x;
+    const uint2 en = lut[(size_t)h * p.lut_stride + bid];
+    const size_t rowA = (((size_t)b * p.nb_a + en.x) * BS + r0) * HD + (size_t)h * p.d, rowB = (((size_t)b * p.nb_b + en.y) * BS + c0) * HD + (size_t)h * p.d;
+    float *bufs = sm + team * 2 * Cfg::buf;
+    Staged<AB_DT, TT, (int)kChunk> held_b;
+    Raw4<AB_DT> held_a[8];                                   // [16-element half of the chunk][row 16 m + 8 half + g]
+    const uint32_t chunks = (p.d + kChunk - 1) / kChunk;
+    auto load_a = [&](uint32_t c) {
 #pragma unroll
-        for (uint32_t k = 0; k < PER; k++) {
-            const uint2 en = k < nblk ? e[k] : e[0];
-            offA[k] = ((size_t)b * p.nb_a + en.x) * BS * HD + head;
-            offB[k] = ((size_t)b * p.nb_b + en.y) * BS * HD + head;
-            shared_rows = shared_rows && en.x == x0;
+        for (int i = 0; i < 8; i++) {
+            const uint32_t k = c * kChunk + 16 * (i >> 2) + 4 * t;
+            load_raw4<AB_DT>(held_a[i], A, rowA + (size_t)(8 * (i & 3) + g) * HD + k, k < p.d ? p.d - k : 0u, vec);
         }
-    }
+    };
     auto issue = [&](uint32_t c) {
-        float *buf = sm + (c & 1) * BUF;
-        const uint32_t k0 = c * kChunk, left = p.d - k0;
-#pragma unroll
-        for (uint32_t g = 0; g < PER; g++)
-            if (g < nblk) {
-                if (g == 0 || !shared_rows) stage<AB_DT, BS, (int)kChunk>(buf + g * BS * kStride, kStride, A, offA[g] + k0, HD, left, vec);
-                stage<AB_DT, BS, (int)kChunk>(buf + (ROWS + g * BS) * kStride, kStride, Bm, offB[g] + k0, HD, left, vec);
-            }
+        stage_begin(held_b, rank, bufs + (c & 1) * Cfg::buf, kStride, Bm, rowB + c * kChunk, HD, p.d - c * kChunk, vec);
         cp_commit();
     };
-    const bool live = BS == 64 || warp < nblk;
-    const uint32_t r0 = BS == 64 ? 32 * (warp >> 1) : (shared_rows ? 0 : 32 * warp), c0 = BS == 64 ? 32 * (warp & 1) : 32 * warp;
-    uint64_t acc[4][8];
-#pragma unroll
-    for (int m = 0; m < 4; m++)
-#pragma unroll
-        for (int n = 0; n < 8; n++) acc[m][n] = 0;
-    const uint32_t chunks = (p.d + kChunk - 1) / kChunk;
+    float acc[2][4][4] = {};
     issue(0);
+    load_a(0);
+    stage_end(held_b, rank, bufs, kStride, vec);
     for (uint32_t c = 0; c < chunks; c++) {
-        cp_wait_all();
-        __syncthreads();
+        cp_wait<0>();
+        meet<TT, (int)kThreads>(1 + team);
         if (c + 1 < chunks) issue(c + 1);
-        const float *buf = sm + (c & 1) * BUF;
-        if (live) mma_nt(acc, buf + (r0 + lr) * kStride, kStride, buf + (ROWS + c0 + lc) * kStride, kStride);
-    }
-    __syncthreads();
-    if (!live) return;
-    float *t = sm + warp * 32 * kStride;
+        Frag<T> fa[2][2];
 #pragma unroll
-    for (int m = 0; m < 4; m++)
+        for (int k = 0; k < 2; k++)
 #pragma unroll
-        for (int n = 0; n < 8; n++) t[(lr + 8 * m) * kStride + lc + 4 * n] = half_sum(acc[m][n]);
-    __syncwarp();
-    const size_t baseC = (((size_t)b * p.H + h) * p.blocks + bid0 + (BS == 64 ? 0 : warp)) * BS * BS + (BS == 64 ? (size_t)r0 * BS + c0 : 0);
-#pragma unroll
-    for (int m = 0; m < 4; m++) {
-        const float *row = t + (lr + 8 * m) * kStride + lc * 8;
-        const float4 u = *(const float4 *)row, w = *(const float4 *)(row + 4);
-        const float v[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
-        const size_t at = baseC + (size_t)(lr + 8 * m) * BS + lc * 8;
-        if (vec) {
-            if (C_DT == SFB_F32) {
-                *(float4 *)((float *)C + at) = u;
-                *(float4 *)((float *)C + at + 4) = w;
-            } else {
-                uint32_t q[4];
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    if (C_DT == SFB_BF16) q[k] = to_bhalf_bits(v[2 * k]) | ((uint32_t)to_bhalf_bits(v[2 * k + 1]) << 16);
-                    else {
-                        __half2 hh = __floats2half2_rn(v[2 * k], v[2 * k + 1]);
-                        q[k] = *reinterpret_cast<uint32_t *>(&hh);
-                    }
-                }
-                *(uint4 *)((uint16_t *)C + at) = make_uint4(q[0], q[1], q[2], q[3]);
+            for (int m = 0; m < 2; m++) {
+                float x0[4], x1[4];
+                widen4<AB_DT>(x0, held_a[4 * k + 2 * m]);
+                widen4<AB_DT>(x1, held_a[4 * k + 2 * m + 1]);
+                split_rows<T>(fa[k][m], x0, x1);
             }
-        } else {
+        if (c + 1 < chunks) load_a(c + 1);
 #pragma unroll
-            for (int k = 0; k < 8; k++) Elem<C_DT>::store(C, at + k, v[k]);
+        for (int k = 0; k < 2; k++) {
+            Four<T> fb[4];
+            load_keys<T, true>(fb, bufs + (c & 1) * Cfg::buf, 16 * k, g, t);
+#pragma unroll
+            for (int m = 0; m < 2; m++) mma16<4, T, T>(acc[m], fa[k][m], fb);
+        }
+        if (c + 1 < chunks) stage_end(held_b, rank, bufs + ((c + 1) & 1) * Cfg::buf, kStride, vec);
+    }
+    if (T > 1 && !(zero_if_finite<4>(acc[1], zero_if_finite<4>(acc[0], 0.f)) == 0.f)) {
+#pragma unroll
+        for (int x = 0; x < 32; x++) {
+            float &v = acc[x >> 4][(x >> 2) & 3][x & 3];
+            if (!finite(v))
+                v = dot_again<AB_DT>(A, Bm, rowA + (16 * (x >> 4) + 8 * ((x >> 1) & 1) + g) * HD, rowB + score_key<true>(t, (x >> 2) & 3, x & 1) * HD, p.d);
         }
     }
+    const size_t baseC = (((size_t)b * p.H + h) * p.blocks + bid) * BS * BS + (size_t)r0 * BS + c0;
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = acc[m][k >> 1][2 * half + (k & 1)];
+            const size_t at = baseC + (size_t)(16 * m + 8 * half + g) * BS + 8 * t;
+            if (vec) {
+                if (C_DT == SFB_F32) {
+                    *(float4 *)((float *)C + at) = make_float4(v[0], v[1], v[2], v[3]);
+                    *(float4 *)((float *)C + at + 4) = make_float4(v[4], v[5], v[6], v[7]);
+                } else {
+                    uint32_t q[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        if (C_DT == SFB_BF16) q[k] = to_bhalf_bits(v[2 * k]) | ((uint32_t)to_bhalf_bits(v[2 * k + 1]) << 16);
+                        else {
+                            __half2 hh = __floats2half2_rn(v[2 * k], v[2 * k + 1]);
+                            q[k] = *reinterpret_cast<uint32_t *>(&hh);
+                        }
+                    }
+                    *(uint4 *)((uint16_t *)C + at) = make_uint4(q[0], q[1], q[2], q[3]);
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < 8; k++) Elem<C_DT>::store(C, at + k, v[k]);
+            }
+        }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -498,74 +521,149 @@ __global__ void __launch_bounds__(BS * BS / 8 / SPLIT) softmax_grad_kernel(const
 }
 
 // ------------------------------------------------------------------------------------------------
+// An output that is not finite, made again by plain FMAs.  pbase: first block of the (batch, head); vbase: this column in its first row.
+template <int BS, int A_DT, int BC_DT, bool TRANS>
+__device__ __noinline__ float spmm_again(const uint2 *ent, uint32_t cnt, const void *Pm, const void *V, size_t pbase, size_t vbase, size_t HD, uint32_t r)
+{
+    float s = 0.f;
+    for (uint32_t e = 0; e < cnt; e++)
+        for (uint32_t k = 0; k < BS; k++)
+            s = fmaf(Elem<A_DT>::load(Pm, pbase + ((size_t)ent[e].x * BS + (TRANS ? k : r)) * BS + (TRANS ? r : k)),
+                     Elem<BC_DT>::load(V, vbase + ((size_t)ent[e].y * BS + k) * HD), s);
+    return s;
+}
+
 // SpMM: one CTA per (block-row, slice of up to 128 of d).  TRANS = false: O = sum over the row's blocks of P . V (NN, the
 // lut is the nn_lut).  TRANS = true: the backward products dV = P^T dO and dK = dS^T Q -- the lut is the tn_lut,
 // "row" i is a block COLUMN, an entry names a block of that column and the block-row its B rows come from, and
 // the block is used transposed (read as it lies, four neighbouring rows of P^T per 16-byte load).
-// A chunk is 32 elements of the contraction: one 32x32 block, or half of a 64x64 one, with its 32 rows of V.
+// A chunk is 32 elements of the contraction: one 32x32 block, or half of a 64x64 one, with its 32 rows of V.  A warp owns 32
+// output rows and a share of the columns; it stages its own columns of V (with the other warp that has them, where blocks
+// are 64 rows) and reads P straight into fragments, a chunk ahead in registers: P is small beside V, and L1 has it for
+// the other warps.
 template <int BS, int DS> struct SpmmCfg {
-    static constexpr int WC = BS == 32 ? 4 : 2;                          // warps side by side along d
-    static constexpr int TN = DS / WC / 4;                               // columns per thread
-    static constexpr uint32_t a_floats = BS == 32 ? 32 * tile::kStride : 64 * tile::kStride > 32 * (64 + 4) ? 64 * tile::kStride : 32 * (64 + 4);
-    static constexpr uint32_t buf = a_floats + 32 * (DS + 4);
+    static constexpr int WC = BS == 32 ? 4 : 2;                          // warps side by side along d: each is a team with the ones below it
+    static constexpr int TT = 128 / WC, NW = DS / WC, N = NW / 8;        // a team's threads and columns, n-tiles of 8 columns
+    static constexpr uint32_t v_stride = NW + 8, buf = 32 * v_stride;
 };
 template <int BS, int DS, int A_DT, int BC_DT, bool TRANS>
-__global__ void __launch_bounds__(tile::kThreads, 4) spmm_nn_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Pm,
-                                                                  const void *__restrict__ V, void *__restrict__ O, AttnDims p, bool avec,
-                                                                  bool vec)
+__global__ void __launch_bounds__(tile::kThreads, (BS == 64 && DS == 128) || A_DT == SFB_F32 ? 3 : 4)
+spmm_nn_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Pm, const void *__restrict__ V, void *__restrict__ O, AttnDims p, bool avec, bool vec)
 {
     using namespace tile;
     typedef SpmmCfg<BS, DS> Cfg;
-    constexpr int TN = Cfg::TN;
+    constexpr int N = Cfg::N, TT = Cfg::TT, VN = Cols<N>::VN;
+    constexpr int TP = kTerms<A_DT>, TV = kTerms<BC_DT>;
     constexpr uint32_t PARTS = BS / 32;                                  // chunks per block
-    constexpr uint32_t a_stride = TRANS ? BS + 4 : kStride;
-    extern __shared__ __align__(16) float sm[];                          // [2][P chunk | V chunk]
+    extern __shared__ __align__(16) float sm[];                          // [team][3][32 rows of V]
     grid_dependency_wait();
     grid_launch_dependents();
     const uint32_t nslice = (p.d + DS - 1) / DS;
     const uint32_t i = blockIdx.x / nslice, d0 = (blockIdx.x % nslice) * DS;
     const uint32_t b = blockIdx.y, h = blockIdx.z;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane_row(lane), lc = lane_quad(lane);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const uint2 *nn = lut + (size_t)h * p.lut_stride;
     const uint2 head = nn[i];
     const size_t HD = (size_t)p.H * p.d;
     const size_t bh = (size_t)b * p.H + h;
-    const uint32_t r0 = BS == 64 ? 32 * (warp >> 1) : 0, n0 = (BS == 64 ? warp & 1 : warp) * (DS / Cfg::WC);
-    const uint32_t chunks = head.y * PARTS;
+    const uint32_t r0 = BS == 64 ? 32 * (warp >> 1) : 0, team = BS == 64 ? warp & 1 : warp, n0 = d0 + team * Cfg::NW;
+    const uint32_t rank = BS == 64 ? 32 * (warp >> 1) + lane : lane;
+    const uint32_t chunks = head.y * PARTS, left = p.d > n0 ? p.d - n0 : 0;
+    float *bufs = sm + team * 3 * Cfg::buf;
 
-    auto issue = [&](uint32_t c) {
-        const uint2 ent = nn[head.x + c / PARTS];
-        const uint32_t part = c % PARTS;
-        float *buf = sm + (c & 1) * Cfg::buf;
-        const size_t baseP = (bh * p.blocks + ent.x) * BS * BS, baseV = ((size_t)b * p.nb_b + ent.y) * BS * HD + (size_t)h * p.d + d0;
-        if (TRANS) stage<A_DT, 32, BS>(buf, a_stride, Pm, baseP + part * 32 * BS, BS, BS, avec);
-        else stage<A_DT, BS, 32>(buf, a_stride, Pm, baseP + part * 32, BS, 32, avec);
-        stage<BC_DT, 32, DS>(buf + Cfg::a_floats, DS + 4, V, baseV + (size_t)part * 32 * HD, HD, p.d - d0, vec);
+    // the row's entries, 32 at a time, one per lane, the next 32 ahead
+    uint2 ent = lane < head.y ? nn[head.x + lane] : make_uint2(0u, 0u), ent2 = 32 + lane < head.y ? nn[head.x + 32 + lane] : make_uint2(0u, 0u);
+    auto entry = [&](uint32_t c, uint32_t &part) {                       // called for c = 0, 1, 2, ... in turn
+        const uint32_t e = c / PARTS;
+        part = c % PARTS;
+        if (e && e % 32 == 0 && part == 0) {
+            ent = ent2;
+            ent2 = e + 32 + lane < head.y ? nn[head.x + e + 32 + lane] : make_uint2(0u, 0u);
+        }
+        return make_uint2(__shfl_sync(0xffffffffu, ent.x, e % 32), __shfl_sync(0xffffffffu, ent.y, e % 32));
+    };
+    Staged<BC_DT, TT, Cfg::NW> held_v;
+    Raw4<A_DT> held_p[8];                                                // [k16][row 16 m + 8 half + g], TRANS: [k16][element 4 t + i], rows 4 g to 4 g + 3
+    size_t next_p = 0;                                                   // chunk c + 1's place in P
+    auto issue = [&](uint32_t c) {                                       // V of chunk c; its P is asked for one chunk later
+        if (c < chunks) {
+            uint32_t part;
+            const uint2 en = entry(c, part);
+            next_p = (bh * p.blocks + en.x) * BS * BS + (TRANS ? (size_t)part * 32 * BS + r0 : (size_t)r0 * BS + part * 32);
+            if (left) stage_begin(held_v, rank, bufs + (c % 3) * Cfg::buf, Cfg::v_stride, V, ((size_t)b * p.nb_b + en.y) * BS * HD + (size_t)part * 32 * HD + (size_t)h * p.d + n0, HD, left, vec);
+        }
         cp_commit();
     };
-    uint64_t acc[4][TN / 2];
+    auto land = [&](uint32_t c) {                                        // the pieces of chunk c that are converted on the way
+        if (c < chunks && left) stage_end(held_v, rank, bufs + (c % 3) * Cfg::buf, Cfg::v_stride, vec);
+    };
+    auto load_p = [&](size_t at) {
 #pragma unroll
-    for (int m = 0; m < 4; m++)
-#pragma unroll
-        for (int n = 0; n < TN / 2; n++) acc[m][n] = 0;
-    if (chunks) issue(0);
+        for (int x = 0; x < 8; x++)
+            load_raw4<A_DT>(held_p[x], Pm, at + (TRANS ? (size_t)(16 * (x >> 2) + 4 * t + (x & 3)) * BS + 4 * g : (size_t)(8 * (x & 3) + g) * BS + 16 * (x >> 2) + 4 * t), 4, avec);
+    };
+    float acc[2][N][4] = {};
+    if (chunks) {
+        issue(0);
+        land(0);
+        load_p(next_p);
+        issue(1);
+        land(1);
+    }
     for (uint32_t c = 0; c < chunks; c++) {
-        cp_wait_all();
-        __syncthreads();
-        if (c + 1 < chunks) issue(c + 1);
-        const float *buf = sm + (c & 1) * Cfg::buf;
-        const float *v = buf + Cfg::a_floats + n0 + lane_col<TN>(lc);
-        if (TRANS) mma_tn<TN>(acc, buf + r0 + 4 * lr, a_stride, v, DS + 4);
-        else mma_nn<TN>(acc, buf + (r0 + lr) * a_stride, a_stride, v, DS + 4);
+        cp_wait<1>();
+        meet<TT, (int)kThreads>(1 + team);
+        Frag<TP> fp[2][2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            float x[4][4];
+#pragma unroll
+            for (int r = 0; r < 4; r++) widen4<A_DT>(x[r], held_p[4 * k + r]);
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+                if (TRANS) {
+                    const float y0[4] = {x[0][2 * m], x[1][2 * m], x[2][2 * m], x[3][2 * m]}, y1[4] = {x[0][2 * m + 1], x[1][2 * m + 1], x[2][2 * m + 1], x[3][2 * m + 1]};
+                    split_rows<TP>(fp[k][m], y0, y1);
+                } else {
+                    split_rows<TP>(fp[k][m], x[2 * m], x[2 * m + 1]);
+                }
+            }
+        }
+        if (c + 1 < chunks) load_p(next_p);
+        issue(c + 2);
+        if (left) {
+            const float *v = bufs + (c % 3) * Cfg::buf;
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+#pragma unroll
+                for (int q = 0; q < Cols<N>::GROUPS; q++) {
+                    Four<TV> fb[VN];
+                    load_values<VN, TV>(fb, v + 16 * k * Cfg::v_stride + 32 * q, Cfg::v_stride, g, t);
+#pragma unroll
+                    for (int m = 0; m < 2; m++) mma16<VN, TP, TV>(&acc[m][VN * q], fp[k][m], fb);
+                }
+        }
+        land(c + 2);
     }
     // rows without blocks are written as zeros (blocksparse.h:949-962)
-    const size_t baseO = ((size_t)b * p.nb_a + i) * BS * HD + (size_t)h * p.d + d0 + n0;
-    const uint32_t left = p.d > d0 + n0 ? p.d - d0 - n0 : 0;
+    const size_t baseO = ((size_t)b * p.nb_a + i) * BS * HD + (size_t)h * p.d + n0;
+    if ((TP > 1 || TV > 1) && !(zero_if_finite<N>(acc[1], zero_if_finite<N>(acc[0], 0.f)) == 0.f)) {
 #pragma unroll
-    for (int m = 0; m < 4; m++) {
-        const uint32_t r = r0 + (TRANS ? 4 * lr + m : lr + 8 * m);
-        store_cols<BC_DT, TN>(O, baseO + (size_t)r * HD, lc, acc[m], 1.f, left, vec);
+        for (int x = 0; x < 8 * N; x++) {
+            float &o = acc[x / (4 * N)][(x >> 2) % N][x & 3];
+            const uint32_t r = r0 + (TRANS ? 4 * g + 2 * (x / (4 * N)) + ((x >> 1) & 1) : 16 * (x / (4 * N)) + 8 * ((x >> 1) & 1) + g);
+            const uint32_t col = out_col<N>(t, (x >> 2) % N, x & 1);
+            if (!finite(o) && col < left)
+                o = spmm_again<BS, A_DT, BC_DT, TRANS>(nn + head.x, head.y, Pm, V, bh * p.blocks * BS * BS, (size_t)b * p.nb_b * BS * HD + (size_t)h * p.d + n0 + col, HD, r);
+        }
     }
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            const uint32_t r = r0 + (TRANS ? 4 * g + 2 * m + half : 16 * m + 8 * half + g);
+            store_cols<BC_DT, N>(O, baseO + (size_t)r * HD, t, acc[m], half, 1.f, left, vec);
+        }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -693,38 +791,205 @@ __global__ void __launch_bounds__(256) fused_sddmm_softmax_kernel(const uint2 *_
     }
 }
 
-// SDDMM + softmax + SpMM with an online softmax; S and P never leave the SM.  One CTA (four warps) per block-row.
-// A step takes four 32x32 key blocks (a 32x32 score tile per warp) or one 64x64 block (a quarter per warp): Q . K^T over
-// chunks of 32 of d, the softmax in registers (row maxima meet in shared memory), P to shared memory, then O += P . V in
-// chunks of 32 keys, each warp on its share of O's columns (and, for 64 rows, of its rows).  Keys and values flow through
-// the same two buffers as one sequence of chunks.  Score and O rows of a thread are the same, so O is rescaled in place.
-// ST chunk buffers: two let three CTAs share an SM; four keep three chunks on their way, for launches that do not fill the SMs
-// anyway and wait for L2 chunk by chunk.
-template <int BS, int D, int ST = 2> struct FaCfg {
-    static constexpr uint32_t G = BS == 32 ? 4 : 1;                      // key blocks per step
-    static constexpr uint32_t NK = G * BS;                               // keys per step
-    static constexpr uint32_t WC = BS == 32 ? 4 : 2;                     // warps side by side (score columns, O columns)
-    static constexpr int TN = D / (int)WC / 4;
-    static constexpr uint32_t kbuf = NK * tile::kStride, vbuf = 32 * (D + 4), buf = kbuf > vbuf ? kbuf : vbuf;
-    static constexpr uint32_t p_stride = NK + 4, q_stride = D + 4;
-    static constexpr uint32_t floats = BS * q_stride + ST * buf + BS * p_stride + WC * BS;
-    static constexpr int ctas = ST > 2 || (BS == 64 && D == 128) ? 2 : 3;            // what registers and shared memory allow per SM
+// A query row whose output is not finite, made again by one warp with plain FMAs (simt_tile.cuh says why): a key per lane for the
+// scores, a share of the columns per lane for the output.  mask: this row's word of block 0.
+template <int BS, int DT>
+__device__ __noinline__ void attention_row_again(const uint2 *ent, uint32_t cnt, const void *Q, const void *K, const void *V, void *O,
+                                                 const typename MaskWord<BS>::type *mask, size_t qrow, size_t kv, size_t orow, size_t HD, uint32_t d, float scale_log2e)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    float m = -INFINITY, l = 0.f, acc[4] = {};
+    for (uint32_t e = 0; e < cnt; e++)
+        for (uint32_t part = 0; part < BS; part += 32) {
+            const size_t rows = kv + ((size_t)ent[e].y * BS + part) * HD;
+            float s = 0.f;
+            for (uint32_t k = 0; k < d; k++) s = fmaf(Elem<DT>::load(Q, qrow + k), Elem<DT>::load(K, rows + lane * HD + k), s);
+            s = !mask || ((mask[(size_t)ent[e].x * BS] >> (part + lane)) & 1u) ? s * scale_log2e : -INFINITY;
+            const float mn = fmaxf(m, warp_max(s)), alpha = mn > m ? exp2f(m - mn) : 1.f;
+            const float pv = exp2f(s - (mn > -INFINITY ? mn : 0.f));
+            m = mn;
+            l = fmaf(l, alpha, warp_sum(pv));
+#pragma unroll
+            for (int c = 0; c < 4; c++) acc[c] *= alpha;
+            for (uint32_t k = 0; k < 32; k++) {
+                const float pk = __shfl_sync(0xffffffffu, pv, k);
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    if (lane + 32 * c < d) acc[c] = fmaf(pk, Elem<DT>::load(V, rows + k * HD + lane + 32 * c), acc[c]);
+            }
+        }
+    const float inv = l > 0.f ? 1.f / l : l;                             // nothing kept: 0; NaN stays NaN
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+        if (lane + 32 * c < d) Elem<DT>::store(O, orow + lane + 32 * c, acc[c] * inv);
+}
+
+// SDDMM + softmax + SpMM with an online softmax; S and P never leave the SM.  One CTA (eight warps) per block-row.
+//
+// A step takes four 32x32 key blocks or one 64x64 block: Q . K^T, the softmax in registers (row maxima meet in shared
+// memory), P to shared memory as fragments, then O += P . V.  For the scores a warp owns 32 query rows and 16 keys: two n-tiles of
+// eight, of different blocks where blocks are 32 (tiles w and w + 8 of the step's 16, so that a step of one or two blocks is
+// still shared by many warps).  For the output it owns 32 rows, 16 or 32 columns and, where the head is too narrow for all
+// warps, every KG-th chunk of 32 keys; such shares of O are added up at the end.
+//
+// Eight warps and not four: the work of a row (a few key blocks) is a chain of loads, products, maxima and products again, of
+// which each warp then has a shorter piece, and sixteen warps of 128 registers per SM wait for one another's latencies.
+// B 32, H 4, L 1024, d 128, sawtooth, fp32: 305 us on the FMA pipe (four warps, 4 x 8 outputs per thread), 265 now; B 1, H 4, L 512, d 64, fixed (64 CTAs):
+// 14.8 -> 11.4.  At 265 us the tensor pipe is 41 % busy and half of the issue slots are used, a quarter of them by
+// the splits: warps wait for fixed latencies and for the tensor pipe in turn.  Measured beside it: four warps of 250 registers, two CTAs per SM 265 / 12.1;
+// keys and values straight to fragments without the ring 282 / 12.2 with eight warps, 291 with four and three CTAs per SM.
+//
+// A warp stages the keys of its own scores and the values of its own columns (for 64 rows together with the warp that has the
+// other half of the rows) as one sequence of chunks, 32 of d or 32 keys, through a ring of ST buffers.  All warps of a row meet twice
+// per step, for the maxima and for P.
+template <int BS, int D, int DT> struct FaCfg {
+    static constexpr uint32_t RH = BS / 32, GW = 8 / RH;                 // halves of the block-row's 32 rows each, warps of a half
+    static constexpr int TT = 32 * RH;                                   // threads that stage together: the warps with the same keys and columns
+    static constexpr uint32_t G = BS == 32 ? 4 : 1, NK = G * BS;         // key blocks and keys per step
+    static constexpr int N = BS == 64 && D == 128 ? 4 : 2, NW = 8 * N;   // n-tiles of 8 columns per warp, its columns
+    static constexpr uint32_t CG = D / NW, KG = GW / CG;                 // column groups, key groups
+    static constexpr uint32_t v_stride = NW + 8;
+    static constexpr uint32_t kbuf = 16 * tile::kStride, vbuf = 32 * v_stride, buf = kbuf > vbuf ? kbuf : vbuf;
+    static constexpr uint32_t T = tile::kTerms<DT>;
+    static constexpr uint32_t qfrags = BS / 16 * (D / 16) * T * 32, pfrags = BS / 16 * (NK / 16) * 3 * 32;      // uint4
+    static constexpr int ST = D == 128 ? 2 : 3;
+    static constexpr size_t bytes = 16 * (qfrags + pfrags) + 4 * (GW * ST * buf + GW * BS);
+    static_assert(2 * (bytes + 1024) <= 228 * 1024, "two CTAs per SM");
 };
-template <int BS, int D, int DT, int ST>
-__global__ void __launch_bounds__(tile::kThreads, (FaCfg<BS, D, ST>::ctas))
+constexpr uint32_t kFaThreads = 256;
+
+// The staged row of key n of tile j (two tiles of eight): lanes read neighbouring keys four rows apart (simt_tile.cuh: tile_row)
+__device__ __forceinline__ constexpr uint32_t key_place(uint32_t j, uint32_t n) { return 8 * j + (n >> 1) + 4 * (n & 1); }
+// Key n of a tile in its 32 keys, for the tile's place sub in them: keys 16 (sub >> 1) to + 15 are one k16 of the product with the values, of
+// which a lane's four elements are neighbours
+__device__ __forceinline__ constexpr uint32_t tile_key(uint32_t sub, uint32_t n) { return 16 * (sub >> 1) + 2 * (sub & 1) + 4 * (n >> 1) + (n & 1); }
+
+// One chunk of scores: 32 rows (fragments at q, pitch from one 16 rows to the next) x tiles staged at `keys`
+template <int T>
+__device__ __forceinline__ void score_chunk(float (&s)[2][2][4], const uint4 *q, uint32_t pitch, const float *keys, uint32_t tiles, uint32_t lane)
+{
+    using namespace tile;
+    const float *p = keys + key_place(0, lane >> 2) * kStride + 4 * (lane & 3);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        Frag<T> a[2];
+        load_frag<T>(a[0], q + k * T * 32, lane);
+        load_frag<T>(a[1], q + pitch + k * T * 32, lane);
+        Four<T> b[2];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const float4 v = *(const float4 *)(p + key_place(j, 0) * kStride + 16 * k);
+            const float x[4] = {v.x, v.y, v.z, v.w};
+            split4<T>(b[j], x);
+        }
+        if (tiles == 2) mma16<2, 2, 2, T, T>(s[0], a, b);
+        else mma16<2, 1, 2, T, T>(s[0], a, b);
+    }
+}
+// Softmax of a step: the maxima of this warp's scores meet those of the other warps, the scores become probabilities.  red: [row][warp]
+template <int GW, int ROWT, int N>
+__device__ __forceinline__ void softmax_step(float (&s)[2][2][4], float (&mx)[4], float (&sum)[4], float (&acc)[2][N][4], float *red, uint32_t w, uint32_t g, uint32_t t, uint32_t bar)
+{
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        float bm = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 2; j++) bm = fmaxf(bm, fmaxf(s[q >> 1][j][2 * (q & 1)], s[q >> 1][j][2 * (q & 1) + 1]));
+        bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
+        bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 2));
+        if (t == 0) red[(g + 8 * q) * GW + w] = bm;
+    }
+    tile::meet<ROWT, kFaThreads>(bar);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        float mn = mx[q];
+#pragma unroll
+        for (int k = 0; k < GW; k += 4) {
+            const float4 r = *(const float4 *)(red + (g + 8 * q) * GW + k);
+            mn = fmaxf(fmaxf(fmaxf(mn, r.x), fmaxf(r.y, r.z)), r.w);
+        }
+        const float alpha = mn > mx[q] ? ex2_fast(mx[q] - mn) : 1.f;
+        mx[q] = mn;
+        const float off = mn > -INFINITY ? mn : 0.f;                     // nothing kept so far: exp2(-inf) = 0, and NaN stays NaN
+        float ps = 0.f;
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                float &v = s[q >> 1][j][2 * (q & 1) + k];
+                v = ex2_fast(v - off);
+                ps += v;
+            }
+        sum[q] = fmaf(sum[q], alpha, ps);                                // this thread's columns only; the shares meet at the end
+#pragma unroll
+        for (int n = 0; n < N; n++) {
+            acc[q >> 1][n][2 * (q & 1)] *= alpha;
+            acc[q >> 1][n][2 * (q & 1) + 1] *= alpha;
+        }
+    }
+}
+// P of 32x32 blocks: tile j is half (sub & 1) of the k16 at `at` + j * step; pitch: from one 16 rows to the next
+__device__ __forceinline__ void put_halves(uint4 *at, uint32_t step, uint32_t pitch, const float (&s)[2][2][4], uint32_t half, uint32_t lane)
+{
+    using namespace tile;
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            uint32_t lo[3], hi[3];
+            split2<3>(lo, s[m][j][0], s[m][j][1]);
+            split2<3>(hi, s[m][j][2], s[m][j][3]);
+#pragma unroll
+            for (int i = 0; i < 3; i++) ((uint2 *)(at + m * pitch + j * step + i * 32 + lane))[half] = make_uint2(lo[i], hi[i]);
+        }
+}
+// the same where a warp's two tiles are one k16
+__device__ __forceinline__ void put_whole(uint4 *at, uint32_t pitch, const float (&s)[2][2][4], uint32_t lane)
+{
+    using namespace tile;
+#pragma unroll
+    for (int m = 0; m < 2; m++) {
+        const float x0[4] = {s[m][0][0], s[m][0][1], s[m][1][0], s[m][1][1]}, x1[4] = {s[m][0][2], s[m][0][3], s[m][1][2], s[m][1][3]};
+        Frag<3> f;
+        split_rows<3>(f, x0, x1);
+        store_frag<3>(at + m * pitch, lane, f);
+    }
+}
+// the key groups' shares of O meet in the first group: at: room for (KG - 1) * groups shares
+template <int N, int KG>
+__device__ __forceinline__ void add_shares(float (&acc)[2][N][4], float *at, uint32_t kg, uint32_t group, uint32_t groups, uint32_t lane)
+{
+    if (KG == 1) return;
+    if (kg) {
+#pragma unroll
+        for (int x = 0; x < 8 * N; x++) at[(((kg - 1) * groups + group) * 8 * N + x) * 32 + lane] = acc[x / (4 * N)][(x >> 2) % N][x & 3];
+    }
+    __syncthreads();
+    if (kg == 0) {
+        for (int k = 0; k < KG - 1; k++)
+#pragma unroll
+            for (int x = 0; x < 8 * N; x++) acc[x / (4 * N)][(x >> 2) % N][x & 3] += at[((k * groups + group) * 8 * N + x) * 32 + lane];
+    }
+}
+
+template <int BS, int D, int DT>
+__global__ void __launch_bounds__(kFaThreads, 2)
 fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q, const void *__restrict__ K, const void *__restrict__ V,
                        void *__restrict__ O, const typename MaskWord<BS>::type *__restrict__ mask, AttnDims p, float scale_log2e, bool vec)
 {
     using namespace tile;
     typedef typename MaskWord<BS>::type W;
-    typedef FaCfg<BS, D, ST> Cfg;
-    constexpr int TN = Cfg::TN;
-    constexpr uint32_t G = Cfg::G, WC = Cfg::WC, QS = Cfg::q_stride, PS = Cfg::p_stride;
+    typedef FaCfg<BS, D, DT> Cfg;
+    constexpr int N = Cfg::N, T = Cfg::T, TT = Cfg::TT, ST = Cfg::ST, ROWT = 32 * Cfg::GW;      // ROWT: threads that share query rows
+    constexpr uint32_t G = Cfg::G, GW = Cfg::GW, KG = Cfg::KG, KQ = D / 16, KP = Cfg::NK / 16;
     extern __shared__ __align__(16) float sm[];
-    float *Qs = sm, *bufs = Qs + BS * QS, *Ps = bufs + ST * Cfg::buf, *red = Ps + BS * PS;
+    uint4 *Qf = (uint4 *)sm, *Pf = Qf + Cfg::qfrags;
+    float *bufs = (float *)(Pf + Cfg::pfrags), *red = bufs + GW * ST * Cfg::buf;
     grid_dependency_wait();
     grid_launch_dependents();
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane_row(lane), lc = lane_quad(lane);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const uint32_t rh = warp / GW, w = warp % GW, r0 = 32 * rh, rank = 32 * rh + lane;
+    const uint32_t cg = w % Cfg::CG, kg = w / Cfg::CG, n0 = cg * Cfg::NW;
     // rows are dealt from both ends: the long rows of the layouts at hand sit there and start first
     const uint32_t i = (blockIdx.x & 1u) ? p.nb_a - 1u - (blockIdx.x >> 1) : blockIdx.x >> 1, b = blockIdx.y, h = blockIdx.z;
     const uint2 *nn = lut + (size_t)h * p.lut_stride;
@@ -732,297 +997,388 @@ fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q
     const size_t HD = p.in_pitch ? (size_t)p.in_pitch : (size_t)p.H * p.d;      // row pitch of q, k, v
     const size_t HDo = p.out_pitch ? (size_t)p.out_pitch : (size_t)p.H * p.d;   // row pitch of o
     const W *mh = mask ? mask + (size_t)h * p.mask_stride : nullptr;
-    const uint32_t r0 = BS == 64 ? 32 * (warp >> 1) : 0, wc = BS == 64 ? warp & 1 : warp;   // this warp's rows and column share
-    const uint32_t n0 = wc * (D / WC);
     const uint32_t kchunks = (p.d + kChunk - 1) / kChunk;
-    const uint32_t cnt = head.y;
+    const uint32_t cnt = head.y, left = p.d > n0 ? p.d - n0 : 0;
+    const size_t kv = (size_t)b * p.nb_b * BS * HD + (size_t)h * p.d;
+    bufs += w * ST * Cfg::buf;
+    red += r0 * GW;
+    // this warp's tiles: block and place in its 32 keys of tile j (the step's 32-key parts where blocks are 64)
+    const uint32_t blk0 = BS == 32 ? w >> 2 : 0, sub0 = BS == 32 ? w & 3 : 2 * (w & 1), part = BS == 32 ? 0 : 32 * (w >> 1);
+    auto tiles_of = [&](uint32_t nblk) { return BS == 64 ? 2u : (blk0 < nblk ? 1u : 0u) + (blk0 + 2 < nblk ? 1u : 0u); };
 
-    // the sequence of chunks: per step the key chunks, then the value chunks
-    uint32_t is_e = 0, is_k = 0, is_n = 0;                               // next chunk to issue: step's first entry, index in the step, overall
-    size_t koff[G];
+    // the row's entries, 32 at a time, one per lane, the next 32 ahead
+    uint32_t ent = lane < cnt ? nn[head.x + lane].y : 0u, ent2 = 32 + lane < cnt ? nn[head.x + 32 + lane].y : 0u;
+    // the team's sequence of chunks: per step the key chunks of its tiles (if the step has any for it), then its value chunks
+    uint32_t is_e = 0, is_k = 0;                                         // next chunk to issue: step's first entry, index in the step
+    constexpr uint32_t NPART = G * (BS / 32);                            // 32-key parts of a step
+    constexpr int KE = DT == SFB_F32 ? 4 : 8, KPR = (int)kChunk / KE, KSTEP = TT / KPR, KN = 16 / KSTEP;      // 16-byte pieces of 16 keys x 32 elements
+    uint4 held_k[DT == SFB_F32 ? 1 : KN];
+    Staged<DT, TT, Cfg::NW> held_v;
+    uint32_t held = 0;                                                   // 16-bit pieces wait in registers: 1 keys, 2 values
+    float *held_at = nullptr;
+    const uint32_t kr = rank / KPR, kc = rank % KPR * KE;
+    uint32_t is_tiles = tiles_of(min(G, cnt)), is_mine = is_tiles ? kchunks : 0, is_all = is_mine + (min(cnt * (BS / 32), NPART) + KG - 1 - kg) / KG;
+    uint32_t slot = 0;                                                   // ring buffer of the next chunk
+    const typename Elem<DT>::type *krow[2];                              // this thread's piece of tile j's keys, chunk is_k
+    auto key_rows = [&]() {
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const uint32_t row = __shfl_sync(0xffffffffu, ent, (is_e + (BS == 32 ? blk0 + 2 * j : 0)) % 32) * BS + part + tile_key(BS == 32 ? sub0 : sub0 + j, 0);
+            krow[j] = (const typename Elem<DT>::type *)K + kv + (size_t)row * HD + (vec ? (size_t)tile_key(0, kr & 7) * HD + kc : 0);
+        }
+    };
     auto issue = [&]() {
-        if (is_e >= cnt) {                                               // nothing left: an empty group keeps the count
-            cp_commit();
-            return;
-        }
-        const uint32_t nblk = min(G, cnt - is_e);
-        if (is_k == 0) {
+        held = 0;
+        if (is_e < cnt) {
+            if (is_all) {
+                float *buf = bufs + slot * Cfg::buf;
+                held_at = buf;
+                if (is_k < is_mine) {
+                    held = 1;
+                    const uint32_t k0 = is_k * kChunk;
+                    if (is_k == 0) key_rows();
+                    if (vec) {
+                        // rows kr, kr + KSTEP, ... of 16: a tile has eight, KSTEP is 4 or 8 or 16 rows on, that is 8 rows of K or the other tile
+                        const bool in = k0 + kc < p.d;
 #pragma unroll
-            for (uint32_t g = 0; g < G; g++)
-                koff[g] = ((size_t)b * p.nb_b + nn[head.x + is_e + (g < nblk ? g : 0)].y) * BS * HD + (size_t)h * p.d;
+                        for (int x = 0; x < KN; x++) {
+                            const int j = KSTEP >= 8 ? (KSTEP == 8 ? x : -1) : x >> 1;      // -1: by this thread's row
+                            const uint32_t jj = j < 0 ? kr >> 3 : (uint32_t)j;
+                            const typename Elem<DT>::type *src = (jj ? krow[1] : krow[0]) + (KSTEP == 4 && (x & 1) ? 8 * HD : 0);
+                            const uint32_t r = kr + x * KSTEP;
+                            if constexpr (DT == SFB_F32) {
+                                if (jj < is_tiles) cp_async16(buf + key_place(r >> 3, r & 7) * kStride + kc, in ? src : (const float *)K, in ? 16u : 0u);
+                            } else {
+                                held_k[x] = in && jj < is_tiles ? __ldg((const uint4 *)src) : make_uint4(0u, 0u, 0u, 0u);
+                            }
+                        }
+                    } else {
+                        for (uint32_t x = rank; x < 16 * kChunk; x += TT) {
+                            const uint32_t r = x / kChunk, k = x % kChunk, j = r >> 3;
+                            if (j < is_tiles) buf[key_place(j, r & 7) * kStride + k] = k0 + k < p.d ? Elem<DT>::load(j ? krow[1] : krow[0], (size_t)tile_key(0, r & 7) * HD + k) : 0.f;
+                        }
+                    }
+                    krow[0] += kChunk;
+                    krow[1] += kChunk;
+                } else {
+                    held = 2;
+                    const uint32_t vc = kg + (is_k - is_mine) * KG;
+                    const uint32_t row = __shfl_sync(0xffffffffu, ent, (is_e + (BS == 32 ? vc : 0)) % 32) * BS + (BS == 32 ? 0 : 32 * vc);
+                    if (left) stage_begin(held_v, rank, buf, Cfg::v_stride, V, kv + (size_t)row * HD + n0, HD, left, vec);
+                }
+                slot = slot + 1 == ST ? 0 : slot + 1;
+                is_k++;
+            }
+            if (is_k == is_all) {
+                is_k = 0;
+                is_e += G;
+                if (is_e % 32 == 0) {
+                    ent = ent2;
+                    ent2 = is_e + 32 + lane < cnt ? nn[head.x + is_e + 32 + lane].y : 0u;
+                }
+                if (is_e + G > cnt && is_e < cnt) {                      // the last step may have fewer blocks
+                    is_tiles = tiles_of(cnt - is_e);
+                    is_mine = is_tiles ? kchunks : 0;
+                    is_all = is_mine + ((cnt - is_e) * (BS / 32) + KG - 1 - kg) / KG;
+                }
+            }
         }
-        float *buf = bufs + (is_n % ST) * Cfg::buf;
-        if (is_k < kchunks) {
-            const uint32_t k0 = is_k * kChunk;
+        cp_commit();                                                     // nothing left: an empty group keeps the count
+    };
+    auto land = [&]() {
+        if constexpr (DT != SFB_F32) {
+            if (!vec) return;
+            if (held == 1) {
 #pragma unroll
-            for (uint32_t g = 0; g < G; g++)
-                if (g < nblk) stage<DT, BS, (int)kChunk>(buf + g * BS * kStride, kStride, K, koff[g] + k0, HD, p.d - k0, vec);
-        } else {
-            const uint32_t vc = is_k - kchunks;
-            const size_t base = G > 1 ? (vc == 0 ? koff[0] : vc == 1 ? koff[1 % G] : vc == 2 ? koff[2 % G] : koff[3 % G]) : koff[0] + (size_t)vc * 32 * HD;
-            stage<DT, 32, D>(buf, D + 4, V, base, HD, p.d, vec);
-        }
-        cp_commit();
-        is_n++;
-        if (++is_k == kchunks + nblk * (BS / 32)) {
-            is_k = 0;
-            is_e += G;
+                for (int x = 0; x < KN; x++) {
+                    const uint32_t r = kr + x * KSTEP;
+                    widen8_to<DT>(held_at + key_place(r >> 3, r & 7) * kStride + kc, held_k[x]);
+                }
+            } else if (held == 2 && left) {
+                stage_end(held_v, rank, held_at, Cfg::v_stride, vec);
+            }
         }
     };
 
     if (cnt) {
-        stage<DT, BS, D>(Qs, QS, Q, ((size_t)b * p.nb_a + i) * BS * HD + (size_t)h * p.d, HD, p.d, vec);
 #pragma unroll
-        for (int i = 0; i < ST - 1; i++) issue();
+        for (int k = 0; k < ST - 1; k++) {
+            issue();
+            land();
+        }
+        const size_t q0 = ((size_t)b * p.nb_a + i) * BS * HD + (size_t)h * p.d;
+#pragma unroll 2
+        for (uint32_t f = warp; f < BS / 16 * KQ; f += 8) {              // fragment f: rows 16 (f / KQ), elements 16 (f % KQ)
+            const uint32_t k = 16 * (f % KQ) + 4 * t, n = k < p.d ? p.d - k : 0u;
+            Raw4<DT> a0, a1;
+            load_raw4<DT>(a0, Q, q0 + (size_t)(16 * (f / KQ) + g) * HD + k, n, vec);
+            load_raw4<DT>(a1, Q, q0 + (size_t)(16 * (f / KQ) + 8 + g) * HD + k, n, vec);
+            float x0[4], x1[4];
+            widen4<DT>(x0, a0);
+            widen4<DT>(x1, a1);
+            Frag<T> fr;
+            split_rows<T>(fr, x0, x1);
+            store_frag<T>(Qf + f * T * 32, lane, fr);
+        }
     }
-    float mx[4], sum[4];
-    uint64_t acc[4][TN / 2];
+    __syncthreads();
+    const uint4 *Qw = Qf + rh * 2 * KQ * T * 32;                         // this warp's rows
+    uint4 *Pw = Pf + rh * 2 * KP * 3 * 32;
+    float mx[4], sum[4];                                                 // of rows r0 + g + 8 q
+    float acc[2][N][4] = {};
 #pragma unroll
-    for (int m = 0; m < 4; m++) {
-        mx[m] = -INFINITY;
-        sum[m] = 0.f;
-#pragma unroll
-        for (int n = 0; n < TN / 2; n++) acc[m][n] = 0;
+    for (int q = 0; q < 4; q++) {
+        mx[q] = -INFINITY;
+        sum[q] = 0.f;
     }
-    uint32_t c = 0;
+    uint32_t at = 0;                                                     // ring buffer of the chunk at hand
+    auto next = [&]() {
+        cp_wait<ST - 2>();
+        meet<TT, kFaThreads>(1 + w);
+        issue();
+        const float *buf = bufs + at * Cfg::buf;
+        at = at + 1 == ST ? 0 : at + 1;
+        return buf;
+    };
     for (uint32_t e = 0; e < cnt; e += G) {
-        const uint32_t nblk = min(G, cnt - e);
-        const bool live = G == 1 || warp < nblk;
-        uint64_t s2[4][8];
-#pragma unroll
-        for (int m = 0; m < 4; m++)
-#pragma unroll
-            for (int n = 0; n < 8; n++) s2[m][n] = 0;
-        for (uint32_t kc = 0; kc < kchunks; kc++, c++) {
-            cp_wait<ST - 2>();
-            __syncthreads();
-            issue();
-            const float *buf = bufs + (c % ST) * Cfg::buf;
-            if (live) mma_nt(s2, Qs + (r0 + lr) * QS + kc * kChunk, QS, buf + (32 * wc + lc) * kStride, kStride);
-        }
-        const uint32_t blk = nn[head.x + e + (G > 1 && live ? warp : 0)].x;
-        float s[4][8], bm[4];
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-            const W w = live ? (mh ? __ldg(mh + (size_t)blk * BS + r0 + lr + 8 * m) : ~(W)0) : (W)0;
-            bm[m] = -INFINITY;
-#pragma unroll
-            for (int n = 0; n < 8; n++) {
-                const uint32_t col = (BS == 64 ? 32 * wc : 0) + lc + 4 * n;
-                s[m][n] = ((w >> col) & 1) ? half_sum(s2[m][n]) * scale_log2e : -INFINITY;
-                bm[m] = fmaxf(bm[m], s[m][n]);
+        const uint32_t nblk = min(G, cnt - e), tiles = tiles_of(nblk);
+        float s[2][2][4] = {};
+        if (tiles)
+            for (uint32_t kk = 0; kk < kchunks; kk++) {
+                const float *keys = next();
+                score_chunk<T>(s, Qw + 2 * kk * T * 32, KQ * T * 32, keys, tiles, lane);
+                land();
             }
-            bm[m] = fmaxf(bm[m], __shfl_xor_sync(0xffffffffu, bm[m], 1));
-            bm[m] = fmaxf(bm[m], __shfl_xor_sync(0xffffffffu, bm[m], 4));
-            if (lc == 0) red[wc * BS + r0 + lr + 8 * m] = bm[m];
-        }
-        __syncthreads();
+        if (!mh) {
 #pragma unroll
-        for (int m = 0; m < 4; m++) {
-            const uint32_t r = r0 + lr + 8 * m;
-            float mn = mx[m];
-#pragma unroll
-            for (uint32_t k = 0; k < WC; k++) mn = fmaxf(mn, red[k * BS + r]);
-            const float alpha = mn > mx[m] ? exp2f(mx[m] - mn) : 1.f;
-            mx[m] = mn;
-            float ps = 0.f;
-#pragma unroll
-            for (int n = 0; n < 8; n++) {
-                const float pv = mn > -INFINITY ? exp2f(s[m][n] - mn) : 0.f;
-                Ps[r * PS + 32 * wc + lc + 4 * n] = pv;
-                ps += pv;
+            for (int x = 0; x < 16; x++) {
+                float &v = s[x >> 3][(x >> 2) & 1][x & 3];
+                v = (uint32_t)((x >> 2) & 1) < tiles ? v * scale_log2e : -INFINITY;
             }
-            sum[m] = fmaf(sum[m], alpha, ps);                            // this thread's columns only; the shares meet at the end
-            const uint64_t a2 = pair(alpha, alpha);
+        } else
 #pragma unroll
-            for (int n = 0; n < TN / 2; n++) acc[m][n] = fma2(acc[m][n], a2, 0ull);
+        for (int j = 0; j < 2; j++) {
+            const bool live = (uint32_t)j < tiles;
+            const W *mw = live ? mh + (size_t)nn[head.x + e + (BS == 32 ? blk0 + 2 * j : 0)].x * BS + r0 + g : nullptr;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const W word = live ? __ldg(mw + 8 * q) : (W)0;
+                const uint32_t bits = (uint32_t)(word >> (part + tile_key(BS == 32 ? sub0 : sub0 + j, 2 * t)));
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    float &v = s[q >> 1][j][2 * (q & 1) + k];
+                    v = (bits >> k) & 1u ? v * scale_log2e : -INFINITY;
+                }
+            }
         }
-        const uint32_t vchunks = nblk * (BS / 32);
-        for (uint32_t vc = 0; vc < vchunks; vc++, c++) {
-            cp_wait<ST - 2>();
-            __syncthreads();
-            issue();
-            const float *buf = bufs + (c % ST) * Cfg::buf;
-            mma_nn<TN>(acc, Ps + (r0 + lr) * PS + vc * 32, PS, buf + n0 + lane_col<TN>(lc), D + 4);
+        softmax_step<GW, ROWT, N>(s, mx, sum, acc, red, w, g, t, 1 + GW + rh);
+        if (BS == 32) put_halves(Pw + (2 * blk0 + (sub0 >> 1)) * 3 * 32, 4 * 3 * 32, KP * 3 * 32, s, sub0 & 1, lane);
+        else put_whole(Pw + w * 3 * 32, KP * 3 * 32, s, lane);
+        meet<ROWT, kFaThreads>(1 + GW + rh);
+        for (uint32_t vc = kg; vc < nblk * (BS / 32); vc += KG) {
+            const float *values = next();
+            if (left) mma_values<N, 3, T>(acc, Pw + 2 * vc * 3 * 32, KP * 3 * 32, values, Cfg::v_stride, lane);
+            land();
         }
     }
     __syncthreads();
+    add_shares<N, KG>(acc, (float *)Pf, kg, rh * Cfg::CG + cg, Cfg::RH * Cfg::CG, lane);
 #pragma unroll
-    for (int m = 0; m < 4; m++) {
-        sum[m] += __shfl_xor_sync(0xffffffffu, sum[m], 1);
-        sum[m] += __shfl_xor_sync(0xffffffffu, sum[m], 4);
-        if (lc == 0) red[wc * BS + r0 + lr + 8 * m] = sum[m];
+    for (int q = 0; q < 4; q++) {
+        sum[q] += __shfl_xor_sync(0xffffffffu, sum[q], 1);
+        sum[q] += __shfl_xor_sync(0xffffffffu, sum[q], 2);
+        if (t == 0) red[(g + 8 * q) * GW + w] = sum[q];
     }
     __syncthreads();
-    const size_t baseO = (((size_t)b * p.nb_a + i) * BS) * HDo + (size_t)h * p.d + n0;
-    const uint32_t left = p.d > n0 ? p.d - n0 : 0;
+    const size_t baseO = (((size_t)b * p.nb_a + i) * BS) * HDo + (size_t)h * p.d;
+    uint32_t odd = 0;                                                    // this thread's rows with an output that is not finite
+    if (kg == 0) {
 #pragma unroll
-    for (int m = 0; m < 4; m++) {
-        const uint32_t r = r0 + lr + 8 * m;
-        float l = 0.f;
+        for (int q = 0; q < 4; q++) {
+            const uint32_t r = r0 + g + 8 * q;
+            float l = 0.f;
 #pragma unroll
-        for (uint32_t k = 0; k < WC; k++) l += red[k * BS + r];
-        store_cols<DT, TN>(O, baseO + (size_t)r * HDo, lc, acc[m], l > 0.f ? 1.f / l : 0.f, left, vec);
+            for (uint32_t k = 0; k < GW; k++) l += red[(g + 8 * q) * GW + k];
+            store_cols<DT, N>(O, baseO + (size_t)r * HDo + n0, t, acc[q >> 1], q & 1, l > 0.f ? 1.f / l : 0.f, left, vec);
+            float zero = l * 0.f;
+#pragma unroll
+            for (int n = 0; n < N; n++) zero = fmaf(acc[q >> 1][n][2 * (q & 1)], 0.f, fmaf(acc[q >> 1][n][2 * (q & 1) + 1], 0.f, zero));
+            if (!(zero == 0.f)) odd |= 1u << q;
+        }
     }
+    if (!__syncthreads_or(odd != 0)) return;
+    // such rows are made again by plain FMAs, once every warp has written its columns of them
+    uint32_t *again = (uint32_t *)Pf;
+    for (uint32_t r = threadIdx.x; r < BS; r += kFaThreads) again[r] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        if ((odd >> q) & 1u) again[r0 + g + 8 * q] = 1;
+    __syncthreads();
+    for (uint32_t r = warp; r < BS; r += kFaThreads / 32)
+        if (again[r])
+            attention_row_again<BS, DT>(nn + head.x, cnt, Q, K, V, O, mh ? mh + r : nullptr, (((size_t)b * p.nb_a + i) * BS + r) * HD + (size_t)h * p.d,
+                                        (size_t)b * p.nb_b * BS * HD + (size_t)h * p.d, baseO + (size_t)r * HDo, HD, p.d, scale_log2e);
 }
 
 // ------------------------------------------------------------------------------------------------
 // Element-sparse attention of one tile of 32 query rows on fp32 operands (csr.cu makes the tile's list of columns and
 // row masks): the kernel above on keys gathered by column, 128 of them per step, a 32x32 score tile per warp.
-template <int ROWS, int COLS>
-__device__ __forceinline__ void stage_gather(float *dst, uint32_t stride, const float *src, const CsrTileArgs &a, uint32_t base, uint32_t top,
-                                             uint32_t distinct, uint32_t first, uint32_t n, size_t pitch)
+// 32 gathered rows x COLS elements by one warp: lane r has the column of row r, or -1 (zeros)
+template <int COLS>
+__device__ __forceinline__ void stage_gather(float *dst, uint32_t stride, const float *src, int32_t col, uint32_t lane, size_t pitch)
 {
     using namespace tile;
-    constexpr int P = COLS / 4, STEP = (int)kThreads / P;
-    const uint32_t r0 = threadIdx.x / P, c = (threadIdx.x % P) * 4;
+    constexpr int P = COLS / 4, STEP = 32 / P;
+    const uint32_t r0 = lane / P, c = (lane % P) * 4;
 #pragma unroll
-    for (int i = 0; i < ROWS / STEP; i++) {
-        const uint32_t r = r0 + i * STEP;
-        const bool in = first + r < n;                                   // rows behind the list arrive as zeros
-        const uint32_t col = in ? csr_entry(a.entries, base, top, distinct, first + r).x : 0u;
-        cp_async16(dst + r * stride + c, src + (size_t)col * pitch + c, in ? 16u : 0u);
+    for (int i = 0; i < 32 / STEP; i++) {
+        const int32_t j = __shfl_sync(0xffffffffu, col, r0 + i * STEP);
+        cp_async16(dst + (tile_row(r0) + tile_row(i * STEP)) * stride + c, src + (size_t)max(j, 0) * pitch + c, j < 0 ? 0u : 16u);
     }
 }
 template <int D>
-__global__ void __launch_bounds__(tile::kThreads, 3) csr_tile_f32_kernel(const CsrTileArgs a)
+__global__ void __launch_bounds__(kFaThreads, 2) csr_tile_f32_kernel(const CsrTileArgs a)
 {
     using namespace tile;
-    typedef FaCfg<32, D> Cfg;
-    constexpr int TN = Cfg::TN;
-    constexpr uint32_t NK = Cfg::NK, QS = Cfg::q_stride, PS = Cfg::p_stride, kchunks = D / kChunk;
+    typedef FaCfg<32, D, SFB_F32> Cfg;
+    constexpr int N = Cfg::N, ST = Cfg::ST;
+    constexpr uint32_t NK = Cfg::NK, GW = Cfg::GW, KG = Cfg::KG, KQ = D / 16, KP = NK / 16, kchunks = D / kChunk;
     extern __shared__ __align__(16) float sm[];
-    float *Qs = sm, *bufs = Qs + 32 * QS, *Ps = bufs + 2 * Cfg::buf, *red = Ps + 32 * PS;
+    uint4 *Qf = (uint4 *)sm, *Pf = Qf + Cfg::qfrags;
+    float *bufs = (float *)(Pf + Cfg::pfrags), *red = bufs + GW * ST * Cfg::buf;
     grid_dependency_wait();
     grid_launch_dependents();
     csr_write_bad(a);
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane_row(lane), lc = lane_quad(lane);
+    const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const uint32_t cg = w % Cfg::CG, kg = w / Cfg::CG, n0 = cg * Cfg::NW;
     const uint32_t tl = a.tiles - 1u - blockIdx.x, h = blockIdx.y, b = blockIdx.z;
     const uint32_t *cnt = a.counts + kCsrCounts * tl;
     const uint32_t distinct = cnt[0], base = cnt[2], top = cnt[3], n = distinct + cnt[1];
     const size_t HD = (size_t)a.H * D, head = (size_t)b * a.L * HD + (size_t)h * D;
     const float *K = (const float *)a.K + head, *V = (const float *)a.V + head;
-    const uint32_t n0 = warp * (D / 4);
+    bufs += w * ST * Cfg::buf;
+    const uint32_t sub = w & 3;
+    auto tile_at = [&](uint32_t j, uint32_t x) { return 32 * ((w >> 2) + 2 * j) + tile_key(sub, x); };       // key x of this warp's tile j in the step
+    auto tiles_of = [&](uint32_t left) { return (tile_at(0, 0) < left ? 1u : 0u) + (tile_at(1, 0) < left ? 1u : 0u); };
 
+    // This warp's sequence of chunks: per step the key chunks of its two tiles (if the step has any for it), then its value chunks.
+    // Lane r has the column of staged key r (of 16) and of value row r; the next ones are asked for when the last chunk of these is issued.
     uint32_t is_e = 0, is_k = 0, is_n = 0;                               // next chunk to issue: step's first key, index in the step, overall
+    auto column = [&](uint32_t at) { return at < n ? (int32_t)csr_entry(a.entries, base, top, distinct, at).x : -1; };
+    auto key_column = [&](uint32_t e) { return lane < 16 ? column(e + tile_at(lane >> 3, lane & 7)) : -1; };
+    int32_t kcol = key_column(0), vcol = column(32 * kg + lane);
     auto issue = [&]() {
-        float *buf = bufs + (is_n & 1) * Cfg::buf;
-        if (is_k < kchunks) stage_gather<(int)NK, (int)kChunk>(buf, kStride, K + is_k * kChunk, a, base, top, distinct, is_e, n, HD);
-        else stage_gather<32, D>(buf, D + 4, V, a, base, top, distinct, is_e + (is_k - kchunks) * 32, n, HD);
-        cp_commit();
-        is_n++;
-        if (++is_k == kchunks + (min(NK, n - is_e) + 31) / 32) {
-            is_k = 0;
-            is_e += NK;
+        if (is_e < n) {
+            const uint32_t left = min(NK, n - is_e), mine = tiles_of(left) ? kchunks : 0, parts = (left + 31) / 32, vmine = (parts + KG - 1 - kg) / KG;
+            if (mine + vmine) {
+                float *buf = bufs + (is_n % ST) * Cfg::buf;
+                if (is_k < mine) {
+#pragma unroll
+                    for (int x = 0; x < 4; x++) {
+                        const uint32_t r = lane / 8 + 4 * x, kc = lane % 8 * 4;
+                        const int32_t col = __shfl_sync(0xffffffffu, kcol, r);
+                        cp_async16(buf + key_place(r >> 3, r & 7) * kStride + kc, K + (size_t)max(col, 0) * HD + is_k * kChunk + kc, col < 0 ? 0u : 16u);
+                    }
+                    if (is_k + 1 == mine) kcol = key_column(is_e + NK);
+                } else {
+                    stage_gather<Cfg::NW>(buf, Cfg::v_stride, V + n0, vcol, lane, HD);
+                    vcol = column((is_k + 1 < mine + vmine ? is_e + 32 * (kg + (is_k + 1 - mine) * KG) : is_e + NK + 32 * kg) + lane);
+                }
+                is_n++;
+                is_k++;
+            }
+            if (is_k == mine + vmine) {
+                is_k = 0;
+                is_e += NK;
+            }
         }
+        cp_commit();                                                     // nothing left: an empty group keeps the count
     };
     if (n) {
+#pragma unroll
+        for (int k = 0; k < ST - 1; k++) issue();
         const uint32_t rows = min(32u, a.L - tl * 32);                   // rows behind the sequence: the last one again, not written
-        constexpr int P = D / 4, STEP = (int)kThreads / P;
+#pragma unroll 2
+        for (uint32_t f = w; f < 2 * KQ; f += 8) {
+            float x[2][4];
 #pragma unroll
-        for (int i = 0; i < 32 / STEP; i++) {
-            const uint32_t r = threadIdx.x / P + i * STEP, c = (threadIdx.x % P) * 4;
-            cp_async16(Qs + r * QS + c, (const float *)a.Q + head + (size_t)(tl * 32 + min(r, rows - 1)) * HD + c, 16u);
+            for (int half = 0; half < 2; half++) {
+                const uint32_t r = min(16 * (f / KQ) + 8 * half + g, rows - 1);
+                const float4 v = __ldg((const float4 *)((const float *)a.Q + head + (size_t)(tl * 32 + r) * HD + 16 * (f % KQ) + 4 * t));
+                x[half][0] = v.x; x[half][1] = v.y; x[half][2] = v.z; x[half][3] = v.w;
+            }
+            Frag<3> fr;
+            split_rows<3>(fr, x[0], x[1]);
+            store_frag<3>(Qf + f * 3 * 32, lane, fr);
         }
-        issue();
     }
-    float mx[4], sum[4];
-    uint64_t acc[4][TN / 2];
+    __syncthreads();
+    float mx[4], sum[4];                                                 // of rows g + 8 q
+    float acc[2][N][4] = {};
 #pragma unroll
-    for (int m = 0; m < 4; m++) {
-        mx[m] = -INFINITY;
-        sum[m] = 0.f;
-#pragma unroll
-        for (int j = 0; j < TN / 2; j++) acc[m][j] = 0;
+    for (int q = 0; q < 4; q++) {
+        mx[q] = -INFINITY;
+        sum[q] = 0.f;
     }
     uint32_t c = 0;
     for (uint32_t e = 0; e < n; e += NK) {
-        const uint32_t left = min(NK, n - e);
-        const bool live = 32 * warp < left;
-        uint64_t s2[4][8];
+        const uint32_t left = min(NK, n - e), tiles = tiles_of(left);
+        float s[2][2][4] = {};
+        uint32_t mk[4];                                                  // the rows of this thread's four columns
 #pragma unroll
-        for (int m = 0; m < 4; m++)
-#pragma unroll
-            for (int j = 0; j < 8; j++) s2[m][j] = 0;
-        uint32_t mk[8];                                                  // the rows of this thread's eight columns
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const uint32_t col = 32 * warp + lc + 4 * j;
-            mk[j] = col < left ? csr_entry(a.entries, base, top, distinct, e + col).y : 0u;
+        for (int j = 0; j < 4; j++) {
+            const uint32_t at = tile_at(j >> 1, 2 * t + (j & 1));
+            mk[j] = at < left ? csr_entry(a.entries, base, top, distinct, e + at).y : 0u;
         }
-        for (uint32_t kc = 0; kc < kchunks; kc++, c++) {
-            cp_wait_all();
-            __syncthreads();
-            issue();                                                     // a value chunk follows every key chunk of a step
-            if (live) mma_nt(s2, Qs + lr * QS + kc * kChunk, QS, bufs + (c & 1) * Cfg::buf + (32 * warp + lc) * kStride, kStride);
-        }
-        float s[4][8], bm[4];
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-            bm[m] = -INFINITY;
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                s[m][j] = (mk[j] >> (lr + 8 * m)) & 1u ? half_sum(s2[m][j]) * a.scale_log2e : -INFINITY;
-                bm[m] = fmaxf(bm[m], s[m][j]);
+        if (tiles)
+            for (uint32_t kk = 0; kk < kchunks; kk++, c++) {
+                cp_wait<ST - 2>();
+                __syncwarp();
+                issue();
+                score_chunk<3>(s, Qf + 2 * kk * 3 * 32, KQ * 3 * 32, bufs + (c % ST) * Cfg::buf, tiles, lane);
             }
-            bm[m] = fmaxf(bm[m], __shfl_xor_sync(0xffffffffu, bm[m], 1));
-            bm[m] = fmaxf(bm[m], __shfl_xor_sync(0xffffffffu, bm[m], 4));
-            if (lc == 0) red[warp * 32 + lr + 8 * m] = bm[m];
-        }
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                float &v = s[q >> 1][j >> 1][2 * (q & 1) + (j & 1)];
+                v = (mk[j] >> (g + 8 * q)) & 1u ? v * a.scale_log2e : -INFINITY;
+            }
+        softmax_step<GW, (int)kFaThreads, N>(s, mx, sum, acc, red, w, g, t, 0);
+        put_halves(Pf + (2 * (w >> 2) + (sub >> 1)) * 3 * 32, 4 * 3 * 32, KP * 3 * 32, s, sub & 1, lane);
         __syncthreads();
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-            const uint32_t r = lr + 8 * m;
-            float mn = mx[m];
-#pragma unroll
-            for (uint32_t k = 0; k < 4; k++) mn = fmaxf(mn, red[k * 32 + r]);
-            const float alpha = mn > mx[m] ? exp2f(mx[m] - mn) : 1.f;
-            mx[m] = mn;
-            const float off = mn > -INFINITY ? mn : 0.f;                 // nothing kept so far: exp2(-inf) = 0, and NaN stays NaN
-            float ps = 0.f;
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const float pv = exp2f(s[m][j] - off);
-                Ps[r * PS + 32 * warp + lc + 4 * j] = pv;
-                ps += pv;
-            }
-            sum[m] = fmaf(sum[m], alpha, ps);                            // this thread's columns only; the shares meet at the end
-            const uint64_t a2 = pair(alpha, alpha);
-#pragma unroll
-            for (int j = 0; j < TN / 2; j++) acc[m][j] = fma2(acc[m][j], a2, 0ull);
-        }
-        const uint32_t vchunks = (left + 31) / 32;
-        for (uint32_t vc = 0; vc < vchunks; vc++, c++) {
-            cp_wait_all();
-            __syncthreads();
-            if (vc + 1 < vchunks || e + NK < n) issue();
-            mma_nn<TN>(acc, Ps + lr * PS + vc * 32, PS, bufs + (c & 1) * Cfg::buf + n0 + lane_col<TN>(lc), D + 4);
+        for (uint32_t vc = kg; vc < (left + 31) / 32; vc += KG, c++) {
+            cp_wait<ST - 2>();
+            __syncwarp();
+            issue();
+            mma_values<N, 3, 3>(acc, Pf + 2 * vc * 3 * 32, KP * 3 * 32, bufs + (c % ST) * Cfg::buf, Cfg::v_stride, lane);
         }
     }
     __syncthreads();
+    add_shares<N, KG>(acc, (float *)Pf, kg, cg, Cfg::CG, lane);
 #pragma unroll
-    for (int m = 0; m < 4; m++) {
-        sum[m] += __shfl_xor_sync(0xffffffffu, sum[m], 1);
-        sum[m] += __shfl_xor_sync(0xffffffffu, sum[m], 4);
-        if (lc == 0) red[warp * 32 + lr + 8 * m] = sum[m];
+    for (int q = 0; q < 4; q++) {
+        sum[q] += __shfl_xor_sync(0xffffffffu, sum[q], 1);
+        sum[q] += __shfl_xor_sync(0xffffffffu, sum[q], 2);
+        if (t == 0) red[(g + 8 * q) * GW + w] = sum[q];
     }
     __syncthreads();
     uint32_t odd = 0;                                                    // this thread's rows with an output that is not finite
+    if (kg == 0) {
 #pragma unroll
-    for (int m = 0; m < 4; m++) {
-        const uint32_t r = lr + 8 * m;
-        float l = 0.f;
+        for (int q = 0; q < 4; q++) {
+            const uint32_t r = g + 8 * q;
+            float l = 0.f;
 #pragma unroll
-        for (uint32_t k = 0; k < 4; k++) l += red[k * 32 + r];
-        const float inv = l > 0.f ? 1.f / (l + 1e-6f) : 0.f;             // the reference's denominator (ewops.h:93, cuda_kernels.h:1022)
-        if (tl * 32 + r < a.L) store_cols<SFB_F32, TN>(a.O, head + (size_t)(tl * 32 + r) * HD + n0, lc, acc[m], inv, D / 4, true);
-        float zero = 0.f;                                                // stays 0 as long as every output is finite
+            for (uint32_t k = 0; k < GW; k++) l += red[r * GW + k];
+            const float inv = l > 0.f ? 1.f / (l + 1e-6f) : 0.f;         // the reference's denominator (ewops.h:93, cuda_kernels.h:1022)
+            if (tl * 32 + r < a.L) store_cols<SFB_F32, N>(a.O, head + (size_t)(tl * 32 + r) * HD + n0, t, acc[q >> 1], q & 1, inv, Cfg::NW, true);
+            float zero = 0.f;                                            // stays 0 as long as every output is finite
 #pragma unroll
-        for (int j = 0; j < TN / 2; j++) {
-            const float2 f = unpair(acc[m][j]);
-            zero = fmaf(f.x, 0.f, fmaf(f.y, 0.f, zero));
+            for (int j = 0; j < N; j++) zero = fmaf(acc[q >> 1][j][2 * (q & 1)], 0.f, fmaf(acc[q >> 1][j][2 * (q & 1) + 1], 0.f, zero));
+            if (!(zero == 0.f) && tl * 32 + r < a.L) odd |= 1u << r;
         }
-        if (!(zero == 0.f) && tl * 32 + r < a.L) odd |= 1u << r;
     }
     if (!__syncthreads_or(odd != 0)) return;
     // rows that are not finite are made again (csr_row_again), once every warp has written its columns of them
@@ -1032,7 +1388,7 @@ __global__ void __launch_bounds__(tile::kThreads, 3) csr_tile_f32_kernel(const C
     if (odd) atomicOr(again, odd);
     __syncthreads();
     const uint32_t rows = *again;
-    for (uint32_t r = warp; r < 32; r += 4)
+    for (uint32_t r = w; r < 32; r += 8)
         if ((rows >> r) & 1u) csr_row_again<SFB_F32, D>(a.rowptr, a.colidx, a.nnz, a.Q, a.K, a.V, a.O, a.L, a.H, b, h, tl * 32 + r, a.scale_log2e);
 }
 
@@ -1073,7 +1429,7 @@ int simt_sddmm_nt(cudaStream_t s, const void *lut, const void *a, const void *b,
 #define SD_LAUNCH(CD)                                                                                             \
     {                                                                                                             \
         constexpr uint32_t per = BS == 32 ? 4 : 1;                                                                \
-        const size_t bytes = sizeof(float) * 4 * per * BS * tile::kStride;                                        \
+        const size_t bytes = sizeof(float) * 2 * SddmmCfg<BS>::TEAMS * SddmmCfg<BS>::buf;                         \
         auto kern = sddmm_nt_kernel<BS, AB, CD>;                                                                  \
         static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                                                      \
         launch_overlapped(kern, dim3((p.blocks + per - 1) / per, p.B, p.H), dim3(tile::kThreads), bytes, s, (const uint2 *)lut, a, b, c, p, vec); \
@@ -1133,7 +1489,7 @@ int simt_spmm_nn(cudaStream_t s, const void *lut, const void *a, const void *b, 
     const bool avec = ((uintptr_t)a & 15) == 0, vec = rows_vec(b, bc_dtype, HD, p.d) && rows_vec(c, bc_dtype, HD, p.d);
 #define SP_LAUNCH(DSV)                                                                                            \
     {                                                                                                             \
-        const size_t bytes = sizeof(float) * 2 * SpmmCfg<BS, DSV>::buf;                                           \
+        const size_t bytes = sizeof(float) * 3 * SpmmCfg<BS, DSV>::WC * SpmmCfg<BS, DSV>::buf;                                           \
         const dim3 grid(p.nb_a * ((p.d + DSV - 1) / DSV), p.B, p.H);                                              \
         if (trans) {                                                                                              \
             auto kern = spmm_nn_kernel<BS, DSV, AD, BD, true>;                                                    \
@@ -1202,23 +1558,17 @@ int simt_fused_attention(cudaStream_t s, const void *nn_lut, const void *q, cons
     const float sl = scale * LOG2E_F;
     const uint64_t HD = (uint64_t)p.H * p.d, in = p.in_pitch ? p.in_pitch : HD, on = p.out_pitch ? p.out_pitch : HD;
     const bool vec = rows_vec(q, dtype, in, p.d) && rows_vec(k, dtype, in, p.d) && rows_vec(v, dtype, in, p.d) && rows_vec(o, dtype, on, p.d);
-    // a launch that two CTAs per SM hold at once waits for its chunks one after another: more of them on their way
-    // (B 1, H 4, L 512, d 64: 64 CTAs)
-    const int sms = device_sm_count(current_device());
-    const bool few = (uint64_t)p.nb_a * p.B * p.H <= 2ull * (uint64_t)(sms > 0 ? sms : 0);
-#define LAUNCH_FA_ST(DV, STV)                                                                                    \
+#define LAUNCH_FA(DV)                                                                                            \
     {                                                                                                            \
         typedef typename MaskWord<BS>::type W;                                                                   \
-        const size_t bytes = sizeof(float) * FaCfg<BS, DV, STV>::floats;                                         \
-        auto kern = fused_attention_kernel<BS, DV, DT, STV>;                                                     \
+        const size_t bytes = FaCfg<BS, DV, DT>::bytes;                                                           \
+        auto kern = fused_attention_kernel<BS, DV, DT>;                                                          \
         static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                       \
-        launch_overlapped(kern, grid, dim3(tile::kThreads), bytes, s, (const uint2 *)nn_lut, q, k, v, o, (const W *)mask, p, sl, vec); \
+        launch_overlapped(kern, grid, dim3(kFaThreads), bytes, s, (const uint2 *)nn_lut, q, k, v, o, (const W *)mask, p, sl, vec); \
     }
-#define LAUNCH_FA(DV) { if (few) LAUNCH_FA_ST(DV, 4) else LAUNCH_FA_ST(DV, 2) }
     DISPATCH_BS(bs, DISPATCH_DT(dtype, DT, {
         if (p.d <= 32) LAUNCH_FA(32) else if (p.d <= 64) LAUNCH_FA(64) else LAUNCH_FA(128)
     }))
-#undef LAUNCH_FA_ST
 #undef LAUNCH_FA
     return check_launch("sfb_fused_attention");
 }
@@ -1227,10 +1577,10 @@ int csr_tile_f32(cudaStream_t s, const CsrTileArgs &a, uint32_t B, uint32_t d)
 {
 #define LAUNCH_CT(DV)                                                                                            \
     {                                                                                                            \
-        const size_t bytes = sizeof(float) * FaCfg<32, DV>::floats;                                              \
+        const size_t bytes = FaCfg<32, DV, SFB_F32>::bytes;                                                      \
         auto kern = csr_tile_f32_kernel<DV>;                                                                     \
         static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                       \
-        launch_overlapped(kern, dim3(a.tiles, a.H, B), dim3(tile::kThreads), bytes, s, a);                       \
+        launch_overlapped(kern, dim3(a.tiles, a.H, B), dim3(kFaThreads), bytes, s, a);                       \
     }
     if (d == 32) LAUNCH_CT(32) else if (d == 64) LAUNCH_CT(64) else LAUNCH_CT(128)
 #undef LAUNCH_CT

@@ -1,0 +1,140 @@
+"""The kernels whose fp32 products are sums of bf16 products, against 64-bit arithmetic: tile edges (rows of 1 to 9 blocks, so that a
+step has 1 to 4 of them, every block size and head width, widths that are no multiple of a unit), every operand type, and what is
+not finite or close to it, which must come out as plain fp32 arithmetic gives it."""
+import math
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+TD = {"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}
+# Unit roundoff of what leaves a kernel, and of its fp32 sums.  A product of two split numbers is off by 2^-24 of it (three terms
+# of 8 bits each, the products of the smallest left out), a sum of 16 of them is truncated at most six times by 2^-23 of the
+# largest partial sum, and sums of 16 are added with one rounding each.
+EPS = 2.0 ** -24
+
+
+def _bound(terms):
+    return (1 + 6 * 2 + math.ceil(terms / 16) + 1) * EPS
+
+
+def _layout(sfb, nb, bs, seed):
+    rng = np.random.RandomState(seed)
+    keep = np.zeros((1, nb, nb), np.uint8)
+    for i in range(nb):
+        keep[0, i, rng.choice(nb, size=min(nb, i + 1), replace=False)] = 1     # rows of 1, 2, ... nb blocks
+    lay = sfb.BlockLayout(torch.from_numpy(keep).cuda(), bs)
+    return lay, keep[0].astype(bool)
+
+
+def _blocks(keep, bs, x):
+    """[B, H, L, L] -> [B, H, blocks, bs, bs] in row-major block order."""
+    nb = keep.shape[0]
+    i, j = np.nonzero(keep)
+    return x.reshape(x.shape[0], x.shape[1], nb, bs, nb, bs)[:, :, i, :, j].permute(1, 2, 0, 3, 4)
+
+
+def _dense(keep, bs, p):
+    nb = keep.shape[0]
+    i, j = np.nonzero(keep)
+    out = torch.zeros(p.shape[0], p.shape[1], nb, nb, bs, bs, dtype=torch.float64, device="cuda")
+    out[:, :, i, j] = p.double()
+    return out.permute(0, 1, 2, 4, 3, 5).reshape(p.shape[0], p.shape[1], nb * bs, nb * bs)
+
+
+def _heads(x):
+    return x.double().permute(0, 2, 1, 3)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("bs,d,nb", [(32, 128, 9), (32, 64, 7), (32, 32, 5), (32, 40, 3), (64, 128, 5), (64, 64, 4), (64, 32, 3), (64, 72, 2), (32, 30, 2)])
+def test_products_against_64_bits(sfb, bs, d, nb, dtype):
+    if dtype != "f32" and bs == 64 and d == 64:
+        pytest.skip("taken by the tcgen05 kernels")
+    lay, keep = _layout(sfb, nb, bs, nb + d)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn(2, nb * bs, 3, d, device="cuda", generator=g).to(TD[dtype]) for _ in range(3))
+    Q, K, V = map(_heads, (q, k, v))
+    S, A = Q @ K.transpose(-1, -2), Q.abs() @ K.abs().transpose(-1, -2)
+    s = sfb.bst_sgemm_nt(q, k, lay, torch.float32)
+    assert ((s.double() - _blocks(keep, bs, S)).abs() <= _bound(d) * _blocks(keep, bs, A)).all()
+    for pt in ("f32", "bf16", "f16"):
+        p = torch.randn(s.shape, device="cuda", generator=g).to(TD[pt])
+        P = _dense(keep, bs, p)
+        u = EPS if dtype == "f32" else 2.0 ** -8 if dtype == "bf16" else 2.0 ** -11
+        for M, got in ((P, sfb.bst_sgemm_xn(p, v, lay)), (P.transpose(-1, -2), sfb.bst_sgemm_tn(p, v, lay))):
+            want, size = M @ V, M.abs() @ V.abs()
+            assert ((_heads(got) - want).abs() <= _bound(nb * bs) * size + u * want.abs() + (2.0 ** -25 if dtype == "f16" else 0)).all()
+    scale = 1 / math.sqrt(d)
+    full = torch.from_numpy(np.kron(keep, np.ones((bs, bs), bool))).cuda()
+    W = torch.softmax((S * scale).masked_fill(~full, -math.inf), -1)
+    want, size = W @ V, W @ V.abs()
+    # a score off by e moves its probability by e of it; ex2.approx and its argument: 2^-22 and the argument's rounding
+    off = (_bound(d) * A * scale + (S * scale).abs() * 4 * EPS + 2.0 ** -21).masked_fill(~full, 0)
+    err = (W * off) @ V.abs() + off.amax(-1, keepdim=True) * size + _bound(nb * bs) * size + u * want.abs()
+    assert ((_heads(sfb.fused_attention(q, k, v, lay, scale)) - want).abs() <= err).all()
+    if d in (32, 64, 128):
+        rowptr, colidx = sfb.csr_from_layout(lay)
+        got = _heads(sfb.csr_attention(q, k, v, rowptr, colidx, scale)[0])
+        if dtype == "f32":
+            assert ((got - want).abs() <= err + 2e-6 * size).all()           # the denominator's 1e-6
+
+
+def _same(got, want, tol):
+    """Finite where `want` is and close there; the same infinities and NaN elsewhere."""
+    fin = torch.isfinite(want)
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    assert torch.equal(got[~fin & ~torch.isnan(want)], want[~fin & ~torch.isnan(want)])
+    assert ((got[fin] - want[fin]).abs() <= tol * want[fin].abs().clamp_min(1)).all()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+@pytest.mark.parametrize("bs,d", [(32, 64), (64, 128)])
+@pytest.mark.parametrize("value", [math.inf, -math.inf, math.nan, 3.4e38])
+def test_values_that_are_not_finite_or_nearly(sfb, bs, d, value, dtype):
+    if dtype == "f16" and value == 3.4e38:
+        pytest.skip("not an fp16 number")
+    nb = 4
+    lay, keep = _layout(sfb, nb, bs, 1)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    q, k, v = (torch.randn(1, nb * bs, 2, d, device="cuda", generator=g).to(TD[dtype]) for _ in range(3))
+    q = q.where(q.abs() > 1e-2, torch.ones_like(q))
+    k[0, 5, 0, 3] = value
+    q[0, 2 * bs + 1, 1] = 0
+    q[0, 2 * bs + 1, 1, 0] = 0.5
+    k[0, bs + 2, 1, 0] = value
+    full = torch.from_numpy(np.kron(keep, np.ones((bs, bs), bool))).cuda()
+    S32 = (q.float().permute(0, 2, 1, 3)[..., None, :] * k.float().permute(0, 2, 1, 3)[:, :, None]).sum(-1)     # element by element: inf * 0 is NaN
+    _same(sfb.bst_sgemm_nt(q, k, lay, torch.float32), _blocks(keep, bs, S32), 1e-4)
+    if math.isinf(value):
+        # a score of -inf is a probability of 0, one of +inf or NaN a row of NaN
+        W = torch.softmax((S32 / math.sqrt(d)).masked_fill(~full, -math.inf), -1)
+        want = (W @ v.float().permute(0, 2, 1, 3)).permute(0, 2, 1, 3)
+        _same(sfb.fused_attention(q, k, v, lay, 1 / math.sqrt(d)).float(), want, 1e-5 if dtype == "f32" else 2.0 ** -9)
+    # one value: the rows that keep its block, and no other
+    k = torch.randn(k.shape, device="cuda", generator=g).to(TD[dtype])
+    v[0, bs + 3, 1, d - 1] = value
+    p = torch.rand(1, 2, int(keep.sum()), bs, bs, device="cuda", generator=g) + 0.01
+    M = _dense(keep, bs, p).float()
+    want = torch.where(full[None, None, :, :, None], M[..., None] * v.float().permute(0, 2, 1, 3)[:, :, None], torch.zeros((), device="cuda")).sum(3).permute(0, 2, 1, 3)
+    got = sfb.bst_sgemm_xn(p if dtype == "f32" else p.to(TD[dtype]), v, lay).float()
+    if dtype == "f16":
+        assert torch.equal(torch.isfinite(got), torch.isfinite(want))
+    else:
+        _same(got, want, 1e-4)
+    o = sfb.fused_attention(q, k, v, lay, 1 / math.sqrt(d)).float()
+    touched = torch.zeros_like(o, dtype=torch.bool)
+    touched[0, :, 1, d - 1] = full[:, bs + 3]
+    assert torch.isfinite(o[~touched]).all()
+    if not math.isfinite(value):
+        assert not torch.isfinite(o[touched]).any()
+
+
+def test_a_row_of_scores_that_are_not_numbers_is_not_a_row_of_zeros(sfb):
+    lay = sfb.BlockLayout.generate(sfb.LAYOUT_FULL, 1, 2, 32)
+    q, k, v = (torch.ones(1, 64, 1, 32, device="cuda") for _ in range(3))
+    q[0, 7, 0, 0] = math.nan
+    o = sfb.fused_attention(q, k, v, lay, 0.1)
+    assert torch.isnan(o[0, 7]).all() and torch.isfinite(o[0, :7]).all() and torch.isfinite(o[0, 8:]).all()
