@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(tile::kThreads, 3) sddmm_nt_kernel(const uint2
     stage_end(held_b, rank, bufs, kStride, vec);
     for (uint32_t c = 0; c < chunks; c++) {
         cp_wait<0>();
-        meet<TT, (int)kThreads>(1 + team);
+        meet<TT>(1 + team);
         if (c + 1 < chunks) issue(c + 1);
         Frag<T> fa[2][2];
 #pragma unroll
@@ -612,7 +612,7 @@ spmm_nn_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Pm, const
     }
     for (uint32_t c = 0; c < chunks; c++) {
         cp_wait<1>();
-        meet<TT, (int)kThreads>(1 + team);
+        meet<TT>(1 + team);
         Frag<TP> fp[2][2];
 #pragma unroll
         for (int k = 0; k < 2; k++) {
@@ -824,172 +824,65 @@ __device__ __noinline__ void attention_row_again(const uint2 *ent, uint32_t cnt,
         if (lane + 32 * c < d) Elem<DT>::store(O, orow + lane + 32 * c, acc[c] * inv);
 }
 
-// SDDMM + softmax + SpMM with an online softmax; S and P never leave the SM.  One CTA (eight warps) per block-row.
-//
-// A step takes four 32x32 key blocks or one 64x64 block: Q . K^T, the softmax in registers (row maxima meet in shared
-// memory), P to shared memory as fragments, then O += P . V.  For the scores a warp owns 32 query rows and 16 keys: two n-tiles of
-// eight, of different blocks where blocks are 32 (tiles w and w + 8 of the step's 16, so that a step of one or two blocks is
-// still shared by many warps).  For the output it owns 32 rows, 16 or 32 columns and, where the head is too narrow for all
-// warps, every KG-th chunk of 32 keys; such shares of O are added up at the end.
-//
-// Eight warps and not four: the work of a row (a few key blocks) is a chain of loads, products, maxima and products again, of
-// which each warp then has a shorter piece, and sixteen warps of 128 registers per SM wait for one another's latencies.
-// B 32, H 4, L 1024, d 128, sawtooth, fp32: 305 us on the FMA pipe (four warps, 4 x 8 outputs per thread), 265 now; B 1, H 4, L 512, d 64, fixed (64 CTAs):
-// 14.8 -> 11.4.  At 265 us the tensor pipe is 41 % busy and half of the issue slots are used, a quarter of them by
-// the splits: warps wait for fixed latencies and for the tensor pipe in turn.  Measured beside it: four warps of 250 registers, two CTAs per SM 265 / 12.1;
-// keys and values straight to fragments without the ring 282 / 12.2 with eight warps, 291 with four and three CTAs per SM.
-//
-// A warp stages the keys of its own scores and the values of its own columns (for 64 rows together with the warp that has the
-// other half of the rows) as one sequence of chunks, 32 of d or 32 keys, through a ring of ST buffers.  All warps of a row meet twice
-// per step, for the maxima and for P.
-template <int BS, int D, int DT> struct FaCfg {
-    static constexpr uint32_t RH = BS / 32, GW = 8 / RH;                 // halves of the block-row's 32 rows each, warps of a half
-    static constexpr int TT = 32 * RH;                                   // threads that stage together: the warps with the same keys and columns
-    static constexpr uint32_t G = BS == 32 ? 4 : 1, NK = G * BS;         // key blocks and keys per step
-    static constexpr int N = BS == 64 && D == 128 ? 4 : 2, NW = 8 * N;   // n-tiles of 8 columns per warp, its columns
-    static constexpr uint32_t CG = D / NW, KG = GW / CG;                 // column groups, key groups
-    static constexpr uint32_t v_stride = NW + 8;
-    static constexpr uint32_t kbuf = 16 * tile::kStride, vbuf = 32 * v_stride, buf = kbuf > vbuf ? kbuf : vbuf;
-    static constexpr uint32_t T = tile::kTerms<DT>;
-    static constexpr uint32_t qfrags = BS / 16 * (D / 16) * T * 32, pfrags = BS / 16 * (NK / 16) * 3 * 32;      // uint4
-    static constexpr int ST = D == 128 ? 2 : 3;
-    static constexpr size_t bytes = 16 * (qfrags + pfrags) + 4 * (GW * ST * buf + GW * BS);
-    static_assert(2 * (bytes + 1024) <= 228 * 1024, "two CTAs per SM");
-};
-constexpr uint32_t kFaThreads = 256;
-
-// The staged row of key n of tile j (two tiles of eight): lanes read neighbouring keys four rows apart (simt_tile.cuh: tile_row)
-__device__ __forceinline__ constexpr uint32_t key_place(uint32_t j, uint32_t n) { return 8 * j + (n >> 1) + 4 * (n & 1); }
-// Key n of a tile in its 32 keys, for the tile's place sub in them: keys 16 (sub >> 1) to + 15 are one k16 of the product with the values, of
-// which a lane's four elements are neighbours
-__device__ __forceinline__ constexpr uint32_t tile_key(uint32_t sub, uint32_t n) { return 16 * (sub >> 1) + 2 * (sub & 1) + 4 * (n >> 1) + (n & 1); }
-
-// One chunk of scores: 32 rows (fragments at q, pitch from one 16 rows to the next) x tiles staged at `keys`
-template <int T>
-__device__ __forceinline__ void score_chunk(float (&s)[2][2][4], const uint4 *q, uint32_t pitch, const float *keys, uint32_t tiles, uint32_t lane)
-{
-    using namespace tile;
-    const float *p = keys + key_place(0, lane >> 2) * kStride + 4 * (lane & 3);
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        Frag<T> a[2];
-        load_frag<T>(a[0], q + k * T * 32, lane);
-        load_frag<T>(a[1], q + pitch + k * T * 32, lane);
-        Four<T> b[2];
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const float4 v = *(const float4 *)(p + key_place(j, 0) * kStride + 16 * k);
-            const float x[4] = {v.x, v.y, v.z, v.w};
-            split4<T>(b[j], x);
-        }
-        if (tiles == 2) mma16<2, 2, 2, T, T>(s[0], a, b);
-        else mma16<2, 1, 2, T, T>(s[0], a, b);
-    }
-}
-// Softmax of a step: the maxima of this warp's scores meet those of the other warps, the scores become probabilities.  red: [row][warp]
-template <int GW, int ROWT, int N>
-__device__ __forceinline__ void softmax_step(float (&s)[2][2][4], float (&mx)[4], float (&sum)[4], float (&acc)[2][N][4], float *red, uint32_t w, uint32_t g, uint32_t t, uint32_t bar)
-{
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        float bm = -INFINITY;
-#pragma unroll
-        for (int j = 0; j < 2; j++) bm = fmaxf(bm, fmaxf(s[q >> 1][j][2 * (q & 1)], s[q >> 1][j][2 * (q & 1) + 1]));
-        bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
-        bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 2));
-        if (t == 0) red[(g + 8 * q) * GW + w] = bm;
-    }
-    tile::meet<ROWT, kFaThreads>(bar);
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        float mn = mx[q];
-#pragma unroll
-        for (int k = 0; k < GW; k += 4) {
-            const float4 r = *(const float4 *)(red + (g + 8 * q) * GW + k);
-            mn = fmaxf(fmaxf(fmaxf(mn, r.x), fmaxf(r.y, r.z)), r.w);
-        }
-        const float alpha = mn > mx[q] ? ex2_fast(mx[q] - mn) : 1.f;
-        mx[q] = mn;
-        const float off = mn > -INFINITY ? mn : 0.f;                     // nothing kept so far: exp2(-inf) = 0, and NaN stays NaN
-        float ps = 0.f;
-#pragma unroll
-        for (int j = 0; j < 2; j++)
-#pragma unroll
-            for (int k = 0; k < 2; k++) {
-                float &v = s[q >> 1][j][2 * (q & 1) + k];
-                v = ex2_fast(v - off);
-                ps += v;
-            }
-        sum[q] = fmaf(sum[q], alpha, ps);                                // this thread's columns only; the shares meet at the end
-#pragma unroll
-        for (int n = 0; n < N; n++) {
-            acc[q >> 1][n][2 * (q & 1)] *= alpha;
-            acc[q >> 1][n][2 * (q & 1) + 1] *= alpha;
-        }
-    }
-}
-// P of 32x32 blocks: tile j is half (sub & 1) of the k16 at `at` + j * step; pitch: from one 16 rows to the next
-__device__ __forceinline__ void put_halves(uint4 *at, uint32_t step, uint32_t pitch, const float (&s)[2][2][4], uint32_t half, uint32_t lane)
+// This warp's 32 x 32 probabilities as the A fragments of their product with the values: two of 16 keys per 16 rows (pitch: from
+// one 16 rows to the next)
+__device__ __forceinline__ void put_p(uint4 *at, uint32_t pitch, const float (&s)[2][4][4], uint32_t lane)
 {
     using namespace tile;
 #pragma unroll
     for (int m = 0; m < 2; m++)
 #pragma unroll
         for (int j = 0; j < 2; j++) {
-            uint32_t lo[3], hi[3];
-            split2<3>(lo, s[m][j][0], s[m][j][1]);
-            split2<3>(hi, s[m][j][2], s[m][j][3]);
-#pragma unroll
-            for (int i = 0; i < 3; i++) ((uint2 *)(at + m * pitch + j * step + i * 32 + lane))[half] = make_uint2(lo[i], hi[i]);
+            const float x0[4] = {s[m][2 * j][0], s[m][2 * j][1], s[m][2 * j + 1][0], s[m][2 * j + 1][1]};
+            const float x1[4] = {s[m][2 * j][2], s[m][2 * j][3], s[m][2 * j + 1][2], s[m][2 * j + 1][3]};
+            Frag<3> f;
+            split_rows<3>(f, x0, x1);
+            store_frag<3>(at + m * pitch + j * 3 * 32, lane, f);
         }
 }
-// the same where a warp's two tiles are one k16
-__device__ __forceinline__ void put_whole(uint4 *at, uint32_t pitch, const float (&s)[2][2][4], uint32_t lane)
-{
-    using namespace tile;
-#pragma unroll
-    for (int m = 0; m < 2; m++) {
-        const float x0[4] = {s[m][0][0], s[m][0][1], s[m][1][0], s[m][1][1]}, x1[4] = {s[m][0][2], s[m][0][3], s[m][1][2], s[m][1][3]};
-        Frag<3> f;
-        split_rows<3>(f, x0, x1);
-        store_frag<3>(at + m * pitch, lane, f);
-    }
-}
-// the key groups' shares of O meet in the first group: at: room for (KG - 1) * groups shares
-template <int N, int KG>
-__device__ __forceinline__ void add_shares(float (&acc)[2][N][4], float *at, uint32_t kg, uint32_t group, uint32_t groups, uint32_t lane)
-{
-    if (KG == 1) return;
-    if (kg) {
-#pragma unroll
-        for (int x = 0; x < 8 * N; x++) at[(((kg - 1) * groups + group) * 8 * N + x) * 32 + lane] = acc[x / (4 * N)][(x >> 2) % N][x & 3];
-    }
-    __syncthreads();
-    if (kg == 0) {
-        for (int k = 0; k < KG - 1; k++)
-#pragma unroll
-            for (int x = 0; x < 8 * N; x++) acc[x / (4 * N)][(x >> 2) % N][x & 3] += at[((k * groups + group) * 8 * N + x) * 32 + lane];
-    }
-}
 
-template <int BS, int D, int DT>
-__global__ void __launch_bounds__(kFaThreads, 2)
+// SDDMM + softmax + SpMM with an online softmax; S and P never leave the SM.  One CTA (four warps) per block-row.
+// A step takes four 32x32 key blocks (a 32x32 score tile per warp) or one 64x64 block (a quarter per warp): Q . K^T over
+// chunks of 32 of d, the softmax in registers (row maxima meet in shared memory), P to shared memory as fragments, then
+// O += P . V in chunks of 32 keys, each warp on its share of O's columns (and, for 64 rows, of its rows).  A warp stages
+// the keys of its own scores and its own columns of the values (for 64 rows together with the warp that has the other half
+// of the rows) as one sequence of chunks through a ring of ST buffers; all warps of a row meet twice per step, for the
+// maxima and for P.  Score and O rows of a thread are the same, so O is rescaled in place.
+// ST: two chunk buffers where three CTAs share an SM, three where two do; four for launches that the SMs hold at once: each CTA then waits alone.
+// Measured (fp32, us, the FMA-pipe kernel before / now): B 1, H 4, L 512, d 64, fixed (64 CTAs) 14.8 / 12.1; B 8, H 4, L 2048, d 64, stride 179 / 136;
+// d 128 317 / 245; blocks of 64, d 64 198 / 160; B 2, H 4, L 1024, d 64, full with a mask 77.5 / 57; B 32, H 4, L 1024, d 128, sawtooth 304 / 264.  At the
+// last the tensor pipe is 41 % busy and a third of the issue slots are used, a quarter of them by the splits: the warps wait for fixed
+// latencies, for their chunks and for the tensor pipe in turn.  Beside it were measured: eight warps of 16 keys and 16 columns 11.5 / 156 / 267 / 168 / 60 / 265;
+// every warp a share of every key block of a step (no idle warps in a step of fewer than four) 13.2 / 138 / 254 / 159 / 71 / 267; keys and values
+// straight to fragments without the ring, three CTAs per SM 291 at the last.
+template <int BS, int D, int DT, int ST> struct FaCfg {
+    static constexpr uint32_t G = BS == 32 ? 4 : 1;                      // key blocks per step
+    static constexpr uint32_t NK = G * BS;                               // keys per step
+    static constexpr uint32_t WC = BS == 32 ? 4 : 2;                     // teams: warps side by side (score columns, O columns)
+    static constexpr int TT = 128 / WC, NW = D / WC, N = NW / 8;         // a team's threads and columns of O, n-tiles of 8 columns
+    static constexpr uint32_t v_stride = NW + 8;
+    static constexpr uint32_t kbuf = 32 * tile::kStride, vbuf = 32 * v_stride, buf = kbuf > vbuf ? kbuf : vbuf;
+    static constexpr uint32_t T = tile::kTerms<DT>;
+    static constexpr uint32_t qfrags = BS / 16 * (D / 16) * T * 32, pfrags = BS / 16 * (NK / 16) * 3 * 32;      // uint4
+    static constexpr size_t bytes = 16 * (qfrags + pfrags) + 4 * (WC * ST * buf + WC * BS);
+    static constexpr int ctas = bytes <= 75 * 1024 && N <= 4 ? 3 : bytes <= 113 * 1024 ? 2 : 1;       // what shared memory and registers allow per SM
+};
+template <int BS, int D, int DT, int ST>
+__global__ void __launch_bounds__(tile::kThreads, (FaCfg<BS, D, DT, ST>::ctas))
 fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q, const void *__restrict__ K, const void *__restrict__ V,
                        void *__restrict__ O, const typename MaskWord<BS>::type *__restrict__ mask, AttnDims p, float scale_log2e, bool vec)
 {
     using namespace tile;
     typedef typename MaskWord<BS>::type W;
-    typedef FaCfg<BS, D, DT> Cfg;
-    constexpr int N = Cfg::N, T = Cfg::T, TT = Cfg::TT, ST = Cfg::ST, ROWT = 32 * Cfg::GW;      // ROWT: threads that share query rows
-    constexpr uint32_t G = Cfg::G, GW = Cfg::GW, KG = Cfg::KG, KQ = D / 16, KP = Cfg::NK / 16;
+    typedef FaCfg<BS, D, DT, ST> Cfg;
+    constexpr int N = Cfg::N, T = Cfg::T, TT = Cfg::TT, ROWT = BS == 32 ? 128 : 64;      // ROWT: threads that share query rows
+    constexpr uint32_t G = Cfg::G, WC = Cfg::WC, KQ = D / 16, KP = Cfg::NK / 16;
     extern __shared__ __align__(16) float sm[];
     uint4 *Qf = (uint4 *)sm, *Pf = Qf + Cfg::qfrags;
-    float *bufs = (float *)(Pf + Cfg::pfrags), *red = bufs + GW * ST * Cfg::buf;
+    float *bufs = (float *)(Pf + Cfg::pfrags), *red = bufs + WC * ST * Cfg::buf;
     grid_dependency_wait();
     grid_launch_dependents();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const uint32_t rh = warp / GW, w = warp % GW, r0 = 32 * rh, rank = 32 * rh + lane;
-    const uint32_t cg = w % Cfg::CG, kg = w / Cfg::CG, n0 = cg * Cfg::NW;
     // rows are dealt from both ends: the long rows of the layouts at hand sit there and start first
     const uint32_t i = (blockIdx.x & 1u) ? p.nb_a - 1u - (blockIdx.x >> 1) : blockIdx.x >> 1, b = blockIdx.y, h = blockIdx.z;
     const uint2 *nn = lut + (size_t)h * p.lut_stride;
@@ -997,107 +890,52 @@ fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q
     const size_t HD = p.in_pitch ? (size_t)p.in_pitch : (size_t)p.H * p.d;      // row pitch of q, k, v
     const size_t HDo = p.out_pitch ? (size_t)p.out_pitch : (size_t)p.H * p.d;   // row pitch of o
     const W *mh = mask ? mask + (size_t)h * p.mask_stride : nullptr;
+    const uint32_t r0 = BS == 64 ? 32 * (warp >> 1) : 0, wc = BS == 64 ? warp & 1 : warp;   // this warp's rows and its team: score columns, columns of O
+    const uint32_t rank = BS == 64 ? 32 * (warp >> 1) + lane : lane, n0 = wc * Cfg::NW;
     const uint32_t kchunks = (p.d + kChunk - 1) / kChunk;
     const uint32_t cnt = head.y, left = p.d > n0 ? p.d - n0 : 0;
     const size_t kv = (size_t)b * p.nb_b * BS * HD + (size_t)h * p.d;
-    bufs += w * ST * Cfg::buf;
-    red += r0 * GW;
-    // this warp's tiles: block and place in its 32 keys of tile j (the step's 32-key parts where blocks are 64)
-    const uint32_t blk0 = BS == 32 ? w >> 2 : 0, sub0 = BS == 32 ? w & 3 : 2 * (w & 1), part = BS == 32 ? 0 : 32 * (w >> 1);
-    auto tiles_of = [&](uint32_t nblk) { return BS == 64 ? 2u : (blk0 < nblk ? 1u : 0u) + (blk0 + 2 < nblk ? 1u : 0u); };
+    bufs += wc * ST * Cfg::buf;
 
     // the row's entries, 32 at a time, one per lane, the next 32 ahead
     uint32_t ent = lane < cnt ? nn[head.x + lane].y : 0u, ent2 = 32 + lane < cnt ? nn[head.x + 32 + lane].y : 0u;
-    // the team's sequence of chunks: per step the key chunks of its tiles (if the step has any for it), then its value chunks
-    uint32_t is_e = 0, is_k = 0;                                         // next chunk to issue: step's first entry, index in the step
-    constexpr uint32_t NPART = G * (BS / 32);                            // 32-key parts of a step
-    constexpr int KE = DT == SFB_F32 ? 4 : 8, KPR = (int)kChunk / KE, KSTEP = TT / KPR, KN = 16 / KSTEP;      // 16-byte pieces of 16 keys x 32 elements
-    uint4 held_k[DT == SFB_F32 ? 1 : KN];
+    // the team's sequence of chunks: per step the key chunks of its block (if the step has one for it), then the value chunks
+    uint32_t is_e = 0, is_k = 0, is_n = 0;                               // next chunk to issue: step's first entry, index in the step, overall
+    Staged<DT, TT, (int)kChunk> held_k;
     Staged<DT, TT, Cfg::NW> held_v;
     uint32_t held = 0;                                                   // 16-bit pieces wait in registers: 1 keys, 2 values
     float *held_at = nullptr;
-    const uint32_t kr = rank / KPR, kc = rank % KPR * KE;
-    uint32_t is_tiles = tiles_of(min(G, cnt)), is_mine = is_tiles ? kchunks : 0, is_all = is_mine + (min(cnt * (BS / 32), NPART) + KG - 1 - kg) / KG;
-    uint32_t slot = 0;                                                   // ring buffer of the next chunk
-    const typename Elem<DT>::type *krow[2];                              // this thread's piece of tile j's keys, chunk is_k
-    auto key_rows = [&]() {
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const uint32_t row = __shfl_sync(0xffffffffu, ent, (is_e + (BS == 32 ? blk0 + 2 * j : 0)) % 32) * BS + part + tile_key(BS == 32 ? sub0 : sub0 + j, 0);
-            krow[j] = (const typename Elem<DT>::type *)K + kv + (size_t)row * HD + (vec ? (size_t)tile_key(0, kr & 7) * HD + kc : 0);
-        }
-    };
     auto issue = [&]() {
         held = 0;
         if (is_e < cnt) {
-            if (is_all) {
-                float *buf = bufs + slot * Cfg::buf;
-                held_at = buf;
-                if (is_k < is_mine) {
-                    held = 1;
-                    const uint32_t k0 = is_k * kChunk;
-                    if (is_k == 0) key_rows();
-                    if (vec) {
-                        // rows kr, kr + KSTEP, ... of 16: a tile has eight, KSTEP is 4 or 8 or 16 rows on, that is 8 rows of K or the other tile
-                        const bool in = k0 + kc < p.d;
-#pragma unroll
-                        for (int x = 0; x < KN; x++) {
-                            const int j = KSTEP >= 8 ? (KSTEP == 8 ? x : -1) : x >> 1;      // -1: by this thread's row
-                            const uint32_t jj = j < 0 ? kr >> 3 : (uint32_t)j;
-                            const typename Elem<DT>::type *src = (jj ? krow[1] : krow[0]) + (KSTEP == 4 && (x & 1) ? 8 * HD : 0);
-                            const uint32_t r = kr + x * KSTEP;
-                            if constexpr (DT == SFB_F32) {
-                                if (jj < is_tiles) cp_async16(buf + key_place(r >> 3, r & 7) * kStride + kc, in ? src : (const float *)K, in ? 16u : 0u);
-                            } else {
-                                held_k[x] = in && jj < is_tiles ? __ldg((const uint4 *)src) : make_uint4(0u, 0u, 0u, 0u);
-                            }
-                        }
-                    } else {
-                        for (uint32_t x = rank; x < 16 * kChunk; x += TT) {
-                            const uint32_t r = x / kChunk, k = x % kChunk, j = r >> 3;
-                            if (j < is_tiles) buf[key_place(j, r & 7) * kStride + k] = k0 + k < p.d ? Elem<DT>::load(j ? krow[1] : krow[0], (size_t)tile_key(0, r & 7) * HD + k) : 0.f;
-                        }
-                    }
-                    krow[0] += kChunk;
-                    krow[1] += kChunk;
-                } else {
-                    held = 2;
-                    const uint32_t vc = kg + (is_k - is_mine) * KG;
-                    const uint32_t row = __shfl_sync(0xffffffffu, ent, (is_e + (BS == 32 ? vc : 0)) % 32) * BS + (BS == 32 ? 0 : 32 * vc);
-                    if (left) stage_begin(held_v, rank, buf, Cfg::v_stride, V, kv + (size_t)row * HD + n0, HD, left, vec);
-                }
-                slot = slot + 1 == ST ? 0 : slot + 1;
-                is_k++;
+            const uint32_t nblk = min(G, cnt - is_e), mine = G == 1 || wc < nblk ? kchunks : 0;
+            float *buf = bufs + (is_n % ST) * Cfg::buf;
+            held_at = buf;
+            if (is_k < mine) {
+                const uint32_t key = __shfl_sync(0xffffffffu, ent, (is_e + (G == 1 ? 0 : wc)) % 32) * BS + (G == 1 ? 32 * wc : 0), k0 = is_k * kChunk;
+                held = 1;
+                stage_begin(held_k, rank, buf, kStride, K, kv + (size_t)key * HD + k0, HD, p.d - k0, vec);
+            } else {
+                const uint32_t vc = is_k - mine, key = __shfl_sync(0xffffffffu, ent, (is_e + (G == 1 ? 0 : vc)) % 32) * BS + (G == 1 ? 32 * vc : 0);
+                held = 2;
+                if (left) stage_begin(held_v, rank, buf, Cfg::v_stride, V, kv + (size_t)key * HD + n0, HD, left, vec);
             }
-            if (is_k == is_all) {
+            is_n++;
+            if (++is_k == mine + nblk * (BS / 32)) {
                 is_k = 0;
                 is_e += G;
                 if (is_e % 32 == 0) {
                     ent = ent2;
                     ent2 = is_e + 32 + lane < cnt ? nn[head.x + is_e + 32 + lane].y : 0u;
                 }
-                if (is_e + G > cnt && is_e < cnt) {                      // the last step may have fewer blocks
-                    is_tiles = tiles_of(cnt - is_e);
-                    is_mine = is_tiles ? kchunks : 0;
-                    is_all = is_mine + ((cnt - is_e) * (BS / 32) + KG - 1 - kg) / KG;
-                }
             }
         }
         cp_commit();                                                     // nothing left: an empty group keeps the count
     };
     auto land = [&]() {
-        if constexpr (DT != SFB_F32) {
-            if (!vec) return;
-            if (held == 1) {
-#pragma unroll
-                for (int x = 0; x < KN; x++) {
-                    const uint32_t r = kr + x * KSTEP;
-                    widen8_to<DT>(held_at + key_place(r >> 3, r & 7) * kStride + kc, held_k[x]);
-                }
-            } else if (held == 2 && left) {
-                stage_end(held_v, rank, held_at, Cfg::v_stride, vec);
-            }
-        }
+        if (DT == SFB_F32) return;
+        if (held == 1) stage_end(held_k, rank, held_at, kStride, vec);
+        else if (held == 2 && left) stage_end(held_v, rank, held_at, Cfg::v_stride, vec);
     };
 
     if (cnt) {
@@ -1107,8 +945,8 @@ fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q
             land();
         }
         const size_t q0 = ((size_t)b * p.nb_a + i) * BS * HD + (size_t)h * p.d;
-#pragma unroll 2
-        for (uint32_t f = warp; f < BS / 16 * KQ; f += 8) {              // fragment f: rows 16 (f / KQ), elements 16 (f % KQ)
+#pragma unroll 4
+        for (uint32_t f = warp; f < BS / 16 * KQ; f += 4) {              // fragment f: rows 16 (f / KQ), elements 16 (f % KQ)
             const uint32_t k = 16 * (f % KQ) + 4 * t, n = k < p.d ? p.d - k : 0u;
             Raw4<DT> a0, a1;
             load_raw4<DT>(a0, Q, q0 + (size_t)(16 * (f / KQ) + g) * HD + k, n, vec);
@@ -1122,8 +960,6 @@ fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q
         }
     }
     __syncthreads();
-    const uint4 *Qw = Qf + rh * 2 * KQ * T * 32;                         // this warp's rows
-    uint4 *Pw = Pf + rh * 2 * KP * 3 * 32;
     float mx[4], sum[4];                                                 // of rows r0 + g + 8 q
     float acc[2][N][4] = {};
 #pragma unroll
@@ -1131,91 +967,129 @@ fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q
         mx[q] = -INFINITY;
         sum[q] = 0.f;
     }
-    uint32_t at = 0;                                                     // ring buffer of the chunk at hand
-    auto next = [&]() {
-        cp_wait<ST - 2>();
-        meet<TT, kFaThreads>(1 + w);
-        issue();
-        const float *buf = bufs + at * Cfg::buf;
-        at = at + 1 == ST ? 0 : at + 1;
-        return buf;
-    };
+    uint32_t c = 0;
     for (uint32_t e = 0; e < cnt; e += G) {
-        const uint32_t nblk = min(G, cnt - e), tiles = tiles_of(nblk);
-        float s[2][2][4] = {};
-        if (tiles)
-            for (uint32_t kk = 0; kk < kchunks; kk++) {
-                const float *keys = next();
-                score_chunk<T>(s, Qw + 2 * kk * T * 32, KQ * T * 32, keys, tiles, lane);
+        const uint32_t nblk = min(G, cnt - e);
+        const bool live = G == 1 || warp < nblk;
+        float s[2][4][4] = {};
+        if (live)
+            for (uint32_t kc = 0; kc < kchunks; kc++, c++) {
+                cp_wait<ST - 2>();
+                meet<TT>(1 + wc);
+                issue();
+                const float *keys = bufs + (c % ST) * Cfg::buf;
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    Four<T> fb[4];
+                    load_keys<T, false>(fb, keys, 16 * k, g, t);
+#pragma unroll
+                    for (int m = 0; m < 2; m++) {
+                        Frag<T> fa;
+                        load_frag<T>(fa, Qf + ((r0 / 16 + m) * KQ + 2 * kc + k) * T * 32, lane);
+                        mma16<4, T, T>(s[m], fa, fb);
+                    }
+                }
                 land();
             }
-        if (!mh) {
+        const uint32_t blk = mh ? nn[head.x + e + (G > 1 && live ? warp : 0)].x : 0u;
 #pragma unroll
-            for (int x = 0; x < 16; x++) {
-                float &v = s[x >> 3][(x >> 2) & 1][x & 3];
-                v = (uint32_t)((x >> 2) & 1) < tiles ? v * scale_log2e : -INFINITY;
+        for (int q = 0; q < 4; q++) {
+            const uint32_t r = r0 + g + 8 * q;
+            float bm = -INFINITY;
+            if (mh) {
+                const W w = live ? __ldg(mh + (size_t)blk * BS + r) : (W)0;
+                const uint32_t bits = (uint32_t)(w >> (BS == 64 ? 32 * wc : 0));
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+#pragma unroll
+                    for (int k = 0; k < 2; k++) {
+                        float &v = s[q >> 1][j][2 * (q & 1) + k];
+                        v = (bits >> score_key<false>(t, j, k)) & 1u ? v * scale_log2e : -INFINITY;
+                        bm = fmaxf(bm, v);
+                    }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+#pragma unroll
+                    for (int k = 0; k < 2; k++) {
+                        float &v = s[q >> 1][j][2 * (q & 1) + k];
+                        v = live ? v * scale_log2e : -INFINITY;
+                        bm = fmaxf(bm, v);
+                    }
             }
-        } else
+            bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
+            bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 2));
+            if (t == 0) red[wc * BS + r] = bm;
+        }
+        meet<ROWT>(5 + (r0 >> 5));
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const bool live = (uint32_t)j < tiles;
-            const W *mw = live ? mh + (size_t)nn[head.x + e + (BS == 32 ? blk0 + 2 * j : 0)].x * BS + r0 + g : nullptr;
+        for (int q = 0; q < 4; q++) {
+            const uint32_t r = r0 + g + 8 * q;
+            float mn = mx[q];
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const W word = live ? __ldg(mw + 8 * q) : (W)0;
-                const uint32_t bits = (uint32_t)(word >> (part + tile_key(BS == 32 ? sub0 : sub0 + j, 2 * t)));
+            for (uint32_t k = 0; k < WC; k++) mn = fmaxf(mn, red[k * BS + r]);
+            const float alpha = mn > mx[q] ? ex2_fast(mx[q] - mn) : 1.f;
+            mx[q] = mn;
+            const float off = mn > -INFINITY ? mn : 0.f;                 // nothing kept so far: exp2(-inf) = 0, and NaN stays NaN
+            float ps = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
 #pragma unroll
                 for (int k = 0; k < 2; k++) {
                     float &v = s[q >> 1][j][2 * (q & 1) + k];
-                    v = (bits >> k) & 1u ? v * scale_log2e : -INFINITY;
+                    v = ex2_fast(v - off);
+                    ps += v;
                 }
+            sum[q] = fmaf(sum[q], alpha, ps);                            // this thread's columns only; the shares meet at the end
+#pragma unroll
+            for (int n = 0; n < N; n++) {
+                acc[q >> 1][n][2 * (q & 1)] *= alpha;
+                acc[q >> 1][n][2 * (q & 1) + 1] *= alpha;
             }
         }
-        softmax_step<GW, ROWT, N>(s, mx, sum, acc, red, w, g, t, 1 + GW + rh);
-        if (BS == 32) put_halves(Pw + (2 * blk0 + (sub0 >> 1)) * 3 * 32, 4 * 3 * 32, KP * 3 * 32, s, sub0 & 1, lane);
-        else put_whole(Pw + w * 3 * 32, KP * 3 * 32, s, lane);
-        meet<ROWT, kFaThreads>(1 + GW + rh);
-        for (uint32_t vc = kg; vc < nblk * (BS / 32); vc += KG) {
-            const float *values = next();
-            if (left) mma_values<N, 3, T>(acc, Pw + 2 * vc * 3 * 32, KP * 3 * 32, values, Cfg::v_stride, lane);
+        put_p(Pf + (r0 / 16 * KP + 2 * wc) * 3 * 32, KP * 3 * 32, s, lane);
+        meet<ROWT>(5 + (r0 >> 5));
+        const uint32_t vchunks = nblk * (BS / 32);
+        for (uint32_t vc = 0; vc < vchunks; vc++, c++) {
+            cp_wait<ST - 2>();
+            meet<TT>(1 + wc);
+            issue();
+            if (left) mma_values<N, 3, T>(acc, Pf + (r0 / 16 * KP + 2 * vc) * 3 * 32, KP * 3 * 32, bufs + (c % ST) * Cfg::buf, Cfg::v_stride, lane);
             land();
         }
     }
     __syncthreads();
-    add_shares<N, KG>(acc, (float *)Pf, kg, rh * Cfg::CG + cg, Cfg::RH * Cfg::CG, lane);
 #pragma unroll
     for (int q = 0; q < 4; q++) {
         sum[q] += __shfl_xor_sync(0xffffffffu, sum[q], 1);
         sum[q] += __shfl_xor_sync(0xffffffffu, sum[q], 2);
-        if (t == 0) red[(g + 8 * q) * GW + w] = sum[q];
+        if (t == 0) red[wc * BS + r0 + g + 8 * q] = sum[q];
     }
     __syncthreads();
     const size_t baseO = (((size_t)b * p.nb_a + i) * BS) * HDo + (size_t)h * p.d;
     uint32_t odd = 0;                                                    // this thread's rows with an output that is not finite
-    if (kg == 0) {
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const uint32_t r = r0 + g + 8 * q;
-            float l = 0.f;
+    for (int q = 0; q < 4; q++) {
+        const uint32_t r = r0 + g + 8 * q;
+        float l = 0.f;
 #pragma unroll
-            for (uint32_t k = 0; k < GW; k++) l += red[(g + 8 * q) * GW + k];
-            store_cols<DT, N>(O, baseO + (size_t)r * HDo + n0, t, acc[q >> 1], q & 1, l > 0.f ? 1.f / l : 0.f, left, vec);
-            float zero = l * 0.f;
+        for (uint32_t k = 0; k < WC; k++) l += red[k * BS + r];
+        store_cols<DT, N>(O, baseO + (size_t)r * HDo + n0, t, acc[q >> 1], q & 1, l > 0.f ? 1.f / l : 0.f, left, vec);
+        float zero = l * 0.f;
 #pragma unroll
-            for (int n = 0; n < N; n++) zero = fmaf(acc[q >> 1][n][2 * (q & 1)], 0.f, fmaf(acc[q >> 1][n][2 * (q & 1) + 1], 0.f, zero));
-            if (!(zero == 0.f)) odd |= 1u << q;
-        }
+        for (int n = 0; n < N; n++) zero = fmaf(acc[q >> 1][n][2 * (q & 1)], 0.f, fmaf(acc[q >> 1][n][2 * (q & 1) + 1], 0.f, zero));
+        if (!(zero == 0.f)) odd |= 1u << q;
     }
     if (!__syncthreads_or(odd != 0)) return;
     // such rows are made again by plain FMAs, once every warp has written its columns of them
     uint32_t *again = (uint32_t *)Pf;
-    for (uint32_t r = threadIdx.x; r < BS; r += kFaThreads) again[r] = 0;
+    for (uint32_t r = threadIdx.x; r < BS; r += kThreads) again[r] = 0;
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < 4; q++)
         if ((odd >> q) & 1u) again[r0 + g + 8 * q] = 1;
     __syncthreads();
-    for (uint32_t r = warp; r < BS; r += kFaThreads / 32)
+    for (uint32_t r = warp; r < BS; r += kThreads / 32)
         if (again[r])
             attention_row_again<BS, DT>(nn + head.x, cnt, Q, K, V, O, mh ? mh + r : nullptr, (((size_t)b * p.nb_a + i) * BS + r) * HD + (size_t)h * p.d,
                                         (size_t)b * p.nb_b * BS * HD + (size_t)h * p.d, baseO + (size_t)r * HDo, HD, p.d, scale_log2e);
@@ -1224,6 +1098,9 @@ fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q
 // ------------------------------------------------------------------------------------------------
 // Element-sparse attention of one tile of 32 query rows on fp32 operands (csr.cu makes the tile's list of columns and
 // row masks): the kernel above on keys gathered by column, 128 of them per step, a 32x32 score tile per warp.
+template <int D> struct CsrF32Cfg : FaCfg<32, D, SFB_F32, D == 128 ? 3 : 2> {
+    static constexpr int ST = D == 128 ? 3 : 2;
+};
 // 32 gathered rows x COLS elements by one warp: lane r has the column of row r, or -1 (zeros)
 template <int COLS>
 __device__ __forceinline__ void stage_gather(float *dst, uint32_t stride, const float *src, int32_t col, uint32_t lane, size_t pitch)
@@ -1238,57 +1115,46 @@ __device__ __forceinline__ void stage_gather(float *dst, uint32_t stride, const 
     }
 }
 template <int D>
-__global__ void __launch_bounds__(kFaThreads, 2) csr_tile_f32_kernel(const CsrTileArgs a)
+__global__ void __launch_bounds__(tile::kThreads, CsrF32Cfg<D>::ctas) csr_tile_f32_kernel(const CsrTileArgs a)
 {
     using namespace tile;
-    typedef FaCfg<32, D, SFB_F32> Cfg;
+    typedef CsrF32Cfg<D> Cfg;
     constexpr int N = Cfg::N, ST = Cfg::ST;
-    constexpr uint32_t NK = Cfg::NK, GW = Cfg::GW, KG = Cfg::KG, KQ = D / 16, KP = NK / 16, kchunks = D / kChunk;
+    constexpr uint32_t NK = Cfg::NK, KQ = D / 16, KP = NK / 16, kchunks = D / kChunk;
     extern __shared__ __align__(16) float sm[];
     uint4 *Qf = (uint4 *)sm, *Pf = Qf + Cfg::qfrags;
-    float *bufs = (float *)(Pf + Cfg::pfrags), *red = bufs + GW * ST * Cfg::buf;
+    float *bufs = (float *)(Pf + Cfg::pfrags), *red = bufs + 4 * ST * Cfg::buf;
     grid_dependency_wait();
     grid_launch_dependents();
     csr_write_bad(a);
-    const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const uint32_t cg = w % Cfg::CG, kg = w / Cfg::CG, n0 = cg * Cfg::NW;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const uint32_t tl = a.tiles - 1u - blockIdx.x, h = blockIdx.y, b = blockIdx.z;
     const uint32_t *cnt = a.counts + kCsrCounts * tl;
     const uint32_t distinct = cnt[0], base = cnt[2], top = cnt[3], n = distinct + cnt[1];
     const size_t HD = (size_t)a.H * D, head = (size_t)b * a.L * HD + (size_t)h * D;
     const float *K = (const float *)a.K + head, *V = (const float *)a.V + head;
-    bufs += w * ST * Cfg::buf;
-    const uint32_t sub = w & 3;
-    auto tile_at = [&](uint32_t j, uint32_t x) { return 32 * ((w >> 2) + 2 * j) + tile_key(sub, x); };       // key x of this warp's tile j in the step
-    auto tiles_of = [&](uint32_t left) { return (tile_at(0, 0) < left ? 1u : 0u) + (tile_at(1, 0) < left ? 1u : 0u); };
+    const uint32_t n0 = warp * (D / 4);
+    bufs += warp * ST * Cfg::buf;
 
-    // This warp's sequence of chunks: per step the key chunks of its two tiles (if the step has any for it), then its value chunks.
-    // Lane r has the column of staged key r (of 16) and of value row r; the next ones are asked for when the last chunk of these is issued.
+    // this warp's sequence of chunks: per step the key chunks of its 32 columns (if the step has any for it), then the value
+    // chunks.  A chunk's columns are asked for when the one before is issued.
     uint32_t is_e = 0, is_k = 0, is_n = 0;                               // next chunk to issue: step's first key, index in the step, overall
-    auto column = [&](uint32_t at) { return at < n ? (int32_t)csr_entry(a.entries, base, top, distinct, at).x : -1; };
-    auto key_column = [&](uint32_t e) { return lane < 16 ? column(e + tile_at(lane >> 3, lane & 7)) : -1; };
-    int32_t kcol = key_column(0), vcol = column(32 * kg + lane);
+    auto column = [&](uint32_t first) { return first + lane < n ? (int32_t)csr_entry(a.entries, base, top, distinct, first + lane).x : -1; };
+    int32_t kcol = column(32 * warp), vcol = column(0);                  // of the key chunks at hand, of the next value chunk
     auto issue = [&]() {
         if (is_e < n) {
-            const uint32_t left = min(NK, n - is_e), mine = tiles_of(left) ? kchunks : 0, parts = (left + 31) / 32, vmine = (parts + KG - 1 - kg) / KG;
-            if (mine + vmine) {
-                float *buf = bufs + (is_n % ST) * Cfg::buf;
-                if (is_k < mine) {
-#pragma unroll
-                    for (int x = 0; x < 4; x++) {
-                        const uint32_t r = lane / 8 + 4 * x, kc = lane % 8 * 4;
-                        const int32_t col = __shfl_sync(0xffffffffu, kcol, r);
-                        cp_async16(buf + key_place(r >> 3, r & 7) * kStride + kc, K + (size_t)max(col, 0) * HD + is_k * kChunk + kc, col < 0 ? 0u : 16u);
-                    }
-                    if (is_k + 1 == mine) kcol = key_column(is_e + NK);
-                } else {
-                    stage_gather<Cfg::NW>(buf, Cfg::v_stride, V + n0, vcol, lane, HD);
-                    vcol = column((is_k + 1 < mine + vmine ? is_e + 32 * (kg + (is_k + 1 - mine) * KG) : is_e + NK + 32 * kg) + lane);
-                }
-                is_n++;
-                is_k++;
+            const uint32_t left = min(NK, n - is_e), mine = 32 * warp < left ? kchunks : 0, vchunks = (left + 31) / 32;
+            float *buf = bufs + (is_n % ST) * Cfg::buf;
+            if (is_k < mine) {
+                stage_gather<(int)kChunk>(buf, kStride, K + is_k * kChunk, kcol, lane, HD);
+                if (is_k + 1 == mine) kcol = column(is_e + NK + 32 * warp);
+            } else {
+                const uint32_t vc = is_k - mine;
+                stage_gather<(int)Cfg::NW>(buf, Cfg::v_stride, V + n0, vcol, lane, HD);
+                vcol = column(vc + 1 < vchunks ? is_e + 32 * (vc + 1) : is_e + NK);
             }
-            if (is_k == mine + vmine) {
+            is_n++;
+            if (++is_k == mine + vchunks) {
                 is_k = 0;
                 is_e += NK;
             }
@@ -1299,8 +1165,8 @@ __global__ void __launch_bounds__(kFaThreads, 2) csr_tile_f32_kernel(const CsrTi
 #pragma unroll
         for (int k = 0; k < ST - 1; k++) issue();
         const uint32_t rows = min(32u, a.L - tl * 32);                   // rows behind the sequence: the last one again, not written
-#pragma unroll 2
-        for (uint32_t f = w; f < 2 * KQ; f += 8) {
+#pragma unroll 4
+        for (uint32_t f = warp; f < 2 * KQ; f += 4) {
             float x[2][4];
 #pragma unroll
             for (int half = 0; half < 2; half++) {
@@ -1323,32 +1189,74 @@ __global__ void __launch_bounds__(kFaThreads, 2) csr_tile_f32_kernel(const CsrTi
     }
     uint32_t c = 0;
     for (uint32_t e = 0; e < n; e += NK) {
-        const uint32_t left = min(NK, n - e), tiles = tiles_of(left);
-        float s[2][2][4] = {};
-        uint32_t mk[4];                                                  // the rows of this thread's four columns
+        const uint32_t left = min(NK, n - e);
+        const bool live = 32 * warp < left;
+        float s[2][4][4] = {};
+        uint32_t mk[8];                                                  // the rows of this thread's eight columns
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const uint32_t at = tile_at(j >> 1, 2 * t + (j & 1));
-            mk[j] = at < left ? csr_entry(a.entries, base, top, distinct, e + at).y : 0u;
+        for (int j = 0; j < 8; j++) {
+            const uint32_t col = 32 * warp + score_key<false>(t, j >> 1, j & 1);
+            mk[j] = col < left ? csr_entry(a.entries, base, top, distinct, e + col).y : 0u;
         }
-        if (tiles)
-            for (uint32_t kk = 0; kk < kchunks; kk++, c++) {
+        if (live)
+            for (uint32_t kc = 0; kc < kchunks; kc++, c++) {
                 cp_wait<ST - 2>();
                 __syncwarp();
                 issue();
-                score_chunk<3>(s, Qf + 2 * kk * 3 * 32, KQ * 3 * 32, bufs + (c % ST) * Cfg::buf, tiles, lane);
+                const float *keys = bufs + (c % ST) * Cfg::buf;
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    Four<3> fb[4];
+                    load_keys<3, false>(fb, keys, 16 * k, g, t);
+#pragma unroll
+                    for (int m = 0; m < 2; m++) {
+                        Frag<3> fa;
+                        load_frag<3>(fa, Qf + (m * KQ + 2 * kc + k) * 3 * 32, lane);
+                        mma16<4, 3, 3>(s[m], fa, fb);
+                    }
+                }
             }
 #pragma unroll
-        for (int q = 0; q < 4; q++)
+        for (int q = 0; q < 4; q++) {
+            float bm = -INFINITY;
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
+            for (int j = 0; j < 8; j++) {
                 float &v = s[q >> 1][j >> 1][2 * (q & 1) + (j & 1)];
                 v = (mk[j] >> (g + 8 * q)) & 1u ? v * a.scale_log2e : -INFINITY;
+                bm = fmaxf(bm, v);
             }
-        softmax_step<GW, (int)kFaThreads, N>(s, mx, sum, acc, red, w, g, t, 0);
-        put_halves(Pf + (2 * (w >> 2) + (sub >> 1)) * 3 * 32, 4 * 3 * 32, KP * 3 * 32, s, sub & 1, lane);
+            bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
+            bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 2));
+            if (t == 0) red[warp * 32 + g + 8 * q] = bm;
+        }
         __syncthreads();
-        for (uint32_t vc = kg; vc < (left + 31) / 32; vc += KG, c++) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint32_t r = g + 8 * q;
+            float mn = mx[q];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) mn = fmaxf(mn, red[k * 32 + r]);
+            const float alpha = mn > mx[q] ? ex2_fast(mx[q] - mn) : 1.f;
+            mx[q] = mn;
+            const float off = mn > -INFINITY ? mn : 0.f;                 // nothing kept so far: exp2(-inf) = 0, and NaN stays NaN
+            float ps = 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                float &v = s[q >> 1][j >> 1][2 * (q & 1) + (j & 1)];
+                v = ex2_fast(v - off);
+                ps += v;
+            }
+            sum[q] = fmaf(sum[q], alpha, ps);                            // this thread's columns only; the shares meet at the end
+#pragma unroll
+            for (int j = 0; j < N; j++) {
+                acc[q >> 1][j][2 * (q & 1)] *= alpha;
+                acc[q >> 1][j][2 * (q & 1) + 1] *= alpha;
+            }
+        }
+        put_p(Pf + 2 * warp * 3 * 32, KP * 3 * 32, s, lane);
+        __syncthreads();
+        const uint32_t vchunks = (left + 31) / 32;
+        for (uint32_t vc = 0; vc < vchunks; vc++, c++) {
             cp_wait<ST - 2>();
             __syncwarp();
             issue();
@@ -1356,29 +1264,26 @@ __global__ void __launch_bounds__(kFaThreads, 2) csr_tile_f32_kernel(const CsrTi
         }
     }
     __syncthreads();
-    add_shares<N, KG>(acc, (float *)Pf, kg, cg, Cfg::CG, lane);
 #pragma unroll
     for (int q = 0; q < 4; q++) {
         sum[q] += __shfl_xor_sync(0xffffffffu, sum[q], 1);
         sum[q] += __shfl_xor_sync(0xffffffffu, sum[q], 2);
-        if (t == 0) red[(g + 8 * q) * GW + w] = sum[q];
+        if (t == 0) red[warp * 32 + g + 8 * q] = sum[q];
     }
     __syncthreads();
     uint32_t odd = 0;                                                    // this thread's rows with an output that is not finite
-    if (kg == 0) {
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const uint32_t r = g + 8 * q;
-            float l = 0.f;
+    for (int q = 0; q < 4; q++) {
+        const uint32_t r = g + 8 * q;
+        float l = 0.f;
 #pragma unroll
-            for (uint32_t k = 0; k < GW; k++) l += red[r * GW + k];
-            const float inv = l > 0.f ? 1.f / (l + 1e-6f) : 0.f;         // the reference's denominator (ewops.h:93, cuda_kernels.h:1022)
-            if (tl * 32 + r < a.L) store_cols<SFB_F32, N>(a.O, head + (size_t)(tl * 32 + r) * HD + n0, t, acc[q >> 1], q & 1, inv, Cfg::NW, true);
-            float zero = 0.f;                                            // stays 0 as long as every output is finite
+        for (uint32_t k = 0; k < 4; k++) l += red[k * 32 + r];
+        const float inv = l > 0.f ? 1.f / (l + 1e-6f) : 0.f;             // the reference's denominator (ewops.h:93, cuda_kernels.h:1022)
+        if (tl * 32 + r < a.L) store_cols<SFB_F32, N>(a.O, head + (size_t)(tl * 32 + r) * HD + n0, t, acc[q >> 1], q & 1, inv, D / 4, true);
+        float zero = 0.f;                                                // stays 0 as long as every output is finite
 #pragma unroll
-            for (int j = 0; j < N; j++) zero = fmaf(acc[q >> 1][j][2 * (q & 1)], 0.f, fmaf(acc[q >> 1][j][2 * (q & 1) + 1], 0.f, zero));
-            if (!(zero == 0.f) && tl * 32 + r < a.L) odd |= 1u << r;
-        }
+        for (int j = 0; j < N; j++) zero = fmaf(acc[q >> 1][j][2 * (q & 1)], 0.f, fmaf(acc[q >> 1][j][2 * (q & 1) + 1], 0.f, zero));
+        if (!(zero == 0.f) && tl * 32 + r < a.L) odd |= 1u << r;
     }
     if (!__syncthreads_or(odd != 0)) return;
     // rows that are not finite are made again (csr_row_again), once every warp has written its columns of them
@@ -1388,7 +1293,7 @@ __global__ void __launch_bounds__(kFaThreads, 2) csr_tile_f32_kernel(const CsrTi
     if (odd) atomicOr(again, odd);
     __syncthreads();
     const uint32_t rows = *again;
-    for (uint32_t r = w; r < 32; r += 8)
+    for (uint32_t r = warp; r < 32; r += 4)
         if ((rows >> r) & 1u) csr_row_again<SFB_F32, D>(a.rowptr, a.colidx, a.nnz, a.Q, a.K, a.V, a.O, a.L, a.H, b, h, tl * 32 + r, a.scale_log2e);
 }
 
@@ -1558,17 +1463,23 @@ int simt_fused_attention(cudaStream_t s, const void *nn_lut, const void *q, cons
     const float sl = scale * LOG2E_F;
     const uint64_t HD = (uint64_t)p.H * p.d, in = p.in_pitch ? p.in_pitch : HD, on = p.out_pitch ? p.out_pitch : HD;
     const bool vec = rows_vec(q, dtype, in, p.d) && rows_vec(k, dtype, in, p.d) && rows_vec(v, dtype, in, p.d) && rows_vec(o, dtype, on, p.d);
-#define LAUNCH_FA(DV)                                                                                            \
+    // a launch that the SMs hold at once waits for its chunks one after another: more of them on their way
+    // (B 1, H 4, L 512, d 64: 64 CTAs)
+    const int sms = device_sm_count(current_device());
+    const uint64_t ctas = (uint64_t)p.nb_a * p.B * p.H;
+#define LAUNCH_FA_ST(DV, STV)                                                                                    \
     {                                                                                                            \
         typedef typename MaskWord<BS>::type W;                                                                   \
-        const size_t bytes = FaCfg<BS, DV, DT>::bytes;                                                           \
-        auto kern = fused_attention_kernel<BS, DV, DT>;                                                          \
+        const size_t bytes = FaCfg<BS, DV, DT, STV>::bytes;                                                      \
+        auto kern = fused_attention_kernel<BS, DV, DT, STV>;                                                     \
         static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                       \
-        launch_overlapped(kern, grid, dim3(kFaThreads), bytes, s, (const uint2 *)nn_lut, q, k, v, o, (const W *)mask, p, sl, vec); \
+        launch_overlapped(kern, grid, dim3(tile::kThreads), bytes, s, (const uint2 *)nn_lut, q, k, v, o, (const W *)mask, p, sl, vec); \
     }
+#define LAUNCH_FA(DV) { if (ctas <= (uint64_t)(sms > 0 ? sms : 0) * FaCfg<BS, DV, DT, 4>::ctas) LAUNCH_FA_ST(DV, 4) else LAUNCH_FA_ST(DV, (BS == 32 && DV == 128 ? 3 : 2)) }
     DISPATCH_BS(bs, DISPATCH_DT(dtype, DT, {
         if (p.d <= 32) LAUNCH_FA(32) else if (p.d <= 64) LAUNCH_FA(64) else LAUNCH_FA(128)
     }))
+#undef LAUNCH_FA_ST
 #undef LAUNCH_FA
     return check_launch("sfb_fused_attention");
 }
@@ -1577,10 +1488,10 @@ int csr_tile_f32(cudaStream_t s, const CsrTileArgs &a, uint32_t B, uint32_t d)
 {
 #define LAUNCH_CT(DV)                                                                                            \
     {                                                                                                            \
-        const size_t bytes = FaCfg<32, DV, SFB_F32>::bytes;                                                      \
+        const size_t bytes = CsrF32Cfg<DV>::bytes;                                                               \
         auto kern = csr_tile_f32_kernel<DV>;                                                                     \
         static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                       \
-        launch_overlapped(kern, dim3(a.tiles, a.H, B), dim3(kFaThreads), bytes, s, a);                       \
+        launch_overlapped(kern, dim3(a.tiles, a.H, B), dim3(tile::kThreads), bytes, s, a);                       \
     }
     if (d == 32) LAUNCH_CT(32) else if (d == 64) LAUNCH_CT(64) else LAUNCH_CT(128)
 #undef LAUNCH_CT

@@ -45,15 +45,15 @@ __device__ __forceinline__ void cp_async16(float *dst, const void *src, uint32_t
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// THREADS threads (whole warps) of a CTA of ALL meet; id: 1 to 15, the same for all of them and nobody else at the time
-template <int THREADS, int ALL> __device__ __forceinline__ void meet(uint32_t id)
+// THREADS threads (whole warps) meet; id: 1 to 15, the same for all of them and nobody else at the time
+template <int THREADS> __device__ __forceinline__ void meet(uint32_t id)
 {
     if (THREADS == 32) __syncwarp();
-    else if (THREADS == ALL) __syncthreads();
+    else if (THREADS == (int)kThreads) __syncthreads();
     else asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(THREADS) : "memory");
 }
 
-// two elements of a 16-bit type
+// 16-byte piece of a 16-bit type -> eight floats
 template <int DT> __device__ __forceinline__ void widen2(float &a, float &b, uint32_t w)
 {
     if (DT == SFB_BF16) {
@@ -64,18 +64,6 @@ template <int DT> __device__ __forceinline__ void widen2(float &a, float &b, uin
         a = f.x;
         b = f.y;
     }
-}
-
-// a 16-byte piece of a 16-bit type -> eight floats in shared memory
-template <int DT> __device__ __forceinline__ void widen8_to(float *d, const uint4 &u)
-{
-    float v[8];
-    widen2<DT>(v[0], v[1], u.x);
-    widen2<DT>(v[2], v[3], u.y);
-    widen2<DT>(v[4], v[5], u.z);
-    widen2<DT>(v[6], v[7], u.w);
-    *(float4 *)d = make_float4(v[0], v[1], v[2], v[3]);
-    *(float4 *)(d + 4) = make_float4(v[4], v[5], v[6], v[7]);
 }
 
 // 32 rows x COLS elements -> dst[tile_row(r) * stride + c] as fp32, by a team of TT threads (rank: this thread's place in it);
@@ -132,7 +120,14 @@ __device__ __forceinline__ void stage_end(const Staged<DT, TT, COLS> &st, uint32
 #pragma unroll
     for (int i = 0; i < S::N; i++)
         if (32 % S::STEP == 0 || r0 + i * S::STEP < 32) {
-            widen8_to<DT == SFB_F32 ? SFB_F16 : DT>(d + tile_row(i * S::STEP) * stride, st.held[DT == SFB_F32 ? 0 : i]);
+            const uint4 u = st.held[DT == SFB_F32 ? 0 : i];
+            float v[8];
+            widen2<DT>(v[0], v[1], u.x);
+            widen2<DT>(v[2], v[3], u.y);
+            widen2<DT>(v[4], v[5], u.z);
+            widen2<DT>(v[6], v[7], u.w);
+            *(float4 *)(d + tile_row(i * S::STEP) * stride) = make_float4(v[0], v[1], v[2], v[3]);
+            *(float4 *)(d + tile_row(i * S::STEP) * stride + 4) = make_float4(v[4], v[5], v[6], v[7]);
         }
 }
 
@@ -244,12 +239,12 @@ template <int T> __device__ __forceinline__ void load_frag(Frag<T> &f, const uin
 #pragma unroll
     for (int i = 0; i < T; i++) f.w[i] = at[i * 32 + lane];
 }
-// acc[m][n] += a[m] . b[n], 16 elements of the contraction: small products first, from zero.  A: accumulators from one m to the next
-template <int M, int N, int A, int TA, int TB>
-__device__ __forceinline__ void mma16(float (*acc)[4], const Frag<TA> (&a)[M], const Four<TB> *b)
+// acc[n] += a . b[n], 16 elements of the contraction: small products first, from zero
+template <int N, int TA, int TB>
+__device__ __forceinline__ void mma16(float (*acc)[4], const Frag<TA> &a, const Four<TB> *b)
 {
     constexpr int TOP = TA + TB - 2 < 2 ? TA + TB - 2 : 2;
-    float t[M][N][4];
+    float t[N][4];
 #pragma unroll
     for (int s = TOP; s >= 0; s--)
 #pragma unroll
@@ -258,25 +253,15 @@ __device__ __forceinline__ void mma16(float (*acc)[4], const Frag<TA> (&a)[M], c
             if (j < 0 || j >= TB) continue;
             const bool first = s == TOP && (i == TA - 1 || s - (i + 1) < 0);
 #pragma unroll
-            for (int m = 0; m < M; m++)
-#pragma unroll
-                for (int n = 0; n < N; n++)
-                    if (first) mma_zero(t[m][n], a[m].w[i], b[n].w[j]);
-                    else mma_add(t[m][n], a[m].w[i], b[n].w[j]);
+            for (int n = 0; n < N; n++)
+                if (first) mma_zero(t[n], a.w[i], b[n].w[j]);
+                else mma_add(t[n], a.w[i], b[n].w[j]);
         }
 #pragma unroll
-    for (int m = 0; m < M; m++)
-#pragma unroll
-        for (int n = 0; n < N; n++) {
-            add2(acc[m * A + n][0], acc[m * A + n][1], t[m][n][0], t[m][n][1]);
-            add2(acc[m * A + n][2], acc[m * A + n][3], t[m][n][2], t[m][n][3]);
-        }
-}
-template <int N, int TA, int TB>
-__device__ __forceinline__ void mma16(float (*acc)[4], const Frag<TA> &a, const Four<TB> *b)
-{
-    const Frag<TA> a1[1] = {a};
-    mma16<1, N, N, TA, TB>(acc, a1, b);
+    for (int n = 0; n < N; n++) {
+        add2(acc[n][0], acc[n][1], t[n][0], t[n][1]);
+        add2(acc[n][2], acc[n][3], t[n][2], t[n][3]);
+    }
 }
 
 // Scores.  acc[m][j][2 * half + e] is row 16 m + 8 half + g and key score_key<WIDE>(t, j, e): a thread's keys of a row are two
@@ -333,26 +318,20 @@ template <int N, int TP, int TV>
 __device__ __forceinline__ void mma_values(float (&acc)[2][N][4], const uint4 *p, uint32_t pitch, const float *v, uint32_t stride, uint32_t lane)
 {
     constexpr int VN = Cols<N>::VN;
-    static_assert(N == VN, "one group of columns");
     const uint32_t g = lane >> 2, t = lane & 3;
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
-        Four<TV> b[VN];
-        load_values<VN, TV>(b, v + 16 * k * stride, stride, g, t);
-        if (N <= 2) {
-            Frag<TP> a[2];
-            load_frag<TP>(a[0], p + k * TP * 32, lane);
-            load_frag<TP>(a[1], p + pitch + k * TP * 32, lane);
-            mma16<2, VN, N, TP, TV>(acc[0], a, b);
-        } else {
+    for (int k = 0; k < 2; k++)
+#pragma unroll
+        for (int q = 0; q < Cols<N>::GROUPS; q++) {
+            Four<TV> b[VN];
+            load_values<VN, TV>(b, v + 16 * k * stride + 32 * q, stride, g, t);
 #pragma unroll
             for (int m = 0; m < 2; m++) {
                 Frag<TP> a;
                 load_frag<TP>(a, p + m * pitch + k * TP * 32, lane);
-                mma16<VN, TP, TV>(acc[m], a, b);
+                mma16<VN, TP, TV>(&acc[m][VN * q], a, b);
             }
         }
-    }
 }
 // stays 0 while every v is finite
 template <int N>
