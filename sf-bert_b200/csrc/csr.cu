@@ -160,6 +160,7 @@ __global__ void __launch_bounds__(kPlanThreads) csr_plan_kernel(const int32_t *_
 // per SM 119).
 // P enters P.V as two 16-bit terms (the rounded value and what the rounding left), so the product keeps the fp32
 // probabilities to 16 bits (bf16) and 22 bits (fp16).
+constexpr float kCsrGrow = 8.f;
 template <int D> struct CsrCfg {
     static constexpr int MT = D == 128 ? 1 : 2;              // 16-row tiles per warp
     static constexpr int SPLITS = D == 128 ? 2 : 4;          // warps that take different chunks
@@ -333,28 +334,32 @@ __global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const Cs
                 }
             }
         }
-        // running maximum of every row over its quad of lanes, in units of log2 after the scale
-        float nm[MT][2];
+        // The reference maximum of a row (shared by its quad of lanes, in units of log2 after the scale) moves only when a score
+        // outgrows it by 2^8: P stays below that, its two terms are as precise there, and a chunk of 16 columns, in which nearly
+        // always one of 32 rows has a new maximum, needs neither the row's shuffles nor a rescaled output.
+        float x[MT][2];
         bool grow = false;
 #pragma unroll
         for (int mt = 0; mt < MT; mt++)
 #pragma unroll
             for (int e = 0; e < 2; e++) {
-                float x = fmaxf(sc[mt][0][2 * e], sc[mt][0][2 * e + 1]);
+                x[mt][e] = fmaxf(sc[mt][0][2 * e], sc[mt][0][2 * e + 1]);
 #pragma unroll
-                for (int t = 1; t < NT; t++) x = fmaxf(x, fmaxf(sc[mt][t][2 * e], sc[mt][t][2 * e + 1]));
-                x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
-                x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
-                nm[mt][e] = fmaxf(m[mt][e], x * a.scale_log2e);
-                grow |= nm[mt][e] > m[mt][e];
+                for (int t = 1; t < NT; t++) x[mt][e] = fmaxf(x[mt][e], fmaxf(sc[mt][t][2 * e], sc[mt][t][2 * e + 1]));
+                x[mt][e] *= a.scale_log2e;
+                grow |= x[mt][e] > m[mt][e] + kCsrGrow;
             }
         if (__any_sync(0xffffffffu, grow)) {
 #pragma unroll
             for (int mt = 0; mt < MT; mt++)
 #pragma unroll
                 for (int e = 0; e < 2; e++) {
-                    const float f = m[mt][e] > -INFINITY ? ex2f(m[mt][e] - nm[mt][e]) : 0.f;
-                    m[mt][e] = nm[mt][e];
+                    float top = x[mt][e];
+                    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+                    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+                    const float old = m[mt][e], nm = top > old + kCsrGrow ? top : old;
+                    const float f = old > -INFINITY ? ex2f(old - nm) : 0.f;
+                    m[mt][e] = nm;
                     l[mt][e] *= f;
 #pragma unroll
                     for (int d = 0; d < DN; d++) {
