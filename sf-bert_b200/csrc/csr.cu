@@ -211,6 +211,26 @@ __device__ __forceinline__ float ex2f(float x)
     return y;
 }
 
+// pairs of floats: one issue slot for two operations
+__device__ __forceinline__ uint64_t pair2(float a, float b)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpair2(uint64_t v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
 template <bool BF16, int D>
 __global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const CsrTileArgs a)
 {
@@ -242,11 +262,12 @@ __global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const Cs
         const uint16_t *src = (const uint16_t *)a.Q + ((size_t)b * a.L + row) * HD + (size_t)h * D + t % CH * 8;
         q_piece[i] = row < a.L ? __ldg((const uint4 *)src) : make_uint4(0u, 0u, 0u, 0u);
     }
-    float o[MT][DN][4], m[MT][2], l[MT][2];
+    float o[MT][DN][4], m[MT][2];
+    uint64_t l[MT][2];                                       // two partial sums of a row, one per column of a pair
 #pragma unroll
     for (int mt = 0; mt < MT; mt++) {
         m[mt][0] = m[mt][1] = -INFINITY;
-        l[mt][0] = l[mt][1] = 0.f;
+        l[mt][0] = l[mt][1] = 0ull;
 #pragma unroll
         for (int d = 0; d < DN; d++)
 #pragma unroll
@@ -258,19 +279,23 @@ __global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const Cs
     };
     // 16-byte chunk c of row r of a tile sits at chunk c ^ (r % 8) (64-byte rows: c ^ (r / 2 % 4)): no bank twice in a ldmatrix
     auto place = [](uint32_t r, uint32_t c) { return r * (D * 2) + ((c ^ (D == 32 ? (r >> 1) & 3u : r & 7u)) << 4); };
+    static_assert(32 % CH == 0, "a lane keeps its piece of the row");
+    const uint32_t pitch = (uint32_t)(HD * 2);               // bytes; 32 bits, so that an address is one wide multiply-add
+    const uint64_t klane = (uint64_t)(K + lane % CH * 8), vlane = (uint64_t)(V + lane % CH * 8);
     auto issue = [&](const uint2 &e, uint32_t s) {
         const uint32_t kt = (uint32_t)__cvta_generic_to_shared(buf + s * 2 * Cfg::tile_bytes), vt = kt + Cfg::tile_bytes;
 #pragma unroll
         for (int i = 0; i < KC * CH / 32; i++) {
-            const uint32_t t = i * 32 + lane, r = t / CH, c = t % CH;
-            const size_t at = (size_t)__shfl_sync(0xffffffffu, e.x, r) * HD + c * 8;
-            const uint32_t off = place(r, c);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(kt + off), "l"(K + at) : "memory");
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(vt + off), "l"(V + at) : "memory");
+            const uint32_t r = i * (32 / CH) + lane / CH;
+            const uint64_t at = (uint64_t)__shfl_sync(0xffffffffu, e.x, r) * pitch;
+            const uint32_t off = place(r, lane % CH);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(kt + off), "l"(klane + at) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(vt + off), "l"(vlane + at) : "memory");
         }
         if (KC == 32 || lane < KC) masks[warp][s][lane % KC] = e.y;
     };
     const uint32_t qt = (uint32_t)__cvta_generic_to_shared(sm + 4 * Cfg::warp_bytes);
+    const uint64_t scale2 = pair2(a.scale_log2e, a.scale_log2e), one2 = pair2(1.f, 1.f), minus2 = pair2(-1.f, -1.f);
     uint2 e_next = make_uint2(0u, 0u);
     if (split < chunks) {
         issue(entry(split), 0);
@@ -360,7 +385,7 @@ __global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const Cs
                     const float old = m[mt][e], nm = top > old + kCsrGrow ? top : old;
                     const float f = old > -INFINITY ? ex2f(old - nm) : 0.f;
                     m[mt][e] = nm;
-                    l[mt][e] *= f;
+                    l[mt][e] = fma2(l[mt][e], pair2(f, f), 0ull);
 #pragma unroll
                     for (int d = 0; d < DN; d++) {
                         o[mt][d][2 * e] *= f;
@@ -383,13 +408,14 @@ __global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const Cs
                 for (int t = 0; t < 2; t++)
 #pragma unroll
                     for (int e = 0; e < 2; e++) {
-                        const float p0 = ex2f(fmaf(sc[mt][2 * j + t][2 * e], a.scale_log2e, neg[mt][e]));
-                        const float p1 = ex2f(fmaf(sc[mt][2 * j + t][2 * e + 1], a.scale_log2e, neg[mt][e]));
-                        l[mt][e] += p0 + p1;
+                        const float2 z = unpair2(fma2(pair2(sc[mt][2 * j + t][2 * e], sc[mt][2 * j + t][2 * e + 1]), scale2, pair2(neg[mt][e], neg[mt][e])));
+                        const float p0 = ex2f(z.x), p1 = ex2f(z.y);
+                        const uint64_t p2 = pair2(p0, p1);
+                        l[mt][e] = fma2(p2, one2, l[mt][e]);
                         const uint32_t w = pack16<BF16>(p0, p1);
-                        const float2 r = unpack16<BF16>(w);
+                        const float2 r = unpack16<BF16>(w), d = unpair2(fma2(pair2(r.x, r.y), minus2, p2));
                         hi[mt][2 * t + e] = w;
-                        lo[mt][2 * t + e] = pack16<BF16>(p0 - r.x, p1 - r.y);
+                        lo[mt][2 * t + e] = pack16<BF16>(d.x, d.y);
                     }
             uint32_t f[DN / 2][4];
 #pragma unroll
@@ -411,7 +437,8 @@ __global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const Cs
     for (int mt = 0; mt < MT; mt++)
 #pragma unroll
         for (int e = 0; e < 2; e++) {
-            float sum = l[mt][e];
+            const float2 l2 = unpair2(l[mt][e]);
+            float sum = l2.x + l2.y;
             sum += __shfl_xor_sync(0xffffffffu, sum, 1);
             sum += __shfl_xor_sync(0xffffffffu, sum, 2);
             const uint32_t r = mt * 16 + quad + 8 * e;
