@@ -642,24 +642,40 @@ static bool tc_shape_ok(uint32_t bs, const AttnDims &p, uint32_t max_lut)
 
 bool tc_sddmm_supported(int ab_dtype, uint32_t bs, const AttnDims &p, const void *a, const void *b, const void *c)
 {
-    // what the kernel cannot take goes to the CUDA-core kernel instead of failing: unequal block grids, operands the TMA
+    // what the kernel cannot take goes to attn_simt.cu instead of failing: unequal block grids, operands the TMA
     // cannot address (16-byte aligned a, b; 32-byte aligned c)
     if ((((uintptr_t)a | (uintptr_t)b) & 15) != 0 || ((uintptr_t)c & 31) != 0 || p.nb_a != p.nb_b) return false;
     return (ab_dtype == SFB_BF16 || ab_dtype == SFB_F16) && bs == 64 && p.d == 64 && p.blocks > 0 &&
            (uint64_t)p.B * (p.nb_a > p.nb_b ? p.nb_a : p.nb_b) * 64 < (1ull << 31);
 }
 
-// Blocks per CTA: the fewest with which the launch is still one wave of two CTAs per SM, which is what shared memory admits,
-// and kChunk for what is longer.  A launch of 544 blocks was CTAs of 32 blocks one after the other: 17.0 us, 6.6 now.  At
-// least 4, under which a CTA is all set-up.  A few CTAs beyond the wave cost more than the shorter ones save: 8576 blocks
-// in 288 CTAs take 20.5 us, in 320 of them 24.1.
-static uint32_t sddmm_chunk(const AttnDims &p)
+// Blocks per CTA.  GRAD: the fewest with which the launch is still one wave of the two CTAs per SM that shared memory admits, and
+// kChunk for what is longer; at least 4, under which a CTA is all set-up.
+static uint32_t sddmm_grad_chunk(const AttnDims &p)
 {
     const int sms = device_sm_count(current_device());
     const uint64_t bh = (uint64_t)p.B * p.H, slots = 2ull * (uint64_t)(sms > 0 ? sms : 1);
     uint32_t chunk = 4;
     while (chunk < tc::kChunk && (p.blocks + chunk - 1) / chunk * bh > slots) chunk++;
     return chunk;
+}
+// Without it three CTAs share an SM, and what counts is how full the last wave is: the chunk with the least estimated time, in microseconds.
+// A block takes a CTA 0.89 with three on the SM and 0.62 with one or two, a CTA's set-up 1.  Fitted to nine launches of 1024 to
+// 70080 blocks with chunks of 8 to 32: 16256 blocks in CTAs of 32 (512 of them on 444 places) 48.4, of 20 36.3; 32512 74.1 / 67.8; 14850
+// 48.2 / 36.0; 13824 28.6 / 34.4; 70080 129.6 / 135.3.
+static uint32_t sddmm_chunk(const AttnDims &p)
+{
+    const int sms = device_sm_count(current_device());
+    const uint64_t bh = (uint64_t)p.B * p.H, sm = (uint64_t)(sms > 0 ? sms : 1), slots = 3 * sm;
+    uint32_t best = tc::kChunk;
+    double t_best = 1e30;
+    for (uint32_t chunk = tc::kChunk; chunk >= 4; chunk--) {
+        const uint64_t ctas = (p.blocks + chunk - 1) / chunk * bh, rest = ctas % slots;
+        double t = (double)(ctas / slots) * (0.89 * chunk + 1.0);
+        if (rest) t += (rest > 2 * sm ? 0.89 : 0.62) * chunk + 1.0;
+        if (t < t_best) { t_best = t; best = chunk; }
+    }
+    return best;
 }
 
 int tc_sddmm(cudaStream_t s, const void *nt_lut, const void *a, const void *b, void *c, int ab_dtype, int c_dtype, const AttnDims &p)
@@ -701,7 +717,7 @@ int tc_sddmm_softmax_grad(cudaStream_t s, const void *nt_lut, const void *dout, 
     if (make_map(&qm, dout, rows, p.H, is_bf16, 64) || make_map(&km, v, rows, p.H, is_bf16, 64) || make_map_2d(&om, ds, prow, 64, is_bf16, 64) ||
         make_map_2d(&pm, pblk, prow, 64, is_bf16, 64))
         return 1;
-    UParams prm = {(const uint2 *)nt_lut, ds, p.B, p.H, p.nb_a, p.blocks, p.lut_stride, dtype, is_bf16, 0, 0, delta, scale, sddmm_chunk(p)};
+    UParams prm = {(const uint2 *)nt_lut, ds, p.B, p.H, p.nb_a, p.blocks, p.lut_stride, dtype, is_bf16, 0, 0, delta, scale, sddmm_grad_chunk(p)};
     static DeviceOnce once;
     const int dev = current_device();
     if (!once.done(dev)) {
@@ -715,7 +731,7 @@ int tc_sddmm_softmax_grad(cudaStream_t s, const void *nt_lut, const void *dout, 
 
 bool tc_fused_p_supported(int ab_dtype, uint32_t bs, const AttnDims &p, float scale, const void *a, const void *b, const void *y)
 {
-    if ((((uintptr_t)a | (uintptr_t)b | (uintptr_t)y) & 31) != 0) return false;     // the CUDA-core kernel takes any alignment
+    if ((((uintptr_t)a | (uintptr_t)b | (uintptr_t)y) & 31) != 0) return false;     // attn_simt.cu takes any alignment
     // the longest row is not an argument of the fused entry points: any row of the block grid must fit the union list
     return (ab_dtype == SFB_BF16 || ab_dtype == SFB_F16) && scale > 0.f && p.blocks > 0 &&
            tc_shape_ok(bs, p, p.nb_a <= tc::kMaxUnion / 2 ? p.nb_a : 0);
@@ -746,7 +762,7 @@ int tc_fused_p(cudaStream_t s, const void *nn_lut, const void *a, const void *b,
 bool tc_spmm_supported(int a_dtype, int bc_dtype, uint32_t bs, const AttnDims &p, uint32_t max_lut, const void *a, const void *b,
                        const void *c)
 {
-    if ((((uintptr_t)a | (uintptr_t)b) & 15) != 0 || ((uintptr_t)c & 31) != 0) return false;    // the CUDA-core kernel takes any alignment
+    if ((((uintptr_t)a | (uintptr_t)b) & 15) != 0 || ((uintptr_t)c & 31) != 0) return false;    // attn_simt.cu takes any alignment
     return a_dtype == bc_dtype && (a_dtype == SFB_BF16 || a_dtype == SFB_F16) && p.blocks > 0 && tc_shape_ok(bs, p, max_lut);
 }
 

@@ -376,3 +376,17 @@ def test_sddmm_blocks_per_cta(sfb, B, H, nb):
     want = p.float() * (want - rows) * 0.125
     assert sfb.device_status() == 0
     assert float((ds - want).abs().max()) <= 2.0 ** -7 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("B,H,nb", [(1, 16, 23), (2, 12, 24), (1, 15, 31), (1, 16, 32), (2, 13, 35)])
+def test_sddmm_blocks_per_cta_beyond_a_wave(sfb, B, H, nb):
+    """Launches of more than one wave, where the blocks per CTA follow from how full the last wave is (the last CTA of a head
+    has fewer): each block's scores against fp32."""
+    g = torch.Generator(device="cuda").manual_seed(nb)
+    lay = sfb.BlockLayout(torch.ones(1, nb, nb, dtype=torch.uint8, device="cuda"), 64)
+    q, k = (torch.randn(B, nb * 64, H, 64, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    want = torch.einsum("bihd,bjhd->bhij", q.float(), k.float())
+    want = want.reshape(B, H, nb, 64, nb, 64).permute(0, 1, 2, 4, 3, 5).reshape(B, H, lay.blocks, 64, 64)
+    s = sfb.bst_sgemm_nt(q, k, lay, torch.float32)
+    assert sfb.device_status() == 0
+    assert float((s - want).abs().max()) <= 1e-3 * 8         # sqrt(64) * 1e-3: operands are exact in fp32, sums of 64
