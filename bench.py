@@ -893,7 +893,7 @@ def run_dropin(args):
     includes include/blocksparse.h / include/fusion_blocksparse.h reaches (their bodies are one-line forwarders to the
     C ABI entry points called here with the same arguments) timed beside the reference's own unfused GPU operators
     compiled for sm_100a (oracle/_ref/libsfb_ref_gpu.so) on the same inputs.  fp32 operands run on this library's
-    CUDA-core kernels (tensor-core arithmetic cannot meet fp32 parity); the reference's fused kernels spin on global
+    kernels of attn_simt.cu (fp32 products as sums of bf16 products on the tensor cores); the reference's fused kernels spin on global
     flags without a bound and are not run."""
     import torch
     import __graft_entry__ as ge

@@ -12,7 +12,7 @@ struct AttnDims {
     uint64_t out_pitch;    // the same for o
 };
 
-// CUDA-core kernels (attn_simt.cu)
+// fp32 operands and the shapes that the tcgen05 kernels do not take (attn_simt.cu)
 int simt_sddmm_nt(cudaStream_t s, const void *lut, const void *a, const void *b, void *c, int ab_dtype, int c_dtype,
                   uint32_t bs, const AttnDims &p);
 int simt_softmax(cudaStream_t s, const void *lut, const void *mask, const void *x, void *y, int x_dtype, int y_dtype,

@@ -6,7 +6,7 @@
 //   csr_plan_kernel          the pattern by tiles of 32 query rows: the columns any of them has, in ascending order, each with
 //                            a 32-bit mask of the rows that have it
 //   csr_tile_kernel          O for one tile and (batch, head) over those columns, 16-bit operands, on warp MMAs
-//   csr_tile_f32_kernel      (attn_simt.cu) the same on the CUDA cores, for fp32 operands
+//   csr_tile_f32_kernel      (attn_simt.cu) the same for fp32 operands, split into bf16 terms
 //   csr_attention_split_kernel   one warp per query row, four lanes per key: callers without a workspace for the plan, and
 //                            sequences whose columns do not fit the plan's shared memory
 // Row by row every query gathers its own keys through L2 (294 keys, 75 KB, per row of a 256-token window with strided and
@@ -155,7 +155,8 @@ __global__ void __launch_bounds__(kPlanThreads) csr_plan_kernel(const int32_t *_
 // the end.  Warp MMAs rather than tcgen05: the columns of a tile are rows scattered over K and V, and 32 rows is where
 // neighbouring queries still share them.
 // The queries are read from shared memory as they are needed and the chunks are small: what bounds the kernel is latency
-// (42 % of the issue slots, L2 16 %), so the registers go to more CTAs (D 128: two per SM became three, 226 -> 170 us for
+// (40 % of the issue slots, tensor pipe 43 %, L2 18 %: a chunk is 360 instructions of 7.5 cycles each on one of three warps; 32 columns per
+// chunk 96.8 us instead of 95.1), so the registers go to more CTAs (D 128: two per SM became three, 226 -> 170 us for
 // the window pattern at B 2, H 12, L 4096) or keep the accumulators out of local memory (D 64: 114.4 -> 105.8, at four CTAs
 // per SM 119).
 // P enters P.V as two 16-bit terms (the rounded value and what the rounding left), so the product keeps the fp32

@@ -1,5 +1,5 @@
 // C ABI of the attention operators: argument checks and the choice between the tensor-core
-// (tcgen05) kernels and the CUDA-core kernels.  No path leaves the GPU.
+// (tcgen05) kernels and the kernels of attn_simt.cu.  No path leaves the GPU.
 #include "attn.cuh"
 
 using namespace sfb;
@@ -123,7 +123,7 @@ static int fused_attention_common(const char *who, sfb_stream_t stream, const vo
     AttnDims p = {batch_dim, head_dim, state_dim, ctx_blks, ctx_blks, blocks, lut_heads > 1 ? lut_dim + ctx_blks : 0,
                   mask_heads > 1 ? blocks * block_size : 0, in_pitch, out_pitch};
     // 16-bit operands with 64x64 blocks and 64-wide heads run on the tensor cores, when the TMA can address them
-    // (16-byte aligned bases and row pitches); everything else runs on the CUDA cores
+    // (16-byte aligned bases and row pitches); everything else goes to attn_simt.cu
     const bool tma_ok = ((((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)o) & 15) == 0) && in_pitch % 8 == 0 && out_pitch % 8 == 0;
     if (tma_ok && tc_fused_attention_supported(dtype, block_size, p, scale, max_lut))
         return tc_fused_attention(as_stream(stream), nn_lut, q, k, v, o, mask, dtype, p, scale, max_lut);
