@@ -22,9 +22,7 @@ constexpr uint32_t kGBBytes = kGBK * kGBN * 2;           // 32 KB: four 64 x 64 
 constexpr uint32_t kBiasBytes = 2 * 2 * 128 * 4;          // the epilogue's bias: [accumulator][column half][128]
 constexpr int kGStages = 4, kGBufs = 2;
 constexpr uint32_t kGStageBytes = kGABytes + kGBBytes;
-constexpr uint32_t kGStagingBytes = 8 * 32 * 128;     // one 32-row x 64-column tile per epilogue warp
-constexpr size_t kGSmem = kGStages * kGStageBytes + kGStagingBytes + kBiasBytes + 256;
-static_assert(kGSmem <= 227 * 1024, "shared memory budget");
+constexpr size_t kGSmem = 1024 + kGStages * kGStageBytes + kBiasBytes + 256;
 
 struct GShared {
     uint64_t full[kGStages], empty[kGStages], acc_full[2], acc_empty[2], drained;
@@ -32,17 +30,12 @@ struct GShared {
 };
 static_assert(sizeof(GShared) <= 256, "GShared outgrew its slot");
 
-// kWRows: w is [n, k] row-major (out = x . w^T, the tied-embedding logits), its tile is a K-major B operand and one box of
-// rows.  Otherwise w is [k, n] and its tile an MN-major operand of 64 x 64 pieces: one box of neighbouring groups of 64 columns
-// (kWGroups), or, where n is no multiple of 64, a box per piece (kWBoxes).
-enum { kWRows = 0, kWGroups = 1, kWBoxes = 2 };
-
 struct GParams {
     void *out;
     const float *bias;
     uint32_t M, N, K, tiles_m, tiles_n;
     int is_bf16, act;
-    int w_kind;         // how a tile of w is fetched: kWRows, kWGroups, kWBoxes
+    int w_transposed;   // w is [n, k] row-major (out = x . w^T, the tied-embedding logits): its tile is a K-major B operand
     uint32_t band;      // CTA-pair kernel: column tiles per band of the tile order (tile_coords)
     const void *resid;  // split kernel: [m, n] of x's type, added to the product (not out itself), or NULL
 };
@@ -82,8 +75,50 @@ __device__ __forceinline__ float gelu_ref(float t)
     return fmaf(h, th, h);
 }
 
-// A warp's share of a 128-row accumulator: its 32 rows, 128 columns from n0 on, read from TMEM at tcol 32 columns at a time (the
-// next 32 travel while these are written), bias and activation applied, leaving through shared memory: 64 columns are packed into a
+// One thread's share of a 128-row accumulator: row `row` of the output, 128 columns from n0 on, read from TMEM at
+// tcol 32 columns at a time (the next 32 travel while these are written), bias and activation applied, 32-byte stores.
+__device__ __forceinline__ void drain_rows(const GParams &p, uint32_t tcol, const float *bias, uint32_t row, uint32_t n0)
+{
+    const bool row_ok = row < p.M;
+    const size_t off = (size_t)row * p.N + n0;
+    uint32_t v[2][32];
+    TMEM_LD_32((v[0]), tcol);
+#pragma unroll
+    for (uint32_t c = 0; c < 4; c++) {
+        const uint32_t c0 = c * 32;
+        tmem_wait_ld();
+        if (c + 1 < 4) TMEM_LD_32((v[(c + 1) & 1]), tcol + c0 + 32);
+        uint32_t(&cur)[32] = v[c & 1];
+#pragma unroll
+        for (uint32_t q = 0; q < 2; q++) {
+            const uint32_t col = n0 + c0 + q * 16;
+            if (row_ok && col < p.N) {      // N is a multiple of 16: a group of 16 is inside or outside as a whole
+                float x[16];
+#pragma unroll
+                for (int j = 0; j < 16; j++) x[j] = __uint_as_float(cur[q * 16 + j]);
+                if (p.bias) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const float4 bb = *(const float4 *)(bias + c0 + q * 16 + 4 * j);   // the same address in every lane: one broadcast
+                        x[4 * j] += bb.x; x[4 * j + 1] += bb.y; x[4 * j + 2] += bb.z; x[4 * j + 3] += bb.w;
+                    }
+                }
+                if (p.act == 1) {
+#pragma unroll
+                    for (int j = 0; j < 16; j++) x[j] = gelu_ref(x[j]);
+                }
+                uint32_t w[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) w[j] = pack2(x[2 * j], x[2 * j + 1], p.is_bf16);
+                asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"((uint16_t *)p.out + off + c0 + q * 16),
+                             "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                             : "memory");
+            }
+        }
+    }
+}
+
+// The same share of an accumulator, leaving through shared memory: the warp's 32 rows x 64 columns are packed into a
 // staging tile in the tensor map's 128-byte swizzle (16-byte chunk c of row r at chunk c ^ (r % 8)) and one lane hands
 // the tile to the TMA, twice per 128 columns.  The writes reach memory as whole 128-byte rows instead of 32 bytes per
 // thread and instruction, and the storing threads are free as soon as the tile is in shared memory.
@@ -140,28 +175,13 @@ __device__ __forceinline__ void drain_rows_staged(const GParams &p, const CUtens
     }
 }
 
-// 64 x COLS elements of w, k from k0 on, columns from n0 on
-template <uint32_t COLS>
-__device__ __forceinline__ void load_w(const GParams &p, uint32_t dst, const CUtensorMap *map, uint64_t *bar, uint32_t k0, uint32_t n0)
-{
-    if (p.w_kind == kWGroups) {
-        tma_load_3d(dst, map, bar, 0, (int32_t)k0, (int32_t)(n0 / 64));
-    } else if (p.w_kind == kWRows) {
-        tma_load_2d(dst, map, bar, (int32_t)k0, (int32_t)n0);
-    } else {
-#pragma unroll
-        for (uint32_t j = 0; j < COLS / 64; j++) tma_load_2d(dst + j * kTileBytes, map, bar, (int32_t)(n0 + j * 64), (int32_t)k0);
-    }
-}
-
 __global__ void __launch_bounds__(320, 1)
-linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap,
-                 const __grid_constant__ CUtensorMap omap, const GParams p)
+linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap, const GParams p)
 {
-    extern __shared__ __align__(1024) uint8_t smem_aligned[];
-    uint8_t *tiles = smem_aligned;                           // stage s: A (16 KB) then B (32 KB)
-    uint8_t *staging = tiles + kGStages * kGStageBytes;      // the epilogue warps' output tiles (4 KB each)
-    float *bias_s = (float *)(staging + kGStagingBytes);
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t *tiles = smem;                                   // stage s: A (16 KB) then B (32 KB)
+    float *bias_s = (float *)(tiles + kGStages * kGStageBytes);
     GShared *st = (GShared *)((uint8_t *)bias_s + kBiasBytes);
 
     const uint32_t warp = uniform_warp(), lane = threadIdx.x & 31;
@@ -173,7 +193,6 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
     if (threadIdx.x == 0) {
         prefetch_map(amap);
         prefetch_map(bmap);
-        prefetch_map(omap);
         for (int s = 0; s < kGStages; s++) { mbar_init(&st->full[s], 1); mbar_init(&st->empty[s], 1); }
         for (int s = 0; s < 2; s++) { mbar_init(&st->acc_full[s], 1); mbar_init(&st->acc_empty[s], 256); }
         mbar_init(&st->drained, 1);
@@ -205,7 +224,14 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
                     const uint32_t base = smem_u32(tiles + s * kGStageBytes);
                     mbar_expect_tx(&st->full[s], kGStageBytes);   // boxes beyond the tensor arrive as zeros and still count
                     tma_load_2d(base, &amap, &st->full[s], (int32_t)(kb * kGBK), m0);
-                    load_w<kGBN>(p, base + kGABytes, &bmap, &st->full[s], kb * kGBK, (uint32_t)n0);
+                    if (p.w_transposed) {
+                        // 256 rows of w, 64 of k: one box
+                        tma_load_2d(base + kGABytes, &bmap, &st->full[s], (int32_t)(kb * kGBK), n0);
+                    } else {
+#pragma unroll
+                        for (uint32_t j = 0; j < 4; j++)
+                            tma_load_2d(base + kGABytes + j * kTileBytes, &bmap, &st->full[s], n0 + (int32_t)(j * 64), (int32_t)(kb * kGBK));
+                    }
                 }
                 if (!alive) break;
             }
@@ -213,8 +239,8 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
     } else if (warp == 1) {
         // ===== MMA issuer =====
         if (elect_one()) {
-            const uint32_t idesc = instr_desc(fmt, fmt, kGBM, kGBN, p.w_kind == kWRows ? 0 : 1);
-            const uint32_t b_step = p.w_kind == kWRows ? 2u : 128u;   // descriptor units of 16 bytes per 16 of K
+            const uint32_t idesc = instr_desc(fmt, fmt, kGBM, kGBN, p.w_transposed ? 0 : 1);
+            const uint32_t b_step = p.w_transposed ? 2u : 128u;   // descriptor units of 16 bytes per 16 of K
             uint32_t g = 0, i = 0;
             for (uint32_t t = blockIdx.x; t < n_tiles; t += gridDim.x, i++) {
                 const uint32_t buf = i % kGBufs;
@@ -227,7 +253,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
                     tcgen05_fence_after();
                     const uint32_t base = smem_u32(tiles + s * kGStageBytes);
                     // MN-major: the next 64 columns are one box further on; K-major: 256 rows of 128 bytes
-                    const uint64_t b_desc = p.w_kind == kWRows ? smem_desc_sw128(base + kGABytes) : smem_desc_sw128(base + kGABytes, kTileBytes);
+                    const uint64_t b_desc = p.w_transposed ? smem_desc_sw128(base + kGABytes) : smem_desc_sw128(base + kGABytes, kTileBytes);
                     const uint64_t a_desc = smem_desc_sw128(base);
 #pragma unroll
                     for (uint32_t kk = 0; kk < 4; kk++)   // 16 of K per MMA: +32 bytes in A's swizzled rows, +16 rows (2048 bytes) in B
@@ -242,6 +268,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
         // ===== epilogue: eight warps; a thread takes one output row and half of the tile's 256 columns, 32 at a time =====
         const uint32_t quarter = warp & 3;                 // TMEM lanes this warp may touch
         const uint32_t chalf = (warp - 2) >> 2;            // which 128 columns
+        const uint32_t r = quarter * 32 + lane;
         const uint32_t lane_field = (quarter * 32) << 16;
         uint32_t i = 0;
         float4 next = fetch_bias(p, (blockIdx.x / p.tiles_m) * kGBN + chalf * 128, lane);
@@ -254,11 +281,10 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
             __syncwarp();
             if (t + gridDim.x < n_tiles) next = fetch_bias(p, ((t + gridDim.x) / p.tiles_m) * kGBN + chalf * 128, lane);
             tcgen05_fence_after();
-            drain_rows_staged(p, &omap, tmem + buf * kGBN + chalf * 128 + lane_field, staging + (warp - 2) * 4096, bias, (t % p.tiles_m) * kGBM + quarter * 32, n0, lane);
+            drain_rows(p, tmem + buf * kGBN + chalf * 128 + lane_field, bias, (t % p.tiles_m) * kGBM + r, n0);
             tcgen05_fence_before();
             mbar_arrive(&st->acc_empty[buf]);
         }
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the last tile has left shared memory
     }
 
     // ---- teardown (also the way out after a timeout) ----
@@ -347,13 +373,6 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
         ::"r"(dst), "l"((uint64_t)map), "r"(bar_cluster_addr), "r"(x), "r"(y)
         : "memory");
 }
-__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap *map, uint32_t bar_cluster_addr, int32_t x, int32_t y, int32_t z)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-        ::"r"(dst), "l"((uint64_t)map), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z)
-        : "memory");
-}
 __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
 {
     asm volatile(
@@ -430,9 +449,7 @@ linear_tc_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_con
                     const uint32_t bar = mapa_rank(smem_u32(&st->full[s]), 0);
                     if (rank == 0) mbar_expect_tx(&st->full[s], 2 * kPStageBytes);   // both CTAs' bytes; boxes beyond the tensor arrive as zeros and still count
                     tma_load_2d_pair(base, &amap, bar, (int32_t)(kb * kGBK), m0);
-                    if (p.w_kind == kWGroups) {
-                        tma_load_3d_pair(base + kPABytes, &bmap, bar, 0, (int32_t)(kb * kGBK), n0 / 64);
-                    } else if (p.w_kind == kWRows) {
+                    if (p.w_transposed) {
                         tma_load_2d_pair(base + kPABytes, &bmap, bar, (int32_t)(kb * kGBK), n0);      // 128 rows of w, 64 of k
                     } else {
 #pragma unroll
@@ -446,8 +463,8 @@ linear_tc_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_con
     } else if (warp == 1) {
         // ===== MMA issuer: one thread of the even CTA for the pair =====
         if (rank == 0 && elect_one()) {
-            const uint32_t idesc = instr_desc(fmt, fmt, 256, kGBN, p.w_kind == kWRows ? 0 : 1);
-            const uint32_t b_step = p.w_kind == kWRows ? 2u : 128u;
+            const uint32_t idesc = instr_desc(fmt, fmt, 256, kGBN, p.w_transposed ? 0 : 1);
+            const uint32_t b_step = p.w_transposed ? 2u : 128u;
             uint32_t g = 0, i = 0;
             for (uint32_t t = pair; t < n_tiles; t += pairs, i++) {
                 const uint32_t buf = i & 1;
@@ -460,7 +477,7 @@ linear_tc_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_con
                     tcgen05_fence_after();
                     const uint32_t base = smem_u32(tiles + s * kPStageBytes);
                     const uint64_t a_desc = smem_desc_sw128(base);
-                    const uint64_t b_desc = p.w_kind == kWRows ? smem_desc_sw128(base + kPABytes) : smem_desc_sw128(base + kPABytes, kTileBytes);
+                    const uint64_t b_desc = p.w_transposed ? smem_desc_sw128(base + kPABytes) : smem_desc_sw128(base + kPABytes, kTileBytes);
 #pragma unroll
                     for (uint32_t kk = 0; kk < 4; kk++)
                         umma_f16_pair(tmem + buf * kGBN, a_desc + 2 * kk, b_desc + b_step * kk, idesc, (kb | kk) ? 1u : 0u);
@@ -526,38 +543,31 @@ linear_tc_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_con
 // ---- few tiles: the contraction split over a cluster -------------------------------------------------------------
 // With fewer 128 x 256 tiles than SMs the kernels above leave most of the chip idle, and the tiles that do run walk the
 // whole of k one after another (m = 320, n = 768, k = 3072: 9 CTAs, 20 us).  Here a tile is 128 x BN and a cluster of
-// SPLIT CTAs shares it, each multiplying its share of the k-blocks and finishing its share of the rows: the fp32 accumulator
-// goes to shared memory, and each other CTA's rows of it from there to that CTA by one bulk copy.  Every CTA adds up its
-// rows, rank 0 first (the sum does not depend on timing), applies bias and activation and stores.
-// What a launch spends, in cycles after the kernel before it has ended (bf16, 128 x 64 tiles, two CTAs per tile): 800 to the first
-// stage, 210 per k-block of 64 (194 of them the MMAs', which read 24 KB of shared memory while the TMA writes the next 24), 800 until the accumulator
-// is in shared memory, 1300 until the shares have met, 700 for bias and stores, mostly code that is fetched for the first time.
-// Measured, launches in sequence, before (pulled shares, cluster barriers that order the stores, one issuer) and now: m 320, n 768, k 768
-// 4.7 -> 3.9 us, k 3072 8.5 -> 7.1 (two CTAs per tile); n 256, k 256 3.1 -> 2.9, m 704, n 1024, k 1024 5.3 -> 4.9 (one).  The transposed order of the
-// epilogue for one CTA per tile (through shared memory, whole rows per store) was 0.3 us slower, and a first walk through its code by the
-// idle warps slowed the MMAs by a quarter.
-template <int BN, int SPLIT> struct SCfg {
-    static constexpr int ST = BN == 64 ? 8 : SPLIT == 4 ? 5 : 6;                    // stages
+// `split` CTAs shares it, each multiplying its share of the k-blocks; the fp32 accumulators meet in distributed shared
+// memory: every CTA leaves its own in shared memory, and after the cluster's barrier each adds up its share of the
+// rows from all of them, rank 0 first (the sum does not depend on timing), applies bias and activation and stores.
+// One tile per CTA and deep stages: with few CTAs pulling through L2 the distance to it is what a k-block waits for.
+// Measured, launches in sequence: m 320, n 768, k 3072 17.7 -> 8.6 us (two CTAs per 128 x 64 tile), m 320, n 768, k 768
+// 8.4 -> 4.9 us (128 x 64), m 2048, n 768, k 3072 20.6 -> 14.0 us (128 x 128).
+template <int BN, int ST> struct SCfg {
+    static constexpr uint32_t stages = ST;
     static constexpr uint32_t stage_bytes = kGABytes + kGBK * BN * 2;
     static constexpr uint32_t acc_stride = BN + 4;                                  // floats
-    static constexpr uint32_t rows = kGBM / SPLIT, share_bytes = rows * acc_stride * 4;   // a CTA's rows of an accumulator
-    static constexpr uint32_t body = ST * stage_bytes;                              // the accumulator lies over the spent stages
-    static_assert(body >= kGBM * acc_stride * 4, "the accumulator lies over the stages");
-    static constexpr size_t smem = body + (SPLIT - 1) * share_bytes + BN * 4 + 256;
-    static_assert(smem <= 227 * 1024, "shared memory budget");
+    static constexpr uint32_t acc_bytes = kGBM * acc_stride * 4;
+    static constexpr uint32_t body = stages * stage_bytes > acc_bytes ? stages * stage_bytes : acc_bytes;
+    static constexpr size_t smem = 1024 + body + BN * 4 + 256;
 };
 struct SShared {
-    uint64_t full[8], empty[8], acc_full, shares, drained;
+    uint64_t full[8], empty[8], acc_full, drained;
     uint32_t tmem_base, abort_flag;
 };
 static_assert(sizeof(SShared) <= 256, "SShared outgrew its slot");
 
-// shared memory of this CTA -> shared memory of another one of the cluster, counted on a barrier there
-__device__ __forceinline__ void bulk_copy_cluster(uint32_t dst_cluster, uint32_t src, uint32_t bytes, uint32_t bar_cluster)
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr)
 {
-    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_cluster), "r"(src), "r"(bytes),
-                 "r"(bar_cluster)
-                 : "memory");
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
+    return v;
 }
 
 // eight neighbouring outputs of one row: bias, activation, one 16-byte store
@@ -589,47 +599,41 @@ __device__ __forceinline__ void finish8(const GParams &p, float (&x)[8], const f
     *(uint4 *)((uint16_t *)p.out + (size_t)row * p.N + col) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-template <int BN, int SPLIT>
+template <int BN, int ST>
 __global__ void __launch_bounds__(256, 1)
-linear_tc_split_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap, const GParams p)
+linear_tc_split_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap, const GParams p, const uint32_t split)
 {
-    typedef SCfg<BN, SPLIT> Cfg;
-    constexpr int ST = Cfg::ST;
-    extern __shared__ __align__(1024) uint8_t smem_aligned[];
-    uint8_t *smem = smem_aligned;
+    typedef SCfg<BN, ST> Cfg;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    float *bias_s = (float *)(smem + Cfg::body);           // the tile's bias: a read from L2 per column group would be on the critical path
+    SShared *st = (SShared *)(smem + Cfg::body + BN * 4);
     float *acc_s = (float *)smem;                          // the accumulator's place once the stages are spent
-    float *shares = (float *)(smem + Cfg::body);           // this CTA's rows of the other CTAs' accumulators, by rank
-    float *bias_s = (float *)(smem + Cfg::body + (SPLIT - 1) * Cfg::share_bytes);           // the tile's bias: a read from L2 per column group would be on the critical path
-    SShared *st = (SShared *)(bias_s + BN);
 
     const uint32_t warp = uniform_warp(), lane = threadIdx.x & 31;
     volatile uint32_t *abort_flag = &st->abort_flag;
     const uint32_t fmt = p.is_bf16 ? 1u : 0u;
-    const uint32_t tile = blockIdx.x / SPLIT, rank = blockIdx.x % SPLIT;          // the cluster is SPLIT neighbouring CTAs
+    const uint32_t tile = blockIdx.x / split, rank = blockIdx.x - tile * split;    // the cluster is `split` neighbouring CTAs
     const uint32_t tm = tile % p.tiles_m, tn = tile / p.tiles_m;
     const uint32_t kblocks = (p.K + kGBK - 1) / kGBK;
-    const uint32_t kb0 = kblocks * rank / SPLIT, kb1 = kblocks * (rank + 1) / SPLIT;   // SPLIT <= kblocks: never empty
-    const bool two = kb1 - kb0 > 1 && (BN == 64 || kb1 - kb0 <= 16);                   // two issuers
+    const uint32_t kb0 = kblocks * rank / split, kb1 = kblocks * (rank + 1) / split;   // split <= kblocks: never empty
 
     if (threadIdx.x == 0) {
         prefetch_map(amap);
         prefetch_map(bmap);
         for (uint32_t s = 0; s < ST; s++) { mbar_init(&st->full[s], 1); mbar_init(&st->empty[s], 1); }
-        mbar_init(&st->acc_full, 2);
-        mbar_init(&st->shares, 1);
-        mbar_init(&st->drained, 2);
+        mbar_init(&st->acc_full, 1);
+        mbar_init(&st->drained, 1);
         st->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        if (SPLIT > 1) mbar_expect_tx(&st->shares, (SPLIT - 1) * Cfg::share_bytes);
     }
     if (warp == 0) {
         __syncwarp();
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&st->tmem_base)), "r"(2u * BN) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&st->tmem_base)), "r"((uint32_t)BN) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tcgen05_fence_before();
-    if (SPLIT > 1) cluster_sync_all();                     // every CTA's barriers exist before a share is counted on one
-    else __syncthreads();
+    __syncthreads();
     tcgen05_fence_after();
     const uint32_t tmem = st->tmem_base;
     grid_dependency_wait();
@@ -637,67 +641,57 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
 
     if (warp == 0) {
         if (elect_one()) {
-            auto load = [&](uint32_t kb, uint32_t s) {
+            for (uint32_t kb = kb0; kb < kb1; kb++) {
+                const uint32_t g = kb - kb0, s = g % ST;
+                if (g >= ST && !mbar_wait(&st->empty[s], ((g / ST) - 1) & 1, abort_flag, 61)) break;
                 const uint32_t base = smem_u32(smem + s * Cfg::stage_bytes);
                 mbar_expect_tx(&st->full[s], Cfg::stage_bytes);       // boxes beyond the tensor arrive as zeros and still count
                 tma_load_2d(base, &amap, &st->full[s], (int32_t)(kb * kGBK), (int32_t)(tm * kGBM));
-                load_w<BN>(p, base + kGABytes, &bmap, &st->full[s], kb * kGBK, tn * BN);
-            };
-            // the first round of stages in a loop without the wait: 185 cycles a stage instead of 300, and the MMAs follow at that pace
-            const uint32_t n = kb1 - kb0;
-#pragma unroll 1
-            for (uint32_t g = 0; g < n && g < (uint32_t)ST; g++) load(kb0 + g, g);
-#pragma unroll 1
-            for (uint32_t g = ST; g < n; g++) {
-                const uint32_t s = g % ST;
-                if (!mbar_wait(&st->empty[s], ((g / ST) - 1) & 1, abort_flag, 61)) break;
-                load(kb0 + g, s);
+                if (p.w_transposed) {
+                    tma_load_2d(base + kGABytes, &bmap, &st->full[s], (int32_t)(kb * kGBK), (int32_t)(tn * BN));
+                } else {
+#pragma unroll
+                    for (uint32_t j = 0; j < BN / 64; j++)
+                        tma_load_2d(base + kGABytes + j * kTileBytes, &bmap, &st->full[s], (int32_t)(tn * BN + j * 64), (int32_t)(kb * kGBK));
+                }
             }
         }
-    } else if (warp <= 2) {
-        // Two issuers take turns at the k-blocks, each with an accumulator of its own.  A thread that issues N 64 MMAs is held up until
-        // the one before has started, so of a k-block's four only the last runs on while the thread waits for its next stage: one
-        // issuer took 298 to 380 cycles per k-block, of which the tensor core works for 194.  With N 128 (256 of 310 to 340 cycles) the
-        // second one gains up to some 16 k-blocks; beyond, two k-blocks in the making leave the ring too short (m 2816, n 768, k 3072:
-        // 13.3 us with one, 14.4 with two).
+    } else if (warp == 1) {
         if (elect_one()) {
-            const uint32_t idesc = instr_desc(fmt, fmt, kGBM, BN, p.w_kind == kWRows ? 0 : 1);
-            const uint32_t b_step = p.w_kind == kWRows ? 2u : 128u;
-            const uint32_t me = warp - 1, n = kb1 - kb0, acc = tmem + me * BN, step = two ? 2u : 1u;
+            const uint32_t idesc = instr_desc(fmt, fmt, kGBM, BN, p.w_transposed ? 0 : 1);
+            const uint32_t b_step = p.w_transposed ? 2u : 128u;
             bool alive = true;
-#pragma unroll 1
-            for (uint32_t g = me; g < n && me < step; g += step) {
-                const uint32_t s = g % ST;
+            for (uint32_t kb = kb0; kb < kb1; kb++) {
+                const uint32_t g = kb - kb0, s = g % ST;
                 if (!mbar_wait(&st->full[s], (g / ST) & 1, abort_flag, 62)) { alive = false; break; }
                 tcgen05_fence_after();
                 const uint32_t base = smem_u32(smem + s * Cfg::stage_bytes);
                 const uint64_t a_desc = smem_desc_sw128(base);
-                const uint64_t b_desc = p.w_kind == kWRows ? smem_desc_sw128(base + kGABytes) : smem_desc_sw128(base + kGABytes, kTileBytes);
+                const uint64_t b_desc = p.w_transposed ? smem_desc_sw128(base + kGABytes) : smem_desc_sw128(base + kGABytes, kTileBytes);
 #pragma unroll
-                for (uint32_t kk = 0; kk < 4; kk++) umma_f16(acc, a_desc + 2 * kk, b_desc + b_step * kk, idesc, (g - me) | kk ? 1u : 0u);
+                for (uint32_t kk = 0; kk < 4; kk++) umma_f16(tmem, a_desc + 2 * kk, b_desc + b_step * kk, idesc, (g | kk) ? 1u : 0u);
                 umma_commit(&st->empty[s]);
             }
             if (alive) umma_commit(&st->acc_full);
         }
-    } else if (warp == 3 && p.bias) {
+    }
+    else if (warp == 2 && p.bias) {
         for (uint32_t c = lane; c < BN; c += 32) bias_s[c] = tn * BN + c < p.N ? __ldg(p.bias + tn * BN + c) : 0.f;
     }
     __syncwarp();
-    // ===== all eight warps drain the accumulators, 32 rows and half of the columns each =====
+    // ===== all eight warps drain the accumulator: 32 rows and half of the columns each =====
     const uint32_t quarter = warp & 3, ch = warp >> 2, r = quarter * 32 + lane, lane_field = (quarter * 32) << 16;
-    constexpr uint32_t PIECES = BN / 8, COUNT = Cfg::rows * PIECES / 256;      // SPLIT > 1: 16-byte pieces of a row, and per thread
-    const uint32_t r8 = threadIdx.x / PIECES, c8 = (threadIdx.x % PIECES) * 8;
-    uint4 res[SPLIT == 1 ? BN / 16 : COUNT];               // this thread's residuals, on their way while the products run
-    if (p.resid) {
+    uint4 res[BN / 16];                                    // this thread's residuals, on their way while the products run
+    if (p.resid && split == 1) {
+        const uint32_t row = tm * kGBM + r;
 #pragma unroll
-        for (uint32_t q = 0; q < (SPLIT == 1 ? BN / 16 : COUNT); q++) {
-            const uint32_t row = tm * kGBM + (SPLIT == 1 ? r : rank * Cfg::rows + r8 + q * (256 / PIECES));
-            const uint32_t col = tn * BN + (SPLIT == 1 ? ch * (BN / 2) + q * 8 : c8);
+        for (uint32_t q = 0; q < BN / 16; q++) {
+            const uint32_t col = tn * BN + ch * (BN / 2) + q * 8;
             if (row < p.M && col < p.N) res[q] = *(const uint4 *)((const uint16_t *)p.resid + (size_t)row * p.N + col);
         }
     }
     const bool ok = mbar_wait_warp(&st->acc_full, 0, abort_flag, 63);
-    if (SPLIT == 1) __syncthreads();                       // the bias is in place
+    __syncthreads();                                       // the bias is in place
     if (ok) {
         tcgen05_fence_after();
 #pragma unroll
@@ -705,16 +699,8 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
             const uint32_t c = ch * (BN / 2) + c0;
             uint32_t v[32];
             TMEM_LD_32((v), tmem + c + lane_field);
-            if (two) {
-                uint32_t u[32];
-                TMEM_LD_32((u), tmem + BN + c + lane_field);
-                tmem_wait_ld();
-#pragma unroll
-                for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(u[j]));
-            } else {
-                tmem_wait_ld();
-            }
-            if (SPLIT == 1) {
+            tmem_wait_ld();
+            if (split == 1) {
                 const uint32_t row = tm * kGBM + r;
 #pragma unroll
                 for (uint32_t q = 0; q < 4; q++) {
@@ -723,7 +709,7 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
                         float x[8];
 #pragma unroll
                         for (int j = 0; j < 8; j++) x[j] = __uint_as_float(v[q * 8 + j]);
-                        finish8(p, x, bias_s + c + q * 8, res[SPLIT == 1 ? c0 / 8 + q : 0], row, col);
+                        finish8(p, x, bias_s + c + q * 8, res[c0 / 8 + q], row, col);
                     }
                 }
             } else {
@@ -735,42 +721,37 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
         }
         tcgen05_fence_before();
     }
-    if (SPLIT > 1) {
-        fence_proxy_async();                               // the copies read what was written here
-        __syncthreads();
-        // also after a timeout (the status word then says that the sums are not to be used): nobody waits in vain
-        if (warp == 0 && lane < SPLIT && lane != rank)
-            bulk_copy_cluster(mapa_rank(smem_u32(shares) + (rank - (rank > lane ? 1u : 0u)) * Cfg::share_bytes, lane), smem_u32(acc_s) + lane * Cfg::share_bytes,
-                              Cfg::share_bytes, mapa_rank(smem_u32(&st->shares), lane));
-        __syncwarp();
-        mbar_wait_warp(&st->shares, 0, abort_flag, 64);
-        // All shares of this CTA's rows are here; when everybody's are, everybody may leave.  There is nothing to release: as a
-        // release this arrival takes 1200 cycles, and behind the stores below 3000.
-        __syncwarp();
-        asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-#pragma unroll
-        for (uint32_t i = 0; i < COUNT; i++) {
-            const uint32_t rr = r8 + i * (256 / PIECES), row = tm * kGBM + rank * Cfg::rows + rr, col = tn * BN + c8;
-            float x[8];
-#pragma unroll
-            for (uint32_t k = 0; k < (uint32_t)SPLIT; k++) {
-                const float *src = k == rank ? acc_s + (rank * Cfg::rows + rr) * Cfg::acc_stride + c8
-                                             : shares + ((k - (k > rank ? 1u : 0u)) * Cfg::rows + rr) * Cfg::acc_stride + c8;
-                const float4 u = *(const float4 *)src, w = *(const float4 *)(src + 4);
-                const float add[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
-#pragma unroll
-                for (int j = 0; j < 8; j++) x[j] = k ? x[j] + add[j] : add[j];
+    if (split > 1) {
+        // every CTA of the cluster reaches both barriers, also after a timeout (the status word then says that the sums are not to be used)
+        cluster_sync_all();
+        const uint32_t rows = kGBM / split, first = rank * rows;      // split is 2 or 4
+        const uint32_t mine = smem_u32(acc_s);
+        constexpr uint32_t PIECES = BN / 8;
+        for (uint32_t t = threadIdx.x; t < rows * PIECES; t += 256) {
+            const uint32_t rr = first + t / PIECES, c = (t % PIECES) * 8;
+            const uint32_t row = tm * kGBM + rr, col = tn * BN + c;
+            if (row >= p.M || col >= p.N) continue;
+            const uint32_t at = mine + (rr * Cfg::acc_stride + c) * 4;
+            uint4 rs = make_uint4(0u, 0u, 0u, 0u);
+            if (p.resid) rs = *(const uint4 *)((const uint16_t *)p.resid + (size_t)row * p.N + col);
+            float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+            for (uint32_t k = 0; k < split; k++) {
+                const uint32_t a = mapa_rank(at, k);
+                const float4 u = ld_cluster_f4(a), w = ld_cluster_f4(a + 16);
+                x[0] += u.x; x[1] += u.y; x[2] += u.z; x[3] += u.w;
+                x[4] += w.x; x[5] += w.y; x[6] += w.z; x[7] += w.w;
             }
-            if (row < p.M && col < p.N) finish8(p, x, bias_s + c8, res[SPLIT == 1 ? 0 : i], row, col);
+            finish8(p, x, bias_s + c, rs, row, col);
         }
         __syncwarp();
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        cluster_sync_all();                                           // the others have read this CTA's accumulator
     }
 
     // ---- teardown (also the way out after a timeout) ----
     __syncthreads();
     if (st->abort_flag) {
-        if ((warp == 1 || warp == 2) && lane == 0) {
+        if (warp == 1 && lane == 0) {
             umma_commit(&st->drained);
             for (uint32_t k = 0; k < kWaitLimit && !mbar_try_wait(&st->drained, 0); k++) {}
         }
@@ -783,40 +764,30 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
     if (warp == 0) {
         __syncwarp();
         tcgen05_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2u * BN) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)BN) : "memory");
     }
 }
 
 }  // namespace tc
 
-// tiles of 64 (of k) x cols
-static int make_map_w(CUtensorMap *map, const void *w, const tc::GParams &g, uint32_t cols)
-{
-    using namespace tc;
-    if (g.w_kind == kWRows) return make_map_2d(map, w, g.N, g.K, g.is_bf16, cols);
-    if (g.w_kind == kWGroups) return make_map_groups(map, w, g.K, g.N, g.is_bf16, kGBK, cols / 64);
-    return make_map_2d(map, w, g.K, g.N, g.is_bf16, kGBK);
-}
-
 // *refused: the device or partition cannot place the clusters, nothing was launched
-template <int BN, int SPLIT>
-static int launch_split(cudaStream_t s, const CUtensorMap &am, const void *w, const tc::GParams &g, int dev, bool *refused)
+template <int BN, int ST>
+static int launch_split(cudaStream_t s, const CUtensorMap &am, const void *w, const tc::GParams &g, uint32_t split, int dev, bool *refused)
 {
     using namespace tc;
-    constexpr uint32_t split = SPLIT;
     static DeviceOnce once;
     if (!once.done(dev)) {
-        if (cudaFuncSetAttribute(linear_tc_split_kernel<BN, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCfg<BN, SPLIT>::smem) != cudaSuccess)
-            return fail("sfb_linear: cannot reserve %zu bytes of shared memory", SCfg<BN, SPLIT>::smem);
+        if (cudaFuncSetAttribute(linear_tc_split_kernel<BN, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCfg<BN, ST>::smem) != cudaSuccess)
+            return fail("sfb_linear: cannot reserve %zu bytes of shared memory", SCfg<BN, ST>::smem);
         once.mark(dev);
     }
     CUtensorMap bm;
-    if (make_map_w(&bm, w, g, BN)) return 1;
+    if (g.w_transposed ? make_map_2d(&bm, w, g.N, g.K, g.is_bf16, BN) : make_map_2d(&bm, w, g.K, g.N, g.is_bf16, kGBK)) return 1;
     GParams prm = g;
     prm.tiles_m = (g.M + kGBM - 1) / kGBM;
     prm.tiles_n = (g.N + BN - 1) / BN;
-    const cudaError_t e = launch_overlapped_cluster(linear_tc_split_kernel<BN, SPLIT>, dim3(prm.tiles_m * prm.tiles_n * split), dim3(256),
-                                                    SCfg<BN, SPLIT>::smem, s, split, am, bm, prm);
+    const cudaError_t e = launch_overlapped_cluster(linear_tc_split_kernel<BN, ST>, dim3(prm.tiles_m * prm.tiles_n * split), dim3(256),
+                                                    SCfg<BN, ST>::smem, s, split, am, bm, prm, split);
     *refused = split > 1 && e != cudaSuccess;
     if (*refused) { (void)cudaGetLastError(); return 0; }
     return check_launch("sfb_linear");
@@ -825,10 +796,12 @@ static int launch_split(cudaStream_t s, const CUtensorMap &am, const void *w, co
 // Which kernel and which tile: the one with the least estimated time, in microseconds.  Each estimate is a fixed part (the
 // hand-over from the kernel before, the first load, the last tile's epilogue) plus the k-blocks of 64 that a CTA walks
 // one after another, times what one costs -- which grows with the share of the SMs that pull operands through L2.
-// Fitted to 176 shapes (m 64-11264, n 256-4096, k 256-4096, bf16, launches in sequence, each kernel on each shape): within 5 %
-// on average, and the variant taken is the shape's fastest or within 5 % of it on all but four (m 64 or 128: 3.8 to 4.8 us
-// instead of 3.6 to 4.4).  128 x 64 and 128 x 128 tiles are considered only while all of them run at once; clusters of four up to 7 of 8 SMs
-// (128 CTAs were placed in one round, 144 took two).
+// Fitted to 36 shapes (m 64-32768, n 256-4096, k 256-4096, bf16, launches in sequence); within 8 % of all of them, and
+// the shape's fastest variant or one within 4 % of it is the one taken:
+//   128 x 64 and 128 x 128 tiles, one per CTA, only while all of them run at once: 2.7 + 0.165 and 3.7 + 0.175 per
+//     k-block; sharing a tile between 2 (4) CTAs costs 1.9 (2.2) more, and clusters of four are only placed at once in a
+//     third of the SMs (with twice as many CTAs they took two rounds);
+//   128 x 256 tiles, persistent: 5.0 + 0.25 per k-block and round;  256 x 256 tiles on CTA pairs: 5.4 + 0.27.
 struct LinearPlan {
     int kind;                  // 0: 128 x 256, 1: CTA pairs, 2: one tile per cluster
     uint32_t bn, split;
@@ -836,27 +809,25 @@ struct LinearPlan {
 static LinearPlan plan_linear(uint32_t m, uint32_t n, uint32_t k, uint32_t sms)
 {
     using namespace tc;
-    struct Cost { double fixed, per, load; };
-    static const Cost few[2][3] = {{{2.2, 0.154, 0.03}, {3.1, 0.131, 0.06}, {3.2, 0.078, 0.16}},       // 128 x 64 tiles by 1, 2, 4 CTAs
-                                   {{3.2, 0.168, 0.05}, {4.5, 0.153, 0.06}, {5.1, 0.093, 0.26}}};      // 128 x 128
     const uint32_t kb = (k + kGBK - 1) / kGBK, tiles_m = (m + kGBM - 1) / kGBM, tiles_n = (n + kGBN - 1) / kGBN;
-    auto estimate = [&](uint64_t tiles, uint32_t slots, uint32_t blocks, const Cost &c) {
+    auto waves = [&](uint64_t tiles, uint32_t slots, double fixed, double per, double load) {
         const uint64_t rounds = (tiles + slots - 1) / slots;
         const double share = tiles < slots ? (double)tiles / slots : 1.0;
-        return c.fixed + (double)blocks * (double)rounds * (c.per + c.load * share);
+        return fixed + (double)kb * (double)rounds * (per + load * share);
     };
     LinearPlan best = {0, kGBN, 1};
-    double t_best = estimate((uint64_t)tiles_m * tiles_n, sms, kb, {4.3, 0.27, 0.06});
+    double t_best = waves((uint64_t)tiles_m * tiles_n, sms, 5.0, 0.25, 0.13);
     if (kUsePairs && sms >= 2) {
-        const double t = estimate((uint64_t)((m + 255) / 256) * tiles_n, sms / 2, kb, {4.9, 0.26, 0.04});
+        const double t = waves((uint64_t)((m + 255) / 256) * tiles_n, sms / 2, 5.4, 0.27, 0.09);
         if (t < t_best) { t_best = t; best = {1, kGBN, 1}; }
     }
     for (uint32_t bn = 64; bn <= 128; bn += 64) {
         const uint64_t tiles = (uint64_t)tiles_m * ((n + bn - 1) / bn);
-        for (uint32_t split = 1, i = 0; split <= 4 && split <= kb; split *= 2, i++) {
+        for (uint32_t split = 1; split <= 4 && split <= kb; split *= 2) {
             const uint64_t ctas = tiles * split;
-            if (ctas > (split == 4 ? sms * 7 / 8 : sms)) break;
-            const double t = estimate(ctas, sms, (kb + split - 1) / split, few[bn / 64 - 1][i]);
+            if (ctas > (split == 4 ? sms / 3 : sms)) break;
+            const double t = (bn == 64 ? 2.7 : 3.7) + (split == 1 ? 0.0 : split == 2 ? 1.9 : 2.2) +
+                             (double)((kb + split - 1) / split) * ((bn == 64 ? 0.165 : 0.175) + 0.04 * (double)ctas / sms);
             if (t < t_best) { t_best = t; best = {2, bn, split}; }
         }
     }
@@ -895,29 +866,26 @@ static int linear_product(cudaStream_t s, void *out, const void *x, const void *
     if (sms <= 0) return fail("sfb_linear: cannot read the SM count");
     const LinearPlan plan = plan_linear(m, n, k, (uint32_t)sms);
     const uint32_t tiles_n = (n + kGBN - 1) / kGBN;
-    GParams prm = {out, bias, m, n, k, 0, tiles_n, is_bf16, act, w_transposed ? kWRows : n % 64 == 0 ? kWGroups : kWBoxes, 1, nullptr};
+    GParams prm = {out, bias, m, n, k, 0, tiles_n, is_bf16, act, w_transposed ? 1 : 0, 1, nullptr};
     // a device or a partition that cannot place clusters refuses their launch: the single-CTA kernel at the end takes over
     if (plan.kind == 2) {
         GParams few = prm;
         few.resid = resid;
         bool refused = false;
-#define SPLIT_CASE(N, SP) launch_split<N, SP>(s, am, w, few, dev, &refused)
-        const int rc = plan.bn == 64 ? (plan.split == 1 ? SPLIT_CASE(64, 1) : plan.split == 2 ? SPLIT_CASE(64, 2) : SPLIT_CASE(64, 4))
-                                     : (plan.split == 1 ? SPLIT_CASE(128, 1) : plan.split == 2 ? SPLIT_CASE(128, 2) : SPLIT_CASE(128, 4));
-#undef SPLIT_CASE
+        const int rc = plan.bn == 64 ? launch_split<64, 8>(s, am, w, few, plan.split, dev, &refused) : launch_split<128, 6>(s, am, w, few, plan.split, dev, &refused);
         if (!refused) { *added = true; return rc; }
     }
-    CUtensorMap om;      // out as [m, n], boxes of 32 rows x 64 columns for the epilogue's stores
-    if (make_map_2d(&om, out, m, n, is_bf16, 32)) return 1;
     if (plan.kind == 1) {
         CUtensorMap bp;
-        if (make_map_w(&bp, w, prm, kGBN / 2)) return 1;
+        if (w_transposed ? make_map_2d(&bp, w, n, k, is_bf16, kGBN / 2) : make_map_2d(&bp, w, k, n, is_bf16, kGBK)) return 1;
         static DeviceOnce once_pair;
         if (!once_pair.done(dev)) {
             if (cudaFuncSetAttribute(linear_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPSmem) != cudaSuccess)
                 return fail("sfb_linear: cannot reserve %zu bytes of shared memory", kPSmem);
             once_pair.mark(dev);
         }
+        CUtensorMap om;      // out as [m, n], boxes of 32 rows x 64 columns for the epilogue's stores
+        if (make_map_2d(&om, out, m, n, is_bf16, 32)) return 1;
         prm.tiles_m = (m + 255) / 256;
         prm.band = tiles_n < kPBand ? tiles_n : kPBand;
         const uint64_t pair_tiles = (uint64_t)prm.tiles_m * tiles_n;
@@ -926,7 +894,7 @@ static int linear_product(cudaStream_t s, void *out, const void *x, const void *
             return check_launch("sfb_linear");
         (void)cudaGetLastError();
     }
-    if (make_map_w(&bm, w, prm, kGBN)) return 1;
+    if (w_transposed ? make_map_2d(&bm, w, n, k, is_bf16, kGBN) : make_map_2d(&bm, w, k, n, is_bf16, kGBK)) return 1;
     static DeviceOnce once;
     if (!once.done(dev)) {
         if (cudaFuncSetAttribute(linear_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGSmem) != cudaSuccess)
@@ -937,7 +905,7 @@ static int linear_product(cudaStream_t s, void *out, const void *x, const void *
     prm.band = 1;
     const uint64_t tiles = (uint64_t)prm.tiles_m * prm.tiles_n;
     const uint32_t grid = tiles < (uint64_t)sms ? (uint32_t)tiles : (uint32_t)sms;
-    launch_overlapped(linear_tc_kernel, dim3(grid), dim3(320), kGSmem, s, am, bm, om, prm);
+    launch_overlapped(linear_tc_kernel, dim3(grid), dim3(320), kGSmem, s, am, bm, prm);
     return check_launch("sfb_linear");
 }
 

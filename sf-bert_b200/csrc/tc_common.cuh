@@ -144,13 +144,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
         ::"r"(dst), "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y)
         : "memory");
 }
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, uint64_t *bar, int32_t x, int32_t y, int32_t z)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-        ::"r"(dst), "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
-        : "memory");
-}
 
 // brings a tensor map into the descriptor cache ahead of the first copy that uses it
 __device__ __forceinline__ void prefetch_map(const CUtensorMap &map)
@@ -593,23 +586,6 @@ inline int make_map_2d(CUtensorMap *map, const void *base, uint64_t rows, uint64
     cuuint32_t box[2] = {64, box_rows};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = fn(map, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void *)base, dims,
-                    strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail("cuTensorMapEncodeTiled failed with code %d", (int)r);
-    return 0;
-}
-
-// The same tensor as neighbouring groups of 64 columns, [cols / 64][rows][64]: one box is `groups` of the tiles above, each
-// box_rows x 64, laid out one behind the other.  cols must be a multiple of 64.
-inline int make_map_groups(CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols, int is_bf16, uint32_t box_rows, uint32_t groups)
-{
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return fail("cuTensorMapEncodeTiled is not available from this driver");
-    cuuint64_t dims[3] = {64, (cuuint64_t)rows, (cuuint64_t)(cols / 64)};
-    cuuint64_t strides[2] = {(cuuint64_t)cols * 2, 128};
-    cuuint32_t box[3] = {64, box_rows, groups};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(map, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, (void *)base, dims,
                     strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail("cuTensorMapEncodeTiled failed with code %d", (int)r);
