@@ -63,7 +63,8 @@ template <> struct Piece<SFB_F16> {
 
 // Query row i of (batch b, head h) over the elements lo to hi - 1 of colidx: one warp, LPK lanes per key, each owning a share of the head dimension; the key's K and V pieces are all
 // requested before the first is used.  The lanes of a key join their partial scores by shuffles and carry the same running
-// max and sum; the groups' softmaxes are merged at the end.
+// max and sum; the groups' softmaxes are merged at the end.  A score of -inf is a weight of 0, also while nothing else has
+// been met; one of +inf makes the row NaN.
 template <int DT, int D, int LPK>
 __device__ __forceinline__ void csr_row(const int32_t *__restrict__ colidx, int32_t lo, int32_t hi, const void *__restrict__ Q, const void *__restrict__ K,
                                         const void *__restrict__ V, void *__restrict__ O, uint32_t L, uint32_t H, uint32_t b, uint32_t h, uint32_t i,
@@ -81,6 +82,11 @@ __device__ __forceinline__ void csr_row(const int32_t *__restrict__ colidx, int3
         const uint4 *src = (const uint4 *)((const uint8_t *)Q + row_off * ESZ);
 #pragma unroll
         for (int n = 0; n < NP; n++) Piece<DT>::unpack(q + n * Piece<DT>::N, __ldg(src + n));
+    }
+    if (scale_log2e < 0.f) {                         // the largest score is the one that counts, so the sign goes to the query
+        scale_log2e = -scale_log2e;
+#pragma unroll
+        for (int x = 0; x < HD2; x++) q[x] = -q[x];
     }
 #pragma unroll
     for (int x = 0; x < HD2; x++) acc[x] = 0.f;
@@ -126,7 +132,7 @@ __device__ __forceinline__ void csr_row(const int32_t *__restrict__ colidx, int3
                 for (int x = 0; x < HD2; x++) acc[x] *= f;
                 m = sc;
             }
-            const float p = exp2f((sc - m) * scale_log2e);
+            const float p = exp2f((sc - (m > -INFINITY ? m : 0.f)) * scale_log2e);
             l += p;
 #pragma unroll
             for (int n = 0; n < NP; n++) {

@@ -179,3 +179,52 @@ def test_csr_values_that_are_not_finite_stay_in_the_rows_that_have_them(sfb, ora
     keep = ~np.broadcast_to(has[None, :, None], got.shape)
     # two sums in a different order, rounded to the type of the output
     assert np.abs(got - clean)[keep].max() <= (1e-5 if dtype == "f32" else 2.0 ** -7) * np.abs(clean).max()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("what", ["inf", "-inf", "product"])
+@pytest.mark.parametrize("scale", [0.125, -0.125])
+def test_csr_keys_that_are_not_finite(sfb, dtype, d, what, scale):
+    """A score that the scale makes -inf is a probability of 0 wherever in its row the column stands, among the first that a warp
+    takes or behind them; one that it makes +inf gives NaN in the rows that have the column and in no other.
+    what: the key's element, or `product`: finite operands whose product overflows fp32."""
+    if what == "product" and dtype == "f16":
+        pytest.skip("no product of fp16 numbers overflows fp32")
+    L = 160
+    gen = torch.Generator(device="cuda").manual_seed(60 + d)
+    q, k, v = (torch.randn(1, L, 2, d, device="cuda", generator=gen).to(TD[dtype]) for _ in range(3))
+    # rows of 1 to 97 columns, the bad one first, in place i, or last
+    rng = np.random.RandomState(d)
+    bad, rows = 5, []
+    for i in range(L):
+        r = rng.choice(np.delete(np.arange(L), bad), size=i % 97, replace=False)
+        rows.append(np.insert(r, {0: 0, 1: min(i, len(r)), 2: len(r)}[i % 3], bad) if i % 4 else r)
+    rowptr = torch.from_numpy(np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)).cuda()
+    colidx = torch.from_numpy(np.concatenate(rows).astype(np.int32)).cuda()
+    if what == "product":
+        q[..., 3] = -2.0 ** 70
+        k[..., 3] = 0
+        k[0, bad, :, 3] = 2.0 ** 70
+        sign = -1
+    else:
+        q[..., 3] = q[..., 3].abs() + 1
+        k[0, bad, :, 3] = float(what)
+        sign = 1 if what == "inf" else -1
+    has = torch.zeros(L, L, device="cuda")
+    has.index_put_((torch.repeat_interleave(torch.arange(L, device="cuda"), (rowptr[1:] - rowptr[:-1]).long()), colidx.long()), torch.ones((), device="cuda"), accumulate=True)
+    keep = has.clone()
+    keep[:, bad] = 0                                         # what the rows are without it
+    S = torch.einsum("blhd,bmhd->bhlm", q.double(), k.double().nan_to_num(0, 0, 0)) * scale
+    W = torch.softmax(S.masked_fill(keep == 0, -np.inf), -1).nan_to_num(0)
+    want = torch.einsum("bhlm,bmhd->blhd", W, v.double())
+    got = sfb.csr_attention(q, k, v, rowptr, colidx, scale)[0].double()
+    plain = torch.empty_like(q)
+    p = lambda t: sfb.C.c_void_p(t.data_ptr())
+    n = torch.zeros(1, dtype=torch.int32, device="cuda")
+    sfb._check(sfb.lib.sfb_csr_attention(sfb._stream(), p(rowptr), p(colidx), p(q), p(k), p(v), p(plain), sfb.dtype_tag(q), 1, L, 2, d, scale, p(n)))
+    nan = torch.zeros(L, dtype=torch.bool, device="cuda") if sign * scale < 0 else has[:, bad] > 0
+    for o in (got, plain.double()):
+        assert torch.equal(torch.isnan(o), nan[None, :, None, None].expand_as(o))
+        diff = (o - want)[:, ~nan].abs().max()
+        assert diff <= (1e-5 if dtype == "f32" else 2.0 ** -7) * want.abs().max()
