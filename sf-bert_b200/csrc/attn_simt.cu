@@ -36,13 +36,17 @@ __device__ __forceinline__ void load_tile_kmajor(float (*dst)[BS + 1], const voi
 }
 
 // ------------------------------------------------------------------------------------------------
-// A score that is not finite, made again by plain FMAs (simt_tile.cuh says why).
-template <int DT>
-__device__ __noinline__ float dot_again(const void *A, const void *B, size_t a, size_t b, uint32_t d)
+// The scores of a warp's 32x32 tile that are not finite, made again by plain FMAs (simt_tile.cuh says why), in place.  By a warp at a
+// time and not inlined: the tile's registers are free by then.
+template <int BS, int AB_DT, int C_DT>
+__device__ __noinline__ void sddmm_again(float *buf, const void *A, const void *B, void *C, size_t rowA, size_t rowB, size_t at, size_t HD, uint32_t d)
 {
-    float s = 0.f;
-    for (uint32_t k = 0; k < d; k++) s = fmaf(Elem<DT>::load(A, a + k), Elem<DT>::load(B, b + k), s);
-    return s;
+    const uint32_t lane = threadIdx.x & 31;
+    float s[32];
+    tile::scores_again<AB_DT>(s, buf, A, B, rowA, rowB, HD, d, lane);
+#pragma unroll
+    for (int n = 0; n < 32; n++)
+        if (!tile::finite(Elem<C_DT>::load(C, at + lane * BS + n))) Elem<C_DT>::store(C, at + lane * BS + n, s[n]);
 }
 
 // SDDMM.  A CTA (four warps) makes one 64x64 block, a 32x32 quarter per warp, or four consecutive 32x32 blocks of the LUT,
@@ -53,6 +57,7 @@ __device__ __noinline__ float dot_again(const void *A, const void *B, size_t a, 
 template <int BS> struct SddmmCfg {
     static constexpr int TEAMS = BS == 32 ? 4 : 2, TT = 128 / TEAMS;      // teams that stage keys of their own
     static constexpr uint32_t buf = 32 * tile::kStride;
+    static_assert(TEAMS * 2 * buf / 4 >= tile::kAgainFloats, "a warp's share holds the tiles of sddmm_again");
 };
 template <int BS, int AB_DT, int C_DT>
 __global__ void __launch_bounds__(tile::kThreads, 3) sddmm_nt_kernel(const uint2 *__restrict__ lut, const void *__restrict__ A,
@@ -117,14 +122,7 @@ __global__ void __launch_bounds__(tile::kThreads, 3) sddmm_nt_kernel(const uint2
         }
         if (c + 1 < chunks) stage_end(held_b, rank, bufs + ((c + 1) & 1) * Cfg::buf, kStride, vec);
     }
-    if (T > 1 && !(zero_if_finite<4>(acc[1], zero_if_finite<4>(acc[0], 0.f)) == 0.f)) {
-#pragma unroll
-        for (int x = 0; x < 32; x++) {
-            float &v = acc[x >> 4][(x >> 2) & 3][x & 3];
-            if (!finite(v))
-                v = dot_again<AB_DT>(A, Bm, rowA + (16 * (x >> 4) + 8 * ((x >> 1) & 1) + g) * HD, rowB + score_key<true>(t, (x >> 2) & 3, x & 1) * HD, p.d);
-        }
-    }
+    const bool odd = T > 1 && !(zero_if_finite<4>(acc[1], zero_if_finite<4>(acc[0], 0.f)) == 0.f);
     const size_t baseC = (((size_t)b * p.H + h) * p.blocks + bid) * BS * BS + (size_t)r0 * BS + c0;
 #pragma unroll
     for (int m = 0; m < 2; m++)
@@ -155,6 +153,9 @@ __global__ void __launch_bounds__(tile::kThreads, 3) sddmm_nt_kernel(const uint2
                 for (int k = 0; k < 8; k++) Elem<C_DT>::store(C, at + k, v[k]);
             }
         }
+    // on the team's shared memory, when its other warp is past the products too
+    if (T > 1 && (BS == 64 ? __syncthreads_or(odd) : __any_sync(0xffffffffu, odd)) && __any_sync(0xffffffffu, odd))
+        sddmm_again<BS, AB_DT, C_DT>(sm + warp * (Cfg::TEAMS * 2 * Cfg::buf / 4), A, Bm, C, rowA, rowB, baseC, HD, p.d);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -521,16 +522,28 @@ __global__ void __launch_bounds__(BS * BS / 8 / SPLIT) softmax_grad_kernel(const
 }
 
 // ------------------------------------------------------------------------------------------------
-// An output that is not finite, made again by plain FMAs.  pbase: first block of the (batch, head); vbase: this column in its first row.
-template <int BS, int A_DT, int BC_DT, bool TRANS>
-__device__ __noinline__ float spmm_again(const uint2 *ent, uint32_t cnt, const void *Pm, const void *V, size_t pbase, size_t vbase, size_t HD, uint32_t r)
+// The same for 32 rows x NC columns of the SpMM below.  pbase: first block of the (batch, head); vbase, at: the first column in the first rows of V and
+// of the warp's outputs.
+template <int BS, int A_DT, int BC_DT, bool TRANS, int NC>
+__device__ __noinline__ void spmm_again(float *buf, const uint2 *ent, uint32_t cnt, const void *Pm, const void *V, void *O, size_t pbase, size_t vbase, size_t at, size_t HD,
+                                        uint32_t r0, uint32_t ncols)
 {
-    float s = 0.f;
+    using namespace tile;
+    const uint32_t lane = threadIdx.x & 31;
+    float acc[NC] = {};
     for (uint32_t e = 0; e < cnt; e++)
-        for (uint32_t k = 0; k < BS; k++)
-            s = fmaf(Elem<A_DT>::load(Pm, pbase + ((size_t)ent[e].x * BS + (TRANS ? k : r)) * BS + (TRANS ? r : k)),
-                     Elem<BC_DT>::load(V, vbase + ((size_t)ent[e].y * BS + k) * HD), s);
-    return s;
+        for (uint32_t k = 0; k < BS; k += kAgain) {
+            const size_t pb = pbase + (size_t)ent[e].x * BS * BS;
+            __syncwarp();
+            if (TRANS) copy_again<A_DT, kAgain, 32, kAgainRows, 1>(buf, Pm, pb + (size_t)k * BS + r0, BS, 32, lane);
+            else copy_again<A_DT, 32, kAgain, 1, kAgainRows>(buf, Pm, pb + (size_t)r0 * BS + k, BS, kAgain, lane);
+            copy_again<BC_DT, kAgain, NC, kAgainCols<NC>, 1>(buf + kAgain * kAgainRows, V, vbase + ((size_t)ent[e].y * BS + k) * HD, HD, ncols, lane);
+            __syncwarp();
+            fma_again<NC>(acc, buf, buf + kAgain * kAgainRows, lane);
+        }
+#pragma unroll
+    for (int n = 0; n < NC; n++)
+        if ((uint32_t)n < ncols && !finite(Elem<BC_DT>::load(O, at + lane * HD + n))) Elem<BC_DT>::store(O, at + lane * HD + n, acc[n]);
 }
 
 // SpMM: one CTA per (block-row, slice of up to 128 of d).  TRANS = false: O = sum over the row's blocks of P . V (NN, the
@@ -545,6 +558,8 @@ template <int BS, int DS> struct SpmmCfg {
     static constexpr int WC = BS == 32 ? 4 : 2;                          // warps side by side along d: each is a team with the ones below it
     static constexpr int TT = 128 / WC, NW = DS / WC, N = NW / 8;        // a team's threads and columns, n-tiles of 8 columns
     static constexpr uint32_t v_stride = NW + 8, buf = 32 * v_stride;
+    static constexpr int NC = NW < 32 ? NW : 32;                         // columns that spmm_again takes at a time
+    static_assert(WC * 3 * buf / 4 >= tile::kAgain * (tile::kAgainRows + tile::kAgainCols<NC>), "a warp's share holds the tiles of spmm_again");
 };
 template <int BS, int DS, int A_DT, int BC_DT, bool TRANS>
 __global__ void __launch_bounds__(tile::kThreads, (BS == 64 && DS == 128) || A_DT == SFB_F32 ? 3 : 4)
@@ -647,16 +662,7 @@ spmm_nn_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Pm, const
     }
     // rows without blocks are written as zeros (blocksparse.h:949-962)
     const size_t baseO = ((size_t)b * p.nb_a + i) * BS * HD + (size_t)h * p.d + n0;
-    if ((TP > 1 || TV > 1) && !(zero_if_finite<N>(acc[1], zero_if_finite<N>(acc[0], 0.f)) == 0.f)) {
-#pragma unroll
-        for (int x = 0; x < 8 * N; x++) {
-            float &o = acc[x / (4 * N)][(x >> 2) % N][x & 3];
-            const uint32_t r = r0 + (TRANS ? 4 * g + 2 * (x / (4 * N)) + ((x >> 1) & 1) : 16 * (x / (4 * N)) + 8 * ((x >> 1) & 1) + g);
-            const uint32_t col = out_col<N>(t, (x >> 2) % N, x & 1);
-            if (!finite(o) && col < left)
-                o = spmm_again<BS, A_DT, BC_DT, TRANS>(nn + head.x, head.y, Pm, V, bh * p.blocks * BS * BS, (size_t)b * p.nb_b * BS * HD + (size_t)h * p.d + n0 + col, HD, r);
-        }
-    }
+    const bool odd = (TP > 1 || TV > 1) && !(zero_if_finite<N>(acc[1], zero_if_finite<N>(acc[0], 0.f)) == 0.f);
 #pragma unroll
     for (int m = 0; m < 2; m++)
 #pragma unroll
@@ -664,6 +670,13 @@ spmm_nn_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Pm, const
             const uint32_t r = r0 + (TRANS ? 4 * g + 2 * m + half : 16 * m + 8 * half + g);
             store_cols<BC_DT, N>(O, baseO + (size_t)r * HD, t, acc[m], half, 1.f, left, vec);
         }
+    // on the team's shared memory, when its other warp is past the products too
+    if ((TP > 1 || TV > 1) && (BS == 64 ? __syncthreads_or(odd) : __any_sync(0xffffffffu, odd)) && __any_sync(0xffffffffu, odd)) {
+        cp_wait<0>();
+        for (uint32_t c = 0; c < Cfg::NW && c < left; c += Cfg::NC)
+            spmm_again<BS, A_DT, BC_DT, TRANS, Cfg::NC>(sm + warp * (Cfg::WC * 3 * Cfg::buf / 4), nn + head.x, head.y, Pm, V, O, bh * p.blocks * BS * BS,
+                                                        (size_t)b * p.nb_b * BS * HD + (size_t)h * p.d + n0 + c, baseO + (size_t)r0 * HD + c, HD, r0, left - c);
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -791,37 +804,77 @@ __global__ void __launch_bounds__(256) fused_sddmm_softmax_kernel(const uint2 *_
     }
 }
 
-// A query row whose output is not finite, made again by one warp with plain FMAs (simt_tile.cuh says why): a key per lane for the
-// scores, a share of the columns per lane for the output.  mask: this row's word of block 0.
-template <int BS, int DT>
-__device__ __noinline__ void attention_row_again(const uint2 *ent, uint32_t cnt, const void *Q, const void *K, const void *V, void *O,
-                                                 const typename MaskWord<BS>::type *mask, size_t qrow, size_t kv, size_t orow, size_t HD, uint32_t d, float scale_log2e)
+// The rows of a block-row whose outputs are not finite, made again by plain FMAs (simt_tile.cuh says why): the steps of the kernel
+// below, by the same warps, on its shared memory, where the rows' flags come first.  q0, o0: first elements of the block-row; kv: of the keys and values;
+// mask: this head's.
+template <int BS, int NW> struct AgainCfg {
+    static constexpr uint32_t red = BS, ps = red + 128, stage = ps + 128 * tile::kAgainRows;      // floats
+    static constexpr uint32_t warp_floats = tile::kAgainFloats > tile::kAgain * tile::kAgainCols<NW> ? tile::kAgainFloats : tile::kAgain * tile::kAgainCols<NW>;
+    static constexpr size_t bytes = 4 * (stage + 4 * warp_floats);
+};
+template <int BS, int DT, int NW>
+__device__ __noinline__ void attention_again(float *sm, const uint2 *ent, uint32_t cnt, const void *Q, const void *K, const void *V, void *O,
+                                             const typename MaskWord<BS>::type *mask, size_t q0, size_t kv, size_t o0, size_t HD, size_t HDo, uint32_t d, float scale_log2e)
 {
-    const uint32_t lane = threadIdx.x & 31;
-    float m = -INFINITY, l = 0.f, acc[4] = {};
-    for (uint32_t e = 0; e < cnt; e++)
-        for (uint32_t part = 0; part < BS; part += 32) {
-            const size_t rows = kv + ((size_t)ent[e].y * BS + part) * HD;
-            float s = 0.f;
-            for (uint32_t k = 0; k < d; k++) s = fmaf(Elem<DT>::load(Q, qrow + k), Elem<DT>::load(K, rows + lane * HD + k), s);
-            s = !mask || ((mask[(size_t)ent[e].x * BS] >> (part + lane)) & 1u) ? s * scale_log2e : -INFINITY;
-            const float mn = fmaxf(m, warp_max(s)), alpha = mn > m ? exp2f(m - mn) : 1.f;
-            const float pv = exp2f(s - (mn > -INFINITY ? mn : 0.f));
-            m = mn;
-            l = fmaf(l, alpha, warp_sum(pv));
+    using namespace tile;
+    typedef typename MaskWord<BS>::type W;
+    typedef AgainCfg<BS, NW> Cfg;
+    constexpr uint32_t G = BS == 32 ? 4 : 1, WC = BS == 32 ? 4 : 2;      // key blocks per step, warps per row
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wc = warp % WC, rg = warp / WC, r = 32 * rg + lane;
+    const uint32_t n0 = wc * NW, left = d > n0 ? d - n0 : 0;
+    float *red = sm + Cfg::red, *ps = sm + Cfg::ps + rg * 64 * kAgainRows, *buf = sm + Cfg::stage + warp * Cfg::warp_floats;
+    float m = -INFINITY, l = 0.f, acc[NW] = {};
+    for (uint32_t e = 0; e < cnt; e += G) {
+        const uint32_t nblk = min(G, cnt - e);
+        float s[32];
+        if (G == 1 || wc < nblk) {
+            const uint2 en = ent[e + (G == 1 ? 0 : wc)];
+            scores_again<DT>(s, buf, Q, K, q0 + (size_t)(32 * rg) * HD, kv + ((size_t)en.y * BS + (G == 1 ? 32 * wc : 0)) * HD, HD, d, lane);
+            const W w = mask ? mask[(size_t)en.x * BS + r] : ~(W)0;
 #pragma unroll
-            for (int c = 0; c < 4; c++) acc[c] *= alpha;
-            for (uint32_t k = 0; k < 32; k++) {
-                const float pk = __shfl_sync(0xffffffffu, pv, k);
+            for (int n = 0; n < 32; n++) s[n] = (w >> (n + (G == 1 ? 32 * wc : 0))) & 1u ? s[n] * scale_log2e : -INFINITY;
+        } else {
 #pragma unroll
-                for (int c = 0; c < 4; c++)
-                    if (lane + 32 * c < d) acc[c] = fmaf(pk, Elem<DT>::load(V, rows + k * HD + lane + 32 * c), acc[c]);
-            }
+            for (int n = 0; n < 32; n++) s[n] = -INFINITY;
         }
+        float mn = s[0];
+#pragma unroll
+        for (int n = 1; n < 32; n++) mn = fmaxf(mn, s[n]);
+        red[warp * 32 + lane] = mn;
+        __syncthreads();
+        mn = m;
+#pragma unroll
+        for (uint32_t k = 0; k < WC; k++) mn = fmaxf(mn, red[(rg * WC + k) * 32 + lane]);
+        const float alpha = mn > m ? exp2f(m - mn) : 1.f, off = mn > -INFINITY ? mn : 0.f;
+        m = mn;
+        l *= alpha;
+#pragma unroll
+        for (int n = 0; n < 32; n++) {
+            const float pv = exp2f(s[n] - off);
+            l += pv;
+            ps[(32 * wc + n) * kAgainRows + lane] = pv;
+        }
+#pragma unroll
+        for (int n = 0; n < NW; n++) acc[n] *= alpha;
+        __syncthreads();
+        for (uint32_t k = 0; left && k < nblk * BS; k += kAgain) {
+            __syncwarp();
+            copy_again<DT, kAgain, NW, kAgainCols<NW>, 1>(buf, V, kv + ((size_t)ent[e + k / BS].y * BS + k % BS) * HD + n0, HD, left, lane);
+            __syncwarp();
+            fma_again<NW>(acc, ps + k * kAgainRows, buf, lane);
+        }
+    }
+    __syncthreads();
+    red[warp * 32 + lane] = l;
+    __syncthreads();
+    if (!((const uint32_t *)sm)[r]) return;
+    l = 0.f;
+#pragma unroll
+    for (uint32_t k = 0; k < WC; k++) l += red[(rg * WC + k) * 32 + lane];
     const float inv = l > 0.f ? 1.f / l : l;                             // nothing kept: 0; NaN stays NaN
 #pragma unroll
-    for (int c = 0; c < 4; c++)
-        if (lane + 32 * c < d) Elem<DT>::store(O, orow + lane + 32 * c, acc[c] * inv);
+    for (int n = 0; n < NW; n++)
+        if ((uint32_t)n < left) Elem<DT>::store(O, o0 + (size_t)r * HDo + n0 + n, acc[n] * inv);
 }
 
 // This warp's 32 x 32 probabilities as the A fragments of their product with the values: two of 16 keys per 16 rows (pitch: from
@@ -1082,17 +1135,15 @@ fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q
     }
     if (!__syncthreads_or(odd != 0)) return;
     // such rows are made again by plain FMAs, once every warp has written its columns of them
-    uint32_t *again = (uint32_t *)Pf;
-    for (uint32_t r = threadIdx.x; r < BS; r += kThreads) again[r] = 0;
+    uint32_t *again = (uint32_t *)sm;
+    if (threadIdx.x < BS) again[threadIdx.x] = 0;
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < 4; q++)
         if ((odd >> q) & 1u) again[r0 + g + 8 * q] = 1;
     __syncthreads();
-    for (uint32_t r = warp; r < BS; r += kThreads / 32)
-        if (again[r])
-            attention_row_again<BS, DT>(nn + head.x, cnt, Q, K, V, O, mh ? mh + r : nullptr, (((size_t)b * p.nb_a + i) * BS + r) * HD + (size_t)h * p.d,
-                                        (size_t)b * p.nb_b * BS * HD + (size_t)h * p.d, baseO + (size_t)r * HDo, HD, p.d, scale_log2e);
+    static_assert(Cfg::bytes >= AgainCfg<BS, Cfg::NW>::bytes, "attention_again works in the kernel's shared memory");
+    attention_again<BS, DT, Cfg::NW>(sm, nn + head.x, cnt, Q, K, V, O, mh, ((size_t)b * p.nb_a + i) * BS * HD + (size_t)h * p.d, kv, baseO, HD, HDo, p.d, scale_log2e);
 }
 
 // ------------------------------------------------------------------------------------------------

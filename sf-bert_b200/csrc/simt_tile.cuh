@@ -17,8 +17,8 @@
 // several warps use is split once: the queries when they arrive, the probabilities where they are made, both kept
 // in shared memory as fragments.
 //
-// What is not finite.  inf splits into inf and inf - inf, so products with it come out as NaN; callers make every
-// result that is not finite again with plain FMAs.
+// What is not finite.  inf splits into inf and inf - inf, so products with it come out as NaN, as do those with a finite number
+// that rounds to a bf16 infinity; callers make every result that is not finite again with plain FMAs, a tile at a time (fma_again below).
 //
 // Keys and values travel by cp.async through rings of chunks, and only as far as the warps that use them: a team (one warp, or
 // the two that share columns) stages its own keys and its own columns of the values, and waits for nobody else.
@@ -344,6 +344,53 @@ __device__ __forceinline__ float zero_if_finite(const float (*v)[4], float z)
     return z;
 }
 __device__ __forceinline__ bool finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+
+// ---- results that are not finite, made again by plain FMAs: a warp's 32 rows, one per lane, times N columns, kAgain elements of the
+// contraction at a time from shared memory (the rows' elements at a, the columns' at b, both with the contraction outermost: a lane's own
+// element is one conflict-free load, four columns are one broadcast)
+constexpr uint32_t kAgain = 16, kAgainRows = 33;
+template <int N> constexpr uint32_t kAgainCols = N + 4;
+constexpr uint32_t kAgainFloats = kAgain * (kAgainRows + kAgainCols<32>);
+// element (r, c) = src[at + r * pitch + c] -> dst[r * ROW + c * COL], by one warp; columns from ncols on are zeros
+template <int DT, int ROWS, int COLS, int ROW, int COL>
+__device__ __forceinline__ void copy_again(float *dst, const void *src, size_t at, size_t pitch, uint32_t ncols, uint32_t lane)
+{
+#pragma unroll 8
+    for (uint32_t x = lane; x < ROWS * COLS; x += 32) {
+        const uint32_t r = x / COLS, c = x % COLS;
+        dst[r * ROW + c * COL] = c < ncols ? Elem<DT>::load(src, at + r * pitch + c) : 0.f;
+    }
+}
+template <int N>
+__device__ __forceinline__ void fma_again(float (&acc)[N], const float *a, const float *b, uint32_t lane)
+{
+#pragma unroll 4
+    for (uint32_t k = 0; k < kAgain; k++) {
+        const float x = a[k * kAgainRows + lane];
+#pragma unroll
+        for (int n = 0; n < N; n += 4) {
+            const float4 v = *(const float4 *)(b + k * kAgainCols<N> + n);
+            acc[n] = fmaf(x, v.x, acc[n]);
+            acc[n + 1] = fmaf(x, v.y, acc[n + 1]);
+            acc[n + 2] = fmaf(x, v.z, acc[n + 2]);
+            acc[n + 3] = fmaf(x, v.w, acc[n + 3]);
+        }
+    }
+}
+// scores of the rows at rowA, rowA + HD, ... and the keys at rowB, rowB + HD, ... (element offsets), d elements
+template <int DT>
+__device__ __forceinline__ void scores_again(float (&s)[32], float *buf, const void *A, const void *B, size_t rowA, size_t rowB, size_t HD, uint32_t d, uint32_t lane)
+{
+#pragma unroll
+    for (int n = 0; n < 32; n++) s[n] = 0.f;
+    for (uint32_t k = 0; k < d; k += kAgain) {
+        __syncwarp();
+        copy_again<DT, 32, kAgain, 1, kAgainRows>(buf, A, rowA + k, HD, d - k, lane);
+        copy_again<DT, 32, kAgain, 1, kAgainCols<32>>(buf + kAgain * kAgainRows, B, rowB + k, HD, d - k, lane);
+        __syncwarp();
+        fma_again<32>(s, buf, buf + kAgain * kAgainRows, lane);
+    }
+}
 
 // the column of accumulator n of a row, e = 0 or 1
 template <int N> __device__ __forceinline__ uint32_t out_col(uint32_t t, int n, int e)

@@ -138,3 +138,74 @@ def test_a_row_of_scores_that_are_not_numbers_is_not_a_row_of_zeros(sfb):
     q[0, 7, 0, 0] = math.nan
     o = sfb.fused_attention(q, k, v, lay, 0.1)
     assert torch.isnan(o[0, 7]).all() and torch.isfinite(o[0, :7]).all() and torch.isfinite(o[0, 8:]).all()
+
+
+def _us(f):
+    times = []
+    for _ in range(7):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        f()
+        a.record()
+        for _ in range(5):
+            f()
+        b.record()
+        torch.cuda.synchronize()
+        times.append(a.elapsed_time(b))
+    return min(times)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+@pytest.mark.parametrize("bs,d", [(32, 128), (32, 64), (64, 128)])
+def test_what_is_not_finite_does_not_set_the_time(sfb, bs, d, dtype):
+    """An overflowed gradient or an infinite key must not make a call much longer: every result, or every row, is made again, and the
+    call takes at most five times what it takes on finite operands."""
+    lay = sfb.BlockLayout.generate(sfb.LAYOUT_SAWTOOTH, 1, 1024 // bs, bs, p0=8)
+    lay.tn_lut
+    g = torch.Generator(device="cuda").manual_seed(6)
+    q, k, v = (torch.randn(8, 1024, 4, d, device="cuda", generator=g).to(TD[dtype]) for _ in range(3))
+    p = torch.rand(8, 4, lay.blocks, bs, bs, device="cuda", generator=g).to(torch.bfloat16 if dtype == "f32" else TD[dtype])
+    bad, key = torch.full_like(v, math.nan), k.clone()
+    key[:, ::64, :, 3] = math.inf                            # in every row of blocks
+    scale = 1 / math.sqrt(d)
+    assert _us(lambda: sfb.bst_sgemm_nt(q, bad, lay, torch.float32)) <= 5 * _us(lambda: sfb.bst_sgemm_nt(q, k, lay, torch.float32))
+    assert _us(lambda: sfb.bst_sgemm_xn(p, bad, lay)) <= 5 * _us(lambda: sfb.bst_sgemm_xn(p, v, lay))
+    assert _us(lambda: sfb.bst_sgemm_tn(p, bad, lay)) <= 5 * _us(lambda: sfb.bst_sgemm_tn(p, v, lay))
+    assert _us(lambda: sfb.fused_attention(q, key, v, lay, scale)) <= 5 * _us(lambda: sfb.fused_attention(q, k, v, lay, scale))
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+@pytest.mark.parametrize("bs,d", [(32, 128), (32, 64), (32, 32), (32, 30), (64, 128), (64, 72), (64, 32)])
+def test_rows_made_again(sfb, bs, d, dtype):
+    """Infinities in several places of the keys and of the values, rows of 1 to 9 blocks with and without a mask, widths that are no
+    multiple of a unit: what is not finite is what fp32 arithmetic gives, and what meets no infinity is bit for bit what it is without."""
+    nb = 9
+    lay, keep = _layout(sfb, nb, bs, d)
+    lay.pack_mask(sfb.MASK_CAUSAL_DIAG)
+    g = torch.Generator(device="cuda").manual_seed(7)
+    q, k, v = (torch.randn(2, nb * bs, 3, d, device="cuda", generator=g).to(TD[dtype]) for _ in range(3))
+    q, v = (x.where(x.abs() > 1e-2, torch.ones_like(x)) for x in (q, v))
+    full = torch.from_numpy(np.kron(keep, np.ones((bs, bs), bool))).cuda()
+    scale = 1 / math.sqrt(d)
+    bad = k.clone()
+    for j in range(nb):
+        bad[:, j * bs + 3 * j + 1, :, (5 * j) % d] = math.inf if j % 2 else -math.inf
+    S = torch.einsum("blhd,bmhd->bhlm", q.double(), bad.double())        # one infinity per key: no inf - inf
+    assert not torch.isnan(S).any()
+    _same(sfb.bst_sgemm_nt(q, bad, lay, torch.float32), _blocks(keep, bs, S.float()), 1e-4)
+    inside = torch.ones(nb * bs, nb * bs, dtype=torch.bool, device="cuda")
+    for i in range(nb):
+        inside[i * bs:(i + 1) * bs, i * bs:(i + 1) * bs] = torch.ones(bs, bs, device="cuda").tril().bool()
+    for use_mask in (False, True):
+        W = torch.softmax((S * scale).masked_fill(~(full & inside if use_mask else full), -math.inf), -1)
+        want = torch.einsum("bhlm,bmhd->blhd", W, v.double()).float()
+        _same(sfb.fused_attention(q, bad, v, lay, scale, use_mask=use_mask).float(), want, 1e-5 if dtype == "f32" else 2.0 ** -9)
+    p = torch.rand(2, 3, lay.blocks, bs, bs, device="cuda", generator=g).clamp_min(1e-2).to(torch.bfloat16 if dtype == "f32" else TD[dtype])
+    badv, hit = v.clone(), torch.zeros(nb * bs, d, dtype=torch.float64, device="cuda")
+    for j in range(0, nb, 2):
+        badv[:, j * bs + 2 * j, :, (7 * j) % d] = math.inf
+        hit[j * bs + 2 * j, (7 * j) % d] = 1
+    for rows, f in ((full, sfb.bst_sgemm_xn), (full.T, sfb.bst_sgemm_tn)):
+        got, clean = (f(p, x, lay).permute(0, 2, 1, 3) for x in (badv, v))
+        met = rows.double() @ hit > 0
+        assert (got[:, :, met] == math.inf).all()
+        assert torch.equal(got[:, :, ~met], clean[:, :, ~met])
