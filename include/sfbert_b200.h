@@ -187,8 +187,9 @@ int sfb_fused_sddmm_softmax(sfb_stream_t stream, const void *nn_lut, const void 
                             uint32_t mask_heads, float scale);
 
 /* SDDMM + softmax + SpMM in one launch: O = softmax(scale * Q K^T on the kept blocks) V with S
- * and P never leaving the chip.  dtype is the type of q, k, v and o.  Replaces fusion_attention
- * (fusion_blocksparse.h:2990-3050), whose kernel the reference left unfinished. */
+ * and P never leaving the chip.  dtype is the type of q, k, v and o.  A score of -inf is a probability of 0 (a row that has no
+ * other is zeros); with fp32 operands, and 16-bit ones whose blocks or heads are not 64 wide, a score of +inf or NaN gives a row
+ * of NaN.  Replaces fusion_attention (fusion_blocksparse.h:2990-3050), whose kernel the reference left unfinished. */
 int sfb_fused_attention(sfb_stream_t stream, const void *nn_lut, const void *q, const void *k,
                         const void *v, void *o, const void *mask, int dtype,
                         uint32_t block_size, uint32_t blocks, uint32_t batch_dim,
