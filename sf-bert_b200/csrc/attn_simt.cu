@@ -1081,7 +1081,7 @@ fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q
             float mn = mx[q];
 #pragma unroll
             for (uint32_t k = 0; k < WC; k++) mn = fmaxf(mn, red[k * BS + r]);
-            const float alpha = mn > mx[q] ? ex2_fast(mx[q] - mn) : 1.f;
+            const float alpha = mn > mx[q] ? exp2f(mx[q] - mn) : 1.f;
             mx[q] = mn;
             const float off = mn > -INFINITY ? mn : 0.f;                 // nothing kept so far: exp2(-inf) = 0, and NaN stays NaN
             float ps = 0.f;
@@ -1090,7 +1090,7 @@ fused_attention_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Q
 #pragma unroll
                 for (int k = 0; k < 2; k++) {
                     float &v = s[q >> 1][j][2 * (q & 1) + k];
-                    v = ex2_fast(v - off);
+                    v = exp2f(v - off);                              // not ex2_fast: that flushes weights below 2^-126 of the largest
                     ps += v;
                 }
             sum[q] = fmaf(sum[q], alpha, ps);                            // this thread's columns only; the shares meet at the end
@@ -1287,14 +1287,14 @@ __global__ void __launch_bounds__(tile::kThreads, CsrF32Cfg<D>::ctas) csr_tile_f
             float mn = mx[q];
 #pragma unroll
             for (uint32_t k = 0; k < 4; k++) mn = fmaxf(mn, red[k * 32 + r]);
-            const float alpha = mn > mx[q] ? ex2_fast(mx[q] - mn) : 1.f;
+            const float alpha = mn > mx[q] ? exp2f(mx[q] - mn) : 1.f;
             mx[q] = mn;
             const float off = mn > -INFINITY ? mn : 0.f;                 // nothing kept so far: exp2(-inf) = 0, and NaN stays NaN
             float ps = 0.f;
 #pragma unroll
             for (int j = 0; j < 8; j++) {
                 float &v = s[q >> 1][j >> 1][2 * (q & 1) + (j & 1)];
-                v = ex2_fast(v - off);
+                v = exp2f(v - off);                              // not ex2_fast: that flushes weights below 2^-126 of the largest
                 ps += v;
             }
             sum[q] = fmaf(sum[q], alpha, ps);                            // this thread's columns only; the shares meet at the end

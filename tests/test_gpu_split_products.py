@@ -209,3 +209,26 @@ def test_rows_made_again(sfb, bs, d, dtype):
         met = rows.double() @ hit > 0
         assert (got[:, :, met] == math.inf).all()
         assert torch.equal(got[:, :, ~met], clean[:, :, ~met])
+
+
+@pytest.mark.parametrize("bs,d", [(32, 128), (32, 64), (64, 64)])
+@pytest.mark.parametrize("below", [100, 126, 127, 130, 132])
+def test_weights_that_are_subnormal(sfb, bs, d, below):
+    """A key whose weight is 2^-below of the row's largest, with the only values of its columns: subnormal weights count, as far as the
+    terms of a product do (multiples of 2^-133)."""
+    L = 4 * bs
+    lay = sfb.BlockLayout.generate(sfb.LAYOUT_FULL, 1, 4, bs)
+    q, k, v = (torch.zeros(1, L, 1, d, device="cuda") for _ in range(3))
+    q[..., 0] = 1
+    k[:, :, 0, 0] = -1000                                    # weights of 0
+    k[:, 5, 0, 0] = 0
+    k[:, L - 3, 0, 0] = -below
+    v[:, L - 3, 0, : d // 2] = 2.0 ** 100
+    v[:, 5, 0, d // 2:] = 1
+    want = torch.cat([torch.full((d // 2,), 2.0 ** (100 - below)), torch.ones(d - d // 2)]).cuda()
+    # score * scale is off by 2^-24 of itself, twice (the scale in units of log2), and ex2 by 2^-22
+    tol = 2 * below * EPS + 2.0 ** -21
+    rowptr, colidx = sfb.csr_from_layout(lay)
+    for o in (sfb.fused_attention(q, k, v, lay, math.log(2)), sfb.csr_attention(q, k, v, rowptr, colidx, math.log(2))[0] * (1 + 1e-6)):
+        assert ((o[0, :, 0] - want).abs() <= tol * want + (2.0 ** (100 - 134) if below > 109 else 0) * (want < 1)).all()
+        assert (o[0, :, 0] > 0).all()
