@@ -228,3 +228,38 @@ def test_csr_keys_that_are_not_finite(sfb, dtype, d, what, scale):
         assert torch.equal(torch.isnan(o), nan[None, :, None, None].expand_as(o))
         diff = (o - want)[:, ~nan].abs().max()
         assert diff <= (1e-5 if dtype == "f32" else 2.0 ** -7) * want.abs().max()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("L", [545, 1024])
+def test_csr_scores_that_rise_and_fall(sfb, dtype, d, L):
+    """The reference maximum of a row moves only when a score outgrows it by 2^8 (16-bit tiles): scores that rise or fall along the row by
+    little, by a little less and a little more than 8 (log2) from one of a warp's chunks to its next, and by far more, row by row
+    in the same tile, so that some rows of a tile rescale where others must not, and warps meet with very different maxima."""
+    gen = torch.Generator(device="cuda").manual_seed(L + d)
+    q, k, v = (0.25 * torch.randn(1, L, 2, d, device="cuda", generator=gen) for _ in range(3))
+    v *= 4
+    scale = 0.125
+    # how many columns a warp's chunk and its next are apart, and by what their scores differ then
+    apart = 32 if d == 128 else 128 if d == 32 else 64
+    slopes = torch.tensor([0.5, 3, 7.75, 8.25, 20, 60, -0.5, -3, -7.75, -8.25, -20, -60], device="cuda")
+    q[..., 0] = (slopes / (apart / 16 * scale * 1.4427))[torch.arange(L, device="cuda") % 12][None, :, None]
+    q[..., 1] = q[..., 0] / 16
+    j = torch.arange(L, device="cuda")
+    k[..., 0], k[..., 1] = (j // 16).float()[None, :, None], (j % 16).float()[None, :, None]
+    q, k, v = (x.to(TD[dtype]) for x in (q, k, v))
+    keep = torch.rand(L, L, device="cuda", generator=gen) < 0.7
+    keep[:, 0] = True
+    rowptr = torch.zeros(L + 1, dtype=torch.int32, device="cuda")
+    rowptr[1:] = keep.sum(1).cumsum(0)
+    got = sfb.csr_attention(q, k, v, rowptr, keep.nonzero()[:, 1].to(torch.int32).contiguous(), scale)[0].double()
+    Q, K, V = (x.double().permute(0, 2, 1, 3) for x in (q, k, v))
+    S, A = Q @ K.transpose(-1, -2) * scale, Q.abs() @ K.abs().transpose(-1, -2) * scale
+    W = torch.softmax(S.masked_fill(~keep, -np.inf), -1)
+    want, size = (W @ V).permute(0, 2, 1, 3), (W @ V.abs()).permute(0, 2, 1, 3)
+    # a score: fp32 sums of d products, truncated (2^-23 each), and two roundings of the exponent; P: two 16-bit terms
+    off = ((d * 2.0 ** -23 + 4 * 2.0 ** -24) * A + 2.0 ** -21).masked_fill(~keep, 0).amax(-1)[..., None].permute(0, 2, 1, 3)
+    u = {"f32": 2.0 ** -24, "bf16": 2.0 ** -8, "f16": 2.0 ** -11}[dtype]
+    err = (2 * off + 2e-6 + L * 2.0 ** -23 + (2.0 ** -16 if dtype == "bf16" else 2.0 ** -22)) * size + u * want.abs() + (2.0 ** -25 if dtype == "f16" else 0)
+    assert ((got - want).abs() <= err).all()

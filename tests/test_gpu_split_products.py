@@ -78,12 +78,13 @@ def test_products_against_64_bits(sfb, bs, d, nb, dtype):
     if d in (32, 64, 128):
         rowptr, colidx = sfb.csr_from_layout(lay)
         got = _heads(sfb.csr_attention(q, k, v, rowptr, colidx, scale)[0])
-        if dtype == "f32":
-            assert ((got - want).abs() <= err + 2e-6 * size).all()           # the denominator's 1e-6
+        # the denominator's 1e-6; 16-bit tiles keep P to 16 (bf16) or 22 (fp16) bits and add their products on the tensor core, truncated
+        extra = 2e-6 + (0 if dtype == "f32" else nb * bs * 2 * EPS + (2.0 ** -16 if dtype == "bf16" else 2.0 ** -22))
+        assert ((got - want).abs() <= err + extra * size + (2.0 ** -25 if dtype == "f16" else 0)).all()
 
 
 def _same(got, want, tol):
-    """Finite where `want` is and close there; the same infinities and NaN elsewhere."""
+    """Finite where `want` is and close there (tol: of the value, or absolute below 1); the same infinities and NaN elsewhere."""
     fin = torch.isfinite(want)
     assert torch.equal(torch.isnan(got), torch.isnan(want))
     assert torch.equal(got[~fin & ~torch.isnan(want)], want[~fin & ~torch.isnan(want)])
@@ -108,28 +109,35 @@ def test_values_that_are_not_finite_or_nearly(sfb, bs, d, value, dtype):
     full = torch.from_numpy(np.kron(keep, np.ones((bs, bs), bool))).cuda()
     S32 = (q.float().permute(0, 2, 1, 3)[..., None, :] * k.float().permute(0, 2, 1, 3)[:, :, None]).sum(-1)     # element by element: inf * 0 is NaN
     _same(sfb.bst_sgemm_nt(q, k, lay, torch.float32), _blocks(keep, bs, S32), 1e-4)
-    if math.isinf(value):
-        # a score of -inf is a probability of 0, one of +inf or NaN a row of NaN
-        W = torch.softmax((S32 / math.sqrt(d)).masked_fill(~full, -math.inf), -1)
-        want = (W @ v.float().permute(0, 2, 1, 3)).permute(0, 2, 1, 3)
-        _same(sfb.fused_attention(q, k, v, lay, 1 / math.sqrt(d)).float(), want, 1e-5 if dtype == "f32" else 2.0 ** -9)
+    # a score of -inf is a probability of 0, one of +inf or NaN a row of NaN
+    scale = 1 / math.sqrt(d)
+    W = torch.softmax((S32.double() * scale).masked_fill(~full, -math.inf), -1)
+    want = (W @ v.double().permute(0, 2, 1, 3)).permute(0, 2, 1, 3).float()
+    rowptr, colidx = sfb.csr_from_layout(lay)
+    tol = 1e-5 if dtype == "f32" else 2.0 ** -9
+    _same(sfb.fused_attention(q, k, v, lay, scale).float(), want, tol)
+    _same(sfb.csr_attention(q, k, v, rowptr, colidx, scale)[0].float(), want, tol)
     # one value: the rows that keep its block, and no other
     k = torch.randn(k.shape, device="cuda", generator=g).to(TD[dtype])
     v[0, bs + 3, 1, d - 1] = value
     p = torch.rand(1, 2, int(keep.sum()), bs, bs, device="cuda", generator=g) + 0.01
     M = _dense(keep, bs, p).float()
     want = torch.where(full[None, None, :, :, None], M[..., None] * v.float().permute(0, 2, 1, 3)[:, :, None], torch.zeros((), device="cuda")).sum(3).permute(0, 2, 1, 3)
-    got = sfb.bst_sgemm_xn(p if dtype == "f32" else p.to(TD[dtype]), v, lay).float()
-    if dtype == "f16":
-        assert torch.equal(torch.isfinite(got), torch.isfinite(want))
-    else:
-        _same(got, want, 1e-4)
-    o = sfb.fused_attention(q, k, v, lay, 1 / math.sqrt(d)).float()
-    touched = torch.zeros_like(o, dtype=torch.bool)
+    pt, none = p if dtype == "f32" else p.to(TD[dtype]), torch.zeros((), device="cuda")
+    V = v.float().permute(0, 2, 1, 3)[:, :, None]
+    wantT = torch.where(full.T[None, None, :, :, None], M.transpose(-1, -2)[..., None] * V, none).sum(3).permute(0, 2, 1, 3)
+    for got, ref in ((sfb.bst_sgemm_xn(pt, v, lay).float(), want), (sfb.bst_sgemm_tn(pt, v, lay).float(), wantT)):
+        if dtype == "f16":
+            assert torch.equal(torch.isfinite(got), torch.isfinite(ref))
+        else:
+            _same(got, ref, 1e-4)
+    W = torch.softmax((_heads(q) @ _heads(k).transpose(-1, -2) * scale).masked_fill(~full, -math.inf), -1)
+    want = torch.where(full[None, None, :, :, None], W[..., None] * V.double(), none.double()).sum(3).permute(0, 2, 1, 3).float()
+    touched = torch.zeros_like(want, dtype=torch.bool)
     touched[0, :, 1, d - 1] = full[:, bs + 3]
-    assert torch.isfinite(o[~touched]).all()
-    if not math.isfinite(value):
-        assert not torch.isfinite(o[touched]).any()
+    for o in (sfb.fused_attention(q, k, v, lay, scale).float(), sfb.csr_attention(q, k, v, rowptr, colidx, scale)[0].float()):
+        _same(o[~touched], want[~touched], tol)
+        _same(o[touched], want[touched], 1e-5)
 
 
 def test_a_row_of_scores_that_are_not_numbers_is_not_a_row_of_zeros(sfb):
@@ -232,3 +240,109 @@ def test_weights_that_are_subnormal(sfb, bs, d, below):
     for o in (sfb.fused_attention(q, k, v, lay, math.log(2)), sfb.csr_attention(q, k, v, rowptr, colidx, math.log(2))[0] * (1 + 1e-6)):
         assert ((o[0, :, 0] - want).abs() <= tol * want + (2.0 ** (100 - 134) if below > 109 else 0) * (want < 1)).all()
         assert (o[0, :, 0] > 0).all()
+
+
+@pytest.mark.parametrize("down", [100, 109, 112, 118, 124])
+def test_small_operands(sfb, down):
+    """What is left of an operand below 2^-109 is a multiple of 2^-133, the last place of the smallest bf16 numbers: its products are
+    off by up to 2^-134 of the other operand on top of what larger ones are."""
+    bs, d, nb = 32, 64, 4
+    lay, keep = _layout(sfb, nb, bs, 2)
+    g = torch.Generator(device="cuda").manual_seed(9)
+    q, k, v = (torch.randn(1, nb * bs, 2, d, device="cuda", generator=g) for _ in range(3))
+    q, v = q * 2.0 ** -down, v * 2.0 ** -down
+    Q, K, V = map(_heads, (q, k, v))
+    S, A, lost = Q @ K.transpose(-1, -2), Q.abs() @ K.abs().transpose(-1, -2), torch.ones_like(Q) @ K.abs().transpose(-1, -2) * 2.0 ** -134
+    s = sfb.bst_sgemm_nt(q, k, lay, torch.float32)
+    assert ((s.double() - _blocks(keep, bs, S)).abs() <= _blocks(keep, bs, _bound(d) * A + lost)).all()
+    p = torch.randn(1, 2, lay.blocks, bs, bs, device="cuda", generator=g)
+    P = _dense(keep, bs, p)
+    for M, got in ((P, sfb.bst_sgemm_xn(p, v, lay)), (P.transpose(-1, -2), sfb.bst_sgemm_tn(p, v, lay))):
+        assert ((_heads(got) - M @ V).abs() <= _bound(nb * bs) * (M.abs() @ V.abs()) + 2.0 ** -134 * (M.abs() @ torch.ones_like(V))).all()
+
+
+def _attention64(q, k, v, keep, scale):
+    """Outputs [B, H, L, d] in 64 bits and the error that scores and exponentials of fp32 leave in them."""
+    d, n = q.shape[3], k.shape[1]
+    Q, K, V = map(_heads, (q, k, v))
+    S, A = Q @ K.transpose(-1, -2) * scale, Q.abs() @ K.abs().transpose(-1, -2) * scale
+    W = torch.softmax(S.masked_fill(~keep, -math.inf), -1).nan_to_num(0)
+    size = W @ V.abs()
+    off = (_bound(d) * A + S.abs() * 4 * EPS + 2.0 ** -21).masked_fill(~keep, 0)
+    return W @ V, (W * off) @ V.abs() + off.amax(-1, keepdim=True) * size + _bound(n) * size
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("bs,d", [(32, 32), (32, 64), (32, 128), (64, 32), (64, 64), (64, 128)])
+def test_attention_launches_of_more_than_one_wave(sfb, bs, d, dtype):
+    """More CTAs than the SMs hold at once (up to three each): the kernels with short rings.  Against 64 bits with and without a mask,
+    bit for bit what a slice of one head gives (the kernels with long rings), and with a key that is not finite."""
+    if dtype != "f32" and bs == 64 and d == 64:
+        pytest.skip("taken by the tcgen05 kernels")
+    nb = 7
+    B = 3 * torch.cuda.get_device_properties(0).multi_processor_count // (2 * nb) + 1
+    lay, keep = _layout(sfb, nb, bs, bs + d)
+    lay.pack_mask(sfb.MASK_CAUSAL_DIAG)
+    g = torch.Generator(device="cuda").manual_seed(12)
+    q, k, v = (torch.randn(B, nb * bs, 2, d, device="cuda", generator=g).to(TD[dtype]) for _ in range(3))
+    full = torch.from_numpy(np.kron(keep, np.ones((bs, bs), bool))).cuda()
+    tril = torch.ones(bs, bs, device="cuda").tril().bool()
+    u = EPS if dtype == "f32" else 2.0 ** -8 if dtype == "bf16" else 2.0 ** -11
+    scale = 1 / math.sqrt(d)
+    for use_mask in (False, True):
+        if use_mask:
+            for i in range(nb):
+                full[i * bs:(i + 1) * bs, i * bs:(i + 1) * bs] &= tril
+        want, err = _attention64(q, k, v, full, scale)
+        o = sfb.fused_attention(q, k, v, lay, scale, use_mask=use_mask)
+        assert ((_heads(o) - want).abs() <= err + u * want.abs() + (2.0 ** -25 if dtype == "f16" else 0)).all()
+        for b in (0, B // 2, B - 1):
+            part = sfb.fused_attention_slice(q[b:b + 1, :, 1:], k[b:b + 1, :, 1:], v[b:b + 1, :, 1:], lay, scale, use_mask=use_mask)
+            assert torch.equal(part, o[b:b + 1, :, 1:])
+    bad = k.clone()
+    bad[B // 2, bs + 5, 1, 3] = math.nan
+    again = sfb.fused_attention(q, bad, v, lay, scale, use_mask=True)
+    met = torch.zeros(o.shape[:3], dtype=torch.bool, device="cuda")
+    met[B // 2, :, 1] = full[:, bs + 5]
+    assert met.any() and torch.isnan(again[met]).all() and torch.equal(again[~met], o[~met])
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("d,B", [(64, 1), (128, 1), (32, 1), (64, 5)])
+def test_rows_longer_than_the_lanes(sfb, d, B, dtype):
+    """A row's entries are held one per lane, 32 at a time: rows (and columns) of 31 to 97 blocks in no regular order."""
+    nb, bs, H = 104, 32, 1
+    rng = np.random.RandomState(d)
+    keep = np.zeros((nb, nb), bool)
+    for i, n in enumerate((31, 32, 33, 64, 65, 97, 1, 0)):
+        keep[11 * i, rng.choice(nb, size=n, replace=False)] = True
+    lay, layT = (sfb.BlockLayout(torch.from_numpy(np.ascontiguousarray(x)[None].astype(np.uint8)).cuda(), bs) for x in (keep, keep.T))
+    g = torch.Generator(device="cuda").manual_seed(13)
+    q, k, v = (torch.randn(B, nb * bs, H, d, device="cuda", generator=g).to(TD[dtype]) for _ in range(3))
+    u, floor = (EPS if dtype == "f32" else 2.0 ** -8 if dtype == "bf16" else 2.0 ** -11), (2.0 ** -25 if dtype == "f16" else 0)
+    rows = torch.arange(nb * bs, device="cuda").reshape(nb, bs)[::11][:8].reshape(-1)          # of the block-rows above
+    V = _heads(v)
+    # the blocks in the transposed layout's order
+    at = np.zeros((nb, nb), np.int64)
+    at[np.nonzero(keep)] = np.arange(lay.blocks)
+    i, j = np.nonzero(keep.T)
+    order = torch.from_numpy(at[j, i]).cuda()
+    for pt in ("f32", "bf16"):
+        p = torch.randn(B, H, lay.blocks, bs, bs, device="cuda", generator=g).to(TD[pt])
+        M = _dense(keep, bs, p)
+        want, size = M @ V, M.abs() @ V.abs()
+        for got in (sfb.bst_sgemm_xn(p, v, lay), sfb.bst_sgemm_tn(p[:, :, order].transpose(-1, -2).contiguous(), v, layT)):
+            assert ((_heads(got) - want).abs() <= _bound(97 * bs) * size + u * want.abs() + floor).all()
+    lay.pack_mask(sfb.MASK_CAUSAL_DIAG)
+    full = torch.from_numpy(np.kron(keep, np.ones((bs, bs), bool))).cuda()[rows]
+    rest = torch.ones(nb * bs, dtype=torch.bool, device="cuda")
+    rest[rows] = False
+    scale = 1 / math.sqrt(d)
+    for use_mask in (False, True):
+        if use_mask:
+            for n in range(8):
+                full[n * bs:(n + 1) * bs, 11 * n * bs:(11 * n + 1) * bs] &= torch.ones(bs, bs, device="cuda").tril().bool()
+        want, err = _attention64(q[:, rows], k, v, full, scale)
+        o = _heads(sfb.fused_attention(q, k, v, lay, scale, use_mask=use_mask))
+        assert ((o[:, :, rows] - want).abs() <= err + u * want.abs() + floor).all()
+        assert (o[:, :, rest] == 0).all()
