@@ -460,7 +460,8 @@ __global__ void __launch_bounds__(128, CsrCfg<D>::CTAS) csr_tile_kernel(const Cs
         f[k] = x.x > -INFINITY ? ex2f(x.x - M) : 0.f;
         sum = fmaf(x.y, f[k], sum);
     }
-    const float inv = sum > 0.f ? 1.f / (sum + 1e-6f) : 0.f;   // the reference's denominator (ewops.h:93, cuda_kernels.h:1022)
+    // the reference's denominator (ewops.h:93, cuda_kernels.h:1022); the sum may stand 2^8 above the reference's, where 1e-6 counts less
+    const float inv = sum > 0.f ? 1.f / (sum + 1e-6f) : 0.f;
     uint16_t *dst = (uint16_t *)a.O + ((size_t)b * a.L + row) * HD + (size_t)h * D + d0;
     float zero = 0.f;                                          // stays 0 as long as every output is finite
 #pragma unroll

@@ -3,8 +3,9 @@
 // on warp-level tensor-core instructions.
 //
 // fp32 products on bf16 operands.  An fp32 number is the sum of three bf16 numbers, x = h + m + l (8 + 8 + 8 bits, each
-// rounded from what the one before left), exact down to 2^-109.  x * y is then six products of them, hh + hm + mh + hl + mm + lh,
-// up to 2^-25 of it.  The tensor core's products are exact and its sums truncate (measured: an aligned addend keeps one bit
+// rounded from what the one before left), exact down to 2^-109; of a smaller number a multiple of 2^-133 is left (the last place
+// of the smallest bf16 numbers), so its products are off by up to 2^-134 of the other factor.  x * y is then six products of them,
+// hh + hm + mh + hl + mm + lh, up to 2^-24 of it.  The tensor core's products are exact and its sums truncate (measured: an aligned addend keeps one bit
 // below the last place), which over a long contraction is a bias; so the small products go first, and every 16 elements of
 // the contraction are summed from zero and added to the fp32 accumulator by rounded additions.  Measured relative error of
 // scores against 64 bits at d = 32 / 64 / 128: 5.5e-8 / 6.3e-8 / 7.4e-8; two FMA chains, as the thread tiles before this had
