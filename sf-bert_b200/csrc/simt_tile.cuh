@@ -43,6 +43,10 @@ __device__ __forceinline__ void cp_async16(float *dst, const void *src, uint32_t
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void cp_async4(float *dst, const void *src, uint32_t bytes)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
@@ -105,9 +109,12 @@ __device__ __forceinline__ void stage_begin(Staged<DT, TT, COLS> &st, uint32_t r
             }
         }
     } else {
+#pragma unroll 8
         for (uint32_t t = rank; t < 32 * COLS; t += TT) {
             const uint32_t r = t / COLS, c = t % COLS;
-            dst[tile_row(r) * stride + c] = c < ncols ? Elem<DT>::load(src, at + r * pitch + c) : 0.f;
+            float *d = dst + tile_row(r) * stride + c;
+            if (DT == SFB_F32) cp_async4(d, (const float *)src + at + (c < ncols ? r * pitch + c : 0), c < ncols ? 4u : 0u);
+            else *d = c < ncols ? Elem<DT>::load(src, at + r * pitch + c) : 0.f;
         }
     }
 }
