@@ -6,7 +6,7 @@
 // instructions on operands split into bf16 terms (simt_tile.cuh).  The fused SDDMM + softmax (fused_sddmm_softmax_kernel) is on the
 // FMA pipe: 256 threads as a 16x16 grid; thread (ty,tx) owns rows ty+16m and columns tx+16n of a tile, so the 16
 // lanes of a half-warp own one set of rows and row reductions are four shuffles.
-#include "simt_tile.cuh"
+#include "fma_tile.cuh"
 #include "csr.cuh"
 #include <float.h>
 #include <math.h>
@@ -522,35 +522,93 @@ __global__ void __launch_bounds__(BS * BS / 8 / SPLIT) softmax_grad_kernel(const
 }
 
 // ------------------------------------------------------------------------------------------------
-// The same for 32 rows x NC columns of the SpMM below.  pbase: first block of the (batch, head); vbase, at: the first column in the first rows of V and
-// of the warp's outputs.
-template <int BS, int A_DT, int BC_DT, bool TRANS, int NC>
-__device__ __noinline__ void spmm_again(float *buf, const uint2 *ent, uint32_t cnt, const void *Pm, const void *V, void *O, size_t pbase, size_t vbase, size_t at, size_t HD,
-                                        uint32_t r0, uint32_t ncols)
-{
-    using namespace tile;
-    const uint32_t lane = threadIdx.x & 31;
-    float acc[NC] = {};
-    for (uint32_t e = 0; e < cnt; e++)
-        for (uint32_t k = 0; k < BS; k += kAgain) {
-            const size_t pb = pbase + (size_t)ent[e].x * BS * BS;
-            __syncwarp();
-            if (TRANS) copy_again<A_DT, kAgain, 32, kAgainRows, 1>(buf, Pm, pb + (size_t)k * BS + r0, BS, 32, lane);
-            else copy_again<A_DT, 32, kAgain, 1, kAgainRows>(buf, Pm, pb + (size_t)r0 * BS + k, BS, kAgain, lane);
-            copy_again<BC_DT, kAgain, NC, kAgainCols<NC>, 1>(buf + kAgain * kAgainRows, V, vbase + ((size_t)ent[e].y * BS + k) * HD, HD, ncols, lane);
-            __syncwarp();
-            fma_again<NC>(acc, buf, buf + kAgain * kAgainRows, lane);
-        }
-#pragma unroll
-    for (int n = 0; n < NC; n++)
-        if ((uint32_t)n < ncols && !finite(Elem<BC_DT>::load(O, at + lane * HD + n))) Elem<BC_DT>::store(O, at + lane * HD + n, acc[n]);
-}
-
 // SpMM: one CTA per (block-row, slice of up to 128 of d).  TRANS = false: O = sum over the row's blocks of P . V (NN, the
 // lut is the nn_lut).  TRANS = true: the backward products dV = P^T dO and dK = dS^T Q -- the lut is the tn_lut,
 // "row" i is a block COLUMN, an entry names a block of that column and the block-row its B rows come from, and
 // the block is used transposed (read as it lies, four neighbouring rows of P^T per 16-byte load).
-// A chunk is 32 elements of the contraction: one 32x32 block, or half of a 64x64 one, with its 32 rows of V.  A warp owns 32
+// A chunk is 32 elements of the contraction: one 32x32 block, or half of a 64x64 one, with its 32 rows of V.
+//
+// By FMAs (fma_tile.cuh).  AGAIN: what the kernel below left that is not finite, made again by the same CTA (simt_tile.cuh says why).
+template <int BS, int DS> struct SpmmFmaCfg {
+    static constexpr int WC = BS == 32 ? 4 : 2;                          // warps side by side along d
+    static constexpr int TN = DS / WC / 4;                               // columns per thread
+    static constexpr uint32_t a_floats = BS == 32 ? 32 * tile::kStride : 64 * tile::kStride > 32 * (64 + 4) ? 64 * tile::kStride : 32 * (64 + 4);
+    static constexpr uint32_t buf = a_floats + 32 * (DS + 4);
+    static constexpr size_t bytes = sizeof(float) * 2 * buf;             // [2][P chunk | V chunk]
+};
+template <int BS, int DS, int A_DT, int BC_DT, bool TRANS, bool AGAIN>
+__device__ __forceinline__ void spmm_fma(float *sm, const uint2 *__restrict__ lut, const void *__restrict__ Pm, const void *__restrict__ V, void *__restrict__ O,
+                                         const AttnDims &p, bool avec, bool vec)
+{
+    using namespace fma_tile;
+    typedef SpmmFmaCfg<BS, DS> Cfg;
+    constexpr int TN = Cfg::TN;
+    constexpr uint32_t PARTS = BS / 32;                                  // chunks per block
+    constexpr uint32_t a_stride = TRANS ? BS + 4 : kStride;
+    const uint32_t nslice = (p.d + DS - 1) / DS;
+    const uint32_t i = blockIdx.x / nslice, d0 = (blockIdx.x % nslice) * DS;
+    const uint32_t b = blockIdx.y, h = blockIdx.z;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane_row(lane), lc = lane_quad(lane);
+    const uint2 *nn = lut + (size_t)h * p.lut_stride;
+    const uint2 head = nn[i];
+    const size_t HD = (size_t)p.H * p.d;
+    const size_t bh = (size_t)b * p.H + h;
+    const uint32_t r0 = BS == 64 ? 32 * (warp >> 1) : 0, n0 = (BS == 64 ? warp & 1 : warp) * (DS / Cfg::WC);
+    const uint32_t chunks = head.y * PARTS;
+
+    auto issue = [&](uint32_t c) {
+        const uint2 ent = nn[head.x + c / PARTS];
+        const uint32_t part = c % PARTS;
+        float *buf = sm + (c & 1) * Cfg::buf;
+        const size_t baseP = (bh * p.blocks + ent.x) * BS * BS, baseV = ((size_t)b * p.nb_b + ent.y) * BS * HD + (size_t)h * p.d + d0;
+        if (TRANS) stage<A_DT, 32, BS>(buf, a_stride, Pm, baseP + part * 32 * BS, BS, BS, avec);
+        else stage<A_DT, BS, 32>(buf, a_stride, Pm, baseP + part * 32, BS, 32, avec);
+        stage<BC_DT, 32, DS>(buf + Cfg::a_floats, DS + 4, V, baseV + (size_t)part * 32 * HD, HD, p.d - d0, vec);
+        tile::cp_commit();
+    };
+    uint64_t acc[4][TN / 2];
+#pragma unroll
+    for (int m = 0; m < 4; m++)
+#pragma unroll
+        for (int n = 0; n < TN / 2; n++) acc[m][n] = 0;
+    if (chunks) issue(0);
+    for (uint32_t c = 0; c < chunks; c++) {
+        tile::cp_wait<0>();
+        __syncthreads();
+        if (c + 1 < chunks) issue(c + 1);
+        const float *buf = sm + (c & 1) * Cfg::buf;
+        const float *v = buf + Cfg::a_floats + n0 + lane_col<TN>(lc);
+        if (TRANS) mma_tn<TN>(acc, buf + r0 + 4 * lr, a_stride, v, DS + 4);
+        else mma_nn<TN>(acc, buf + (r0 + lr) * a_stride, a_stride, v, DS + 4);
+    }
+    // rows without blocks are written as zeros (blocksparse.h:949-962)
+    const size_t baseO = ((size_t)b * p.nb_a + i) * BS * HD + (size_t)h * p.d + d0 + n0;
+    const uint32_t left = p.d > d0 + n0 ? p.d - d0 - n0 : 0;
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+        const uint32_t r = r0 + (TRANS ? 4 * lr + m : lr + 8 * m);
+        store_row<BC_DT, TN, AGAIN>(O, baseO + (size_t)r * HD, lc, acc[m], left, vec);
+    }
+}
+template <int BS, int DS, int A_DT, int BC_DT, bool TRANS>
+__global__ void __launch_bounds__(tile::kThreads, 4) spmm_fma_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Pm, const void *__restrict__ V,
+                                                                   void *__restrict__ O, AttnDims p, bool avec, bool vec)
+{
+    extern __shared__ __align__(16) float sm[];
+    grid_dependency_wait();
+    grid_launch_dependents();
+    spmm_fma<BS, DS, A_DT, BC_DT, TRANS, false>(sm, lut, Pm, V, O, p, avec, vec);
+}
+// Not inlined, and from the kernel's parameters alone: nothing is kept for it in registers while the split products are made
+template <int BS, int DS, int A_DT, int BC_DT, bool TRANS>
+__device__ __noinline__ void spmm_again(float *sm, const uint2 *lut, const void *Pm, const void *V, void *O, uint32_t H, uint32_t d, uint32_t nb_a, uint32_t nb_b,
+                                        uint32_t blocks, uint32_t lut_stride, bool avec, bool vec)
+{
+    const AttnDims p = {0, H, d, nb_a, nb_b, blocks, lut_stride, 0, 0, 0};
+    spmm_fma<BS, DS, A_DT, BC_DT, TRANS, true>(sm, lut, Pm, V, O, p, avec, vec);
+}
+
+// As split products.  A warp owns 32
 // output rows and a share of the columns; it stages its own columns of V (with the other warp that has them, where blocks
 // are 64 rows) and reads P straight into fragments, a chunk ahead in registers: P is small beside V, and L1 has it for
 // the other warps.
@@ -558,11 +616,10 @@ template <int BS, int DS> struct SpmmCfg {
     static constexpr int WC = BS == 32 ? 4 : 2;                          // warps side by side along d: each is a team with the ones below it
     static constexpr int TT = 128 / WC, NW = DS / WC, N = NW / 8;        // a team's threads and columns, n-tiles of 8 columns
     static constexpr uint32_t v_stride = NW + 8, buf = 32 * v_stride;
-    static constexpr int NC = NW < 32 ? NW : 32;                         // columns that spmm_again takes at a time
-    static_assert(WC * 3 * buf / 4 >= tile::kAgain * (tile::kAgainRows + tile::kAgainCols<NC>), "a warp's share holds the tiles of spmm_again");
+    static constexpr size_t own = sizeof(float) * 3 * WC * buf, bytes = own > SpmmFmaCfg<BS, DS>::bytes ? own : SpmmFmaCfg<BS, DS>::bytes;      // [team][3][32 rows of V], or spmm_again's
 };
 template <int BS, int DS, int A_DT, int BC_DT, bool TRANS>
-__global__ void __launch_bounds__(tile::kThreads, (BS == 64 && DS == 128) || A_DT == SFB_F32 ? 3 : 4)
+__global__ void __launch_bounds__(tile::kThreads, BS == 64 && DS == 128 ? 3 : 4)
 spmm_nn_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Pm, const void *__restrict__ V, void *__restrict__ O, AttnDims p, bool avec, bool vec)
 {
     using namespace tile;
@@ -670,13 +727,7 @@ spmm_nn_kernel(const uint2 *__restrict__ lut, const void *__restrict__ Pm, const
             const uint32_t r = r0 + (TRANS ? 4 * g + 2 * m + half : 16 * m + 8 * half + g);
             store_cols<BC_DT, N>(O, baseO + (size_t)r * HD, t, acc[m], half, 1.f, left, vec);
         }
-    // on the team's shared memory, when its other warp is past the products too
-    if ((TP > 1 || TV > 1) && (BS == 64 ? __syncthreads_or(odd) : __any_sync(0xffffffffu, odd)) && __any_sync(0xffffffffu, odd)) {
-        cp_wait<0>();
-        for (uint32_t c = 0; c < Cfg::NW && c < left; c += Cfg::NC)
-            spmm_again<BS, A_DT, BC_DT, TRANS, Cfg::NC>(sm + warp * (Cfg::WC * 3 * Cfg::buf / 4), nn + head.x, head.y, Pm, V, O, bh * p.blocks * BS * BS,
-                                                        (size_t)b * p.nb_b * BS * HD + (size_t)h * p.d + n0 + c, baseO + (size_t)r0 * HD + c, HD, r0, left - c);
-    }
+    if ((TP > 1 || TV > 1) && __syncthreads_or(odd)) spmm_again<BS, DS, A_DT, BC_DT, TRANS>(sm, lut, Pm, V, O, p.H, p.d, p.nb_a, p.nb_b, p.blocks, p.lut_stride, avec, vec);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -857,11 +908,17 @@ __device__ __noinline__ void attention_again(float *sm, const uint2 *ent, uint32
 #pragma unroll
         for (int n = 0; n < NW; n++) acc[n] *= alpha;
         __syncthreads();
-        for (uint32_t k = 0; left && k < nblk * BS; k += kAgain) {
-            __syncwarp();
-            copy_again<DT, kAgain, NW, kAgainCols<NW>, 1>(buf, V, kv + ((size_t)ent[e + k / BS].y * BS + k % BS) * HD + n0, HD, left, lane);
-            __syncwarp();
-            fma_again<NW>(acc, ps + k * kAgainRows, buf, lane);
+        if (left) {
+            Again<kAgain, NW> v;
+            v.template load<DT>(V, kv + (size_t)ent[e].y * BS * HD + n0, HD, left, lane);
+            for (uint32_t k = 0; k < nblk * BS; k += kAgain) {
+                __syncwarp();
+                v.template put<kAgainCols<NW>, 1>(buf, lane);
+                __syncwarp();
+                const uint32_t next = k + kAgain;
+                if (next < nblk * BS) v.template load<DT>(V, kv + ((size_t)ent[e + next / BS].y * BS + next % BS) * HD + n0, HD, left, lane);
+                fma_again<NW>(acc, ps + k * kAgainRows, buf, lane);
+            }
         }
     }
     __syncthreads();
@@ -1439,25 +1496,30 @@ int simt_softmax(cudaStream_t s, const void *lut, const void *mask, const void *
     return check_launch("sfb_masked_softmax");
 }
 
+// FMAs: fp32 blocks, whose split every warp makes again for its own columns, and transposed blocks of 32 with heads of up to 32,
+// where a warp has eight columns to spend a fragment of P on.  Split products / FMAs, us: fp32 blocks, sawtooth rows of eight, B 8,
+// H 8, 24 block-rows of 32, d 32 transposed 33.1 / 19.2, d 64 38.1 / 27.8; full rows, B 1, H 4, 16 block-rows of 64, d 128 79.9 / 60.9; fp16,
+// the sawtooth rows, d 32 transposed 28.3 / 23.4
+template <int BS, int DS, int AD, int BD, bool TRANS>
+static int launch_spmm(cudaStream_t s, const void *lut, const void *a, const void *b, void *c, const AttnDims &p, bool avec, bool vec)
+{
+    static DeviceOnce once;
+    const dim3 grid(p.nb_a * ((p.d + DS - 1) / DS), p.B, p.H);
+    if constexpr (AD == SFB_F32 || (TRANS && BS == 32 && DS == 32)) {
+        if (set_smem(once, spmm_fma_kernel<BS, DS, AD, BD, TRANS>, SpmmFmaCfg<BS, DS>::bytes)) return 1;
+        launch_overlapped(spmm_fma_kernel<BS, DS, AD, BD, TRANS>, grid, dim3(tile::kThreads), SpmmFmaCfg<BS, DS>::bytes, s, (const uint2 *)lut, a, b, c, p, avec, vec);
+    } else {
+        if (set_smem(once, spmm_nn_kernel<BS, DS, AD, BD, TRANS>, SpmmCfg<BS, DS>::bytes)) return 1;
+        launch_overlapped(spmm_nn_kernel<BS, DS, AD, BD, TRANS>, grid, dim3(tile::kThreads), SpmmCfg<BS, DS>::bytes, s, (const uint2 *)lut, a, b, c, p, avec, vec);
+    }
+    return 0;
+}
 int simt_spmm_nn(cudaStream_t s, const void *lut, const void *a, const void *b, void *c, int a_dtype, int bc_dtype,
                  uint32_t bs, const AttnDims &p, bool trans)
 {
     const uint64_t HD = (uint64_t)p.H * p.d;
     const bool avec = ((uintptr_t)a & 15) == 0, vec = rows_vec(b, bc_dtype, HD, p.d) && rows_vec(c, bc_dtype, HD, p.d);
-#define SP_LAUNCH(DSV)                                                                                            \
-    {                                                                                                             \
-        const size_t bytes = sizeof(float) * 3 * SpmmCfg<BS, DSV>::WC * SpmmCfg<BS, DSV>::buf;                                           \
-        const dim3 grid(p.nb_a * ((p.d + DSV - 1) / DSV), p.B, p.H);                                              \
-        if (trans) {                                                                                              \
-            auto kern = spmm_nn_kernel<BS, DSV, AD, BD, true>;                                                    \
-            static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                                                  \
-            launch_overlapped(kern, grid, dim3(tile::kThreads), bytes, s, (const uint2 *)lut, a, b, c, p, avec, vec);                  \
-        } else {                                                                                                  \
-            auto kern = spmm_nn_kernel<BS, DSV, AD, BD, false>;                                                   \
-            static DeviceOnce once; if (set_smem(once, kern, bytes)) return 1;                                                                  \
-            launch_overlapped(kern, grid, dim3(tile::kThreads), bytes, s, (const uint2 *)lut, a, b, c, p, avec, vec);                  \
-        }                                                                                                         \
-    }
+#define SP_LAUNCH(DSV) { if (trans ? launch_spmm<BS, DSV, AD, BD, true>(s, lut, a, b, c, p, avec, vec) : launch_spmm<BS, DSV, AD, BD, false>(s, lut, a, b, c, p, avec, vec)) return 1; }
     DISPATCH_BS(bs, DISPATCH_DT(a_dtype, AD, DISPATCH_DT(bc_dtype, BD, {
         if (p.d <= 32) SP_LAUNCH(32) else if (p.d <= 64) SP_LAUNCH(64) else SP_LAUNCH(128)
     })))

@@ -359,16 +359,23 @@ __device__ __forceinline__ bool finite(float v) { return fabsf(v) <= 3.402823466
 constexpr uint32_t kAgain = 16, kAgainRows = 33;
 template <int N> constexpr uint32_t kAgainCols = N + 4;
 constexpr uint32_t kAgainFloats = kAgain * (kAgainRows + kAgainCols<32>);
-// element (r, c) = src[at + r * pitch + c] -> dst[r * ROW + c * COL], by one warp; columns from ncols on are zeros
-template <int DT, int ROWS, int COLS, int ROW, int COL>
-__device__ __forceinline__ void copy_again(float *dst, const void *src, size_t at, size_t pitch, uint32_t ncols, uint32_t lane)
-{
-#pragma unroll 8
-    for (uint32_t x = lane; x < ROWS * COLS; x += 32) {
-        const uint32_t r = x / COLS, c = x % COLS;
-        dst[r * ROW + c * COL] = c < ncols ? Elem<DT>::load(src, at + r * pitch + c) : 0.f;
+// ROWS x COLS elements on their way there, by one warp: element (r, c) = src[at + r * pitch + c] -> dst[r * ROW + c * COL]; columns from ncols on are zeros
+template <int ROWS, int COLS> struct Again {
+    float x[ROWS * COLS / 32];
+    template <int DT> __device__ __forceinline__ void load(const void *src, size_t at, size_t pitch, uint32_t ncols, uint32_t lane)
+    {
+#pragma unroll
+        for (int i = 0; i < ROWS * COLS / 32; i++) {
+            const uint32_t r = (32 * i + lane) / COLS, c = (32 * i + lane) % COLS;
+            x[i] = c < ncols ? Elem<DT>::load(src, at + r * pitch + c) : 0.f;
+        }
     }
-}
+    template <int ROW, int COL> __device__ __forceinline__ void put(float *dst, uint32_t lane) const
+    {
+#pragma unroll
+        for (int i = 0; i < ROWS * COLS / 32; i++) dst[(32 * i + lane) / COLS * ROW + (32 * i + lane) % COLS * COL] = x[i];
+    }
+};
 template <int N>
 __device__ __forceinline__ void fma_again(float (&acc)[N], const float *a, const float *b, uint32_t lane)
 {
@@ -391,11 +398,18 @@ __device__ __forceinline__ void scores_again(float (&s)[32], float *buf, const v
 {
 #pragma unroll
     for (int n = 0; n < 32; n++) s[n] = 0.f;
+    Again<32, kAgain> x, y;
+    x.template load<DT>(A, rowA, HD, d, lane);
+    y.template load<DT>(B, rowB, HD, d, lane);
     for (uint32_t k = 0; k < d; k += kAgain) {
         __syncwarp();
-        copy_again<DT, 32, kAgain, 1, kAgainRows>(buf, A, rowA + k, HD, d - k, lane);
-        copy_again<DT, 32, kAgain, 1, kAgainCols<32>>(buf + kAgain * kAgainRows, B, rowB + k, HD, d - k, lane);
+        x.template put<1, kAgainRows>(buf, lane);
+        y.template put<1, kAgainCols<32>>(buf + kAgain * kAgainRows, lane);
         __syncwarp();
+        if (k + kAgain < d) {
+            x.template load<DT>(A, rowA + k + kAgain, HD, d - k - kAgain, lane);
+            y.template load<DT>(B, rowB + k + kAgain, HD, d - k - kAgain, lane);
+        }
         fma_again<32>(s, buf, buf + kAgain * kAgainRows, lane);
     }
 }

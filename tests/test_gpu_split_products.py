@@ -20,6 +20,11 @@ def _bound(terms):
     return (1 + 6 * 2 + math.ceil(terms / 16) + 1) * EPS
 
 
+def _spmm_bound(terms, bs, d, pt, trans):
+    """fp32 blocks, and transposed ones of 32 beside heads of up to 32, go by FMAs: one rounding per term."""
+    return max(_bound(terms), terms * EPS) if pt == "f32" or (trans and bs == 32 and d <= 32) else _bound(terms)
+
+
 def _layout(sfb, nb, bs, seed):
     rng = np.random.RandomState(seed)
     keep = np.zeros((1, nb, nb), np.uint8)
@@ -64,9 +69,9 @@ def test_products_against_64_bits(sfb, bs, d, nb, dtype):
         p = torch.randn(s.shape, device="cuda", generator=g).to(TD[pt])
         P = _dense(keep, bs, p)
         u = EPS if dtype == "f32" else 2.0 ** -8 if dtype == "bf16" else 2.0 ** -11
-        for M, got in ((P, sfb.bst_sgemm_xn(p, v, lay)), (P.transpose(-1, -2), sfb.bst_sgemm_tn(p, v, lay))):
+        for M, got, trans in ((P, sfb.bst_sgemm_xn(p, v, lay), False), (P.transpose(-1, -2), sfb.bst_sgemm_tn(p, v, lay), True)):
             want, size = M @ V, M.abs() @ V.abs()
-            assert ((_heads(got) - want).abs() <= _bound(nb * bs) * size + u * want.abs() + (2.0 ** -25 if dtype == "f16" else 0)).all()
+            assert ((_heads(got) - want).abs() <= _spmm_bound(nb * bs, bs, d, pt, trans) * size + u * want.abs() + (2.0 ** -25 if dtype == "f16" else 0)).all()
     scale = 1 / math.sqrt(d)
     full = torch.from_numpy(np.kron(keep, np.ones((bs, bs), bool))).cuda()
     W = torch.softmax((S * scale).masked_fill(~full, -math.inf), -1)
@@ -120,17 +125,18 @@ def test_values_that_are_not_finite_or_nearly(sfb, bs, d, value, dtype):
     # one value: the rows that keep its block, and no other
     k = torch.randn(k.shape, device="cuda", generator=g).to(TD[dtype])
     v[0, bs + 3, 1, d - 1] = value
-    p = torch.rand(1, 2, int(keep.sum()), bs, bs, device="cuda", generator=g) + 0.01
+    p = torch.rand(1, 2, int(keep.sum()), bs, bs, device="cuda", generator=g).add(0.01).to(torch.bfloat16)
     M = _dense(keep, bs, p).float()
     want = torch.where(full[None, None, :, :, None], M[..., None] * v.float().permute(0, 2, 1, 3)[:, :, None], torch.zeros((), device="cuda")).sum(3).permute(0, 2, 1, 3)
-    pt, none = p if dtype == "f32" else p.to(TD[dtype]), torch.zeros((), device="cuda")
+    none = torch.zeros((), device="cuda")
     V = v.float().permute(0, 2, 1, 3)[:, :, None]
     wantT = torch.where(full.T[None, None, :, :, None], M.transpose(-1, -2)[..., None] * V, none).sum(3).permute(0, 2, 1, 3)
-    for got, ref in ((sfb.bst_sgemm_xn(pt, v, lay).float(), want), (sfb.bst_sgemm_tn(pt, v, lay).float(), wantT)):
-        if dtype == "f16":
-            assert torch.equal(torch.isfinite(got), torch.isfinite(ref))
-        else:
-            _same(got, ref, 1e-4)
+    for pt in (p.to(TD[dtype]), p):                          # fp32 blocks go by FMAs, others as split products
+        for got, ref in ((sfb.bst_sgemm_xn(pt, v, lay).float(), want), (sfb.bst_sgemm_tn(pt, v, lay).float(), wantT)):
+            if dtype == "f16":
+                assert torch.equal(torch.isfinite(got), torch.isfinite(ref))
+            else:
+                _same(got, ref, 1e-4)
     W = torch.softmax((_heads(q) @ _heads(k).transpose(-1, -2) * scale).masked_fill(~full, -math.inf), -1)
     want = torch.where(full[None, None, :, :, None], W[..., None] * V.double(), none.double()).sum(3).permute(0, 2, 1, 3).float()
     touched = torch.zeros_like(want, dtype=torch.bool)
@@ -255,7 +261,7 @@ def test_small_operands(sfb, down):
     S, A, lost = Q @ K.transpose(-1, -2), Q.abs() @ K.abs().transpose(-1, -2), torch.ones_like(Q) @ K.abs().transpose(-1, -2) * 2.0 ** -134
     s = sfb.bst_sgemm_nt(q, k, lay, torch.float32)
     assert ((s.double() - _blocks(keep, bs, S)).abs() <= _blocks(keep, bs, _bound(d) * A + lost)).all()
-    p = torch.randn(1, 2, lay.blocks, bs, bs, device="cuda", generator=g)
+    p = torch.randn(1, 2, lay.blocks, bs, bs, device="cuda", generator=g).to(torch.bfloat16)
     P = _dense(keep, bs, p)
     for M, got in ((P, sfb.bst_sgemm_xn(p, v, lay)), (P.transpose(-1, -2), sfb.bst_sgemm_tn(p, v, lay))):
         assert ((_heads(got) - M @ V).abs() <= _bound(nb * bs) * (M.abs() @ V.abs()) + 2.0 ** -134 * (M.abs() @ torch.ones_like(V))).all()
@@ -331,8 +337,8 @@ def test_rows_longer_than_the_lanes(sfb, d, B, dtype):
         p = torch.randn(B, H, lay.blocks, bs, bs, device="cuda", generator=g).to(TD[pt])
         M = _dense(keep, bs, p)
         want, size = M @ V, M.abs() @ V.abs()
-        for got in (sfb.bst_sgemm_xn(p, v, lay), sfb.bst_sgemm_tn(p[:, :, order].transpose(-1, -2).contiguous(), v, layT)):
-            assert ((_heads(got) - want).abs() <= _bound(97 * bs) * size + u * want.abs() + floor).all()
+        for got, trans in ((sfb.bst_sgemm_xn(p, v, lay), False), (sfb.bst_sgemm_tn(p[:, :, order].transpose(-1, -2).contiguous(), v, layT), True)):
+            assert ((_heads(got) - want).abs() <= _spmm_bound(97 * bs, bs, d, pt, trans) * size + u * want.abs() + floor).all()
     lay.pack_mask(sfb.MASK_CAUSAL_DIAG)
     full = torch.from_numpy(np.kron(keep, np.ones((bs, bs), bool))).cuda()[rows]
     rest = torch.ones(nb * bs, dtype=torch.bool, device="cuda")
