@@ -44,9 +44,14 @@ __device__ __noinline__ void sddmm_again(float *buf, const void *A, const void *
     const uint32_t lane = threadIdx.x & 31;
     float s[32];
     tile::scores_again<AB_DT>(s, buf, A, B, rowA, rowB, HD, d, lane);
+    // back to where a row's scores lie side by side: a lane per key
+    __syncwarp();
 #pragma unroll
-    for (int n = 0; n < 32; n++)
-        if (!tile::finite(Elem<C_DT>::load(C, at + lane * BS + n))) Elem<C_DT>::store(C, at + lane * BS + n, s[n]);
+    for (int n = 0; n < 32; n++) buf[lane * 33 + n] = s[n];
+    __syncwarp();
+#pragma unroll 8
+    for (uint32_t r = 0; r < 32; r++)
+        if (!tile::finite(Elem<C_DT>::load(C, at + r * BS + lane))) Elem<C_DT>::store(C, at + r * BS + lane, buf[r * 33 + lane]);
 }
 
 // SDDMM.  A CTA (four warps) makes one 64x64 block, a 32x32 quarter per warp, or four consecutive 32x32 blocks of the LUT,
@@ -57,7 +62,7 @@ __device__ __noinline__ void sddmm_again(float *buf, const void *A, const void *
 template <int BS> struct SddmmCfg {
     static constexpr int TEAMS = BS == 32 ? 4 : 2, TT = 128 / TEAMS;      // teams that stage keys of their own
     static constexpr uint32_t buf = 32 * tile::kStride;
-    static_assert(TEAMS * 2 * buf / 4 >= tile::kAgainFloats, "a warp's share holds the tiles of sddmm_again");
+    static_assert(TEAMS * 2 * buf / 4 >= tile::kAgainFloats && tile::kAgainFloats >= 32 * 33, "a warp's share holds the tiles of sddmm_again");
 };
 template <int BS, int AB_DT, int C_DT>
 __global__ void __launch_bounds__(tile::kThreads, 3) sddmm_nt_kernel(const uint2 *__restrict__ lut, const void *__restrict__ A,
@@ -1496,16 +1501,16 @@ int simt_softmax(cudaStream_t s, const void *lut, const void *mask, const void *
     return check_launch("sfb_masked_softmax");
 }
 
-// FMAs: fp32 blocks, whose split every warp makes again for its own columns, and transposed blocks of 32 with heads of up to 32,
-// where a warp has eight columns to spend a fragment of P on.  Split products / FMAs, us: fp32 blocks, sawtooth rows of eight, B 8,
-// H 8, 24 block-rows of 32, d 32 transposed 33.1 / 19.2, d 64 38.1 / 27.8; full rows, B 1, H 4, 16 block-rows of 64, d 128 79.9 / 60.9; fp16,
-// the sawtooth rows, d 32 transposed 28.3 / 23.4
+// FMAs: fp32 blocks, whose split every warp makes again for its own columns.  Split products / FMAs, us, transposed: sawtooth rows of
+// eight, B 8, H 8, 24 block-rows of 32, d 32 33.1 / 19.2, d 64 38.1 / 27.8; full rows, B 1, H 4, 16 block-rows of 64, d 128 84.2 / 57.1;
+// BigBird rows, B 4, H 8, 64 block-rows of 32, d 128, not transposed 184.6 / 211.6.  With 16-bit blocks of 32 at d 32, where a warp has eight columns to
+// spend a fragment of P on, neither is ahead of the other: fp16, transposed, the sawtooth rows 28.3 / 23.4, full rows 11.8 / 15.3.
 template <int BS, int DS, int AD, int BD, bool TRANS>
 static int launch_spmm(cudaStream_t s, const void *lut, const void *a, const void *b, void *c, const AttnDims &p, bool avec, bool vec)
 {
     static DeviceOnce once;
     const dim3 grid(p.nb_a * ((p.d + DS - 1) / DS), p.B, p.H);
-    if constexpr (AD == SFB_F32 || (TRANS && BS == 32 && DS == 32)) {
+    if constexpr (AD == SFB_F32) {
         if (set_smem(once, spmm_fma_kernel<BS, DS, AD, BD, TRANS>, SpmmFmaCfg<BS, DS>::bytes)) return 1;
         launch_overlapped(spmm_fma_kernel<BS, DS, AD, BD, TRANS>, grid, dim3(tile::kThreads), SpmmFmaCfg<BS, DS>::bytes, s, (const uint2 *)lut, a, b, c, p, avec, vec);
     } else {

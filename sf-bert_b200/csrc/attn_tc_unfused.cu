@@ -661,8 +661,9 @@ static uint32_t sddmm_grad_chunk(const AttnDims &p)
 }
 // Without it three CTAs share an SM, and what counts is how full the last wave is: the chunk with the least estimated time, in microseconds.
 // A block takes a CTA 0.89 with three on the SM and 0.62 with one or two, a CTA's set-up 1.  Fitted to nine launches of 1024 to
-// 70080 blocks with chunks of 8 to 32: 16256 blocks in CTAs of 32 (512 of them on 444 places) 48.4, of 20 36.3; 32512 74.1 / 67.8; 14850
-// 48.2 / 36.0; 13824 28.6 / 34.4; 70080 129.6 / 135.3.
+// 70080 blocks.  Measured beside one wave or CTAs of 32 (GRAD's rule), heads with sliding windows: 4352 blocks 11.7 / 11.7, 8576 18.7 / 19.3,
+// 14850 33.7 / 43.2, 16256 36.7 / 48.5 (512 CTAs on 444 places), 32512 70.4 / 83.5, 65024 139.5 / 148.4; of the even chunks from 4 to 32 none
+// was faster in 16 of 19 launches.  The others: 1024 blocks 6.9 (8 per CTA 6.6), 35040 79.9 (28: 78.5), 153600 347 (22: 323).
 static uint32_t sddmm_chunk(const AttnDims &p)
 {
     const int sms = device_sm_count(current_device());

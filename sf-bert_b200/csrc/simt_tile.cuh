@@ -109,7 +109,6 @@ __device__ __forceinline__ void stage_begin(Staged<DT, TT, COLS> &st, uint32_t r
             }
         }
     } else {
-#pragma unroll 8
         for (uint32_t t = rank; t < 32 * COLS; t += TT) {
             const uint32_t r = t / COLS, c = t % COLS;
             float *d = dst + tile_row(r) * stride + c;

@@ -20,9 +20,9 @@ def _bound(terms):
     return (1 + 6 * 2 + math.ceil(terms / 16) + 1) * EPS
 
 
-def _spmm_bound(terms, bs, d, pt, trans):
-    """fp32 blocks, and transposed ones of 32 beside heads of up to 32, go by FMAs: one rounding per term."""
-    return max(_bound(terms), terms * EPS) if pt == "f32" or (trans and bs == 32 and d <= 32) else _bound(terms)
+def _spmm_bound(terms, pt):
+    """fp32 blocks go by FMAs: one rounding per term."""
+    return max(_bound(terms), terms * EPS) if pt == "f32" else _bound(terms)
 
 
 def _layout(sfb, nb, bs, seed):
@@ -69,9 +69,9 @@ def test_products_against_64_bits(sfb, bs, d, nb, dtype):
         p = torch.randn(s.shape, device="cuda", generator=g).to(TD[pt])
         P = _dense(keep, bs, p)
         u = EPS if dtype == "f32" else 2.0 ** -8 if dtype == "bf16" else 2.0 ** -11
-        for M, got, trans in ((P, sfb.bst_sgemm_xn(p, v, lay), False), (P.transpose(-1, -2), sfb.bst_sgemm_tn(p, v, lay), True)):
+        for M, got in ((P, sfb.bst_sgemm_xn(p, v, lay)), (P.transpose(-1, -2), sfb.bst_sgemm_tn(p, v, lay))):
             want, size = M @ V, M.abs() @ V.abs()
-            assert ((_heads(got) - want).abs() <= _spmm_bound(nb * bs, bs, d, pt, trans) * size + u * want.abs() + (2.0 ** -25 if dtype == "f16" else 0)).all()
+            assert ((_heads(got) - want).abs() <= _spmm_bound(nb * bs, pt) * size + u * want.abs() + (2.0 ** -25 if dtype == "f16" else 0)).all()
     scale = 1 / math.sqrt(d)
     full = torch.from_numpy(np.kron(keep, np.ones((bs, bs), bool))).cuda()
     W = torch.softmax((S * scale).masked_fill(~full, -math.inf), -1)
@@ -172,7 +172,7 @@ def _us(f):
 @pytest.mark.parametrize("bs,d", [(32, 128), (32, 64), (64, 128)])
 def test_what_is_not_finite_does_not_set_the_time(sfb, bs, d, dtype):
     """An overflowed gradient or an infinite key must not make a call much longer: every result, or every row, is made again, and the
-    call takes at most five times what it takes on finite operands."""
+    call takes at most eight times what it takes on finite operands (two to five, measured; made again one by one, 10 to 50)."""
     lay = sfb.BlockLayout.generate(sfb.LAYOUT_SAWTOOTH, 1, 1024 // bs, bs, p0=8)
     lay.tn_lut
     g = torch.Generator(device="cuda").manual_seed(6)
@@ -181,10 +181,10 @@ def test_what_is_not_finite_does_not_set_the_time(sfb, bs, d, dtype):
     bad, key = torch.full_like(v, math.nan), k.clone()
     key[:, ::64, :, 3] = math.inf                            # in every row of blocks
     scale = 1 / math.sqrt(d)
-    assert _us(lambda: sfb.bst_sgemm_nt(q, bad, lay, torch.float32)) <= 5 * _us(lambda: sfb.bst_sgemm_nt(q, k, lay, torch.float32))
-    assert _us(lambda: sfb.bst_sgemm_xn(p, bad, lay)) <= 5 * _us(lambda: sfb.bst_sgemm_xn(p, v, lay))
-    assert _us(lambda: sfb.bst_sgemm_tn(p, bad, lay)) <= 5 * _us(lambda: sfb.bst_sgemm_tn(p, v, lay))
-    assert _us(lambda: sfb.fused_attention(q, key, v, lay, scale)) <= 5 * _us(lambda: sfb.fused_attention(q, k, v, lay, scale))
+    assert _us(lambda: sfb.bst_sgemm_nt(q, bad, lay, torch.float32)) <= 8 * _us(lambda: sfb.bst_sgemm_nt(q, k, lay, torch.float32))
+    assert _us(lambda: sfb.bst_sgemm_xn(p, bad, lay)) <= 8 * _us(lambda: sfb.bst_sgemm_xn(p, v, lay))
+    assert _us(lambda: sfb.bst_sgemm_tn(p, bad, lay)) <= 8 * _us(lambda: sfb.bst_sgemm_tn(p, v, lay))
+    assert _us(lambda: sfb.fused_attention(q, key, v, lay, scale)) <= 8 * _us(lambda: sfb.fused_attention(q, k, v, lay, scale))
 
 
 @pytest.mark.parametrize("dtype", ["f32", "f16"])
@@ -337,8 +337,8 @@ def test_rows_longer_than_the_lanes(sfb, d, B, dtype):
         p = torch.randn(B, H, lay.blocks, bs, bs, device="cuda", generator=g).to(TD[pt])
         M = _dense(keep, bs, p)
         want, size = M @ V, M.abs() @ V.abs()
-        for got, trans in ((sfb.bst_sgemm_xn(p, v, lay), False), (sfb.bst_sgemm_tn(p[:, :, order].transpose(-1, -2).contiguous(), v, layT), True)):
-            assert ((_heads(got) - want).abs() <= _spmm_bound(97 * bs, bs, d, pt, trans) * size + u * want.abs() + floor).all()
+        for got in (sfb.bst_sgemm_xn(p, v, lay), sfb.bst_sgemm_tn(p[:, :, order].transpose(-1, -2).contiguous(), v, layT)):
+            assert ((_heads(got) - want).abs() <= _spmm_bound(97 * bs, pt) * size + u * want.abs() + floor).all()
     lay.pack_mask(sfb.MASK_CAUSAL_DIAG)
     full = torch.from_numpy(np.kron(keep, np.ones((bs, bs), bool))).cuda()[rows]
     rest = torch.ones(nb * bs, dtype=torch.bool, device="cuda")
