@@ -965,7 +965,7 @@ __device__ __forceinline__ void put_p(uint4 *at, uint32_t pitch, const float (&s
 // maxima and for P.  Score and O rows of a thread are the same, so O is rescaled in place.
 // ST: two chunk buffers, three at blocks of 32 and d 128, where two CTAs share an SM and their memory has room; four for launches that the
 // SMs hold at once: each CTA then waits alone.
-// Measured (fp32, us, the FMA-pipe kernel before / now): B 1, H 4, L 512, d 64, fixed (64 CTAs) 14.8 / 12.1; B 8, H 4, L 2048, d 64, stride 179 / 136;
+// Measured (fp32, us, the FMA-pipe kernel before / this one with ex2.approx.ftz for the weights; exp2f, for their range, costs 1 to 3 % of it): B 1, H 4, L 512, d 64, fixed (64 CTAs) 14.8 / 12.1; B 8, H 4, L 2048, d 64, stride 179 / 136;
 // d 128 317 / 245; blocks of 64, d 64 198 / 160; B 2, H 4, L 1024, d 64, full with a mask 77.5 / 57; B 32, H 4, L 1024, d 128, sawtooth 304 / 264.  At the
 // last the tensor pipe is 41 % busy and a third of the issue slots are used, a quarter of them by the splits: the warps wait for fixed
 // latencies, for their chunks and for the tensor pipe in turn.  Beside it were measured: eight warps of 16 keys and 16 columns 11.5 / 156 / 267 / 168 / 60 / 265;

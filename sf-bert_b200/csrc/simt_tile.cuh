@@ -109,7 +109,10 @@ __device__ __forceinline__ void stage_begin(Staged<DT, TT, COLS> &st, uint32_t r
             }
         }
     } else {
-        for (uint32_t t = rank; t < 32 * COLS; t += TT) {
+        uint32_t first = rank;
+        asm volatile("" : "+r"(first));      // nothing of this is worked out ahead and kept in registers that the aligned rows need
+#pragma unroll 8
+        for (uint32_t t = first; t < 32 * COLS; t += TT) {
             const uint32_t r = t / COLS, c = t % COLS;
             float *d = dst + tile_row(r) * stride + c;
             if (DT == SFB_F32) cp_async4(d, (const float *)src + at + (c < ncols ? r * pitch + c : 0), c < ncols ? 4u : 0u);
