@@ -3,7 +3,7 @@
 // block-row-owned fusions.
 //
 // SDDMM, SpMM, the fused attention and the fp32 element-sparse tiles take their products from warp-level tensor-core
-// instructions on operands split into bf16 terms (simt_tile.cuh).  The fused SDDMM + softmax (fused_sddmm_softmax_kernel) is on the
+// instructions on operands split into bf16 terms (simt_tile.cuh), the SpMM of fp32 blocks from FMAs (fma_tile.cuh).  The fused SDDMM + softmax (fused_sddmm_softmax_kernel) is on the
 // FMA pipe: 256 threads as a 16x16 grid; thread (ty,tx) owns rows ty+16m and columns tx+16n of a tile, so the 16
 // lanes of a half-warp own one set of rows and row reductions are four shuffles.
 #include "fma_tile.cuh"
@@ -613,10 +613,9 @@ __device__ __noinline__ void spmm_again(float *sm, const uint2 *lut, const void 
     spmm_fma<BS, DS, A_DT, BC_DT, TRANS, true>(sm, lut, Pm, V, O, p, avec, vec);
 }
 
-// As split products.  A warp owns 32
-// output rows and a share of the columns; it stages its own columns of V (with the other warp that has them, where blocks
-// are 64 rows) and reads P straight into fragments, a chunk ahead in registers: P is small beside V, and L1 has it for
-// the other warps.
+// As split products (16-bit blocks).  A warp owns 32 output rows and a share of the columns; it stages its own columns of V (with
+// the other warp that has them, where blocks are 64 rows) and reads P straight into fragments, a chunk ahead in registers: P is
+// small beside V, and L1 has it for the other warps.
 template <int BS, int DS> struct SpmmCfg {
     static constexpr int WC = BS == 32 ? 4 : 2;                          // warps side by side along d: each is a team with the ones below it
     static constexpr int TT = 128 / WC, NW = DS / WC, N = NW / 8;        // a team's threads and columns, n-tiles of 8 columns

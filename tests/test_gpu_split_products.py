@@ -172,7 +172,7 @@ def _us(f):
 @pytest.mark.parametrize("bs,d", [(32, 128), (32, 64), (64, 128)])
 def test_what_is_not_finite_does_not_set_the_time(sfb, bs, d, dtype):
     """An overflowed gradient or an infinite key must not make a call much longer: every result, or every row, is made again, and the
-    call takes at most eight times what it takes on finite operands (two to five, measured; made again one by one, 10 to 50)."""
+    call takes at most eight times what it takes on finite operands (two to five, measured; made again one by one, 7 to 70)."""
     lay = sfb.BlockLayout.generate(sfb.LAYOUT_SAWTOOTH, 1, 1024 // bs, bs, p0=8)
     lay.tn_lut
     g = torch.Generator(device="cuda").manual_seed(6)
